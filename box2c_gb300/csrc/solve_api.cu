@@ -3,10 +3,12 @@
  * device buffers (declared in include/box2d/gpu.h).
  *
  * It builds a world descriptor over the caller's arrays (contacts in order, no joints)
- * and runs the same launch sequence as the world step's solver stage
- * (b2gd_contact_solver: prepare, substeps of integrate / warm start / solve / integrate
- * positions / relax, restitution, store impulses).  The constraint rows are per-call
- * scratch taken from the stream-ordered device allocator.
+ * and runs the solver stage (prepare, substeps of integrate / warm start / solve /
+ * integrate positions / relax, restitution, store impulses) as one resident kernel
+ * (resident.cu), or as one kernel per phase (b2gd_contact_solver) where the device
+ * launches neither a cluster nor a cooperative grid.  The scratch (barrier words, and
+ * rows for sets larger than all shared memory) is taken from the stream-ordered device
+ * allocator for the call.
  */
 #include "b2g_device.h"
 
@@ -20,6 +22,7 @@ static_assert( sizeof( b2gManifold ) == sizeof( b2Manifold ), "device manifold m
 static_assert( sizeof( b2gPoint ) == sizeof( b2ManifoldPoint ), "device manifold point must have the b2ManifoldPoint layout" );
 
 extern "C" int b2gd_contact_solver( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc );
+extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl, int clear );
 
 static void make_soft( float hertz, float zeta, float h, float* out )
 {
@@ -119,15 +122,17 @@ extern "C" int b2SolveContacts( const b2ContactSolveDesc* desc )
 	if ( b2gd_contact_desc( desc, &w, &plan, &sc ) != 0 )
 		return -1;
 	cudaStream_t s = (cudaStream_t)desc->stream;
-	void* rows = nullptr;
+	/* a grid's barrier words, then the rows of a set too large for shared memory */
+	char* scratch = nullptr;
 	int n = desc->contactCount > 0 ? desc->contactCount : 1;
-	cudaError_t e = cudaMallocAsync( &rows, 16u * B2G_ROW_FLOAT4 * (size_t)n, s );
+	cudaError_t e = cudaMallocAsync( (void**)&scratch, 256u + 16u * B2G_ROW_FLOAT4 * (size_t)n, s );
 	if ( e != cudaSuccess )
 		return (int)e;
-	b2gd_contact_rows( &w, rows, n );
-	b2gd_contact_solver( &w, &plan, &sc );
+	b2gd_contact_rows( &w, scratch + 256, n );
+	if ( b2gd_contact_resident( &w, &plan, &sc, (int*)scratch, 1 ) == 0 )
+		b2gd_contact_solver( &w, &plan, &sc );
 	e = cudaGetLastError();
-	cudaError_t f = cudaFreeAsync( rows, s );
+	cudaError_t f = cudaFreeAsync( scratch, s );
 	if ( e != cudaSuccess )
 		return (int)e;
 	return (int)f;

@@ -176,7 +176,8 @@ typedef struct b2ContactSolveDesc
 } b2ContactSolveDesc;
 
 /* Returns 0, or a CUDA error code / -1 for invalid arguments.  Allocates its per-call
- * constraint rows (144 bytes per contact) with stream-ordered device allocation. */
+ * scratch (256 bytes and a constraint row of 144 bytes per contact) with stream-ordered
+ * device allocation. */
 B2_API int b2SolveContacts( const b2ContactSolveDesc* desc );
 
 /* b2SolveContacts that allocates nothing; no counterpart in the reference API.  Its

@@ -1,0 +1,87 @@
+"""The resident contact solver (csrc/resident.cu) at the edges of its spaces: one CTA, a
+cluster, a cooperative grid, body indices that do not fit on chip, overflow rows and an
+empty set.  The reference is the oracle's captured solver stage; tolerance: none."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from box2c_gb300.capi import bind_solve_api
+from tests.test_gpu_solve_api import capture_step, make_desc, solve_on_device
+
+
+def _scene(oracle, name):
+    if name == "plank":  # a plank under sixteen boxes: contacts beyond the graph colours
+        n = 17
+        heights = np.array([0.2] + [0.9 + 0.01 * (k % 3) for k in range(n - 1)], np.float32)
+        kinds = np.array([3] + [0] * (n - 1), np.int32)
+        return oracle.drop_boxes(heights, np.zeros(n), np.zeros(n), 0.6, kinds), 30
+    if name == "many":
+        return oracle.many_pyramids(20, 20, 10), 3
+    size = int(name)
+    return oracle.pyramid(size, 0.01, 5), 12
+
+
+def _spread(cap, stride):
+    """The same set with body indices spread over `stride` times as many states."""
+    n = len(cap["statesIn"])
+    out = dict(cap)
+    for k in ("statesIn", "statesOut", "mass", "force", "damping"):
+        a = np.zeros((n * stride, cap[k].shape[1]), np.float32)
+        a[::stride] = cap[k]
+        out[k] = a
+    out["awake"] = cap["awake"] * stride
+    out["contactBodies"] = np.where(cap["contactBodies"] < 0, -1, cap["contactBodies"] * stride).astype(np.int32)
+    return out
+
+
+# one CTA up to about 1300 contacts, a cluster up to about 22000, a grid above; 30 and 21
+# lie on both sides of the first line, 120 above the second; strides 40 and 90 put the
+# indices beyond the cluster's body slots and beyond 2^16
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene,stride", [("1", 1), ("21", 1), ("30", 1), ("100", 1), ("120", 1), ("many", 1), ("plank", 1),
+                                          ("plank", 700), ("21", 90), ("40", 40), ("40", 90)])
+def test_resident_solver_matches_oracle(gpu, oracle, scene, stride):
+    torch = pytest.importorskip("torch")
+    w, warm = _scene(oracle, scene)
+    oracle.step(w, count=warm)
+    cap = capture_step(oracle, w, body_cap=30000, contact_cap=80000)
+    oracle.destroy(w)
+    if scene == "plank":
+        assert cap["colorStart"][12] > cap["colorStart"][11]
+    cap = _spread(cap, stride)
+    states, manifolds = solve_on_device(gpu, torch, cap)
+    assert np.array_equal(states.view(np.uint32), cap["statesOut"].view(np.uint32))
+    assert np.array_equal(manifolds, cap["manifoldsOut"])
+
+
+@pytest.mark.gpu
+def test_resident_solver_captured(gpu, oracle):
+    """Both entry points inside a stream capture, replayed twice on the same inputs."""
+    torch = pytest.importorskip("torch")
+    bind_solve_api(gpu.lib)
+    gpu.lib.b2SolveContactsNoAlloc.argtypes = gpu.lib.b2SolveContacts.argtypes
+    gpu.lib.b2SolveContactsNoAlloc.restype = C.c_int
+    for size, names in ((21, ("b2SolveContacts", "b2SolveContactsNoAlloc")), (120, ("b2SolveContacts",))):
+        w, warm = _scene(oracle, str(size))
+        oracle.step(w, count=warm)
+        cap = capture_step(oracle, w)
+        oracle.destroy(w)
+        for name in names:
+            fn = getattr(gpu.lib, name)
+            d, t = make_desc(torch, cap, "cuda:0")
+            first = t["statesIn"].clone(), t["manifoldsIn"].clone()
+            assert fn(C.byref(d)) == 0  # set-up outside the capture
+            torch.cuda.synchronize()
+            g = torch.cuda.CUDAGraph()
+            s = torch.cuda.Stream()
+            with torch.cuda.graph(g, stream=s):
+                d.stream = s.cuda_stream
+                assert fn(C.byref(d)) == 0
+            for _ in range(2):
+                t["statesIn"].copy_(first[0])
+                t["manifoldsIn"].copy_(first[1])
+                g.replay()
+                torch.cuda.synchronize()
+                assert np.array_equal(t["statesIn"].cpu().numpy().view(np.uint32), cap["statesOut"].view(np.uint32))
+                assert np.array_equal(t["manifoldsIn"].cpu().numpy(), cap["manifoldsOut"])
