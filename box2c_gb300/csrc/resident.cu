@@ -737,8 +737,88 @@ static bool res_opt_in( K kernel, bool cluster )
 	return ok;
 }
 
-		1,
-		B2G_FUSED_CTAS };
+/* What the current device can launch; looked up once per device (any number of threads
+ * may look at once: they write the same values). */
+static const ResDevice* res_device( void )
+{
+	int dev = 0;
+	if ( cudaGetDevice( &dev ) != cudaSuccess || dev < 0 || dev >= RES_MAX_DEVICES )
+		return nullptr;
+	ResDevice* d = s_devices + dev;
+	if ( __atomic_load_n( &d->looked, __ATOMIC_ACQUIRE ) )
+		return d;
+	int cluster = 0, sms = 0, coop = 0, blocks = 0;
+	auto wide = k_solve_cluster<B2G_FUSED_CTAS, CLUSTER_THREADS>;
+	bool ok = res_opt_in( k_solve_cluster<1, CLUSTER_THREADS>, false ) && res_opt_in( wide, true );
+	if ( ok )
+	{
+		cudaLaunchAttribute attr[1];
+		cudaLaunchConfig_t cfg = res_config( attr, B2G_FUSED_CTAS, B2G_FUSED_CTAS, CLUSTER_THREADS, RES_SMEM_MAX, nullptr );
+		int n = 0;
+		cluster = cudaOccupancyMaxActiveClusters( &n, wide, &cfg ) == cudaSuccess && n >= 1;
+	}
+	ok = res_opt_in( k_solve_grid<GRID_THREADS, true>, false ) && res_opt_in( k_solve_grid<GRID_THREADS, false>, false );
+	cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, dev );
+	cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
+	if ( ok == false || coop == 0 ||
+		 cudaOccupancyMaxActiveBlocksPerMultiprocessor( &blocks, k_solve_grid<GRID_THREADS, true>, GRID_THREADS, RES_SMEM_MAX ) != cudaSuccess || blocks < 1 )
+		sms = 0;
+	cudaGetLastError();
+	d->cluster = cluster;
+	d->sms = sms;
+	__atomic_store_n( &d->looked, 1, __ATOMIC_RELEASE );
+	return d;
+}
+
+/* Row slots of the fullest CTA: every colour splits into shares that differ by one, CTA
+ * 0 also holds the overflow rows. */
+static int res_row_cap( const int* cs, int ctas )
+{
+	int cap = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
+	for ( int c = 0; c < B2G_OVERFLOW; ++c )
+		cap += ( cs[c + 1] - cs[c] + ctas - 1 ) / ctas;
+	return cap > 0 ? cap : 1;
+}
+
+/* Shared memory of CTA 0 with its overflow cache, which is left out when it does not fit. */
+static size_t res_with_overflow( ResidentPlan* P, size_t bytes, int ovRows )
+{
+	P->ovOffset = 0;
+	size_t at = ( bytes + 15 ) / 16;
+	if ( ovRows > 0 && ovRows <= RES_OVERFLOW_MAX && 16 * at + res_overflow_bytes( ovRows ) <= RES_SMEM_MAX )
+	{
+		P->ovOffset = (int)at;
+		bytes = 16 * at + res_overflow_bytes( ovRows );
+	}
+	return bytes;
+}
+
+/* The solver stage of caller buffers in one launch: the number of launches, 0 when this
+ * device or set needs the per-phase kernels, or -1 on a launch error.  ctl: four ints of
+ * device memory, zero, or cleared here when `clear` is set. */
+extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl, int clear )
+{
+	const ResDevice* d = res_device();
+	if ( d == nullptr )
+		return 0;
+	const int* cs = plan->colorStart;
+	const int ovRows = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
+	ResidentPlan P;
+	memset( &P, 0, sizeof( P ) );
+	memcpy( P.colorStart, cs, sizeof( P.colorStart ) );
+	memcpy( P.active, plan->active, sizeof( P.active ) );
+	P.activeCount = plan->activeCount;
+	P.awakeCount = plan->awakeCount;
+	cudaStream_t s = (cudaStream_t)w->stream;
+	cudaLaunchAttribute attr[1];
+
+	/* One CTA, else a whole cluster, when the rows fit with as many bodies as the list
+	 * has and one for every two rows (body indices are the caller's: the kernel copes
+	 * with more, at L2).  One CTA is the faster one as long as it holds the set (1200
+	 * contacts: 58 us, 80 in a cluster); clusters of 2, 4 or 8 take what 16 take (2000
+	 * contacts: 78 to 82 us), so there is no space between the two; a grid is slower
+	 * wherever a cluster holds the set (20000 contacts: 201 us, 110 in a cluster). */
+	const int spaces[] = { 1, B2G_FUSED_CTAS };
 	for ( int ctas : spaces )
 	{
 		if ( ctas > 1 && d->cluster == 0 )
@@ -759,8 +839,7 @@ static bool res_opt_in( K kernel, bool cluster )
 		if ( tail )
 			bytes = res_with_overflow( &P, bytes, ovRows );
 		auto kernel = ctas == 1 ? (ResClusterKernel)k_solve_cluster<1, CLUSTER_THREADS> : (ResClusterKernel)k_solve_cluster<B2G_FUSED_CTAS, CLUSTER_THREADS>;
-		int threads = CLUSTER_THREADS;
-		cudaLaunchConfig_t cfg = res_config( attr, ctas, ctas, threads, bytes, s );
+		cudaLaunchConfig_t cfg = res_config( attr, ctas, ctas, CLUSTER_THREADS, bytes, s );
 		return cudaLaunchKernelEx( &cfg, kernel, *w, P, *sc ) == cudaSuccess ? 1 : -1;
 	}
 
