@@ -158,8 +158,6 @@ extern "C" void b2gd_free( b2gDevWorld* w, b2gHostIO* io )
 		cudaFreeHost( io->hitIds );
 	if ( io->hitOut )
 		cudaFreeHost( io->hitOut );
-	if ( w->stage )
-		cudaFree( w->stage );
 	if ( w->stream )
 		cudaStreamDestroy( (cudaStream_t)w->stream );
 	memset( w, 0, sizeof( *w ) );

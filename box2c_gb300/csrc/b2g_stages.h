@@ -431,9 +431,8 @@ static __device__ void row_phase( const b2gDevWorld& W, int k, int phase, bool s
 /* ------------------------------------------------------------------ joints */
 /* Joint preparation (reference src/joint.c:983-1018 and the per-type prepare functions):
  * gathers the two bodies' mass and pose, then the type's own preparation. */
-static __device__ void prepare_joint( const b2gDevWorld& W, int t, const b2gStepConst& sc )
+static __device__ void prepare_joint_at( const b2gDevWorld& W, b2gJointDev* j, const b2gStepConst& sc )
 {
-	b2gJointDev* j = W.joints + W.jointList[t];
 	const float4* mass = (const float4*)W.mass;
 	const float4* xf = (const float4*)W.xf;
 	const float4* centers = (const float4*)W.centers;
@@ -456,6 +455,11 @@ static __device__ void prepare_joint( const b2gDevWorld& W, int t, const b2gStep
 	jb.lcA = gv( ca.z, ca.w );
 	jb.lcB = gv( cb.z, cb.w );
 	joint_prepare( j, jb, sc );
+}
+
+static __device__ void prepare_joint( const b2gDevWorld& W, int t, const b2gStepConst& sc )
+{
+	prepare_joint_at( W, W.joints + W.jointList[t], sc );
 }
 
 template <class Bodies>

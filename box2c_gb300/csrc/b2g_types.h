@@ -285,8 +285,6 @@ typedef struct b2gDevWorld
 	/* set for a solver stage launched before the host has seen the narrowphase's events:
 	 * its kernels return at once when the narrowphase reported any (counters[0] != 0) */
 	int guardEvents;
-	void* stage;   /* fused solver: per-CTA shared-memory images */
-	size_t stageBytes;
 } b2gDevWorld;
 
 #ifdef __cplusplus

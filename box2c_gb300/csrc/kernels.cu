@@ -289,16 +289,6 @@ extern "C" int b2gd_contact_solver( b2gDevWorld* w, const b2gSolvePlan* plan, co
 	return launches;
 }
 
-/* Prepares the step's joints (all colours); used by the fused solver, which runs
- * everything else of the solver stage. */
-extern "C" int b2gd_prepare_joints( b2gDevWorld* w, int joints, const b2gStepConst* sc )
-{
-	if ( joints <= 0 )
-		return 0;
-	k_prepare_joints<<<blocks_for( joints ), BLOCK, 0, (cudaStream_t)w->stream>>>( *w, joints, *sc );
-	return 1;
-}
-
 extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc );
 
 extern "C" int b2gd_solve( b2gDevWorld* w, b2gHostIO* io, const b2gSolvePlan* plan, const b2gStepConst* scp )

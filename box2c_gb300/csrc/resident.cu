@@ -36,411 +36,9 @@
  * cluster takes 82), 15000 420 -> 102 (a grid takes 199), 60000 424 -> 207; with 17
  * overflow rows at 15000 contacts 799 -> 185.
  */
-#include "b2g_cluster.h"
-#include "b2g_device.h"
-
-#include <cuda_runtime.h>
+#include "b2g_resident.h"
 
 #include <string.h>
-
-/* dynamic shared memory per CTA, leaving 1 KB of the 227 KB opt-in limit for statics */
-#define RES_SMEM_MAX ( 226 * 1024 )
-#define RES_OVERFLOW_MAX 512
-/* polls of a grid barrier before it gives up (seconds; a cooperative launch never gets
- * there) */
-#define RES_SPIN_LIMIT ( 1 << 22 )
-
-struct ResidentPlan
-{
-	int colorStart[B2G_COLORS + 1];
-	int active[B2G_COLORS];
-	int activeCount;
-	int awakeCount;
-	int ctas;
-	int rowCap;	 /* row slots per CTA (0: rows in the row arrays) */
-	int bodyCap; /* body slots per CTA in shared memory; a grid's velocity-term slots */
-	int ovOffset; /* float4 offset of the overflow cache, 0 without one */
-};
-
-/* Overflow cache of CTA 0: for R overflow rows with E = 2 R body ends, the rows' indices
- * with body slots (int4 x R), slot states (2 x float4 x E), slot bodies, first occurrences
- * and slots per end (3 x int x E). */
-struct ResOverflow
-{
-	int4* idx;
-	float4* st0;
-	float4* st1;
-	int* body;
-	int* first;
-	int* slot;
-};
-
-static __host__ __device__ size_t res_overflow_bytes( int R ) { return 16u * 5u * (size_t)R + 24u * (size_t)R; }
-
-__device__ __forceinline__ ResOverflow res_carve_overflow( float4* base, int R )
-{
-	int E = 2 * R;
-	ResOverflow o;
-	o.idx = (int4*)base;
-	o.st0 = base + R;
-	o.st1 = o.st0 + E;
-	o.body = (int*)( o.st1 + E );
-	o.first = o.body + E;
-	o.slot = o.first + E;
-	return o;
-}
-
-/* Bytes of one body slot in shared memory: two state float4, the velocity terms (float4
- * and float), flags and an entry of the awake list. */
-#define RES_BODY_BYTES 60
-
-struct ResBodies
-{
-	float4* st0;  /* v.x v.y w tag */
-	float4* st1;  /* dp.x dp.y dq.c dq.s */
-	float4* term; /* lvd.x lvd.y avd ld */
-	float* ad;	  /* angular damping factor */
-	int* flags;	  /* RES_AWAKE, RES_TOUCHED */
-	int* awake;	  /* local awake slots */
-};
-
-enum
-{
-	RES_AWAKE = 1,
-	RES_TOUCHED = 2,
-};
-
-__device__ __forceinline__ ResBodies res_carve_bodies( float4* base, int cap )
-{
-	ResBodies b;
-	b.st0 = base;
-	b.st1 = base + cap;
-	b.term = base + 2 * cap;
-	b.ad = (float*)( base + 3 * cap );
-	b.flags = (int*)( b.ad + cap );
-	b.awake = b.flags + cap;
-	return b;
-}
-
-__device__ __forceinline__ SmemRows res_carve_rows( float4* base, int n )
-{
-	SmemRows m;
-	m.idx = (int4*)base;
-	m.nf = base + n;
-	m.ms = base + 2 * n;
-	m.anc0 = base + 3 * n;
-	m.anc1 = base + 4 * n;
-	m.coef0 = base + 5 * n;
-	m.coef1 = base + 6 * n;
-	m.imp0 = base + 7 * n;
-	m.imp1 = base + 8 * n;
-	return m;
-}
-
-__device__ __forceinline__ SmemRows res_global_rows( const b2gDevWorld& W )
-{
-	SmemRows m;
-	m.idx = (int4*)W.kIdx;
-	m.nf = (float4*)W.kNF;
-	m.ms = (float4*)W.kMass;
-	m.anc0 = (float4*)W.kAnchor[0];
-	m.anc1 = (float4*)W.kAnchor[1];
-	m.coef0 = (float4*)W.kCoef[0];
-	m.coef1 = (float4*)W.kCoef[1];
-	m.imp0 = (float4*)W.kImp[0];
-	m.imp1 = (float4*)W.kImp[1];
-	return m;
-}
-
-/* Body states in global memory, read and written at L2: other CTAs change them between
- * sweeps. */
-struct L2Bodies
-{
-	float4* st;
-	__device__ __forceinline__ DevState load( int b ) const
-	{
-		return b < 0 ? identity_state() : state_of( __ldcg( st + 2 * b ), __ldcg( st + 2 * b + 1 ) );
-	}
-	__device__ __forceinline__ DevState load_velocity( int b ) const
-	{
-		return b < 0 ? identity_state() : state_of( __ldcg( st + 2 * b ), make_float4( 0.0f, 0.0f, 1.0f, 0.0f ) );
-	}
-	__device__ __forceinline__ void store( int b, const DevState& x ) const
-	{
-		if ( b >= 0 )
-			__stcg( st + 2 * b, velocity_word( x ) );
-	}
-	__device__ __forceinline__ float4 word0( int b ) const { return __ldcg( st + 2 * b ); }
-	__device__ __forceinline__ float4 word1( int b ) const { return __ldcg( st + 2 * b + 1 ); }
-	__device__ __forceinline__ void set_word0( int b, float4 v ) const { __stcg( st + 2 * b, v ); }
-};
-
-/* ClusterBodies with the words the overflow cache copies. */
-struct DsmemBodies : ClusterBodies
-{
-	__device__ __forceinline__ float4 word0( int b ) const { return *word( st0, b ); }
-	__device__ __forceinline__ float4 word1( int b ) const { return *word( st1, b ); }
-	__device__ __forceinline__ void set_word0( int b, float4 v ) const { *word( st0, b ) = v; }
-};
-
-/* The one-CTA space's bodies are already local: the overflow pass needs no cache. */
-struct LocalBodies : SharedBodies
-{
-	__device__ __forceinline__ float4 word0( int b ) const { return st0[b]; }
-	__device__ __forceinline__ float4 word1( int b ) const { return st1[b]; }
-	__device__ __forceinline__ void set_word0( int b, float4 v ) const { st0[b] = v; }
-};
-
-/* Barrier between sweeps.  A grid's barrier counts arrivals in ctl[0]; ctl[2] tells every
- * CTA that one gave up, after which no CTA waits again. */
-template <int CL>
-struct ResBarrier
-{
-	int* ctl;
-	int ctas;
-	unsigned target;
-	__device__ __forceinline__ void sync()
-	{
-		if constexpr ( CL == 1 )
-			__syncthreads();
-		else if constexpr ( CL > 1 )
-			cg::this_cluster().sync();
-		else
-		{
-			__syncthreads();
-			target += (unsigned)ctas;
-			if ( threadIdx.x == 0 )
-			{
-				unsigned* count = (unsigned*)ctl;
-				asm volatile( "red.release.gpu.global.add.u32 [%0], 1;" ::"l"( count ) : "memory" );
-				int left = RES_SPIN_LIMIT;
-				unsigned seen;
-				do
-				{
-					asm volatile( "ld.acquire.gpu.global.u32 %0, [%1];" : "=r"( seen ) : "l"( count ) : "memory" );
-				} while ( (int)( seen - target ) < 0 && --left > 0 && ( ( left & 1023 ) != 0 || *(volatile int*)( ctl + 2 ) == 0 ) );
-				if ( (int)( seen - target ) < 0 )
-					*(volatile int*)( ctl + 2 ) = 1;
-			}
-			__syncthreads();
-		}
-	}
-};
-
-struct ResShare
-{
-	int first, count, base; /* of one colour: rows [first, first + count) at local index base */
-};
-
-__device__ __forceinline__ int res_first( int n, int k, int ctas ) { return (int)( (long long)n * k / ctas ); }
-
-/* One stage over all colours: the overflow set first (serially, CTA 0), then each active
- * colour with a barrier after it. */
-template <int CL, int PHASE, int T, class Bodies>
-__device__ __forceinline__ void res_stage( const ResidentPlan& P, const ResShare* share, const SmemRows& m, const Bodies& B,
-										   ResBarrier<CL>& bar, int rank, const b2gStepConst& sc, const ResOverflow& ov, int ovSlots )
-{
-	const int* cs = P.colorStart;
-	const int R = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
-	if ( R > 0 )
-	{
-		if ( rank == 0 )
-		{
-			const int base = share[B2G_OVERFLOW].base;
-			if ( CL != 1 && P.ovOffset != 0 )
-			{
-				/* the set's bodies to local slots, the serial pass on them, velocities back:
-				 * nothing else touches a body while the set runs */
-				for ( int s = threadIdx.x; s < ovSlots; s += T )
-				{
-					int b = ov.body[s];
-					ov.st0[s] = B.word0( b );
-					ov.st1[s] = B.word1( b );
-				}
-				__syncthreads();
-				if ( threadIdx.x == 0 )
-				{
-					SharedBodies OB{ ov.st0, ov.st1 };
-					SmemRows mo = { ov.idx, m.nf + base, m.ms + base, m.anc0 + base, m.anc1 + base, m.coef0 + base, m.coef1 + base, m.imp0 + base, m.imp1 + base };
-					for ( int i = 0; i < R; ++i )
-						row_step( mo, OB, i, PHASE, true, sc );
-				}
-				__syncthreads();
-				for ( int s = threadIdx.x; s < ovSlots; s += T )
-					B.set_word0( ov.body[s], ov.st0[s] );
-			}
-			else if ( threadIdx.x == 0 )
-			{
-				for ( int i = 0; i < R; ++i )
-					row_step( m, B, base + i, PHASE, true, sc );
-			}
-		}
-		bar.sync();
-	}
-	if ( PHASE == F_WARM && sc.enableWarmStarting == 0 )
-		return;
-	for ( int a = 0; a < P.activeCount; ++a )
-	{
-		const ResShare s = share[P.active[a]];
-		for ( int j = threadIdx.x; j < s.count; j += T )
-			row_step( m, B, s.base + j, PHASE, false, sc );
-		bar.sync();
-	}
-}
-
-/* All substeps over bodies B.  Integration runs over this CTA's awake bodies: with states
- * in shared memory slots b.awake[0 .. awake), in global memory the ids list[0 .. awake). */
-template <int CL, int T, bool SHARED_STATES, class Bodies>
-__device__ __forceinline__ void res_run( const ResidentPlan& P, const ResShare* share, const SmemRows& m, const Bodies& B,
-										 const ResBodies& rb, float4* gst, const int* list, int awake, ResBarrier<CL>& bar, int rank,
-										 const b2gStepConst& sc, const ResOverflow& ov, int ovSlots )
-{
-	for ( int sub = 0; sub < sc.subSteps; ++sub )
-	{
-		for ( int j = threadIdx.x; j < awake; j += T )
-		{
-			const int s = SHARED_STATES ? rb.awake[j] : list[j];
-			const int k = SHARED_STATES ? s : j;
-			float4* p = SHARED_STATES ? rb.st0 + s : gst + 2 * s;
-			DevState x = state_of( SHARED_STATES ? *p : __ldcg( p ), make_float4( 0.0f, 0.0f, 1.0f, 0.0f ) );
-			float4 t4 = rb.term[k];
-			VelocityTerms t;
-			t.lvd = gv( t4.x, t4.y );
-			t.avd = t4.z;
-			t.ld = t4.w;
-			t.ad = rb.ad[k];
-			integrate_velocity( x, t, sc );
-			if ( SHARED_STATES )
-				*p = velocity_word( x );
-			else
-				__stcg( p, velocity_word( x ) );
-		}
-		bar.sync();
-		res_stage<CL, F_WARM, T>( P, share, m, B, bar, rank, sc, ov, ovSlots );
-		res_stage<CL, F_SOLVE, T>( P, share, m, B, bar, rank, sc, ov, ovSlots );
-		for ( int j = threadIdx.x; j < awake; j += T )
-		{
-			const int s = SHARED_STATES ? rb.awake[j] : list[j];
-			float4* p0 = SHARED_STATES ? rb.st0 + s : gst + 2 * s;
-			float4* p1 = SHARED_STATES ? rb.st1 + s : gst + 2 * s + 1;
-			DevState x = state_of( SHARED_STATES ? *p0 : __ldcg( p0 ), SHARED_STATES ? *p1 : __ldcg( p1 ) );
-			integrate_position( x, sc.h );
-			float4 v = make_float4( x.dp.x, x.dp.y, x.dq.c, x.dq.s );
-			if ( SHARED_STATES )
-				*p1 = v;
-			else
-				__stcg( p1, v );
-		}
-		bar.sync();
-		res_stage<CL, F_RELAX, T>( P, share, m, B, bar, rank, sc, ov, ovSlots );
-	}
-	res_stage<CL, F_RESTITUTION, T>( P, share, m, B, bar, rank, sc, ov, ovSlots );
-}
-
-/* Overflow cache: the distinct bodies of the set's ends get slots in end order. */
-template <int T>
-__device__ __forceinline__ void res_index_overflow( const ResOverflow& ov, const SmemRows& m, int base, int R, int* slots )
-{
-	const int E = 2 * R;
-	auto end_body = [&]( int e ) {
-		int4 ix = m.idx[base + ( e >> 1 )];
-		return ( e & 1 ) ? ix.y : ix.x;
-	};
-	for ( int e = threadIdx.x; e < E; e += T )
-	{
-		int b = end_body( e );
-		int f = -1;
-		if ( b >= 0 )
-		{
-			f = e;
-			for ( int e2 = 0; e2 < e; ++e2 )
-			{
-				if ( end_body( e2 ) == b )
-				{
-					f = e2;
-					break;
-				}
-			}
-		}
-		ov.first[e] = f;
-	}
-	__syncthreads();
-	if ( threadIdx.x == 0 )
-	{
-		int K = 0;
-		for ( int e = 0; e < E; ++e )
-		{
-			if ( ov.first[e] == e )
-			{
-				ov.slot[e] = K;
-				ov.body[K++] = end_body( e );
-			}
-		}
-		*slots = K;
-	}
-	__syncthreads();
-	for ( int e = threadIdx.x; e < E; e += T )
-	{
-		int f = ov.first[e];
-		int s = f < 0 ? -1 : ov.slot[f];
-		int r = e >> 1;
-		if ( e & 1 )
-			ov.idx[r].y = s;
-		else
-		{
-			int4 ix = m.idx[base + r];
-			ov.idx[r].x = s;
-			ov.idx[r].z = ix.z;
-			ov.idx[r].w = ix.w;
-		}
-	}
-}
-
-/* Preparation of one row into m (reference src/contact_solver.c:597-808, :21-147). */
-__device__ __forceinline__ int2 res_prepare( const b2gDevWorld& W, const SmemRows& m, int k, int local, const b2gStepConst& sc )
-{
-	const float4* gst = (const float4*)W.state;
-	const float4* mass = (const float4*)W.mass;
-	const float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
-	int cid = W.solveList ? W.solveList[k] : k;
-	int ia = W.cBodies[2 * cid];
-	int ib = W.cBodies[2 * cid + 1];
-	DevState sA = ia >= 0 ? state_of( gst[2 * ia], gst[2 * ia + 1] ) : identity_state();
-	DevState sB = ib >= 0 ? state_of( gst[2 * ib], gst[2 * ib + 1] ) : identity_state();
-	Row r;
-	prepare_row( r, W.manifold + cid, ia, ib, ia >= 0 ? mass[ia] : zero, ib >= 0 ? mass[ib] : zero, sA, sB, W.cMix[2 * cid],
-				 W.cMix[2 * cid + 1], ( ia < 0 || ib < 0 ) ? sc.staticSoft : sc.contactSoft, sc.enableWarmStarting ? 1.0f : 0.0f );
-	store_row_smem( m, local, cid, r );
-	return make_int2( ia, ib );
-}
-
-/* Impulses of local row k back to its manifold (reference src/contact_solver.c:442-471,
- * :1180-1293): colour rows write both point slots, overflow rows their points. */
-__device__ __forceinline__ void res_store( const b2gDevWorld& W, const SmemRows& m, int k, bool overflow )
-{
-	int4 idx = m.idx[k];
-	b2gManifold* mf = W.manifold + idx.z;
-	int n = overflow ? idx.w : 2;
-	float4 imp[2] = { m.imp0[k], m.imp1[k] };
-	float4 coef[2] = { m.coef0[k], m.coef1[k] };
-#pragma unroll
-	for ( int j = 0; j < 2; ++j )
-	{
-		if ( j >= n )
-			break;
-		mf->pts[j].normalImpulse = imp[j].x;
-		mf->pts[j].tangentImpulse = imp[j].y;
-		mf->pts[j].maxNormalImpulse = imp[j].z;
-		mf->pts[j].normalVelocity = coef[j].w;
-	}
-}
-
-__device__ __forceinline__ void res_terms( const b2gDevWorld& W, const ResBodies& rb, int k, int b, const b2gStepConst& sc )
-{
-	VelocityTerms v = velocity_terms( ( (const float4*)W.mass )[b], ( (const float4*)W.force )[b], ( (const float4*)W.extent )[b], sc );
-	rb.term[k] = make_float4( v.lvd.x, v.lvd.y, v.avd, v.ld );
-	rb.ad[k] = v.ad;
-}
 
 /* The solver stage on caller buffers: one CTA or one cluster.  Body indices are whatever
  * the caller numbered, so the CTAs first find the largest one; when the states up to it
@@ -524,10 +122,11 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	}
 
 	ResBarrier<CL> bar{ nullptr, CL, 0 };
-	ResOverflow ov = res_carve_overflow( smem + P.ovOffset, P.ovOffset ? cs[B2G_COLORS] - cs[B2G_OVERFLOW] : 0 );
+	const ResJoints J{};
+	ResOverflow ov = res_carve_overflow( smem + P.ovOffset, P.ovOffset ? cs[B2G_COLORS] - cs[B2G_OVERFLOW] : 0, 0 );
 	if ( CL > 1 && rank == 0 && P.ovOffset )
 	{
-		res_index_overflow<T>( ov, m, share[B2G_OVERFLOW].base, cs[B2G_COLORS] - cs[B2G_OVERFLOW], &s_ovSlots );
+		res_index_overflow<T, false>( ov, m, J, share[B2G_OVERFLOW], 0, cs[B2G_COLORS] - cs[B2G_OVERFLOW], &s_ovSlots );
 		__syncthreads();
 	}
 	const int ids = top + 1;
@@ -586,10 +185,10 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 			LB.st0 = rb.st0;
 			LB.st1 = rb.st1;
 			/* a thread's terms are its own: no barrier before the first integration */
-			res_run<CL, T, true>( P, share, m, LB, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
+			res_run<CL, T, true, false>( P, share, m, J, LB, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 		}
 		else
-			res_run<CL, T, true>( P, share, m, D, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
+			res_run<CL, T, true, false>( P, share, m, J, D, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 		for ( int s = tid; s < owned; s += T )
 		{
 			int b = rank * block + s;
@@ -610,7 +209,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 			for ( int j = tid; j < n; j += T )
 				res_terms( W, rb, j, W.awake[af + j], sc );
 			bar.sync();
-			res_run<CL, T, false>( P, share, m, G, rb, gst, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
+			res_run<CL, T, false, false>( P, share, m, J, G, rb, gst, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
 		}
 	}
 	for ( int k = tid; k < rows; k += T )
@@ -664,16 +263,17 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 	const int n = res_first( P.awakeCount, rank + 1, ctas ) - af;
 	for ( int j = tid; j < n; j += T )
 		res_terms( W, rb, j, W.awake[af + j], sc );
-	ResOverflow ov = res_carve_overflow( smem + P.ovOffset, P.ovOffset ? ovRows : 0 );
+	const ResJoints J{};
+	ResOverflow ov = res_carve_overflow( smem + P.ovOffset, P.ovOffset ? ovRows : 0, 0 );
 	if ( rank == 0 && P.ovOffset )
 	{
 		__syncthreads();
-		res_index_overflow<T>( ov, m, share[B2G_OVERFLOW].base, ovRows, &s_ovSlots );
+		res_index_overflow<T, false>( ov, m, J, share[B2G_OVERFLOW], 0, ovRows, &s_ovSlots );
 	}
 	ResBarrier<0> bar{ ctl, ctas, 0u };
 	bar.sync();
 	L2Bodies G{ (float4*)W.state };
-	res_run<0, T, false>( P, share, m, G, rb, (float4*)W.state, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
+	res_run<0, T, false, false>( P, share, m, J, G, rb, (float4*)W.state, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
 	for ( int c = 0; c < B2G_COLORS; ++c )
 		for ( int j = tid; j < share[c].count; j += T )
 			res_store( W, m, share[c].base + j, c == B2G_OVERFLOW );
@@ -785,10 +385,10 @@ static size_t res_with_overflow( ResidentPlan* P, size_t bytes, int ovRows )
 {
 	P->ovOffset = 0;
 	size_t at = ( bytes + 15 ) / 16;
-	if ( ovRows > 0 && ovRows <= RES_OVERFLOW_MAX && 16 * at + res_overflow_bytes( ovRows ) <= RES_SMEM_MAX )
+	if ( ovRows > 0 && ovRows <= RES_OVERFLOW_MAX && 16 * at + res_overflow_bytes( ovRows, 0 ) <= RES_SMEM_MAX )
 	{
 		P->ovOffset = (int)at;
-		bytes = 16 * at + res_overflow_bytes( ovRows );
+		bytes = 16 * at + res_overflow_bytes( ovRows, 0 );
 	}
 	return bytes;
 }
@@ -828,7 +428,7 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 		int want = P.awakeCount > cs[B2G_COLORS] / 2 ? P.awakeCount : cs[B2G_COLORS] / 2;
 		want = ( want + ctas - 1 ) / ctas + 1;
 		size_t rows = 144u * (size_t)P.rowCap;
-		size_t tail = ctas > 1 && ovRows > 0 && ovRows <= RES_OVERFLOW_MAX ? res_overflow_bytes( ovRows ) + 16 : 0;
+		size_t tail = ctas > 1 && ovRows > 0 && ovRows <= RES_OVERFLOW_MAX ? res_overflow_bytes( ovRows, 0 ) + 16 : 0;
 		if ( rows + RES_BODY_BYTES * (size_t)want + tail > RES_SMEM_MAX )
 			continue;
 		/* the body slots take what the rows leave */

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from box2c_gb300.capi import bind_solve_api
+from tests.helpers import lockstep
 from tests.test_gpu_solve_api import capture_step, make_desc, solve_on_device
 
 
@@ -85,3 +86,17 @@ def test_resident_solver_captured(gpu, oracle):
                 torch.cuda.synchronize()
                 assert np.array_equal(t["statesIn"].cpu().numpy().view(np.uint32), cap["statesOut"].view(np.uint32))
                 assert np.array_equal(t["manifoldsIn"].cpu().numpy(), cap["manifoldsOut"])
+
+
+# a world's stage: on both sides of what one CTA holds (rows and bodies of a pyramid of 31
+# or 32 rows; records of the 760 or 840 joints of a grid), and joints that fit a cluster's
+# shared memory (60) or not (100)
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene,size,steps", [("pyramid", 2, 20), ("pyramid", 31, 25), ("pyramid", 32, 25), ("grid", 20, 25), ("grid", 21, 25),
+                                              ("grid", 60, 8), ("grid", 100, 4)])
+def test_world_stage_spaces(gpu, oracle, scene, size, steps):
+    def make(b):
+        return b.pyramid(size, 0.01, 3) if scene == "pyramid" else b.joint_grid(size, -10.0)
+
+    bad, detail, _ = lockstep(gpu, oracle, make, steps, check_manifolds=True)
+    assert bad is None, detail
