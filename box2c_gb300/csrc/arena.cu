@@ -81,10 +81,13 @@ extern "C" int b2gd_init( b2gDevWorld* w, b2gHostIO* io )
 	e = ok( cudaMallocAsync( (void**)&w->counters, 4 * sizeof( int ), s ) );
 	if ( e )
 		return e;
-	e = ok( cudaHostAlloc( (void**)&io->counters, 4 * sizeof( int ), cudaHostAllocDefault ) );
+	e = ok( cudaHostAlloc( (void**)&io->counters, 4 * sizeof( int ), cudaHostAllocMapped ) );
 	if ( e )
 		return e;
 	memset( io->counters, 0, 4 * sizeof( int ) );
+	e = ok( cudaHostGetDevicePointer( (void**)&w->hostCounters, io->counters, 0 ) );
+	if ( e )
+		return e;
 	e = ok( cudaMemsetAsync( w->counters, 0, 4 * sizeof( int ), s ) );
 	if ( e )
 		return e;

@@ -35,7 +35,7 @@ typedef struct b2gSolvePlan
 /* Pinned host staging owned by the device module (mapped into the device). */
 typedef struct b2gHostIO
 {
-	int* counters;		/* [0] events [1] records [2] status [3] sleepy bodies, copied back each sync */
+	int* counters;		/* mapped: [0] events [1] records [3] sleepy bodies, written by each step's kernels */
 	int* events;		/* mapped: narrowphase events */
 	b2gRecord* records; /* mapped: finalisation records */
 	int* sleepy;		/* mapped: bodies past the sleep time, 2 ints each (awake index, sleep time bits) */
@@ -94,15 +94,15 @@ int b2gd_reserve_hits( b2gHostIO* io, int n );
 int b2gd_download_shapes( b2gDevWorld* w, float* aabb, float* fat, int count );
 int b2gd_download_joints( b2gDevWorld* w, b2gJointDev* joints, int count );
 
-/* Step stages.  b2gd_collide launches contact creation and the narrowphase and copies
- * the event count back; b2gd_solve launches the solver and finalisation and copies the
+/* Step stages.  b2gd_collide launches contact creation and the narrowphase, which sends
+ * the event count back; b2gd_solve launches the solver and finalisation, which send the
  * record count back.  b2gd_sync waits for the stream; returns 0 or a CUDA error. */
 int b2gd_collide( b2gDevWorld* w, b2gHostIO* io, int newContactCount, int contactIdCount );
 int b2gd_solve( b2gDevWorld* w, b2gHostIO* io, const b2gSolvePlan* plan, const b2gStepConst* sc );
 /* The fused solver stage and finalisation launched before the narrowphase's events are
  * known; they do nothing when there were events.  1 launched, 0 not (the world does not
  * fit the fused solver), -1 launch error. */
-int b2gd_solve_speculative( b2gDevWorld* w, b2gHostIO* io, const b2gSolvePlan* plan, const b2gStepConst* sc );
+int b2gd_solve_speculative( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc );
 int b2gd_sync( b2gDevWorld* w );
 
 /* ---------------------------------------------------------------- broadphase query */

@@ -537,8 +537,9 @@ static __device__ void finalize_body( const b2gDevWorld& W, int i, const b2gStep
 {
 	int b = W.awake[i];
 	float4* st = (float4*)W.state;
-	float4 s0 = st[2 * b];
-	float4 s1 = st[2 * b + 1];
+	/* at L2: in the fused solver another CTA has just stored them */
+	float4 s0 = __ldcg( st + 2 * b );
+	float4 s1 = __ldcg( st + 2 * b + 1 );
 	float4* xfs = (float4*)W.xf;
 	float4* cen = (float4*)W.centers;
 	float4* prev = (float4*)W.prev;
@@ -608,7 +609,7 @@ static __device__ void finalize_body( const b2gDevWorld& W, int i, const b2gStep
 	for ( int slot = 0; slot < count; ++slot )
 	{
 		int sid = W.shapeList[start + slot];
-		b2gShapeGeo g = W.geo[sid];
+		const b2gShapeGeo& g = W.geo[sid];
 		b2gBox fat = box_of( fats[sid] );
 		if ( isFast )
 		{

@@ -270,7 +270,11 @@ typedef struct b2gDevWorld
 	/* staging and outputs */
 	b2gContactInit* newContacts;
 	int newCap;
-	int* counters;	   /* device: [0] events, [1] records, [2] status, [3] sleepy bodies */
+	/* device: [0] events, [1] records, [2] finished narrowphase blocks, [3] sleepy bodies;
+	 * hostCounters: the device view of the host's copy, which the kernels write */
+	int* counters;
+	int* hostCounters;
+	int countersClean; /* the events and blocks are zero once the stream gets there */
 	int* events;	   /* device view of the mapped event buffer */
 	b2gRecord* records; /* device view of the mapped record buffer */
 	int* sleepy;	   /* device view of the mapped sleepy-body buffer: 2 ints per body (awake index, sleep time bits) */

@@ -49,7 +49,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 																	 const __grid_constant__ FusedSplit S, const __grid_constant__ b2gStepConst sc )
 {
 	/* every CTA of the cluster takes the same branch: no barrier is left waiting */
-	if ( W.guardEvents && W.counters[0] != 0 )
+	if ( W.guardEvents && __ldcg( W.counters ) != 0 )
 		return;
 	constexpr int T = FUSED_THREADS;
 	extern __shared__ float4 smem[];
@@ -89,7 +89,11 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		share[tid].jcount = jl - jf;
 	}
 	if ( tid == 0 )
+	{
 		s_awake = s_ovSlots = 0;
+		if ( rank == 0 )
+			W.counters[1] = W.counters[3] = 0;
+	}
 	__syncthreads();
 	if ( tid == 0 )
 	{
@@ -193,6 +197,20 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 			( (int*)( W.joints + id ) )[t & 63] = ( (const int*)J.local )[RES_JOINT_WORDS * k + ( t & 63 )];
 		}
 	}
+
+	/* finalisation (reference src/solver.c:165-351), then the counts of its records and
+	 * sleepy bodies to the host */
+	bar.sync();
+	for ( int i = rank * T + tid; i < P.awakeCount; i += CL * T )
+		finalize_body( W, i, sc );
+	bar.sync();
+	if ( rank == 0 && tid == 0 )
+	{
+		W.hostCounters[1] = __ldcg( W.counters + 1 );
+		W.hostCounters[3] = __ldcg( W.counters + 3 );
+		/* every CTA has passed the guard: the next narrowphase starts from zero */
+		W.counters[0] = 0;
+	}
 }
 
 static_assert( sizeof( b2gJointDev ) == 256, "the joint copies move 64 words" );
@@ -245,7 +263,7 @@ static int fused_cluster_ready( void )
 	return ready;
 }
 
-/* Launches the fused solver when the world fits on chip; returns the number of launches,
+/* Launches the fused solver and finalisation when the world fits on chip; returns the number of launches,
  * 0 when it does not fit (or clusters of FUSED_CLUSTER CTAs are unavailable) and the
  * caller must use the per-phase kernels, or -1 on a launch error. */
 extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc )

@@ -47,11 +47,24 @@ __global__ void k_body_ops( b2gDevWorld W, const int* ops, int n )
 		apply_body_op( W, ops[t] );
 }
 
+/* The last block to finish writes the event count to the host, which saves a copy after
+ * the kernel. */
 __global__ void __launch_bounds__( BLOCK ) k_collide( b2gDevWorld W, int idCount )
 {
 	int id = blockIdx.x * blockDim.x + threadIdx.x;
 	if ( id < idCount )
 		collide_contact( W, id );
+	__syncthreads();
+	if ( threadIdx.x == 0 )
+	{
+		__threadfence();
+		if ( atomicAdd( W.counters + 2, 1 ) == (int)gridDim.x - 1 )
+		{
+			__threadfence();
+			W.hostCounters[0] = __ldcg( W.counters );
+			W.counters[2] = 0;
+		}
+	}
 }
 
 __global__ void __launch_bounds__( BLOCK ) k_prepare( b2gDevWorld W, int total, b2gStepConst sc )
@@ -63,8 +76,6 @@ __global__ void __launch_bounds__( BLOCK ) k_prepare( b2gDevWorld W, int total, 
 
 __global__ void k_prepare_joints( b2gDevWorld W, int count, b2gStepConst sc )
 {
-	if ( W.guardEvents && W.counters[0] != 0 )
-		return;
 	int t = blockIdx.x * blockDim.x + threadIdx.x;
 	if ( t < count )
 		prepare_joint( W, t, sc );
@@ -93,8 +104,6 @@ __global__ void __launch_bounds__( BLOCK ) k_store( b2gDevWorld W, int total, in
 
 __global__ void __launch_bounds__( BLOCK ) k_finalize( b2gDevWorld W, int awakeCount, b2gStepConst sc )
 {
-	if ( W.guardEvents && W.counters[0] != 0 )
-		return;
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if ( i < awakeCount )
 		finalize_body( W, i, sc );
@@ -162,7 +171,11 @@ extern "C" int b2gd_collide( b2gDevWorld* w, b2gHostIO* io, int newCount, int id
 	w->launches = 0;
 	if ( w->timing )
 		cudaEventRecord( (cudaEvent_t)w->timers[1], s );
-	cudaMemsetAsync( w->counters, 0, 4 * sizeof( int ), s );
+	/* the fused solver of the last step has left the counters ready */
+	if ( w->countersClean == 0 )
+		cudaMemsetAsync( w->counters, 0, 4 * sizeof( int ), s );
+	w->countersClean = 0;
+	io->counters[0] = 0;
 	if ( newCount > 0 )
 	{
 		cudaMemcpyAsync( w->newContacts, io->newContacts, sizeof( b2gContactInit ) * (size_t)newCount, cudaMemcpyHostToDevice, s );
@@ -177,8 +190,7 @@ extern "C" int b2gd_collide( b2gDevWorld* w, b2gHostIO* io, int newCount, int id
 	}
 	if ( w->timing )
 		cudaEventRecord( (cudaEvent_t)w->timers[2], s );
-	cudaMemcpyAsync( io->counters, w->counters, 4 * sizeof( int ), cudaMemcpyDeviceToHost, s );
-	w->d2hBytes += 4 * sizeof( int );
+	w->d2hBytes += sizeof( int );
 	return check( cudaGetLastError() );
 }
 
@@ -297,13 +309,25 @@ extern "C" int b2gd_solve( b2gDevWorld* w, b2gHostIO* io, const b2gSolvePlan* pl
 	int awake = plan->awakeCount;
 	if ( w->timing )
 		cudaEventRecord( (cudaEvent_t)w->timers[3], s );
-	cudaMemsetAsync( w->counters + 1, 0, sizeof( int ), s );
-	cudaMemsetAsync( w->counters + 3, 0, sizeof( int ), s );
 	int fused = w->fused ? b2gd_solver_fused( w, plan, scp ) : 0;
 	if ( fused < 0 )
 		return check( cudaGetLastError() );
 	w->fusedUsed = fused > 0;
-	w->launches += fused > 0 ? fused : b2gd_contact_solver( w, plan, scp );
+	if ( fused > 0 )
+	{
+		w->launches += fused;
+		w->countersClean = 1;
+		w->d2hBytes += 2 * sizeof( int );
+		if ( w->timing )
+		{
+			cudaEventRecord( (cudaEvent_t)w->timers[4], s );
+			cudaEventRecord( (cudaEvent_t)w->timers[5], s );
+		}
+		return check( cudaGetLastError() );
+	}
+	cudaMemsetAsync( w->counters + 1, 0, sizeof( int ), s );
+	cudaMemsetAsync( w->counters + 3, 0, sizeof( int ), s );
+	w->launches += b2gd_contact_solver( w, plan, scp );
 	if ( w->timing )
 		cudaEventRecord( (cudaEvent_t)w->timers[4], s );
 	if ( awake > 0 )
@@ -324,33 +348,26 @@ extern "C" int b2gd_solve( b2gDevWorld* w, b2gHostIO* io, const b2gSolvePlan* pl
  * event every kernel returns at once and the host solves again after processing them.
  * Returns 1 when launched, 0 when the world does not fit the fused solver (nothing
  * launched), or -1 on a launch error. */
-extern "C" int b2gd_solve_speculative( b2gDevWorld* w, b2gHostIO* io, const b2gSolvePlan* plan, const b2gStepConst* scp )
+extern "C" int b2gd_solve_speculative( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* scp )
 {
 	cudaStream_t s = (cudaStream_t)w->stream;
-	int awake = plan->awakeCount;
-	if ( w->fused == 0 || awake <= 0 )
+	if ( w->fused == 0 || plan->awakeCount <= 0 )
 		return 0;
 	w->guardEvents = 1;
 	if ( w->timing )
 		cudaEventRecord( (cudaEvent_t)w->timers[3], s );
-	cudaMemsetAsync( w->counters + 1, 0, sizeof( int ), s );
-	cudaMemsetAsync( w->counters + 3, 0, sizeof( int ), s );
 	int fused = b2gd_solver_fused( w, plan, scp );
-	if ( fused <= 0 )
-	{
-		w->guardEvents = 0;
-		return fused < 0 ? -1 : 0;
-	}
-	if ( w->timing )
-		cudaEventRecord( (cudaEvent_t)w->timers[4], s );
-	k_finalize<<<blocks_for( awake ), BLOCK, 0, s>>>( *w, awake, *scp );
-	if ( w->timing )
-		cudaEventRecord( (cudaEvent_t)w->timers[5], s );
-	cudaMemcpyAsync( io->counters, w->counters, 4 * sizeof( int ), cudaMemcpyDeviceToHost, s );
-	w->d2hBytes += 4 * sizeof( int );
 	w->guardEvents = 0;
+	if ( fused <= 0 )
+		return fused < 0 ? -1 : 0;
+	if ( w->timing )
+	{
+		cudaEventRecord( (cudaEvent_t)w->timers[4], s );
+		cudaEventRecord( (cudaEvent_t)w->timers[5], s );
+	}
+	w->d2hBytes += 2 * sizeof( int );
 	w->fusedUsed = 1;
-	w->launches += fused + 1;
+	w->launches += fused;
 	return cudaGetLastError() == cudaSuccess ? 1 : -1;
 }
 

@@ -1328,7 +1328,7 @@ void gstep_run( gWorld* w, float dt, int subSteps )
 		plan = w->solvePlan;
 		plan.awakeCount = w->awake.count;
 		plan.bodyIdCount = w->bodyIds.next;
-		speculated = b2gd_solve_speculative( &w->dev, &w->io, &plan, &sc );
+		speculated = b2gd_solve_speculative( &w->dev, &plan, &sc );
 	}
 	/* The partial rebuild of the trees (reference src/world.c:420, finished before the
 	 * proxies are enlarged, src/solver.c:1725) runs on the host while the device works:
@@ -1350,6 +1350,7 @@ void gstep_run( gWorld* w, float dt, int subSteps )
 	if ( speculated > 0 && w->io.counters[0] == 0 )
 	{
 		/* no events: the solver stage has run on the lists the host would have used */
+		w->dev.countersClean = 1;
 		gstep_after_collide( w, dt, subSteps, &sc, &plan );
 		gstep_finish( w );
 		return;
