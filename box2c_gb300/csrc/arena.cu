@@ -392,15 +392,39 @@ extern "C" int b2gd_upload_body_velocity( b2gDevWorld* w, int bodyId, const floa
 	return h2d( w, (char*)w->state + 32u * (size_t)bodyId, v3, 12u, (cudaStream_t)w->stream );
 }
 
-extern "C" int b2gd_download_bodies( b2gDevWorld* w, float* state, float* xf, float* centers, int count )
+/* Body mirrors in one launch that writes pinned host memory: three copies and their
+ * wait took 23 us for 210 bodies and 200 us for 22000, most of it launches and, for the
+ * larger, a walk of the host's body records beside them. */
+__global__ void __launch_bounds__( 128 ) k_download_bodies( b2gDevWorld W, float4* state, float4* xf, float4* centers, int count )
 {
+	int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if ( i < 2 * count )
+		state[i] = ( (const float4*)W.state )[i];
+	if ( i < count )
+	{
+		xf[i] = ( (const float4*)W.xf )[i];
+		centers[i] = ( (const float4*)W.centers )[i];
+	}
+}
+
+extern "C" int b2gd_download_bodies( b2gDevWorld* w, void* state, void* xf, void* centers, int count )
+{
+	if ( count <= 0 )
+		return 0;
 	cudaStream_t s = (cudaStream_t)w->stream;
-	size_t n4 = 16u * (size_t)count;
-	int e = d2h( w, state, w->state, 2 * n4, s );
-	e |= d2h( w, xf, w->xf, n4, s );
-	e |= d2h( w, centers, w->centers, n4, s );
+	k_download_bodies<<<( 2 * count + 127 ) / 128, 128, 0, s>>>( *w, (float4*)state, (float4*)xf, (float4*)centers, count );
+	w->d2hBytes += 64ll * count;
+	int e = ok( cudaGetLastError() );
 	e |= ok( cudaStreamSynchronize( s ) );
 	return e;
+}
+
+extern "C" void* b2gd_device_view( void* pinned )
+{
+	void* d = nullptr;
+	if ( pinned == nullptr || ok( cudaHostGetDevicePointer( &d, pinned, 0 ) ) != 0 )
+		return nullptr;
+	return d;
 }
 
 /* Hit test of one contact (reference src/solver.c:1688-1712): the point with the largest

@@ -83,7 +83,10 @@ int b2gd_upload_pose( b2gDevWorld* w, int bodyId, const float* xf4, const float*
 int b2gd_upload_shape_boxes( b2gDevWorld* w, int shapeId, const float* aabb4, const float* fat4 );
 
 /* Device -> host copies. */
-int b2gd_download_bodies( b2gDevWorld* w, float* state, float* xf, float* centers, int count );
+/* Bodies [0, count) into the pinned mirrors, given as the device sees them. */
+int b2gd_download_bodies( b2gDevWorld* w, void* state, void* xf, void* centers, int count );
+/* The device's view of pinned host memory; null when there is none. */
+void* b2gd_device_view( void* pinned );
 int b2gd_download_manifolds( b2gDevWorld* w, b2gManifold* out, uint32_t* flags, int count );
 /* Hit test of the contacts ids[0..n) after the solver stage (reference
  * src/solver.c:1670-1723): out[8 k ..] = hit flag, approach speed and point of the

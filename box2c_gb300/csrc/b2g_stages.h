@@ -565,6 +565,12 @@ static __device__ void finalize_body( const b2gDevWorld& W, int i, const b2gStep
 	xf.q = q;
 	xfs[b] = make_float4( p.x, p.y, q.c, q.s );
 	cen[b] = make_float4( center.x, center.y, c.z, c.w );
+	if ( W.mirrorXf != nullptr )
+	{
+		( (float4*)W.mirrorXf )[b] = make_float4( p.x, p.y, q.c, q.s );
+		( (float4*)W.mirrorState )[2 * b] = s0;
+		( (float4*)W.mirrorState )[2 * b + 1] = make_float4( 0.0f, 0.0f, 1.0f, 0.0f );
+	}
 	float4* fo = (float4*)W.force;
 	float4 f = fo[b];
 	fo[b] = make_float4( 0.0f, 0.0f, 0.0f, f.w );

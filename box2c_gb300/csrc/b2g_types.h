@@ -281,6 +281,10 @@ typedef struct b2gDevWorld
 	int eventCap, recordCap, sleepyCap;
 	void* stream; /* cudaStream_t */
 	void* timers[8]; /* cudaEvent_t: step start, collide start/end, solve start/end, finalize end, step end */
+	/* the host's pinned mirrors of xf and state as the device sees them, in a step whose
+	 * finalisation writes the bodies' poses and velocities through; else null */
+	void* mirrorXf;
+	void* mirrorState;
 	int timing;
 	int launches;
 	long long h2dBytes, d2hBytes; /* host <-> device bytes of the current step */

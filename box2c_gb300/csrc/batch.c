@@ -82,6 +82,7 @@ static void begin_worlds( int begin, int end, void* arg )
 		w->dev.h2dBytes = 0;
 		w->dev.d2hBytes = 0;
 		gworld_flush( w );
+		gworld_begin_mirrors( w );
 		int staged = gstep_begin( w );
 		if ( staged < 0 )
 			continue;
@@ -169,9 +170,7 @@ static void finish_worlds( int begin, int end, void* arg )
 		w->batching = false;
 		w->dev.launches = 0;
 		w->dev.fusedUsed = 0;
-		w->mirrorStale = true;
-		w->shapeMirrorStale = true;
-		w->jointMirrorStale = true;
+		gworld_end_mirrors( w );
 	}
 }
 

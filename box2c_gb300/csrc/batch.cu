@@ -408,6 +408,7 @@ __global__ void __launch_bounds__( T, MINB ) k_batch_solve( const b2gBatchItem* 
 	}
 }
 
+static_assert( CTA_SHARED_MAX + SOLVE_STATIC_BYTES( 512 ) <= SM_SHARED_BYTES, "the largest solver CTA fits an SM" );
 static_assert( PACK_WORLDS * 32 >= 512, "a pack holds a world for every warp of the largest CTA" );
 
 /* ------------------------------------------------------------------ host side */

@@ -300,6 +300,7 @@ typedef struct gWorld
 	float* hExtent;
 	int* hInfo;
 	int mirrorCap;
+	void *dState, *dXf, *dCenters; /* the device's view of those mirrors */
 	b2gShapeGeo* hGeo;
 	float* hAabb;
 	float* hFat;
@@ -359,6 +360,10 @@ typedef struct gWorld
 	/* dirty / stale tracking */
 	bool bodiesDirty, awakeDirty, shapesDirty, shapeListsDirty, jointsDirty, solveDirty;
 	bool mirrorStale, shapeMirrorStale, jointMirrorStale;
+	/* hState and hXf are the device's although mirrorStale (the last steps' finalisation
+	 * wrote them through); poseReads: steps that still do so, since a read-back asked */
+	bool poseFresh;
+	int poseReads;
 
 	b2ContactBeginTouchEvent* beginEvents;
 	int beginCount, beginCap;
@@ -401,6 +406,9 @@ void gworld_fail( const char* what );
 bool gworld_out_of_memory( gWorld* w, int before );
 
 void gworld_ensure_mirror( gWorld* w );
+void gworld_ensure_pose( gWorld* w );
+void gworld_begin_mirrors( gWorld* w );
+void gworld_end_mirrors( gWorld* w );
 void gworld_ensure_shape_mirror( gWorld* w );
 bool gworld_reserve_mirrors( gWorld* w ); /* false when pinned memory ran out */
 void gworld_flush( gWorld* w );

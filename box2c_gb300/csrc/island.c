@@ -191,7 +191,12 @@ int gbody_flush_ops( gWorld* w )
 	{
 		e |= b2gd_body_ops( &w->dev, w->bodyOps.data, w->bodyOps.count );
 		for ( int i = 0; i < w->bodyOps.count; ++i )
+		{
+			/* waking clears a velocity on the device that the pose mirrors still show */
+			if ( ( w->bodyOps.data[i] & 3 ) == B2G_BODY_WAKE )
+				w->poseFresh = false;
 			w->bodyOpSlot[w->bodyOps.data[i] >> 2] = B2G_NULL;
+		}
 		w->bodyOps.count = 0;
 	}
 	if ( w->awakeDirty )

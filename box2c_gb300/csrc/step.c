@@ -900,6 +900,8 @@ static void solve_continuous( gWorld* w, b2gRecord* recs, int n, bool bullet )
 	float center4[4] = { c.x, c.y, q.sweep.localCenter.x, q.sweep.localCenter.y };
 	float prev4[4] = { c.x, c.y, rq.c, rq.s };
 	int e = b2gd_upload_pose( &w->dev, bodyId, xf4, center4, prev4 );
+	if ( w->mirrorStale && w->dev.mirrorXf != NULL )
+		memcpy( w->hXf + 4 * bodyId, xf4, 16 );
 	if ( w->mirrorStale == false )
 	{
 		memcpy( w->hXf + 4 * bodyId, xf4, 16 );
@@ -1396,12 +1398,11 @@ void b2World_Step( b2WorldId worldId, float timeStep, int subStepCount )
 	memset( w->hostMs, 0, sizeof( w->hostMs ) );
 	b2gd_mark( &w->dev, 0 );
 	gworld_flush( w );
+	gworld_begin_mirrors( w );
 	if ( w->status == 0 )
 		gstep_run( w, timeStep, subStepCount );
 	b2gd_mark( &w->dev, 6 );
-	w->mirrorStale = true;
-	w->shapeMirrorStale = true;
-	w->jointMirrorStale = true;
+	gworld_end_mirrors( w );
 	w->locked = false;
 	w->profile.step = (float)( b2g_now_ms() - t0 );
 	gworld_out_of_memory( w, failures );

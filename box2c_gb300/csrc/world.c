@@ -147,7 +147,7 @@ static bool grow_pinned( void** ptrs[], const size_t oldBytes[], const size_t ne
 	for ( int i = 0; i < n; ++i )
 	{
 		fresh[i] = NULL;
-		if ( cudaHostAlloc( &fresh[i], newBytes[i], cudaHostAllocDefault ) != cudaSuccess )
+		if ( cudaHostAlloc( &fresh[i], newBytes[i], cudaHostAllocMapped ) != cudaSuccess )
 		{
 			for ( int k = 0; k < i; ++k )
 				cudaFreeHost( fresh[k] );
@@ -180,6 +180,9 @@ bool gworld_reserve_mirrors( gWorld* w )
 		size_t nb[] = { 2 * n4, n4, n4, n4, n4, n4, n4, 4u * (size_t)nc };
 		if ( grow_pinned( ptrs, ob, nb, 8 ) == false )
 			return false;
+		w->dState = b2gd_device_view( w->hState );
+		w->dXf = b2gd_device_view( w->hXf );
+		w->dCenters = b2gd_device_view( w->hCenters );
 		w->mirrorCap = nc;
 	}
 	int needS = w->shapeIds.next;
@@ -222,7 +225,7 @@ void gworld_ensure_mirror( gWorld* w )
 	if ( w->mirrorStale == false )
 		return;
 	int n = w->bodyIds.next;
-	int e = b2gd_download_bodies( &w->dev, w->hState, w->hXf, w->hCenters, n );
+	int e = b2gd_download_bodies( &w->dev, w->dState, w->dXf, w->dCenters, n );
 	if ( e )
 		w->status = e;
 	/* finalisation zeroes forces and advances the sweep start to the current pose */
@@ -242,6 +245,44 @@ void gworld_ensure_mirror( gWorld* w )
 		}
 	}
 	w->mirrorStale = false;
+}
+
+/* Poses and velocities in hXf and hState, as the getters of those alone need them.  A
+ * world that is read keeps its finalisation writing them through for the next
+ * POSE_READ_STEPS steps, so a read after each of them costs no device round trip (a step
+ * of the 20-row pyramid with its read: 88 us, 73 so; of the large one 199 and 157; ten
+ * batched steps of 160 pyramids and their reads 8655 and 5420); the writes are 48 bytes a
+ * body, so a rollout may read as seldom as that. */
+#define POSE_READ_STEPS 64
+
+void gworld_ensure_pose( gWorld* w )
+{
+	w->poseReads = POSE_READ_STEPS;
+	if ( w->bodyOps.count == 0 && w->poseFresh )
+		return;
+	gworld_ensure_mirror( w );
+}
+
+/* Before a step's kernels: whether this step's finalisation writes the mirrors. */
+void gworld_begin_mirrors( gWorld* w )
+{
+	if ( w->mirrorStale == false )
+		w->poseFresh = true;
+	bool through = w->poseReads > 0 && w->dXf != NULL && w->dState != NULL && w->bodyIds.next <= w->mirrorCap;
+	w->poseReads -= w->poseReads > 0;
+	w->dev.mirrorXf = through ? w->dXf : NULL;
+	w->dev.mirrorState = through ? w->dState : NULL;
+}
+
+/* After it: the device copy is the authoritative one. */
+void gworld_end_mirrors( gWorld* w )
+{
+	w->poseFresh = w->poseFresh && w->dev.mirrorXf != NULL;
+	w->dev.mirrorXf = NULL;
+	w->dev.mirrorState = NULL;
+	w->mirrorStale = true;
+	w->shapeMirrorStale = true;
+	w->jointMirrorStale = true;
 }
 
 void gworld_ensure_shape_mirror( gWorld* w )
@@ -715,7 +756,7 @@ void* b2Body_GetUserData( b2BodyId id ) { return get_body( id )->userData; }
 b2Transform b2Body_GetTransform( b2BodyId id )
 {
 	gWorld* w = body_world( id );
-	gworld_ensure_mirror( w );
+	gworld_ensure_pose( w );
 	const float* x = w->hXf + 4 * ( id.index1 - 1 );
 	b2Transform t = { { x[0], x[1] }, { x[2], x[3] } };
 	return t;
@@ -732,7 +773,7 @@ b2Vec2 b2Body_GetLinearVelocity( b2BodyId id )
 	gWorld* w = body_world( id );
 	if ( get_body( id )->setIndex != G_SET_AWAKE )
 		return b2Vec2_zero;
-	gworld_ensure_mirror( w );
+	gworld_ensure_pose( w );
 	const float* s = w->hState + 8 * ( id.index1 - 1 );
 	b2Vec2 v = { s[0], s[1] };
 	return v;
@@ -743,7 +784,7 @@ float b2Body_GetAngularVelocity( b2BodyId id )
 	gWorld* w = body_world( id );
 	if ( get_body( id )->setIndex != G_SET_AWAKE )
 		return 0.0f;
-	gworld_ensure_mirror( w );
+	gworld_ensure_pose( w );
 	return w->hState[8 * ( id.index1 - 1 ) + 2];
 }
 
@@ -1613,13 +1654,16 @@ void b2World_EnableFusedSolver( b2WorldId worldId, bool flag )
 int b2World_GetBodyStates( b2WorldId worldId, float* out, int capacity )
 {
 	gWorld* w = gworld_get( worldId );
-	gworld_ensure_mirror( w );
 	int n = w->bodyIds.next;
+	if ( capacity <= 0 )
+		return n;
+	gworld_ensure_pose( w );
 	for ( int i = 0; i < n && i < capacity; ++i )
 	{
 		const float* x = w->hXf + 4 * i;
 		const float* s = w->hState + 8 * i;
-		bool moving = w->bodies[i].id == i && w->bodies[i].type != b2_staticBody;
+		/* static bodies and free slots have type bits of zero */
+		bool moving = ( w->hInfo[i] & B2G_B_TYPE_MASK ) != 0;
 		float* o = out + 7 * i;
 		o[0] = x[0];
 		o[1] = x[1];

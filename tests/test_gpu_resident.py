@@ -100,3 +100,48 @@ def test_world_stage_spaces(gpu, oracle, scene, size, steps):
 
     bad, detail, _ = lockstep(gpu, oracle, make, steps, check_manifolds=True)
     assert bad is None, detail
+
+
+@pytest.mark.gpu
+def test_read_back_follows_every_step(gpu, oracle):
+    """Body states read back after each step, after several steps, after body edits and
+    wakes, and after batched steps are the device's (a second world that is never read
+    between steps, or the oracle, says what they are)."""
+    from box2c_gb300.capi import Vec2, bind_batch_api, bind_gpu_api, world_array
+
+    bind_gpu_api(gpu.lib)
+    bind_batch_api(gpu.lib)
+
+    def read(world):
+        n = gpu.lib.b2World_GetBodyStates(world, None, 0)
+        out = np.zeros((n, 7), np.float32)
+        assert gpu.lib.b2World_GetBodyStates(world, out.ctypes.data, n) == n
+        return out.view(np.uint32)
+
+    scenes = [lambda b: b.pyramid(8, 0.01, 3), lambda b: b.fast_shots(20), lambda b: b.sleep_scene(), lambda b: b.tumbler(80, 5, 0)]
+    for k, make in enumerate(scenes):
+        w, o = make(gpu), make(oracle)
+        for step in range(1, 150 if k == 2 else 90):
+            batched = step % 5 == 0 and k != 2
+            if batched:
+                ids = world_array([w])
+                gpu.lib.b2World_StepBatch(ids, 1, 1.0 / 60.0, 4)
+            else:
+                gpu.step(w)
+            oracle.step(o)
+            if k == 2:  # scripted wakes, destructions and velocity changes
+                gpu.sleep_step(w, step)
+                oracle.sleep_step(o, step)
+            if step % 7 in (0, 1, 2):
+                got = read(w).view(np.float32)
+                want = oracle.bodies(o)[:, :7]
+                live = np.isfinite(want).all(1)
+                cols = 4 if k == 2 else 7  # a sleeping body keeps its last velocity here
+                assert np.array_equal(got[live][:, :cols].view(np.uint32), want[live][:, :cols].view(np.uint32)), (k, step)
+                # a second read is the same, and so is one of the full mirror
+                assert np.array_equal(read(w), got.view(np.uint32))
+                full = gpu.bodies(w)[:, :7]
+                both = np.isfinite(full).all(1)
+                assert np.array_equal(got[both][:, :4].view(np.uint32), full[both][:, :4].view(np.uint32)), (k, step)
+        gpu.destroy(w)
+        oracle.destroy(o)
