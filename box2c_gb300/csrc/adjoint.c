@@ -6,7 +6,7 @@
  * (4 float4 per body id) and solver rows (b2gTapeRow) on the world's stream and keeps a
  * host header (b2gTapeStep) with their offsets, the solve plan and the step constants.
  * The backward call uploads the headers, the loss gradient and the shape frictions of
- * every world, launches the backward kernel (one warp per world) and downloads the
+ * every world, launches the backward kernels, chunk by chunk of steps, and downloads the
  * gradients.
  */
 #include "host.h"
@@ -170,6 +170,10 @@ typedef struct gAdjointCtx
 	size_t scratchCap;
 } gAdjointCtx;
 
+/* Device memory for the replays of a chunk of steps (a step that needs more is replayed
+ * alone). */
+#define ADJOINT_CHUNK_BYTES ( (size_t)512 << 20 )
+
 static gAdjointCtx s_adj;
 static int s_lastCheck[2];
 
@@ -223,7 +227,8 @@ int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStr
 {
 	if ( worldIds == NULL || count <= 0 || gradFinal == NULL || gradInitial == NULL )
 		return -1;
-	size_t headerBytes = 0, scratchFloats = 0;
+	size_t headerBytes = 0, scratchFloats = 0, stepFloats = 0;
+	int steps = 1, bodies = 1, rows = 1, sub = 1;
 	for ( int i = 0; i < count; ++i )
 	{
 		if ( b2World_IsValid( worldIds[i] ) == false )
@@ -233,8 +238,28 @@ int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStr
 		if ( t == NULL || t->steps == 0 || t->bodies > bodyStride || w->shapeIds.next > shapeStride || w->status != 0 )
 			return -1;
 		headerBytes += sizeof( b2gTapeStep ) * (size_t)t->steps;
-		scratchFloats += b2gd_adjoint_scratch( t->bodies, t->maxRows, w->dev.contactCap, 16 );
+		for ( int k = 0; k < t->steps; ++k )
+			sub = t->hdr[k].sc.subSteps > sub ? t->hdr[k].sc.subSteps : sub;
+		steps = t->steps > steps ? t->steps : steps;
+		bodies = t->bodies > bodies ? t->bodies : bodies;
+		rows = t->maxRows > rows ? t->maxRows : rows;
 	}
+	/* a step of more substeps is reported, not replayed */
+	sub = sub > 16 ? 16 : sub;
+	for ( int i = 0; i < count; ++i )
+	{
+		gWorld* w = gworld_get( worldIds[i] );
+		stepFloats += b2gd_adjoint_step_scratch( w->tape->bodies, w->tape->maxRows, w->dev.contactCap, sub );
+	}
+	/* as many steps at a time as fit the budget: the replays of a chunk run side by side */
+	int chunk = (int)( ADJOINT_CHUNK_BYTES / ( sizeof( float ) * stepFloats ) );
+	chunk = chunk < 1 ? 1 : ( chunk > steps ? steps : chunk );
+	for ( int i = 0; i < count; ++i )
+	{
+		gWorld* w = gworld_get( worldIds[i] );
+		scratchFloats += b2gd_adjoint_scratch( w->tape->bodies, w->tape->maxRows, chunk );
+	}
+	scratchFloats += stepFloats * (size_t)chunk;
 	size_t gradBytes = sizeof( float ) * (size_t)count * ( 12u * (size_t)bodyStride + 2u * (size_t)shapeStride );
 	size_t statusBytes = sizeof( int ) * 4u * (size_t)count;
 	size_t bufBytes = round_up( headerBytes, 256 ) + round_up( gradBytes, 256 ) + statusBytes;
@@ -271,25 +296,31 @@ int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStr
 		it->stepCount = t->steps;
 		it->bodies = t->bodies;
 		it->shapes = w->shapeIds.next;
-		it->maxRows = t->maxRows;
+		it->maxRows = t->maxRows > 0 ? t->maxRows : 1;
 		it->contactCap = w->dev.contactCap;
+		it->maxSub = sub;
+		it->chunk = chunk;
 		float* dg = dGrad + perWorld * (size_t)i;
 		it->gradFinal = dg;
 		it->gradInitial = dg + 6u * (size_t)bodyStride;
 		it->shapeFriction = dg + 12u * (size_t)bodyStride;
 		it->gradFriction = dg + 12u * (size_t)bodyStride + (size_t)shapeStride;
+		it->stepFloats = b2gd_adjoint_step_scratch( t->bodies, t->maxRows, w->dev.contactCap, sub );
+		it->stepScratch = s_adj.scratch + scratchOff;
+		scratchOff += it->stepFloats * (size_t)chunk;
 		it->scratch = s_adj.scratch + scratchOff;
 		it->status = (int*)( db + statusOff ) + 4 * i;
 		hdrOff += sizeof( b2gTapeStep ) * (size_t)t->steps;
-		scratchOff += b2gd_adjoint_scratch( t->bodies, t->maxRows, w->dev.contactCap, 16 );
+		scratchOff += b2gd_adjoint_scratch( t->bodies, t->maxRows, chunk );
 	}
 	/* the recordings were made on the worlds' streams */
 	if ( cudaDeviceSynchronize() != cudaSuccess )
 		return (int)cudaGetLastError();
 	cudaStream_t s = s_adj.stream;
 	cudaMemcpyAsync( db, hb, statusOff, cudaMemcpyHostToDevice, s );
+	cudaMemsetAsync( db + statusOff, 0, statusBytes, s );
 	cudaMemcpyAsync( s_adj.dItems, s_adj.hItems, sizeof( b2gAdjointItem ) * (size_t)count, cudaMemcpyHostToDevice, s );
-	int e = b2gd_adjoint_launch( s_adj.dItems, count, (void*)s );
+	int e = b2gd_adjoint_launch( s_adj.dItems, count, steps, chunk, bodies, rows, sub, (void*)s );
 	cudaMemcpyAsync( hb + gradOff, db + gradOff, statusOff + statusBytes - gradOff, cudaMemcpyDeviceToHost, s );
 	cudaError_t se = cudaStreamSynchronize( s );
 	if ( e != 0 )

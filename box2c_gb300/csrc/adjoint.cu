@@ -6,18 +6,33 @@
  * coloured rows with the manifolds the narrowphase produced (warm-start impulses
  * included).
  *
- * Backward (k_adjoint, one warp per world, steps in reverse): each step is first
- * replayed forward from its record -- the same b2g_solve.h arithmetic in the same
- * order, so the replay is bit-identical -- keeping per-substep body snapshots and, for
- * every row and phase, the velocities and impulses the row started from; the contact
- * geometry is recomputed with dual numbers (b2g_dual.h) for its Jacobian.  Then the
- * step is differentiated backwards: finalisation, restitution colours in reverse
- * order, and per substep in reverse: relax colours reversed, position integration,
- * solve colours reversed, warm-start colours reversed, velocity integration; then the
- * row preparation and the narrowphase Jacobian.  Within a colour no two rows share a
- * body, so a colour's row adjoints run in parallel lanes without conflicts.  The
- * adjoint of the warm-start impulses goes to the previous step's stored impulses
- * through the narrowphase's feature-id matching (reference src/contact.c:555-568).
+ * Backward, in chunks of steps from the last to the first:
+ *   k_adjoint_replay   one warp per world and step, all steps of a chunk at once: a step
+ *                      depends only on its record.  It is replayed forward -- the same
+ *                      b2g_solve.h arithmetic in the same order, so the replay is
+ *                      bit-identical -- keeping body snapshots and, for every row and
+ *                      phase, the velocities before each of its impulses; the contact
+ *                      geometry is recomputed with dual numbers (b2g_dual.h) for its
+ *                      Jacobian.
+ *   k_adjoint_reverse  one warp per world, the chunk's steps in reverse: finalisation,
+ *                      restitution colours in reverse order, and per substep in reverse:
+ *                      relax colours reversed, position integration, solve colours
+ *                      reversed, warm-start colours reversed, velocity integration; then
+ *                      the row preparation and the narrowphase Jacobian.  A step's
+ *                      replay comes into shared memory by a bulk copy while the step
+ *                      after it is differentiated.
+ *   k_adjoint_friction one thread per shape: the friction gradient's sums, in step and
+ *                      row order.
+ * Only the reverse pass is a chain over the steps, and it is bound by that chain: about
+ * 18 us a step of some 70 dependent sweeps.  96 worlds of 8 boxes and 120 steps, one warp
+ * a world doing replay, Jacobians and reverse in turn before: 10.9 ms a call; now 3.2 ms
+ * (replay 0.68, reverse 2.13, friction 0.03).  Replaying the next chunk on a second
+ * stream beside the reverse pass took 3.6 ms: the two share the SMs' issue slots.
+ *
+ * Within a colour no two rows share a body, so a colour's row adjoints run in parallel
+ * lanes without conflicts.  The adjoint of the warm-start impulses goes to the previous
+ * step's stored impulses through the narrowphase's feature-id matching (reference
+ * src/contact.c:555-568).
  *
  * Differentiated: body centres, angles, linear and angular velocities, and contact
  * friction (mixed per shape as sqrt(muA * muB), reference src/contact.c:42-45).  The
@@ -50,71 +65,107 @@ extern "C" int b2gd_tape_record( b2gDevWorld* w, void* bodyDst, int bodies, void
 }
 
 /* ------------------------------------------------------------------ scratch layout */
-/* Per body: adjoint (12), replay state (8), step start (12), velocity terms (8).
- * Per body and snapshot: 8.  Per row: Row (64), adjoint (24), Jacobian (72), and 12
- * per phase.  Per contact id: impulse adjoint (4) + stamp, previous-step row + stamp. */
 #define ADJ_BODY 12
 #define ADJ_STATE 8
-#define ADJ_START 12
-#define ADJ_TERMS 8
+#define ADJ_START 9
+#define ADJ_TERMS 5
 #define ADJ_SNAP 8
-#define ADJ_ROW 64
 #define ADJ_RADJ 24
 #define ADJ_JAC 72
-#define ADJ_PHASE 12
 #define ADJ_MAX_SUBSTEPS 16
+/* what the reverse pass reads of a row: bodies, count, normal, friction, restitution,
+ * masses, anchors, coefficients and the link to the previous step's row; of its phases: the impulses and the velocities of
+ * both bodies before each impulse (none for a warm start, four for solve and relax, two
+ * for restitution) */
+#define ADJ_ROW 28
+#define ADJ_WARM 4
+#define ADJ_SOLVE 28
+#define ADJ_REST 16
 
-static_assert( sizeof( Row ) <= ADJ_ROW * 4, "row record must fit its scratch slot" );
-
-struct AdjLayout
+/* One step's replay, as the reverse pass reads it: field f of row k at [f * Rs + k], of
+ * body b at [f * Ns + b], offsets in floats; then the replay's own working arrays. */
+struct AdjStep
 {
-	float* bodyAdj;
-	float* state;
-	float* start;
-	float* terms;
-	float* snap;
-	float* rows;
-	float* radj;
-	float* jac;
-	float* phase;
-	float* lam;	 /* 4 per contact id */
-	int* lamStamp;
-	int* prevRow;
-	int* prevStamp;
+	int Rs, Ns, S;
+	size_t rows, phase, jac, snap, start, terms;
+	size_t copy; /* floats of the parts above */
+	size_t work, state, total;
+
+	__host__ __device__ size_t warm( int sub ) const { return phase + (size_t)sub * ( ADJ_WARM + 2 * ADJ_SOLVE ) * Rs; }
+	__host__ __device__ size_t solve( int sub, int relax ) const { return warm( sub ) + (size_t)( ADJ_WARM + ADJ_SOLVE * relax ) * Rs; }
+	__host__ __device__ size_t rest() const { return warm( S ); }
 };
 
-static __host__ __device__ size_t adj_layout( AdjLayout* L, float* base, int N, int R, int C, int S )
+static __host__ __device__ AdjStep adj_step( int N, int R, int S )
+{
+	AdjStep l;
+	l.Rs = ( R + 3 ) & ~3;
+	l.Ns = ( N + 3 ) & ~3;
+	l.S = S;
+	size_t o = 0, Rs = (size_t)l.Rs, Ns = (size_t)l.Ns;
+	l.rows = o;
+	o += ADJ_ROW * Rs;
+	l.phase = o;
+	o += ( (size_t)S * ( ADJ_WARM + 2 * ADJ_SOLVE ) + ADJ_REST ) * Rs;
+	l.jac = o;
+	o += ADJ_JAC * Rs;
+	l.snap = o;
+	o += (size_t)( 2 * S + 1 ) * ADJ_SNAP * Ns;
+	l.start = o;
+	o += ADJ_START * Ns;
+	l.terms = o;
+	o += ADJ_TERMS * Ns;
+	l.copy = o;
+	l.work = o;
+	o += sizeof( Row ) / 4 * Rs;
+	l.state = o;
+	o += ADJ_STATE * Ns;
+	l.total = o;
+	return l;
+}
+
+/* What a world carries from step to step: body adjoints, rotation and local centre at the
+ * last differentiated step's start (4 per body), impulse adjoints of the step to come and
+ * the one before it (4 per row each), friction adjoints of a chunk's rows. */
+struct AdjWorld
+{
+	float* bodyAdj;
+	float* pose;
+	float* lam;
+	float* mu;
+};
+
+static __host__ __device__ size_t adj_world( AdjWorld* L, float* base, int N, int R, int chunk )
 {
 	size_t o = 0;
-	float* b = base;
 	auto take = [&]( size_t n ) {
-		float* p = b ? b + o : nullptr;
+		float* p = base ? base + o : nullptr;
 		o += ( n + 3 ) & ~(size_t)3;
 		return p;
 	};
-	AdjLayout l;
+	AdjWorld l;
 	l.bodyAdj = take( (size_t)N * ADJ_BODY );
-	l.state = take( (size_t)N * ADJ_STATE );
-	l.start = take( (size_t)N * ADJ_START );
-	l.terms = take( (size_t)N * ADJ_TERMS );
-	l.snap = take( (size_t)( 2 * S + 1 ) * N * ADJ_SNAP );
-	l.rows = take( (size_t)R * ADJ_ROW );
-	l.radj = take( (size_t)R * ADJ_RADJ );
-	l.jac = take( (size_t)R * ADJ_JAC );
-	l.phase = take( (size_t)( 3 * S + 1 ) * R * ADJ_PHASE );
-	l.lam = take( (size_t)C * 4 );
-	l.lamStamp = (int*)take( (size_t)C );
-	l.prevRow = (int*)take( (size_t)C );
-	l.prevStamp = (int*)take( (size_t)C );
+	l.pose = take( (size_t)N * 4 );
+	l.lam = take( (size_t)R * 8 );
+	l.mu = take( (size_t)R * chunk );
 	if ( L )
 		*L = l;
 	return o;
 }
 
-extern "C" size_t b2gd_adjoint_scratch( int bodies, int maxRows, int contactCap, int subSteps )
+static int at_least_one( int v ) { return v < 1 ? 1 : v; }
+
+/* Scratch floats of one world: carried from step to step, and of one step's replay. */
+extern "C" size_t b2gd_adjoint_scratch( int bodies, int maxRows, int chunk )
 {
-	int S = subSteps < 1 ? 1 : subSteps;
-	return adj_layout( nullptr, nullptr, bodies, maxRows < 1 ? 1 : maxRows, contactCap < 1 ? 1 : contactCap, S );
+	AdjStep l = adj_step( bodies, at_least_one( maxRows ), 1 );
+	return adj_world( nullptr, nullptr, l.Ns, l.Rs, chunk );
+}
+
+/* with the table of the previous step's rows by contact id */
+extern "C" size_t b2gd_adjoint_step_scratch( int bodies, int maxRows, int contactCap, int subSteps )
+{
+	return adj_step( bodies, at_least_one( maxRows ), subSteps ).total + ( ( (size_t)at_least_one( contactCap ) + 3 ) & ~(size_t)3 );
 }
 
 /* ------------------------------------------------------------------ helpers */
@@ -202,14 +253,12 @@ __device__ void warm_vjp( const Row& r, const BodyV& aA, const BodyV& aB, RowAdj
 	}
 }
 
-/* Solve / relax.  r holds the impulses before the row ran; a, b the states before it
- * (velocities) and the substep's position deltas.  On entry aA, aB are the adjoints of
- * the velocities after the row; on exit, before it.  dpA.. receive the position-delta
- * adjoints.  scalar: an overflow row, whose speculative points (s > 0) take the rigid
- * mass and no impulse scaling where the 8-lane rows keep the soft ones (reference
- * src/contact_solver.c:266-279 against :905-925). */
-__device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2gStepConst& sc, BodyV& aA, BodyV& aB, RowAdj& ra,
-						   float* dpA, float* dqA, float* dpB, float* dqB, bool scalar = false )
+/* The velocities before each of the row's four impulses (two normal, two friction), from
+ * the impulses and velocities before the row.  scalar: an overflow row, whose speculative
+ * points (s > 0) take the rigid mass and no impulse scaling where the 8-lane rows keep
+ * the soft ones (reference src/contact_solver.c:266-279 against :905-925). */
+__device__ __forceinline__ void solve_trace( Row r, DevState a, DevState b, bool useBias, const b2gStepConst& sc, bool scalar, DevState* sa,
+											 DevState* sb )
 {
 	float biasRate = useBias ? r.biasRate : 0.0f;
 	float massScale = useBias ? r.massScale : 1.0f;
@@ -218,12 +267,7 @@ __device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2
 	b2gVec n = r.n;
 	b2gVec t = gv( n.y, 0.0f - n.x );
 	b2gVec dp = gv( b.dp.x - a.dp.x, b.dp.y - a.dp.y );
-
-	/* forward replay with snapshots before each of the four point updates */
-	DevState sa[4], sb[4];
-	float ni0[2] = { r.ni[0], r.ni[1] };
-	float ti0[2] = { r.ti[0], r.ti[1] };
-	float s_[2], dbds[2], xN[2], ms_[2], is_[2];
+#pragma unroll
 	for ( int j = 0; j < 2; ++j )
 	{
 		sa[j] = a;
@@ -233,33 +277,18 @@ __device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2
 		b2gVec rsB = gv( b.dq.c * aB_.x - b.dq.s * aB_.y, b.dq.s * aB_.x + b.dq.c * aB_.y );
 		b2gVec ds = gv( dp.x + ( rsB.x - rsA.x ), dp.y + ( rsB.y - rsA.y ) );
 		float s = ( n.x * ds.x + n.y * ds.y ) + r.base[j];
-		float bias;
-		if ( s > 0.0f )
-		{
-			bias = s * sc.inv_h;
-			dbds[j] = sc.inv_h;
-		}
-		else
-		{
-			float soft = biasRate * s;
-			bias = gmax( soft, minBias );
-			dbds[j] = soft > minBias ? biasRate : 0.0f;
-		}
-		s_[j] = s;
-		ms_[j] = scalar && s > 0.0f ? 1.0f : massScale;
-		is_[j] = scalar && s > 0.0f ? 0.0f : impulseScale;
+		float bias = s > 0.0f ? s * sc.inv_h : gmax( biasRate * s, minBias );
+		float ms = scalar && s > 0.0f ? 1.0f : massScale;
+		float is = scalar && s > 0.0f ? 0.0f : impulseScale;
 		b2gVec dv = lane_dv( a, b, aA_, aB_ );
 		float vn = dv.x * n.x + dv.y * n.y;
-		float negImpulse = r.nMass[j] * ( ms_[j] * ( vn + bias ) ) + is_[j] * r.ni[j];
-		float x = r.ni[j] - negImpulse;
-		xN[j] = x;
-		float newImpulse = gmax( x, 0.0f );
+		float negImpulse = r.nMass[j] * ( ms * ( vn + bias ) ) + is * r.ni[j];
+		float newImpulse = gmax( r.ni[j] - negImpulse, 0.0f );
 		float impulse = newImpulse - r.ni[j];
 		r.ni[j] = newImpulse;
 		lane_apply( a, b, r, aA_, aB_, impulse * n.x, impulse * n.y );
 	}
-	float xT[2], maxF[2];
-	int clampT[2]; /* 0 interior, 1 upper, -1 lower */
+#pragma unroll
 	for ( int j = 0; j < 2; ++j )
 	{
 		sa[2 + j] = a;
@@ -273,21 +302,111 @@ __device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2
 		float lo = 0.0f - maxFriction;
 		float mn = x < maxFriction ? x : maxFriction;
 		float newImpulse = lo > mn ? lo : mn;
-		clampT[j] = lo > mn ? -1 : ( x < maxFriction ? 0 : 1 );
-		xT[j] = x;
-		maxF[j] = maxFriction;
 		float impulse = newImpulse - r.ti[j];
 		r.ti[j] = newImpulse;
 		lane_apply( a, b, r, aA_, aB_, impulse * t.x, impulse * t.y );
 	}
+}
 
+/* What the reverse of solve / relax needs of that trace and of the row: nothing here
+ * depends on an adjoint, so the rows of all colours take it at once. */
+struct SolveForward
+{
+	float impulseN[2], impulseT[2];
+	float innerN[2];		/* massScale ( vn + bias ) */
+	float massScale[2], impulseScale[2], dbds[2];
+	float vt[2], frictionNi[2]; /* friction's relative velocity and normal impulse */
+	bool active[2];			/* normal impulse above zero */
+	int clampT[2];			/* friction: 0 interior, 1 upper, -1 lower */
+	b2gVec dvN[2], dvT[2], ds[2];
+	float wA[4], wB[4];
+	b2gRot dqA, dqB;
+};
+
+/* r holds the impulses before the row ran; sa, sb the states before each impulse, with the
+ * substep's position deltas. */
+__device__ __forceinline__ void solve_forward( Row r, const DevState* sa, const DevState* sb, bool useBias, const b2gStepConst& sc, bool scalar,
+											   SolveForward& F )
+{
+	float biasRate = useBias ? r.biasRate : 0.0f;
+	float massScale = useBias ? r.massScale : 1.0f;
+	float impulseScale = useBias ? r.impulseScale : 0.0f;
+	float minBias = -sc.pushout;
+	b2gVec n = r.n;
+	b2gVec t = gv( n.y, 0.0f - n.x );
+	b2gVec dp = gv( sb[0].dp.x - sa[0].dp.x, sb[0].dp.y - sa[0].dp.y );
+	F.dqA = sa[0].dq;
+	F.dqB = sb[0].dq;
+#pragma unroll
+	for ( int j = 0; j < 2; ++j )
+	{
+		const DevState& a = sa[j];
+		const DevState& b = sb[j];
+		b2gVec aA_ = r.rA[j], aB_ = r.rB[j];
+		b2gVec rsA = gv( a.dq.c * aA_.x - a.dq.s * aA_.y, a.dq.s * aA_.x + a.dq.c * aA_.y );
+		b2gVec rsB = gv( b.dq.c * aB_.x - b.dq.s * aB_.y, b.dq.s * aB_.x + b.dq.c * aB_.y );
+		b2gVec ds = gv( dp.x + ( rsB.x - rsA.x ), dp.y + ( rsB.y - rsA.y ) );
+		float s = ( n.x * ds.x + n.y * ds.y ) + r.base[j];
+		float bias;
+		if ( s > 0.0f )
+		{
+			bias = s * sc.inv_h;
+			F.dbds[j] = sc.inv_h;
+		}
+		else
+		{
+			float soft = biasRate * s;
+			bias = gmax( soft, minBias );
+			F.dbds[j] = soft > minBias ? biasRate : 0.0f;
+		}
+		F.ds[j] = ds;
+		F.massScale[j] = scalar && s > 0.0f ? 1.0f : massScale;
+		F.impulseScale[j] = scalar && s > 0.0f ? 0.0f : impulseScale;
+		b2gVec dv = lane_dv( a, b, aA_, aB_ );
+		F.dvN[j] = dv;
+		float vn = dv.x * n.x + dv.y * n.y;
+		F.innerN[j] = F.massScale[j] * ( vn + bias );
+		float negImpulse = r.nMass[j] * F.innerN[j] + F.impulseScale[j] * r.ni[j];
+		float x = r.ni[j] - negImpulse;
+		float newImpulse = gmax( x, 0.0f );
+		F.active[j] = x > 0.0f;
+		F.impulseN[j] = newImpulse - r.ni[j];
+		F.frictionNi[j] = newImpulse;
+		F.wA[j] = a.w;
+		F.wB[j] = b.w;
+	}
+#pragma unroll
+	for ( int j = 0; j < 2; ++j )
+	{
+		b2gVec dv = lane_dv( sa[2 + j], sb[2 + j], r.rA[j], r.rB[j] );
+		float vt = dv.x * t.x + dv.y * t.y;
+		float negImpulse = r.tMass[j] * vt;
+		float maxFriction = r.friction * F.frictionNi[j];
+		float x = r.ti[j] - negImpulse;
+		float lo = 0.0f - maxFriction;
+		float mn = x < maxFriction ? x : maxFriction;
+		F.clampT[j] = lo > mn ? -1 : ( x < maxFriction ? 0 : 1 );
+		float newImpulse = F.clampT[j] < 0 ? -maxFriction : ( F.clampT[j] == 0 ? x : maxFriction );
+		F.impulseT[j] = newImpulse - r.ti[j];
+		F.dvT[j] = dv;
+		F.vt[j] = vt;
+		F.wA[2 + j] = sa[2 + j].w;
+		F.wB[2 + j] = sb[2 + j].w;
+	}
+}
+
+/* Reverse of solve / relax.  On entry aA, aB are the adjoints of the velocities after the
+ * row; on exit, before it.  dpA.. receive the position-delta adjoints. */
+__device__ __forceinline__ void solve_reverse( const Row& r, const SolveForward& F, BodyV& aA, BodyV& aB, RowAdj& ra, float* dpA, float* dqA,
+											   float* dpB, float* dqB )
+{
+	b2gVec n = r.n;
+	b2gVec t = gv( n.y, 0.0f - n.x );
 	/* tangent points in reverse */
+#pragma unroll
 	for ( int j = 1; j >= 0; --j )
 	{
-		const DevState& A = sa[2 + j];
-		const DevState& B = sb[2 + j];
-		float newImpulse = clampT[j] < 0 ? -maxF[j] : ( clampT[j] == 0 ? xT[j] : maxF[j] );
-		float impulse = newImpulse - ti0[j];
+		float impulse = F.impulseT[j];
 		b2gVec P = gv( impulse * t.x, impulse * t.y );
 		b2gVec Pb = apply_vjp( P, r.rA[j], r.rB[j], r, aA, aB, ra.rA[j], ra.rB[j] );
 		float impb = Pb.x * t.x + Pb.y * t.y;
@@ -296,33 +415,30 @@ __device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2
 		float newb = ra.ti[j] + impb;
 		float tib = -impb;
 		float xb = 0.0f, maxFb = 0.0f;
-		if ( clampT[j] < 0 )
+		if ( F.clampT[j] < 0 )
 			maxFb = -newb;
-		else if ( clampT[j] == 0 )
+		else if ( F.clampT[j] == 0 )
 			xb = newb;
 		else
 			maxFb = newb;
-		ra.mu += maxFb * r.ni[j];
+		ra.mu += maxFb * F.frictionNi[j];
 		ra.ni[j] += maxFb * r.friction;
 		tib += xb;
 		float negb = -xb;
-		b2gVec dv = lane_dv( A, B, r.rA[j], r.rB[j] );
-		float vt = dv.x * t.x + dv.y * t.y;
-		ra.tMass[j] += negb * vt;
+		b2gVec dv = F.dvT[j];
+		ra.tMass[j] += negb * F.vt[j];
 		float vtb = negb * r.tMass[j];
 		/* vt = dv . t, t = ( n.y, -n.x ) */
 		ra.n[0] += -( vtb * dv.y );
 		ra.n[1] += vtb * dv.x;
-		dv_vjp( gv( vtb * t.x, vtb * t.y ), r.rA[j], r.rB[j], A.w, B.w, aA, aB, ra.rA[j], ra.rB[j] );
+		dv_vjp( gv( vtb * t.x, vtb * t.y ), r.rA[j], r.rB[j], F.wA[2 + j], F.wB[2 + j], aA, aB, ra.rA[j], ra.rB[j] );
 		ra.ti[j] = tib;
 	}
 	/* normal points in reverse */
+#pragma unroll
 	for ( int j = 1; j >= 0; --j )
 	{
-		const DevState& A = sa[j];
-		const DevState& B = sb[j];
-		float newImpulse = gmax( xN[j], 0.0f );
-		float impulse = newImpulse - ni0[j];
+		float impulse = F.impulseN[j];
 		b2gVec P = gv( impulse * n.x, impulse * n.y );
 		b2gVec Pb = apply_vjp( P, r.rA[j], r.rB[j], r, aA, aB, ra.rA[j], ra.rB[j] );
 		float impb = Pb.x * n.x + Pb.y * n.y;
@@ -330,28 +446,22 @@ __device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2
 		ra.n[1] += impulse * Pb.y;
 		float newb = ra.ni[j] + impb;
 		float nib = -impb;
-		float xb = xN[j] > 0.0f ? newb : 0.0f;
+		float xb = F.active[j] ? newb : 0.0f;
 		nib += xb;
 		float negb = -xb;
-		b2gVec dv = lane_dv( A, B, r.rA[j], r.rB[j] );
-		float vn = dv.x * n.x + dv.y * n.y;
+		b2gVec dv = F.dvN[j];
 		/* negImpulse = nMass * ( massScale * ( vn + bias ) ) + impulseScale * ni */
-		float s = s_[j];
-		float bias = s > 0.0f ? s * sc.inv_h : gmax( biasRate * s, minBias );
-		ra.nMass[j] += negb * ( ms_[j] * ( vn + bias ) );
-		float vnb = negb * r.nMass[j] * ms_[j];
-		nib += negb * is_[j];
-		float sb_ = vnb * dbds[j];
+		ra.nMass[j] += negb * F.innerN[j];
+		float vnb = negb * r.nMass[j] * F.massScale[j];
+		nib += negb * F.impulseScale[j];
+		float sb_ = vnb * F.dbds[j];
 		ra.n[0] += vnb * dv.x;
 		ra.n[1] += vnb * dv.y;
-		dv_vjp( gv( vnb * n.x, vnb * n.y ), r.rA[j], r.rB[j], A.w, B.w, aA, aB, ra.rA[j], ra.rB[j] );
+		dv_vjp( gv( vnb * n.x, vnb * n.y ), r.rA[j], r.rB[j], F.wA[j], F.wB[j], aA, aB, ra.rA[j], ra.rB[j] );
 		/* s = n . ( dp + rotate( dqB, rB ) - rotate( dqA, rA ) ) + base */
 		b2gVec aA_ = r.rA[j], aB_ = r.rB[j];
-		b2gVec rsA = gv( A.dq.c * aA_.x - A.dq.s * aA_.y, A.dq.s * aA_.x + A.dq.c * aA_.y );
-		b2gVec rsB = gv( B.dq.c * aB_.x - B.dq.s * aB_.y, B.dq.s * aB_.x + B.dq.c * aB_.y );
-		b2gVec ds = gv( dp.x + ( rsB.x - rsA.x ), dp.y + ( rsB.y - rsA.y ) );
-		ra.n[0] += sb_ * ds.x;
-		ra.n[1] += sb_ * ds.y;
+		ra.n[0] += sb_ * F.ds[j].x;
+		ra.n[1] += sb_ * F.ds[j].y;
 		ra.base[j] += sb_;
 		b2gVec dsb = gv( sb_ * n.x, sb_ * n.y );
 		dpB[0] += dsb.x;
@@ -363,36 +473,61 @@ __device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2
 		dqB[1] += -dsb.x * aB_.y + dsb.y * aB_.x;
 		dqA[0] -= dsb.x * aA_.x + dsb.y * aA_.y;
 		dqA[1] -= -dsb.x * aA_.y + dsb.y * aA_.x;
-		ra.rB[j][0] += B.dq.c * dsb.x + B.dq.s * dsb.y;
-		ra.rB[j][1] += -B.dq.s * dsb.x + B.dq.c * dsb.y;
-		ra.rA[j][0] -= A.dq.c * dsb.x + A.dq.s * dsb.y;
-		ra.rA[j][1] -= -A.dq.s * dsb.x + A.dq.c * dsb.y;
+		ra.rB[j][0] += F.dqB.c * dsb.x + F.dqB.s * dsb.y;
+		ra.rB[j][1] += -F.dqB.s * dsb.x + F.dqB.c * dsb.y;
+		ra.rA[j][0] -= F.dqA.c * dsb.x + F.dqA.s * dsb.y;
+		ra.rA[j][1] -= -F.dqA.s * dsb.x + F.dqA.c * dsb.y;
 		ra.ni[j] = nib;
 	}
 }
 
-/* Restitution (8-lane path). */
-__device__ void restitution_vjp( Row r, DevState a, DevState b, const b2gStepConst& sc, BodyV& aA, BodyV& aB, RowAdj& ra )
+/* Solve / relax from the states before the row: trace, then reverse. */
+__device__ void solve_vjp( Row r, DevState a, DevState b, bool useBias, const b2gStepConst& sc, BodyV& aA, BodyV& aB, RowAdj& ra,
+						   float* dpA, float* dqA, float* dpB, float* dqB, bool scalar = false )
+{
+	DevState sa[4], sb[4];
+	solve_trace( r, a, b, useBias, sc, scalar, sa, sb );
+	SolveForward F;
+	solve_forward( r, sa, sb, useBias, sc, scalar, F );
+	solve_reverse( r, F, aA, aB, ra, dpA, dqA, dpB, dqB );
+}
+
+/* Restitution (8-lane path): the states before its two impulses, and its reverse. */
+__device__ __forceinline__ void restitution_trace( Row r, DevState a, DevState b, const b2gStepConst& sc, DevState* sa, DevState* sb )
 {
 	b2gVec n = r.n;
-	DevState sa[2], sb[2];
-	float xN[2], ni0[2] = { r.ni[0], r.ni[1] }, mass[2];
+#pragma unroll
 	for ( int j = 0; j < 2; ++j )
 	{
 		sa[j] = a;
 		sb[j] = b;
 		bool skip = ( r.relVel[j] + sc.restitutionThreshold > 0.0f ) || ( r.maxNi[j] == 0.0f );
-		mass[j] = skip ? 0.0f : r.nMass[j];
+		float mass = skip ? 0.0f : r.nMass[j];
 		b2gVec dv = lane_dv( a, b, r.rA[j], r.rB[j] );
 		float vn = dv.x * n.x + dv.y * n.y;
-		float negImpulse = mass[j] * ( vn + r.restitution * r.relVel[j] );
-		float x = r.ni[j] - negImpulse;
-		xN[j] = x;
-		float newImpulse = gmax( x, 0.0f );
+		float negImpulse = mass * ( vn + r.restitution * r.relVel[j] );
+		float newImpulse = gmax( r.ni[j] - negImpulse, 0.0f );
 		float impulse = newImpulse - r.ni[j];
-		r.ni[j] = newImpulse;
 		lane_apply( a, b, r, r.rA[j], r.rB[j], impulse * n.x, impulse * n.y );
 	}
+}
+
+__device__ __forceinline__ void restitution_reverse( Row r, const DevState* sa, const DevState* sb, const b2gStepConst& sc, BodyV& aA, BodyV& aB,
+													 RowAdj& ra )
+{
+	b2gVec n = r.n;
+	float xN[2], ni0[2] = { r.ni[0], r.ni[1] }, mass[2];
+#pragma unroll
+	for ( int j = 0; j < 2; ++j )
+	{
+		bool skip = ( r.relVel[j] + sc.restitutionThreshold > 0.0f ) || ( r.maxNi[j] == 0.0f );
+		mass[j] = skip ? 0.0f : r.nMass[j];
+		b2gVec dv = lane_dv( sa[j], sb[j], r.rA[j], r.rB[j] );
+		float vn = dv.x * n.x + dv.y * n.y;
+		float negImpulse = mass[j] * ( vn + r.restitution * r.relVel[j] );
+		xN[j] = r.ni[j] - negImpulse;
+	}
+#pragma unroll
 	for ( int j = 1; j >= 0; --j )
 	{
 		const DevState& A = sa[j];
@@ -420,6 +555,13 @@ __device__ void restitution_vjp( Row r, DevState a, DevState b, const b2gStepCon
 		dv_vjp( gv( inner * n.x, inner * n.y ), r.rA[j], r.rB[j], A.w, B.w, aA, aB, ra.rA[j], ra.rB[j] );
 		ra.ni[j] = nib;
 	}
+}
+
+__device__ void restitution_vjp( Row r, DevState a, DevState b, const b2gStepConst& sc, BodyV& aA, BodyV& aB, RowAdj& ra )
+{
+	DevState sa[2], sb[2];
+	restitution_trace( r, a, b, sc, sa, sb );
+	restitution_reverse( r, sa, sb, sc, aA, aB, ra );
 }
 
 /* ------------------------------------------------------------------ body VJPs */
@@ -490,8 +632,10 @@ __device__ void finalize_vjp( float qc, float qs, float dqc, float dqs, float* g
  * respect to the manifold (normal, centre-relative anchors, separations), the bodies'
  * step-start velocities and the warm-start impulses.  mAdj: n(2), then per point
  * anchorA(2) anchorB(2) separation. */
-__device__ void prepare_vjp( const Row& r, const DevState& sA, const DevState& sB, const RowAdj& ra, float warm, float* mAdj, BodyV& aA,
-							 BodyV& aB, float* lamIn )
+/* The part that does not add to the bodies' velocity adjoints, whose terms of point j are
+ * those of dv_vjp for g[j]. */
+__device__ __forceinline__ void prepare_parts( const Row& r, const DevState& sA, const DevState& sB, const RowAdj& ra, float warm, float* mAdj,
+											   b2gVec* g, float* lamIn )
 {
 	b2gVec n = r.n;
 	b2gVec t = gright( n );
@@ -501,8 +645,12 @@ __device__ void prepare_vjp( const Row& r, const DevState& sA, const DevState& s
 		mAdj[i] = 0.0f;
 	for ( int i = 0; i < 4; ++i )
 		lamIn[i] = 0.0f;
-	for ( int j = 0; j < r.count; ++j )
+#pragma unroll
+	for ( int j = 0; j < 2; ++j )
 	{
+		g[j] = gv( 0.0f, 0.0f );
+		if ( j >= r.count )
+			continue;
 		b2gVec rA = r.rA[j], rB = r.rB[j];
 		float rAb[2] = { ra.rA[j][0], ra.rA[j][1] };
 		float rBb[2] = { ra.rB[j][0], ra.rB[j][1] };
@@ -549,7 +697,11 @@ __device__ void prepare_vjp( const Row& r, const DevState& sA, const DevState& s
 		b2gVec dv = gsub( gadd( sB.v, gcross_sv( sB.w, rB ) ), gadd( sA.v, gcross_sv( sA.w, rA ) ) );
 		nb[0] += gr * dv.x;
 		nb[1] += gr * dv.y;
-		dv_vjp( gv( gr * n.x, gr * n.y ), rA, rB, sA.w, sB.w, aA, aB, rAb, rBb );
+		g[j] = gv( gr * n.x, gr * n.y );
+		rBb[0] += sB.w * g[j].y;
+		rBb[1] += -sB.w * g[j].x;
+		rAb[0] -= sA.w * g[j].y;
+		rAb[1] -= -sA.w * g[j].x;
 		lamIn[j] = warm * ra.ni[j];
 		lamIn[2 + j] = warm * ra.ti[j];
 		mAdj[2 + 5 * j + 0] = rAb[0];
@@ -565,13 +717,33 @@ __device__ void prepare_vjp( const Row& r, const DevState& sA, const DevState& s
 	mAdj[1] = nb[1];
 }
 
+/* The velocity terms of dv_vjp for g. */
+__device__ __forceinline__ void dv_velocities( b2gVec g, b2gVec rA, b2gVec rB, BodyV& aA, BodyV& aB )
+{
+	aB.vx += g.x;
+	aB.vy += g.y;
+	aA.vx -= g.x;
+	aA.vy -= g.y;
+	aB.w += -rB.y * g.x + rB.x * g.y;
+	aA.w -= -rA.y * g.x + rA.x * g.y;
+}
+
+__device__ void prepare_vjp( const Row& r, const DevState& sA, const DevState& sB, const RowAdj& ra, float warm, float* mAdj, BodyV& aA,
+							 BodyV& aB, float* lamIn )
+{
+	b2gVec g[2];
+	prepare_parts( r, sA, sB, ra, warm, mAdj, g, lamIn );
+	for ( int j = 0; j < r.count; ++j )
+		dv_velocities( g[j], r.rA[j], r.rB[j], aA, aB );
+}
+
 /* ------------------------------------------------------------------ narrowphase Jacobian */
 /* Recomputes the manifold of a polygon pair with derivatives in the six directions
  * ( cA.x, cA.y, angleA, cB.x, cB.y, angleB ); writes the 12 x 6 Jacobian of
  * ( normal, per point anchorA anchorB separation ), anchors relative to the centres.
  * Returns false when the replay does not reproduce the recorded manifold. */
 __device__ bool manifold_jacobian( const b2gShapeGeo& gA, const b2gShapeGeo& gB, const float* startA, const float* startB, bool dynA, bool dynB,
-								   const b2gManifold& rec, float* jac )
+								   const b2gManifold& rec, float* jac, int stride = 1 )
 {
 	typedef Dual<6> D;
 	DXf<6> xf[2];
@@ -626,11 +798,11 @@ __device__ bool manifold_jacobian( const b2gShapeGeo& gA, const b2gShapeGeo& gB,
 	DVec<6> offB = drotate( q[1], dvc<6>( gv( startB[4], startB[5] ) ) );
 	bool same = m.count == rec.count && m.normal.x.v == rec.normal.x && m.normal.y.v == rec.normal.y;
 	for ( int i = 0; i < 12 * 6; ++i )
-		jac[i] = 0.0f;
+		jac[(size_t)i * stride] = 0.0f;
 	for ( int d = 0; d < 6; ++d )
 	{
-		jac[0 * 6 + d] = m.normal.x.d[d];
-		jac[1 * 6 + d] = m.normal.y.d[d];
+		jac[(size_t)( 0 * 6 + d ) * stride] = m.normal.x.d[d];
+		jac[(size_t)( 1 * 6 + d ) * stride] = m.normal.y.d[d];
 	}
 	for ( int j = 0; j < m.count && j < 2; ++j )
 	{
@@ -640,615 +812,1119 @@ __device__ bool manifold_jacobian( const b2gShapeGeo& gA, const b2gShapeGeo& gB,
 			   aB.y.v == rec.pts[j].anchorB.y && m.pts[j].separation.v == rec.pts[j].separation && m.pts[j].id == rec.pts[j].id;
 		for ( int d = 0; d < 6; ++d )
 		{
-			jac[( 2 + 5 * j + 0 ) * 6 + d] = aA.x.d[d];
-			jac[( 2 + 5 * j + 1 ) * 6 + d] = aA.y.d[d];
-			jac[( 2 + 5 * j + 2 ) * 6 + d] = aB.x.d[d];
-			jac[( 2 + 5 * j + 3 ) * 6 + d] = aB.y.d[d];
-			jac[( 2 + 5 * j + 4 ) * 6 + d] = m.pts[j].separation.d[d];
+			jac[(size_t)( ( 2 + 5 * j + 0 ) * 6 + d ) * stride] = aA.x.d[d];
+			jac[(size_t)( ( 2 + 5 * j + 1 ) * 6 + d ) * stride] = aA.y.d[d];
+			jac[(size_t)( ( 2 + 5 * j + 2 ) * 6 + d ) * stride] = aB.x.d[d];
+			jac[(size_t)( ( 2 + 5 * j + 3 ) * 6 + d ) * stride] = aB.y.d[d];
+			jac[(size_t)( ( 2 + 5 * j + 4 ) * 6 + d ) * stride] = m.pts[j].separation.d[d];
 		}
 	}
 	return same;
 }
 
-/* ------------------------------------------------------------------ the backward kernel */
+/* ------------------------------------------------------------------ replay */
 #define ADJ_WARP 32
+#define ADJ_LINK_NONE 3
 
-__device__ __forceinline__ DevState replay_state( const AdjLayout& L, int b )
+__device__ __forceinline__ DevState replay_state( const float* state, int b )
 {
 	if ( b < 0 )
 		return identity_state();
-	const float* s = L.state + (size_t)b * ADJ_STATE;
-	return state_of( make_float4( s[0], s[1], s[2], s[3] ), make_float4( s[4], s[5], s[6], s[7] ) );
+	const float4* s = (const float4*)( state + (size_t)b * ADJ_STATE );
+	return state_of( s[0], s[1] );
 }
 
-__device__ __forceinline__ void replay_store_velocity( const AdjLayout& L, int b, const DevState& x )
+__device__ __forceinline__ void replay_store_velocity( float* state, int b, const DevState& x )
 {
 	if ( b < 0 )
 		return;
-	float* s = L.state + (size_t)b * ADJ_STATE;
+	float* s = state + (size_t)b * ADJ_STATE;
 	s[0] = x.v.x;
 	s[1] = x.v.y;
 	s[2] = x.w;
 }
 
-__device__ __forceinline__ Row load_row_rec( const AdjLayout& L, int k ) { return *(const Row*)( L.rows + (size_t)k * ADJ_ROW ); }
-__device__ __forceinline__ void store_row_rec( const AdjLayout& L, int k, const Row& r ) { *(Row*)( L.rows + (size_t)k * ADJ_ROW ) = r; }
-
-/* One forward stage of the replay over the active colours (warm 0, solve 1, relax 2,
- * restitution 3), recording each row's starting velocities and impulses. */
-/* The state a row starts from, kept on the phase tape for its reverse. */
-__device__ __forceinline__ void tape_row_start( float* t, const Row& r, const DevState& A, const DevState& B )
+__device__ __forceinline__ void put_velocity( float* p, int Rs, const DevState& A, const DevState& B )
 {
-	t[0] = A.v.x;
-	t[1] = A.v.y;
-	t[2] = A.w;
-	t[3] = B.v.x;
-	t[4] = B.v.y;
-	t[5] = B.w;
-	t[6] = r.ni[0];
-	t[7] = r.ni[1];
-	t[8] = r.ti[0];
-	t[9] = r.ti[1];
-	t[10] = r.maxNi[0];
-	t[11] = r.maxNi[1];
+	p[0] = A.v.x;
+	p[Rs] = A.v.y;
+	p[2 * Rs] = A.w;
+	p[3 * Rs] = B.v.x;
+	p[4 * Rs] = B.v.y;
+	p[5 * Rs] = B.w;
 }
 
-__device__ void replay_stage( const AdjLayout& L, const b2gTapeStep& h, int R, int phase, int tapeIndex, const b2gStepConst& sc )
+/* One phase of a replayed row (warm 0, solve 1, relax 2, restitution 3): what its reverse
+ * starts from onto the phase tape, then the row itself. */
+__device__ __forceinline__ void replay_row( const AdjStep& L, float* D, int k, int phase, int sub, const b2gStepConst& sc, bool scalar )
 {
-	float* tape = L.phase + (size_t)tapeIndex * R * ADJ_PHASE;
-	/* the overflow colour first, one row after another with the scalar arithmetic
-	 * (reference src/contact_solver.c:149-440) */
-	if ( threadIdx.x == 0 )
+	const int Rs = L.Rs;
+	float* state = D + L.state;
+	Row* work = (Row*)( D + L.work );
+	Row r = work[k];
+	DevState A = replay_state( state, r.ia );
+	DevState B = replay_state( state, r.ib );
+	bool changed = true;
+	if ( phase == 0 )
 	{
-		for ( int k = h.colorStart[B2G_OVERFLOW]; k < h.colorStart[B2G_COLORS]; ++k )
-		{
-			Row r = load_row_rec( L, k );
-			DevState A = replay_state( L, r.ia );
-			DevState B = replay_state( L, r.ib );
-			tape_row_start( tape + (size_t)k * ADJ_PHASE, r, A, B );
-			bool changed = true;
-			if ( phase == 0 )
-				warm_scalar( r, A, B );
-			else if ( phase == 3 )
-				changed = restitution_scalar( r, A, B, sc.restitutionThreshold );
-			else
-				solve_scalar( r, A, B, phase == 1, sc.inv_h, sc.pushout );
-			if ( changed )
-			{
-				replay_store_velocity( L, r.ia, A );
-				replay_store_velocity( L, r.ib, B );
-				store_row_rec( L, k, r );
-			}
-		}
+		float* t = D + L.warm( sub ) + k;
+		t[0] = r.ni[0];
+		t[Rs] = r.ni[1];
+		t[2 * Rs] = r.ti[0];
+		t[3 * Rs] = r.ti[1];
+		scalar ? warm_scalar( r, A, B ) : warm_lane( r, A, B );
 	}
+	else if ( phase == 3 )
+	{
+		DevState sa[2], sb[2];
+		restitution_trace( r, A, B, sc, sa, sb );
+		float* t = D + L.rest() + k;
+		t[0] = r.ni[0];
+		t[Rs] = r.ni[1];
+		t[2 * Rs] = r.maxNi[0];
+		t[3 * Rs] = r.maxNi[1];
+		for ( int j = 0; j < 2; ++j )
+			put_velocity( t + ( 4 + 6 * j ) * Rs, Rs, sa[j], sb[j] );
+		if ( scalar )
+			changed = restitution_scalar( r, A, B, sc.restitutionThreshold );
+		else
+			restitution_lane( r, A, B, sc.restitutionThreshold );
+	}
+	else
+	{
+		DevState sa[4], sb[4];
+		solve_trace( r, A, B, phase == 1, sc, scalar, sa, sb );
+		float* t = D + L.solve( sub, phase == 2 ) + k;
+		t[0] = r.ni[0];
+		t[Rs] = r.ni[1];
+		t[2 * Rs] = r.ti[0];
+		t[3 * Rs] = r.ti[1];
+#pragma unroll
+		for ( int j = 0; j < 4; ++j )
+			put_velocity( t + ( 4 + 6 * j ) * Rs, Rs, sa[j], sb[j] );
+		scalar ? solve_scalar( r, A, B, phase == 1, sc.inv_h, sc.pushout ) : solve_lane( r, A, B, phase == 1, sc.inv_h, sc.pushout );
+	}
+	if ( changed == false )
+		return;
+	replay_store_velocity( state, r.ia, A );
+	replay_store_velocity( state, r.ib, B );
+	for ( int j = 0; j < 2; ++j )
+	{
+		work[k].ni[j] = r.ni[j];
+		work[k].ti[j] = r.ti[j];
+		work[k].maxNi[j] = r.maxNi[j];
+	}
+}
+
+/* One forward stage of the replay over the active colours: the overflow colour first, one
+ * row after another with the scalar arithmetic (reference src/contact_solver.c:149-440). */
+__device__ void replay_stage( const AdjStep& L, float* D, const b2gTapeStep& h, int phase, int sub, const b2gStepConst& sc )
+{
+	if ( threadIdx.x == 0 )
+		for ( int k = h.colorStart[B2G_OVERFLOW]; k < h.colorStart[B2G_COLORS]; ++k )
+			replay_row( L, D, k, phase, sub, sc, true );
 	__syncwarp();
 	for ( int a = 0; a < h.activeCount; ++a )
 	{
 		int c = h.active[a];
 		for ( int k = h.colorStart[c] + (int)threadIdx.x; k < h.colorStart[c + 1]; k += ADJ_WARP )
-		{
-			Row r = load_row_rec( L, k );
-			DevState A = replay_state( L, r.ia );
-			DevState B = replay_state( L, r.ib );
-			tape_row_start( tape + (size_t)k * ADJ_PHASE, r, A, B );
-			if ( phase == 0 )
-				warm_lane( r, A, B );
-			else if ( phase == 3 )
-				restitution_lane( r, A, B, sc.restitutionThreshold );
-			else
-				solve_lane( r, A, B, phase == 1, sc.inv_h, sc.pushout );
-			replay_store_velocity( L, r.ia, A );
-			replay_store_velocity( L, r.ib, B );
-			store_row_rec( L, k, r );
-		}
+			replay_row( L, D, k, phase, sub, sc, false );
 		__syncwarp();
 	}
 }
 
-/* Reverse of one row of a stage (its velocity, impulse and position-delta adjoints).
- * The scalar overflow rows share the lane rows' derivatives: the arithmetic is the same
- * up to operand grouping, a point past the manifold's count is a zero point of the lane
- * layout, and a restitution-free overflow row is skipped as the forward skipped it. */
-__device__ void reverse_row( const AdjLayout& L, const float* tape, int k, int phase, const float* snap, const b2gStepConst& sc,
-							 bool scalar )
+__device__ void snapshot( const AdjStep& L, float* D, int N, int index )
 {
-	Row r = load_row_rec( L, k );
-	if ( scalar && phase == 3 && r.restitution == 0.0f )
-		return;
-	const float* t = tape + (size_t)k * ADJ_PHASE;
-	r.ni[0] = t[6];
-	r.ni[1] = t[7];
-	r.ti[0] = t[8];
-	r.ti[1] = t[9];
-	r.maxNi[0] = t[10];
-	r.maxNi[1] = t[11];
-	DevState A = identity_state(), B = identity_state();
-	A.v = gv( t[0], t[1] );
-	A.w = t[2];
-	B.v = gv( t[3], t[4] );
-	B.w = t[5];
-	if ( snap && r.ia >= 0 )
-	{
-		const float* s = snap + (size_t)r.ia * ADJ_SNAP;
-		A.dp = gv( s[4], s[5] );
-		A.dq = grot( s[6], s[7] );
-	}
-	if ( snap && r.ib >= 0 )
-	{
-		const float* s = snap + (size_t)r.ib * ADJ_SNAP;
-		B.dp = gv( s[4], s[5] );
-		B.dq = grot( s[6], s[7] );
-	}
-	float* gA = r.ia >= 0 ? L.bodyAdj + (size_t)r.ia * ADJ_BODY : nullptr;
-	float* gB = r.ib >= 0 ? L.bodyAdj + (size_t)r.ib * ADJ_BODY : nullptr;
-	BodyV aA = { gA ? gA[4] : 0.0f, gA ? gA[5] : 0.0f, gA ? gA[6] : 0.0f };
-	BodyV aB = { gB ? gB[4] : 0.0f, gB ? gB[5] : 0.0f, gB ? gB[6] : 0.0f };
-	RowAdj* ra = (RowAdj*)( L.radj + (size_t)k * ADJ_RADJ );
-	RowAdj g = *ra;
-	float dpA[2] = { 0.0f, 0.0f }, dqA[2] = { 0.0f, 0.0f }, dpB[2] = { 0.0f, 0.0f }, dqB[2] = { 0.0f, 0.0f };
-	if ( phase == 0 )
-		warm_vjp( r, aA, aB, g );
-	else if ( phase == 3 )
-		restitution_vjp( r, A, B, sc, aA, aB, g );
-	else
-		solve_vjp( r, A, B, phase == 1, sc, aA, aB, g, dpA, dqA, dpB, dqB, scalar );
-	*ra = g;
-	if ( gA )
-	{
-		gA[4] = aA.vx;
-		gA[5] = aA.vy;
-		gA[6] = aA.w;
-		gA[7] += dpA[0];
-		gA[8] += dpA[1];
-		gA[9] += dqA[0];
-		gA[10] += dqA[1];
-	}
-	if ( gB )
-	{
-		gB[4] = aB.vx;
-		gB[5] = aB.vy;
-		gB[6] = aB.w;
-		gB[7] += dpB[0];
-		gB[8] += dpB[1];
-		gB[9] += dqB[0];
-		gB[10] += dqB[1];
-	}
-}
-
-/* Reverse of one stage: colours in reverse order, then the overflow rows in reverse
- * order.  snap: body snapshot holding the position deltas the stage used (solve and
- * relax). */
-__device__ void reverse_stage( const AdjLayout& L, const b2gTapeStep& h, int R, int phase, int tapeIndex, const float* snap,
-							   const b2gStepConst& sc )
-{
-	const float* tape = L.phase + (size_t)tapeIndex * R * ADJ_PHASE;
-	for ( int a = h.activeCount - 1; a >= 0; --a )
-	{
-		int c = h.active[a];
-		for ( int k = h.colorStart[c] + (int)threadIdx.x; k < h.colorStart[c + 1]; k += ADJ_WARP )
-			reverse_row( L, tape, k, phase, snap, sc, false );
-		__syncwarp();
-	}
-	if ( threadIdx.x == 0 )
-	{
-		for ( int k = h.colorStart[B2G_COLORS] - 1; k >= h.colorStart[B2G_OVERFLOW]; --k )
-			reverse_row( L, tape, k, phase, snap, sc, true );
-	}
-	__syncwarp();
-}
-
-__device__ void snapshot( const AdjLayout& L, int N, int index )
-{
-	float* dst = L.snap + (size_t)index * N * ADJ_SNAP;
+	float* dst = D + L.snap + (size_t)index * ADJ_SNAP * L.Ns;
 	for ( int b = threadIdx.x; b < N; b += ADJ_WARP )
 		for ( int i = 0; i < ADJ_SNAP; ++i )
-			dst[(size_t)b * ADJ_SNAP + i] = L.state[(size_t)b * ADJ_STATE + i];
+			dst[(size_t)i * L.Ns + b] = D[L.state + (size_t)b * ADJ_STATE + i];
 	__syncwarp();
 }
 
-__global__ void __launch_bounds__( ADJ_WARP ) k_adjoint( const b2gAdjointItem* items )
+/* The replay of step stepCount - 1 - (first + blockIdx.x) of world blockIdx.y.  Reads the
+ * tape and the world; writes that step's scratch and, added, the world's status. */
+__global__ void __launch_bounds__( ADJ_WARP ) k_adjoint_replay( const b2gAdjointItem* items, int first )
 {
-	const b2gAdjointItem& it = items[blockIdx.x];
+	const b2gAdjointItem& it = items[blockIdx.y];
+	const int ts = it.stepCount - 1 - ( first + (int)blockIdx.x );
+	if ( ts < 0 )
+		return;
 	const b2gDevWorld& W = it.W;
 	const int lane = threadIdx.x;
 	const int N = it.bodies;
-	AdjLayout L;
-	adj_layout( &L, it.scratch, N, it.maxRows < 1 ? 1 : it.maxRows, it.contactCap < 1 ? 1 : it.contactCap, ADJ_MAX_SUBSTEPS );
+	const AdjStep L = adj_step( N, it.maxRows, it.maxSub );
+	float* D = it.stepScratch + (size_t)blockIdx.x * it.stepFloats;
+	int* table = (int*)( D + L.total ); /* rows of the step before by contact id, where set */
+	const b2gTapeStep& h = it.steps[ts];
+	const b2gStepConst& sc = h.sc;
+	const int R = h.rows, Rs = L.Rs, Ns = L.Ns;
+	const int S = sc.subSteps;
 	int unsupported = 0, mismatches = 0, replayDiffs = 0;
-
-	for ( int s = lane; s < it.shapes; s += ADJ_WARP )
-		it.gradFriction[s] = 0.0f;
-	for ( int c = lane; c < it.contactCap; c += ADJ_WARP )
+	if ( h.solve == 0 || S > ADJ_MAX_SUBSTEPS )
 	{
-		L.lamStamp[c] = -1;
-		L.prevStamp[c] = -1;
+		if ( h.solve != 0 && lane == 0 )
+			atomicAdd( it.status, 1 );
+		return;
 	}
+	if ( h.jointStart[B2G_COLORS] > 0 )
+		unsupported += 1;
+	const float* recB = it.tapeBodies + 4 * h.bodyOff;
+	const b2gTapeRow* recR = it.tapeRows + h.rowOff;
+	const b2gTapeRow* oldR = it.tapeRows;
+	int oldRows = 0;
+	if ( ts > 0 )
+	{
+		oldR = it.tapeRows + it.steps[ts - 1].rowOff;
+		oldRows = it.steps[ts - 1].rows;
+		for ( int k = lane; k < oldRows; k += ADJ_WARP )
+			table[oldR[k].cid] = k;
+	}
+
+	/* step start: bodies */
 	for ( int b = lane; b < N; b += ADJ_WARP )
-		for ( int i = 0; i < ADJ_BODY; ++i )
-			L.bodyAdj[(size_t)b * ADJ_BODY + i] = 0.0f;
+	{
+		const float* o = recB + 16 * b;
+		float* st = D + L.start + b;
+		st[0 * Ns] = o[8];
+		st[1 * Ns] = o[9];
+		st[2 * Ns] = o[6];
+		st[3 * Ns] = o[7];
+		st[4 * Ns] = o[10];
+		st[5 * Ns] = o[11];
+		st[6 * Ns] = o[4];
+		st[7 * Ns] = o[5];
+		st[8 * Ns] = o[12];
+		float4* x = (float4*)( D + L.state + (size_t)b * ADJ_STATE );
+		x[0] = make_float4( o[0], o[1], o[2], o[3] );
+		x[1] = make_float4( 0.0f, 0.0f, 1.0f, 0.0f );
+		if ( o[12] != 0.0f )
+		{
+			float4 ms = ( (const float4*)W.mass )[b];
+			float4 fo = ( (const float4*)W.force )[b];
+			fo = make_float4( o[13], o[14], o[15], fo.w );
+			float4 ex = ( (const float4*)W.extent )[b];
+			VelocityTerms v = velocity_terms( ms, fo, ex, sc );
+			float* tm = D + L.terms + b;
+			tm[0 * Ns] = v.lvd.x;
+			tm[1 * Ns] = v.lvd.y;
+			tm[2 * Ns] = v.avd;
+			tm[3 * Ns] = v.ld;
+			tm[4 * Ns] = v.ad;
+		}
+	}
 	__syncwarp();
 
-	for ( int ts = it.stepCount - 1; ts >= 0; --ts )
+	/* rows: manifold Jacobian, preparation, the previous step's row and points */
+	const float4* mass = (const float4*)W.mass;
+	for ( int k = lane; k < R; k += ADJ_WARP )
 	{
-		const b2gTapeStep h = it.steps[ts];
-		const b2gStepConst sc = h.sc;
+		const b2gTapeRow& tr = recR[k];
+		const b2gShapeGeo& gA = W.geo[tr.shapeA];
+		const b2gShapeGeo& gB = W.geo[tr.shapeB];
+		float startA[8], startB[8];
+		for ( int i = 0; i < 8; ++i )
+		{
+			startA[i] = D[L.start + (size_t)i * Ns + gA.bodyId];
+			startB[i] = D[L.start + (size_t)i * Ns + gB.bodyId];
+		}
+		if ( gA.type == 4 )
+			unsupported += 1; /* chain links have no manifold Jacobian here */
+		else if ( manifold_jacobian( gA, gB, startA, startB, tr.ia >= 0, tr.ib >= 0, tr.m, D + L.jac + k, Rs ) == false )
+			mismatches += 1;
+		float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
+		Row r;
+		prepare_row( r, &tr.m, tr.ia, tr.ib, tr.ia >= 0 ? mass[tr.ia] : zero, tr.ib >= 0 ? mass[tr.ib] : zero,
+					 replay_state( D + L.state, tr.ia ), replay_state( D + L.state, tr.ib ), tr.friction, tr.restitution,
+					 ( tr.ia < 0 || tr.ib < 0 ) ? sc.staticSoft : sc.contactSoft, sc.enableWarmStarting ? 1.0f : 0.0f );
+		( (Row*)( D + L.work ) )[k] = r;
+		/* warm-start impulses came from the previous step's stored impulses of the points
+		 * with the same feature id (reference src/contact.c:555-568) */
+		int link = -1;
+		if ( oldRows > 0 )
+		{
+			int o = table[tr.cid];
+			if ( o >= 0 && o < oldRows && oldR[o].cid == tr.cid )
+			{
+				const b2gTapeRow& old = oldR[o];
+				int from[2] = { ADJ_LINK_NONE, ADJ_LINK_NONE };
+				for ( int j = 0; j < tr.m.count; ++j )
+					for ( int jo = old.m.count - 1; jo >= 0; --jo )
+						if ( old.m.pts[jo].id == tr.m.pts[j].id )
+							from[j] = jo;
+				link = o | ( from[0] << 24 ) | ( from[1] << 26 );
+			}
+		}
+		float* f = D + L.rows + k;
+		f[0 * Rs] = __int_as_float( r.ia );
+		f[1 * Rs] = __int_as_float( r.ib );
+		f[2 * Rs] = __int_as_float( r.count );
+		f[3 * Rs] = r.n.x;
+		f[4 * Rs] = r.n.y;
+		f[5 * Rs] = r.friction;
+		f[6 * Rs] = r.restitution;
+		f[7 * Rs] = r.mA;
+		f[8 * Rs] = r.iA;
+		f[9 * Rs] = r.mB;
+		f[10 * Rs] = r.iB;
+		for ( int j = 0; j < 2; ++j )
+		{
+			f[( 11 + 2 * j ) * Rs] = r.rA[j].x;
+			f[( 12 + 2 * j ) * Rs] = r.rA[j].y;
+			f[( 15 + 2 * j ) * Rs] = r.rB[j].x;
+			f[( 16 + 2 * j ) * Rs] = r.rB[j].y;
+			f[( 19 + j ) * Rs] = r.base[j];
+			f[( 21 + j ) * Rs] = r.nMass[j];
+			f[( 23 + j ) * Rs] = r.tMass[j];
+			f[( 25 + j ) * Rs] = r.relVel[j];
+		}
+		f[27 * Rs] = __int_as_float( link );
+	}
+	__syncwarp();
+
+	for ( int sub = 0; sub < S; ++sub )
+	{
+		snapshot( L, D, N, 2 * sub );
+		for ( int b = lane; b < N; b += ADJ_WARP )
+		{
+			if ( D[L.start + 8 * Ns + b] == 0.0f )
+				continue;
+			DevState x = replay_state( D + L.state, b );
+			const float* tm = D + L.terms + b;
+			VelocityTerms v;
+			v.lvd = gv( tm[0 * Ns], tm[1 * Ns] );
+			v.avd = tm[2 * Ns];
+			v.ld = tm[3 * Ns];
+			v.ad = tm[4 * Ns];
+			integrate_velocity( x, v, sc );
+			replay_store_velocity( D + L.state, b, x );
+		}
+		__syncwarp();
+		if ( sc.enableWarmStarting )
+			replay_stage( L, D, h, 0, sub, sc );
+		replay_stage( L, D, h, 1, sub, sc );
+		snapshot( L, D, N, 2 * sub + 1 );
+		for ( int b = lane; b < N; b += ADJ_WARP )
+		{
+			if ( D[L.start + 8 * Ns + b] == 0.0f )
+				continue;
+			DevState x = replay_state( D + L.state, b );
+			integrate_position( x, sc.h );
+			( (float4*)( D + L.state + (size_t)b * ADJ_STATE ) )[1] = make_float4( x.dp.x, x.dp.y, x.dq.c, x.dq.s );
+		}
+		__syncwarp();
+		replay_stage( L, D, h, 2, sub, sc );
+	}
+	snapshot( L, D, N, 2 * S );
+	replay_stage( L, D, h, 3, 0, sc );
+
+	/* the replayed step must end where the next recorded step starts */
+	if ( ts + 1 < it.stepCount )
+	{
+		const float* next = it.tapeBodies + 4 * it.steps[ts + 1].bodyOff;
+		for ( int b = lane; b < N; b += ADJ_WARP )
+		{
+			const float* st = D + L.start + b;
+			if ( st[8 * Ns] == 0.0f )
+				continue;
+			const float* x = D + L.state + (size_t)b * ADJ_STATE;
+			const float* o = next + 16 * b;
+			b2gRot qf = gnormrot( gmulrot( grot( x[6], x[7] ), grot( st[2 * Ns], st[3 * Ns] ) ) );
+			bool same = x[0] == o[0] && x[1] == o[1] && x[2] == o[2] && st[0] + x[4] == o[8] && st[1 * Ns] + x[5] == o[9] && qf.c == o[6] &&
+						qf.s == o[7];
+			replayDiffs += same ? 0 : 1;
+		}
+	}
+	if ( unsupported )
+		atomicAdd( it.status + 0, unsupported );
+	if ( mismatches )
+		atomicAdd( it.status + 2, mismatches );
+	if ( replayDiffs )
+		atomicAdd( it.status + 3, replayDiffs );
+}
+
+/* ------------------------------------------------------------------ reverse */
+/* What the reverse pass holds of a world: the replay of the current step (D), the body
+ * adjoints and the impulse adjoints, in shared memory when the world is small. */
+struct AdjReverse
+{
+	const float* D;
+	float* adj; /* [f * Ns + b], ADJ_BODY fields */
+	AdjStep L;
+};
+
+__device__ __forceinline__ Row reverse_load_row( const AdjReverse& X, int k, const b2gStepConst& sc )
+{
+	const int Rs = X.L.Rs;
+	const float* f = X.D + X.L.rows + k;
+	Row r;
+	r.ia = __float_as_int( f[0] );
+	r.ib = __float_as_int( f[Rs] );
+	r.count = __float_as_int( f[2 * Rs] );
+	r.n = gv( f[3 * Rs], f[4 * Rs] );
+	r.friction = f[5 * Rs];
+	r.restitution = f[6 * Rs];
+	const float* soft = ( r.ia < 0 || r.ib < 0 ) ? sc.staticSoft : sc.contactSoft;
+	r.biasRate = soft[0];
+	r.massScale = soft[1];
+	r.impulseScale = soft[2];
+	r.mA = f[7 * Rs];
+	r.iA = f[8 * Rs];
+	r.mB = f[9 * Rs];
+	r.iB = f[10 * Rs];
+#pragma unroll
+	for ( int j = 0; j < 2; ++j )
+	{
+		r.rA[j] = gv( f[( 11 + 2 * j ) * Rs], f[( 12 + 2 * j ) * Rs] );
+		r.rB[j] = gv( f[( 15 + 2 * j ) * Rs], f[( 16 + 2 * j ) * Rs] );
+		r.base[j] = f[( 19 + j ) * Rs];
+		r.nMass[j] = f[( 21 + j ) * Rs];
+		r.tMass[j] = f[( 23 + j ) * Rs];
+		r.relVel[j] = f[( 25 + j ) * Rs];
+		r.ni[j] = r.ti[j] = r.maxNi[j] = 0.0f;
+	}
+	return r;
+}
+
+__device__ __forceinline__ void get_velocity( const float* p, int Rs, DevState& A, DevState& B )
+{
+	A.v = gv( p[0], p[Rs] );
+	A.w = p[2 * Rs];
+	B.v = gv( p[3 * Rs], p[4 * Rs] );
+	B.w = p[5 * Rs];
+}
+
+/* What one row of a stage needs besides its record and the adjoints. */
+struct RowForward
+{
+	SolveForward F;	   /* solve, relax */
+	DevState sa[2], sb[2]; /* restitution */
+};
+
+/* Takes it from the replay; sets the row's impulses to those before the stage. */
+template <int PHASE>
+__device__ __forceinline__ void reverse_forward( const AdjReverse& X, int k, Row& r, int sub, const b2gStepConst& sc, bool scalar, RowForward& f )
+{
+	const int Rs = X.L.Rs, Ns = X.L.Ns;
+	if ( PHASE == 0 )
+	{
+		const float* t = X.D + X.L.warm( sub ) + k;
+		r.ni[0] = t[0];
+		r.ni[1] = t[Rs];
+		r.ti[0] = t[2 * Rs];
+		r.ti[1] = t[3 * Rs];
+	}
+	else if ( PHASE == 3 )
+	{
+		const float* t = X.D + X.L.rest() + k;
+		r.ni[0] = t[0];
+		r.ni[1] = t[Rs];
+		r.maxNi[0] = t[2 * Rs];
+		r.maxNi[1] = t[3 * Rs];
+#pragma unroll
+		for ( int j = 0; j < 2; ++j )
+		{
+			f.sa[j] = identity_state();
+			f.sb[j] = identity_state();
+			get_velocity( t + ( 4 + 6 * j ) * Rs, Rs, f.sa[j], f.sb[j] );
+		}
+	}
+	else
+	{
+		const float* t = X.D + X.L.solve( sub, PHASE == 2 ) + k;
+		const float* snap = X.D + X.L.snap + (size_t)( 2 * sub + ( PHASE == 2 ? 2 : 0 ) ) * ADJ_SNAP * Ns;
+		DevState sa[4], sb[4];
+		DevState A = identity_state(), B = identity_state();
+		if ( r.ia >= 0 )
+		{
+			A.dp = gv( snap[4 * Ns + r.ia], snap[5 * Ns + r.ia] );
+			A.dq = grot( snap[6 * Ns + r.ia], snap[7 * Ns + r.ia] );
+		}
+		if ( r.ib >= 0 )
+		{
+			B.dp = gv( snap[4 * Ns + r.ib], snap[5 * Ns + r.ib] );
+			B.dq = grot( snap[6 * Ns + r.ib], snap[7 * Ns + r.ib] );
+		}
+		r.ni[0] = t[0];
+		r.ni[1] = t[Rs];
+		r.ti[0] = t[2 * Rs];
+		r.ti[1] = t[3 * Rs];
+#pragma unroll
+		for ( int j = 0; j < 4; ++j )
+		{
+			sa[j] = A;
+			sb[j] = B;
+			get_velocity( t + ( 4 + 6 * j ) * Rs, Rs, sa[j], sb[j] );
+		}
+		solve_forward( r, sa, sb, PHASE == 1, sc, scalar, f.F );
+	}
+}
+
+/* Reverse of one row of a stage (its velocity, impulse and position-delta adjoints).  The
+ * scalar overflow rows share the lane rows' derivatives: the arithmetic is the same up to
+ * operand grouping, a point past the manifold's count is a zero point of the lane layout,
+ * and a restitution-free overflow row is skipped as the forward skipped it. */
+template <int PHASE>
+__device__ __forceinline__ void reverse_row( const AdjReverse& X, const Row& r, const RowForward& f, RowAdj& ra, const b2gStepConst& sc, bool scalar )
+{
+	if ( PHASE == 3 && scalar && r.restitution == 0.0f )
+		return;
+	const int Ns = X.L.Ns;
+	const bool hasA = r.ia >= 0, hasB = r.ib >= 0;
+	float* gA = X.adj + ( hasA ? r.ia : 0 );
+	float* gB = X.adj + ( hasB ? r.ib : 0 );
+	BodyV aA = { 0.0f, 0.0f, 0.0f }, aB = { 0.0f, 0.0f, 0.0f };
+	float dpA[2] = { 0.0f, 0.0f }, dqA[2] = { 0.0f, 0.0f }, dpB[2] = { 0.0f, 0.0f }, dqB[2] = { 0.0f, 0.0f };
+	if ( hasA )
+		aA = { gA[4 * Ns], gA[5 * Ns], gA[6 * Ns] };
+	if ( hasB )
+		aB = { gB[4 * Ns], gB[5 * Ns], gB[6 * Ns] };
+	if ( PHASE == 0 )
+	{
+		/* the velocities before a warm start carry the same adjoints as those after it */
+		warm_vjp( r, aA, aB, ra );
+		return;
+	}
+	if ( PHASE == 3 )
+		restitution_reverse( r, f.sa, f.sb, sc, aA, aB, ra );
+	else
+		solve_reverse( r, f.F, aA, aB, ra, dpA, dqA, dpB, dqB );
+	if ( hasA )
+	{
+		gA[4 * Ns] = aA.vx;
+		gA[5 * Ns] = aA.vy;
+		gA[6 * Ns] = aA.w;
+		if ( PHASE != 3 )
+		{
+			gA[7 * Ns] += dpA[0];
+			gA[8 * Ns] += dpA[1];
+			gA[9 * Ns] += dqA[0];
+			gA[10 * Ns] += dqA[1];
+		}
+	}
+	if ( hasB )
+	{
+		gB[4 * Ns] = aB.vx;
+		gB[5 * Ns] = aB.vy;
+		gB[6 * Ns] = aB.w;
+		if ( PHASE != 3 )
+		{
+			gB[7 * Ns] += dpB[0];
+			gB[8 * Ns] += dpB[1];
+			gB[9 * Ns] += dqB[0];
+			gB[10 * Ns] += dqB[1];
+		}
+	}
+}
+
+/* Row adjoints outside registers: field f of row k at [f * Rs + k]. */
+__device__ __forceinline__ RowAdj radj_load( const float* p, int Rs )
+{
+	RowAdj ra;
+	float* o = (float*)&ra;
+#pragma unroll
+	for ( int i = 0; i < ADJ_RADJ; ++i )
+		o[i] = p[(size_t)i * Rs];
+	return ra;
+}
+__device__ __forceinline__ void radj_store( float* p, int Rs, const RowAdj& ra )
+{
+	const float* o = (const float*)&ra;
+#pragma unroll
+	for ( int i = 0; i < ADJ_RADJ; ++i )
+		p[(size_t)i * Rs] = o[i];
+}
+
+/* Reverse of one stage: colours in reverse order, then the overflow rows in reverse
+ * order.  REG: row k's record and adjoint live in lane k's registers, turn is its place
+ * among the active colours (overflow rows: the number of them and up, serially). */
+template <int PHASE, bool REG>
+__device__ __forceinline__ void reverse_stage( const AdjReverse& X, const b2gTapeStep& h, Row mine, RowAdj& ra, int turn, int turns, float* radj,
+											   int sub, const b2gStepConst& sc )
+{
+	const int lane = threadIdx.x, Rs = X.L.Rs;
+	const int active = h.activeCount;
+	if constexpr ( REG )
+	{
+		/* all rows at once up to their adjoints, which then pass through them in turn */
+		RowForward f;
+		if ( turn >= 0 )
+			reverse_forward<PHASE>( X, lane, mine, sub, sc, turn >= active, f );
+		if ( PHASE == 0 )
+		{
+			/* a warm start changes no velocity adjoint: no turns */
+			if ( turn >= 0 )
+				reverse_row<PHASE>( X, mine, f, ra, sc, false );
+			__syncwarp();
+			return;
+		}
+		for ( int a = active - 1; a >= 0; --a )
+		{
+			if ( turn == a )
+				reverse_row<PHASE>( X, mine, f, ra, sc, false );
+			__syncwarp();
+		}
+		for ( int a = turns - 1; a >= active; --a )
+		{
+			if ( turn == a )
+				reverse_row<PHASE>( X, mine, f, ra, sc, true );
+			__syncwarp();
+		}
+	}
+	else
+	{
+		for ( int a = active - 1; a >= 0; --a )
+		{
+			const int c = h.active[a];
+			for ( int k = h.colorStart[c] + lane; k < h.colorStart[c + 1]; k += ADJ_WARP )
+			{
+				RowForward f;
+				Row r = reverse_load_row( X, k, sc );
+				RowAdj g = radj_load( radj + k, Rs );
+				reverse_forward<PHASE>( X, k, r, sub, sc, false, f );
+				reverse_row<PHASE>( X, r, f, g, sc, false );
+				radj_store( radj + k, Rs, g );
+			}
+			__syncwarp();
+		}
+		if ( lane == 0 )
+		{
+			for ( int k = h.colorStart[B2G_COLORS] - 1; k >= h.colorStart[B2G_OVERFLOW]; --k )
+			{
+				RowForward f;
+				Row r = reverse_load_row( X, k, sc );
+				RowAdj g = radj_load( radj + k, Rs );
+				reverse_forward<PHASE>( X, k, r, sub, sc, true, f );
+				reverse_row<PHASE>( X, r, f, g, sc, true );
+				radj_store( radj + k, Rs, g );
+			}
+		}
+		__syncwarp();
+	}
+}
+
+/* The preparation and manifold Jacobian of one row: adjoints of both bodies' poses
+ * (gpos), the velocity terms (g) and the warm-start impulses, which go to the row of the
+ * step before (lamNext). */
+__device__ __forceinline__ void reverse_prepare( const AdjReverse& X, int k, const Row& r, const RowAdj& ra, const b2gStepConst& sc, float* gpos,
+												 b2gVec* g, float* lamNext )
+{
+	const int Rs = X.L.Rs, Ns = X.L.Ns;
+	const float* s0 = X.D + X.L.snap; /* snapshot 0: step-start velocities */
+	DevState sA = identity_state(), sB = identity_state();
+	if ( r.ia >= 0 )
+	{
+		sA.v = gv( s0[r.ia], s0[Ns + r.ia] );
+		sA.w = s0[2 * Ns + r.ia];
+	}
+	if ( r.ib >= 0 )
+	{
+		sB.v = gv( s0[r.ib], s0[Ns + r.ib] );
+		sB.w = s0[2 * Ns + r.ib];
+	}
+	float mAdj[12], lamIn[4];
+	prepare_parts( r, sA, sB, ra, sc.enableWarmStarting ? 1.0f : 0.0f, mAdj, g, lamIn );
+	const float* J = X.D + X.L.jac + k;
+#pragma unroll
+	for ( int d = 0; d < 6; ++d )
+		gpos[d] = 0.0f;
+#pragma unroll
+	for ( int o = 0; o < 12; ++o )
+#pragma unroll
+		for ( int d = 0; d < 6; ++d )
+			gpos[d] += mAdj[o] * J[( o * 6 + d ) * Rs];
+	const int link = __float_as_int( X.D[X.L.rows + 27 * Rs + k] );
+	if ( link >= 0 )
+	{
+		float* lam = lamNext + ( link & 0xffffff );
+#pragma unroll
+		for ( int j = 0; j < 2; ++j )
+		{
+			const int jo = ( link >> ( 24 + 2 * j ) ) & 3;
+			if ( j < r.count && jo != ADJ_LINK_NONE )
+			{
+				lam[(size_t)jo * Rs] += lamIn[j];
+				lam[(size_t)( 2 + jo ) * Rs] += lamIn[2 + j];
+			}
+		}
+	}
+}
+
+/* Adds a row's preparation adjoints to its bodies. */
+__device__ __forceinline__ void reverse_pose( const AdjReverse& X, const Row& r, const float* gpos, const b2gVec* g )
+{
+	const int Ns = X.L.Ns;
+	float* gA = X.adj + ( r.ia >= 0 ? r.ia : 0 );
+	float* gB = X.adj + ( r.ib >= 0 ? r.ib : 0 );
+	BodyV aA = { 0.0f, 0.0f, 0.0f }, aB = { 0.0f, 0.0f, 0.0f };
+	if ( r.ia >= 0 )
+		aA = { gA[4 * Ns], gA[5 * Ns], gA[6 * Ns] };
+	if ( r.ib >= 0 )
+		aB = { gB[4 * Ns], gB[5 * Ns], gB[6 * Ns] };
+#pragma unroll
+	for ( int j = 0; j < 2; ++j )
+		if ( j < r.count )
+			dv_velocities( g[j], r.rA[j], r.rB[j], aA, aB );
+	if ( r.ia >= 0 )
+	{
+		const float* st = X.D + X.L.start + r.ia;
+		gA[0 * Ns] += gpos[0];
+		gA[1 * Ns] += gpos[1];
+		gA[2 * Ns] += gpos[2] * -st[3 * Ns];
+		gA[3 * Ns] += gpos[2] * st[2 * Ns];
+		gA[4 * Ns] = aA.vx;
+		gA[5 * Ns] = aA.vy;
+		gA[6 * Ns] = aA.w;
+	}
+	if ( r.ib >= 0 )
+	{
+		const float* st = X.D + X.L.start + r.ib;
+		gB[0 * Ns] += gpos[3];
+		gB[1 * Ns] += gpos[4];
+		gB[2 * Ns] += gpos[5] * -st[3 * Ns];
+		gB[3 * Ns] += gpos[5] * st[2 * Ns];
+		gB[4 * Ns] = aB.vx;
+		gB[5 * Ns] = aB.vy;
+		gB[6 * Ns] = aB.w;
+	}
+}
+
+/* Shared memory of the reverse pass: two replays, body adjoints, impulse adjoints of this
+ * step and the next, row adjoints unless they are in registers, step header. */
+static __host__ __device__ size_t adj_reverse_floats( const AdjStep& L, bool reg )
+{
+	return 2 * L.copy + (size_t)ADJ_BODY * L.Ns + 8u * (size_t)L.Rs + ( reg ? 0u : (size_t)ADJ_RADJ * L.Rs );
+}
+
+/* Polls of a bulk copy's barrier before the pass gives up. */
+#define ADJ_SPIN_LIMIT ( 1 << 20 )
+
+__device__ __forceinline__ bool adj_wait( unsigned bar, unsigned parity )
+{
+	for ( int left = ADJ_SPIN_LIMIT; left > 0; --left )
+	{
+		unsigned done;
+		asm volatile( "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+					  : "=r"( done )
+					  : "r"( bar ), "r"( parity )
+					  : "memory" );
+		if ( done )
+			return true;
+	}
+	return false;
+}
+
+/* The reverse pass of one world over steps stepCount - 1 - first - t, t in [0, chunk).
+ * SMEM: replays come to shared memory by bulk copies, one step ahead; else they are read
+ * where they are.  REG: at most 32 rows, one per lane. */
+template <bool SMEM, bool REG>
+__global__ void __launch_bounds__( ADJ_WARP ) k_adjoint_reverse( const b2gAdjointItem* items, int first, int chunk )
+{
+	extern __shared__ __align__( 16 ) float sm[];
+	__shared__ __align__( 8 ) unsigned long long s_bar[2];
+	__shared__ b2gTapeStep s_h;
+	const b2gAdjointItem& it = items[blockIdx.x];
+	const int lane = threadIdx.x;
+	const int N = it.bodies;
+	AdjReverse X;
+	X.L = adj_step( N, it.maxRows, it.maxSub );
+	const int Rs = X.L.Rs, Ns = X.L.Ns;
+	AdjWorld G;
+	adj_world( &G, it.scratch, Ns, Rs, it.chunk );
+	const int left = it.stepCount - first;
+	const int n = left < chunk ? left : chunk;
+	if ( n <= 0 )
+		return;
+	float* lam = G.lam; /* this step's */
+	float* lamNext;
+	float* radjShared = nullptr;
+	if constexpr ( SMEM )
+	{
+		X.adj = sm + 2 * X.L.copy;
+		lam = X.adj + ADJ_BODY * Ns;
+		lamNext = lam + 4 * Rs;
+		radjShared = lamNext + 4 * Rs;
+	}
+	else
+	{
+		X.adj = G.bodyAdj;
+		lamNext = G.lam + 4 * Rs;
+	}
+	const unsigned bar = (unsigned)__cvta_generic_to_shared( s_bar );
+	const unsigned buffer = (unsigned)__cvta_generic_to_shared( sm );
+	const unsigned bytes = 4u * (unsigned)X.L.copy;
+	auto fetch = [&]( int t ) {
+		if ( lane == 0 )
+		{
+			const unsigned b = bar + 8u * (unsigned)( t & 1 );
+			asm volatile( "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"( b ), "r"( bytes ) : "memory" );
+			asm volatile( "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+							  buffer + ( t & 1 ) * bytes ),
+						  "l"( it.stepScratch + (size_t)t * it.stepFloats ), "r"( bytes ), "r"( b )
+						  : "memory" );
+		}
+	};
+	if constexpr ( SMEM )
+	{
+		if ( lane == 0 )
+		{
+			asm volatile( "mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"( bar ) : "memory" );
+			asm volatile( "mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"( bar + 8u ) : "memory" );
+			asm volatile( "fence.proxy.async.shared::cta;" ::: "memory" );
+		}
+		__syncwarp();
+		fetch( 0 );
+	}
+	/* carried from the chunk before, or nothing yet */
+	if ( SMEM || first == 0 )
+	{
+		for ( int i = lane; i < ADJ_BODY * Ns; i += ADJ_WARP )
+			X.adj[i] = first == 0 ? 0.0f : G.bodyAdj[i];
+		for ( int i = lane; i < 4 * Rs; i += ADJ_WARP )
+			lam[i] = first == 0 ? 0.0f : G.lam[i];
+	}
+	if ( first == 0 )
+		for ( int i = lane; i < 4 * N; i += ADJ_WARP )
+			G.pose[i] = 0.0f;
+	for ( int i = lane; i < 4 * Rs; i += ADJ_WARP )
+		lamNext[i] = 0.0f;
+
+	for ( int t = 0; t < n; ++t )
+	{
+		const int ts = it.stepCount - 1 - ( first + t );
+		__syncwarp();
+		for ( int i = lane; i < (int)( sizeof( b2gTapeStep ) / 4 ); i += ADJ_WARP )
+			( (int*)&s_h )[i] = ( (const int*)( it.steps + ts ) )[i];
+		if constexpr ( SMEM )
+		{
+			if ( t + 1 < n )
+				fetch( t + 1 );
+			if ( __all_sync( 0xffffffffu, adj_wait( bar + 8u * (unsigned)( t & 1 ), (unsigned)( t >> 1 ) & 1u ) ) == false )
+			{
+				/* the copy in flight must not outlive the shared memory it writes */
+				if ( t + 1 < n )
+					adj_wait( bar + 8u * (unsigned)( ( t + 1 ) & 1 ), (unsigned)( ( t + 1 ) >> 1 ) & 1u );
+				if ( lane == 0 )
+					atomicAdd( it.status + 3, 1 );
+				return;
+			}
+			X.D = sm + (size_t)( t & 1 ) * X.L.copy;
+		}
+		else
+			X.D = it.stepScratch + (size_t)t * it.stepFloats;
+		__syncwarp();
+		const b2gTapeStep& h = s_h;
+		const b2gStepConst& sc = h.sc;
 		const int R = h.rows;
 		const int S = sc.subSteps;
+		float* mu = G.mu + (size_t)t * Rs;
 		if ( h.solve == 0 || S > ADJ_MAX_SUBSTEPS )
 		{
-			unsupported += h.solve != 0 ? 1 : 0;
+			for ( int i = lane; i < 4 * Rs; i += ADJ_WARP )
+				lam[i] = 0.0f;
+			for ( int k = lane; k < Rs; k += ADJ_WARP )
+				mu[k] = 0.0f;
 			continue;
 		}
-		if ( h.jointStart[B2G_COLORS] > 0 )
-			unsupported += 1;
-		const float* recB = it.tapeBodies + 4 * h.bodyOff;
-		const b2gTapeRow* recR = it.tapeRows + h.rowOff;
+		float* radj = SMEM ? radjShared : it.stepScratch + (size_t)t * it.stepFloats + X.L.work;
 
-		/* rows of the previous step, by contact id (for the warm-start impulse adjoint) */
-		if ( ts > 0 )
-		{
-			const b2gTapeStep& hp = it.steps[ts - 1];
-			for ( int k = lane; k < hp.rows; k += ADJ_WARP )
-			{
-				int cid = it.tapeRows[hp.rowOff + k].cid;
-				L.prevRow[cid] = k;
-				L.prevStamp[cid] = ts - 1;
-			}
-		}
-
-		/* step start: bodies */
 		for ( int b = lane; b < N; b += ADJ_WARP )
 		{
-			const float* o = recB + 16 * b;
-			float* st = L.start + (size_t)b * ADJ_START;
-			st[0] = o[8];
-			st[1] = o[9];
-			st[2] = o[6];
-			st[3] = o[7];
-			st[4] = o[10];
-			st[5] = o[11];
-			st[6] = o[4];
-			st[7] = o[5];
-			st[8] = o[12];
-			float* x = L.state + (size_t)b * ADJ_STATE;
-			x[0] = o[0];
-			x[1] = o[1];
-			x[2] = o[2];
-			x[3] = o[3];
-			x[4] = 0.0f;
-			x[5] = 0.0f;
-			x[6] = 1.0f;
-			x[7] = 0.0f;
-			if ( o[12] != 0.0f )
+			const float* st = X.D + X.L.start + b;
+			float g[ADJ_BODY];
+#pragma unroll
+			for ( int i = 0; i < ADJ_BODY; ++i )
+				g[i] = X.adj[i * Ns + b];
+			const float* fin = X.D + X.L.snap + (size_t)2 * S * ADJ_SNAP * Ns + b;
+			const float qc = st[2 * Ns], qs = st[3 * Ns], lcx = st[4 * Ns], lcy = st[5 * Ns];
+			if ( st[8 * Ns] != 0.0f )
 			{
-				float4 ms = ( (const float4*)W.mass )[b];
-				float4 fo = ( (const float4*)W.force )[b];
-				fo = make_float4( o[13], o[14], o[15], fo.w );
-				float4 ex = ( (const float4*)W.extent )[b];
-				VelocityTerms v = velocity_terms( ms, fo, ex, sc );
-				float* tm = L.terms + (size_t)b * ADJ_TERMS;
-				tm[0] = v.lvd.x;
-				tm[1] = v.lvd.y;
-				tm[2] = v.avd;
-				tm[3] = v.ld;
-				tm[4] = v.ad;
+				/* seed: the loss gradient with respect to the state after the last step */
+				if ( ts == it.stepCount - 1 )
+				{
+					/* final rotation q' = normalize( dq q ) */
+					b2gRot qf = gnormrot( gmulrot( grot( fin[6 * Ns], fin[7 * Ns] ), grot( qc, qs ) ) );
+					const float* gf = it.gradFinal + 6 * b;
+					/* p = c - rotate( q, lc ); angle: dq/dangle = ( -q.s, q.c ) */
+					g[0] = gf[0];
+					g[1] = gf[1];
+					g[2] = gf[2] * -qf.s - ( gf[0] * lcx + gf[1] * lcy );
+					g[3] = gf[2] * qf.c - ( -gf[0] * lcy + gf[1] * lcx );
+					g[4] = gf[3];
+					g[5] = gf[4];
+					g[6] = gf[5];
+				}
+				/* reverse: finalisation */
+				finalize_vjp( qc, qs, fin[6 * Ns], fin[7 * Ns], g );
 			}
-		}
-		__syncwarp();
-
-		/* rows: manifold Jacobian and preparation */
-		const float4* mass = (const float4*)W.mass;
-		for ( int k = lane; k < R; k += ADJ_WARP )
-		{
-			const b2gTapeRow& tr = recR[k];
-			const b2gShapeGeo& gA = W.geo[tr.shapeA];
-			const b2gShapeGeo& gB = W.geo[tr.shapeB];
-			if ( gA.type == 4 )
-				unsupported += 1; /* chain links have no manifold Jacobian here */
-			else if ( manifold_jacobian( gA, gB, L.start + (size_t)gA.bodyId * ADJ_START, L.start + (size_t)gB.bodyId * ADJ_START, tr.ia >= 0,
-										 tr.ib >= 0, tr.m, L.jac + (size_t)k * ADJ_JAC ) == false )
-				mismatches += 1;
-			float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
-			Row r;
-			prepare_row( r, &tr.m, tr.ia, tr.ib, tr.ia >= 0 ? mass[tr.ia] : zero, tr.ib >= 0 ? mass[tr.ib] : zero, replay_state( L, tr.ia ),
-						 replay_state( L, tr.ib ), tr.friction, tr.restitution, ( tr.ia < 0 || tr.ib < 0 ) ? sc.staticSoft : sc.contactSoft,
-						 sc.enableWarmStarting ? 1.0f : 0.0f );
-			store_row_rec( L, k, r );
-			float* ra = L.radj + (size_t)k * ADJ_RADJ;
-			for ( int i = 0; i < ADJ_RADJ; ++i )
-				ra[i] = 0.0f;
-		}
-		__syncwarp();
-
-		/* forward replay */
-		for ( int sub = 0; sub < S; ++sub )
-		{
-			snapshot( L, N, 2 * sub );
-			for ( int b = lane; b < N; b += ADJ_WARP )
+			else
 			{
-				if ( L.start[(size_t)b * ADJ_START + 8] == 0.0f )
-					continue;
-				DevState x = replay_state( L, b );
-				const float* tm = L.terms + (size_t)b * ADJ_TERMS;
-				VelocityTerms v;
-				v.lvd = gv( tm[0], tm[1] );
-				v.avd = tm[2];
-				v.ld = tm[3];
-				v.ad = tm[4];
-				integrate_velocity( x, v, sc );
-				replay_store_velocity( L, b, x );
-			}
-			__syncwarp();
-			if ( sc.enableWarmStarting )
-				replay_stage( L, h, R, 0, 3 * sub + 0, sc );
-			replay_stage( L, h, R, 1, 3 * sub + 1, sc );
-			snapshot( L, N, 2 * sub + 1 );
-			for ( int b = lane; b < N; b += ADJ_WARP )
-			{
-				if ( L.start[(size_t)b * ADJ_START + 8] == 0.0f )
-					continue;
-				DevState x = replay_state( L, b );
-				integrate_position( x, sc.h );
-				float* st = L.state + (size_t)b * ADJ_STATE;
-				st[4] = x.dp.x;
-				st[5] = x.dp.y;
-				st[6] = x.dq.c;
-				st[7] = x.dq.s;
-			}
-			__syncwarp();
-			replay_stage( L, h, R, 2, 3 * sub + 2, sc );
-		}
-		snapshot( L, N, 2 * S );
-		replay_stage( L, h, R, 3, 3 * S, sc );
-
-		/* the replayed step must end where the next recorded step starts */
-		if ( ts + 1 < it.stepCount )
-		{
-			const float* next = it.tapeBodies + 4 * it.steps[ts + 1].bodyOff;
-			for ( int b = lane; b < N; b += ADJ_WARP )
-			{
-				const float* st = L.start + (size_t)b * ADJ_START;
-				if ( st[8] == 0.0f )
-					continue;
-				const float* x = L.state + (size_t)b * ADJ_STATE;
-				const float* o = next + 16 * b;
-				b2gRot qf = gnormrot( gmulrot( grot( x[6], x[7] ), grot( st[2], st[3] ) ) );
-				bool ok = x[0] == o[0] && x[1] == o[1] && x[2] == o[2] && st[0] + x[4] == o[8] && st[1] + x[5] == o[9] && qf.c == o[6] &&
-						  qf.s == o[7];
-				replayDiffs += ok ? 0 : 1;
-			}
-		}
-
-		/* seed: the loss gradient with respect to the state after the last step */
-		if ( ts == it.stepCount - 1 )
-		{
-			for ( int b = lane; b < N; b += ADJ_WARP )
-			{
-				const float* st = L.start + (size_t)b * ADJ_START;
-				if ( st[8] == 0.0f )
-					continue;
-				const float* fin = L.snap + ( (size_t)2 * S * N + b ) * ADJ_SNAP;
-				/* final rotation q' = normalize( dq q ) */
-				float qc = st[2], qs = st[3], dqc = fin[6], dqs = fin[7];
-				b2gRot qf = gnormrot( gmulrot( grot( dqc, dqs ), grot( qc, qs ) ) );
-				const float* gf = it.gradFinal + 6 * b;
-				float* g = L.bodyAdj + (size_t)b * ADJ_BODY;
-				float lcx = st[4], lcy = st[5];
-				/* p = c - rotate( q, lc ); angle: dq/dangle = ( -q.s, q.c ) */
-				g[0] = gf[0];
-				g[1] = gf[1];
-				g[2] = gf[2] * -qf.s - ( gf[0] * lcx + gf[1] * lcy );
-				g[3] = gf[2] * qf.c - ( -gf[0] * lcy + gf[1] * lcx );
-				g[4] = gf[3];
-				g[5] = gf[4];
-				g[6] = gf[5];
-			}
-			__syncwarp();
-		}
-
-		/* reverse: finalisation */
-		for ( int b = lane; b < N; b += ADJ_WARP )
-		{
-			const float* st = L.start + (size_t)b * ADJ_START;
-			float* g = L.bodyAdj + (size_t)b * ADJ_BODY;
-			if ( st[8] == 0.0f )
-			{
+#pragma unroll
 				for ( int i = 0; i < ADJ_BODY; ++i )
 					g[i] = 0.0f;
-				continue;
 			}
-			const float* fin = L.snap + ( (size_t)2 * S * N + b ) * ADJ_SNAP;
-			finalize_vjp( st[2], st[3], fin[6], fin[7], g );
+#pragma unroll
+			for ( int i = 0; i < ADJ_BODY; ++i )
+				X.adj[i * Ns + b] = g[i];
+			float* pose = G.pose + 4 * b;
+			pose[0] = qc;
+			pose[1] = qs;
+			pose[2] = lcx;
+			pose[3] = lcy;
 		}
-		__syncwarp();
 
-		/* reverse: stored impulses receive the next step's warm-start adjoint */
-		for ( int k = lane; k < R; k += ADJ_WARP )
+		/* rows; stored impulses receive the next step's warm-start adjoint */
+		Row mine;
+		RowAdj ra;
+		int turn = -1;
+		const int turns = h.activeCount + h.colorStart[B2G_COLORS] - h.colorStart[B2G_OVERFLOW];
+		if constexpr ( REG )
 		{
-			int cid = recR[k].cid;
-			if ( L.lamStamp[cid] != ts )
-				continue;
-			RowAdj* ra = (RowAdj*)( L.radj + (size_t)k * ADJ_RADJ );
-			const float* lam = L.lam + 4 * (size_t)cid;
-			ra->ni[0] += lam[0];
-			ra->ni[1] += lam[1];
-			ra->ti[0] += lam[2];
-			ra->ti[1] += lam[3];
+			mine = reverse_load_row( X, lane < R ? lane : 0, sc );
+			ra = RowAdj{};
+			for ( int a = 0; a < h.activeCount; ++a )
+				if ( lane >= h.colorStart[h.active[a]] && lane < h.colorStart[h.active[a] + 1] )
+					turn = a;
+			if ( lane >= h.colorStart[B2G_OVERFLOW] && lane < R )
+				turn = h.activeCount + lane - h.colorStart[B2G_OVERFLOW];
+			if ( lane < R )
+			{
+				ra.ni[0] += lam[lane];
+				ra.ni[1] += lam[Rs + lane];
+				ra.ti[0] += lam[2 * Rs + lane];
+				ra.ti[1] += lam[3 * Rs + lane];
+			}
+		}
+		else
+		{
+			for ( int k = lane; k < R; k += ADJ_WARP )
+			{
+				RowAdj g{};
+				g.ni[0] += lam[k];
+				g.ni[1] += lam[Rs + k];
+				g.ti[0] += lam[2 * Rs + k];
+				g.ti[1] += lam[3 * Rs + k];
+				radj_store( radj + k, Rs, g );
+			}
 		}
 		__syncwarp();
 
 		/* reverse: restitution, then the substeps */
-		reverse_stage( L, h, R, 3, 3 * S, nullptr, sc );
+		reverse_stage<3, REG>( X, h, mine, ra, turn, turns, radj, 0, sc );
 		for ( int sub = S - 1; sub >= 0; --sub )
 		{
-			reverse_stage( L, h, R, 2, 3 * sub + 2, L.snap + (size_t)( 2 * sub + 2 ) * N * ADJ_SNAP, sc );
+			reverse_stage<2, REG>( X, h, mine, ra, turn, turns, radj, sub, sc );
 			for ( int b = lane; b < N; b += ADJ_WARP )
 			{
-				if ( L.start[(size_t)b * ADJ_START + 8] == 0.0f )
+				if ( X.D[X.L.start + 8 * Ns + b] == 0.0f )
 					continue;
-				ip_vjp( L.snap + ( (size_t)( 2 * sub + 1 ) * N + b ) * ADJ_SNAP, sc.h, L.bodyAdj + (size_t)b * ADJ_BODY );
+				const float* s = X.D + X.L.snap + (size_t)( 2 * sub + 1 ) * ADJ_SNAP * Ns + b;
+				float pre[8] = { 0.0f, 0.0f, s[2 * Ns], 0.0f, 0.0f, 0.0f, s[6 * Ns], s[7 * Ns] };
+				float g[ADJ_BODY];
+#pragma unroll
+				for ( int i = 4; i < 11; ++i )
+					g[i] = X.adj[i * Ns + b];
+				ip_vjp( pre, sc.h, g );
+#pragma unroll
+				for ( int i = 4; i < 11; ++i )
+					X.adj[i * Ns + b] = g[i];
 			}
 			__syncwarp();
-			reverse_stage( L, h, R, 1, 3 * sub + 1, L.snap + (size_t)( 2 * sub ) * N * ADJ_SNAP, sc );
+			reverse_stage<1, REG>( X, h, mine, ra, turn, turns, radj, sub, sc );
 			if ( sc.enableWarmStarting )
-				reverse_stage( L, h, R, 0, 3 * sub + 0, nullptr, sc );
+				reverse_stage<0, REG>( X, h, mine, ra, turn, turns, radj, sub, sc );
 			for ( int b = lane; b < N; b += ADJ_WARP )
 			{
-				if ( L.start[(size_t)b * ADJ_START + 8] == 0.0f )
+				if ( X.D[X.L.start + 8 * Ns + b] == 0.0f )
 					continue;
-				const float* tm = L.terms + (size_t)b * ADJ_TERMS;
-				iv_vjp( L.snap + ( (size_t)( 2 * sub ) * N + b ) * ADJ_SNAP, make_float4( tm[0], tm[1], tm[2], tm[3] ), tm[4], sc,
-						L.bodyAdj + (size_t)b * ADJ_BODY );
+				const float* s = X.D + X.L.snap + (size_t)( 2 * sub ) * ADJ_SNAP * Ns + b;
+				const float* tm = X.D + X.L.terms + b;
+				float pre[3] = { s[0], s[Ns], s[2 * Ns] };
+				float g[ADJ_BODY];
+#pragma unroll
+				for ( int i = 4; i < 7; ++i )
+					g[i] = X.adj[i * Ns + b];
+				iv_vjp( pre, make_float4( tm[0], tm[Ns], tm[2 * Ns], tm[3 * Ns] ), tm[4 * Ns], sc, g );
+#pragma unroll
+				for ( int i = 4; i < 7; ++i )
+					X.adj[i * Ns + b] = g[i];
 			}
 			__syncwarp();
 		}
 
-		/* reverse: preparation and the manifold Jacobian, colour by colour so that no
-		 * two lanes update one body, then the overflow rows one after another on lane 0 */
-		for ( int a = 0; a <= h.activeCount; ++a )
+		/* reverse: preparation and the manifold Jacobian; the bodies' sums colour by colour
+		 * so that no two lanes update one body, then the overflow rows in order */
+		if constexpr ( REG )
 		{
-			const bool ov = a == h.activeCount;
-			const int c = ov ? B2G_OVERFLOW : h.active[a];
-			const int first = ov ? ( lane == 0 ? h.colorStart[c] : h.colorStart[c + 1] ) : h.colorStart[c] + lane;
-			const int stride = ov ? 1 : ADJ_WARP;
-			for ( int k = first; k < h.colorStart[c + 1]; k += stride )
+			float gpos[6];
+			b2gVec g[2];
+			if ( lane < R )
 			{
-				const b2gTapeRow& tr = recR[k];
-				Row r = load_row_rec( L, k );
-				const RowAdj* ra = (const RowAdj*)( L.radj + (size_t)k * ADJ_RADJ );
-				const float* s0 = L.snap; /* snapshot 0: step-start velocities */
-				DevState sA = identity_state(), sB = identity_state();
-				if ( tr.ia >= 0 )
-				{
-					sA.v = gv( s0[(size_t)tr.ia * ADJ_SNAP + 0], s0[(size_t)tr.ia * ADJ_SNAP + 1] );
-					sA.w = s0[(size_t)tr.ia * ADJ_SNAP + 2];
-				}
-				if ( tr.ib >= 0 )
-				{
-					sB.v = gv( s0[(size_t)tr.ib * ADJ_SNAP + 0], s0[(size_t)tr.ib * ADJ_SNAP + 1] );
-					sB.w = s0[(size_t)tr.ib * ADJ_SNAP + 2];
-				}
-				float* gA = tr.ia >= 0 ? L.bodyAdj + (size_t)tr.ia * ADJ_BODY : nullptr;
-				float* gB = tr.ib >= 0 ? L.bodyAdj + (size_t)tr.ib * ADJ_BODY : nullptr;
-				BodyV aA = { gA ? gA[4] : 0.0f, gA ? gA[5] : 0.0f, gA ? gA[6] : 0.0f };
-				BodyV aB = { gB ? gB[4] : 0.0f, gB ? gB[5] : 0.0f, gB ? gB[6] : 0.0f };
-				float mAdj[12], lamIn[4];
-				prepare_vjp( r, sA, sB, *ra, sc.enableWarmStarting ? 1.0f : 0.0f, mAdj, aA, aB, lamIn );
-				/* manifold adjoint -> body centres and angles */
-				const float* J = L.jac + (size_t)k * ADJ_JAC;
-				float gpos[6] = { 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f };
-				for ( int o = 0; o < 12; ++o )
-					for ( int d = 0; d < 6; ++d )
-						gpos[d] += mAdj[o] * J[o * 6 + d];
-				if ( gA )
-				{
-					const float* st = L.start + (size_t)tr.ia * ADJ_START;
-					gA[0] += gpos[0];
-					gA[1] += gpos[1];
-					gA[2] += gpos[2] * -st[3];
-					gA[3] += gpos[2] * st[2];
-					gA[4] = aA.vx;
-					gA[5] = aA.vy;
-					gA[6] = aA.w;
-				}
-				if ( gB )
-				{
-					const float* st = L.start + (size_t)tr.ib * ADJ_START;
-					gB[0] += gpos[3];
-					gB[1] += gpos[4];
-					gB[2] += gpos[5] * -st[3];
-					gB[3] += gpos[5] * st[2];
-					gB[4] = aB.vx;
-					gB[5] = aB.vy;
-					gB[6] = aB.w;
-				}
-				/* warm-start impulses came from the previous step's stored impulses of
-				 * the points with the same feature id (reference src/contact.c:555-568) */
-				if ( ts > 0 && L.prevStamp[tr.cid] == ts - 1 )
-				{
-					const b2gTapeRow& old = it.tapeRows[it.steps[ts - 1].rowOff + L.prevRow[tr.cid]];
-					float* lam = L.lam + 4 * (size_t)tr.cid;
-					if ( L.lamStamp[tr.cid] != ts - 1 )
-					{
-						lam[0] = lam[1] = lam[2] = lam[3] = 0.0f;
-						L.lamStamp[tr.cid] = ts - 1;
-					}
-					for ( int j = 0; j < tr.m.count; ++j )
-					{
-						for ( int jo = 0; jo < old.m.count; ++jo )
-						{
-							if ( old.m.pts[jo].id == tr.m.pts[j].id )
-							{
-								lam[jo] += lamIn[j];
-								lam[2 + jo] += lamIn[2 + j];
-								break;
-							}
-						}
-					}
-				}
+				reverse_prepare( X, lane, mine, ra, sc, gpos, g, lamNext );
+				mu[lane] = ra.mu;
 			}
-			__syncwarp();
-		}
-
-		/* friction: mu_row = sqrt( muA muB ) */
-		if ( lane == 0 )
-		{
-			for ( int k = 0; k < R; ++k )
+			for ( int a = 0; a < turns; ++a )
 			{
-				const b2gTapeRow& tr = recR[k];
-				float gmu = ( (const RowAdj*)( L.radj + (size_t)k * ADJ_RADJ ) )->mu;
-				if ( gmu == 0.0f )
-					continue;
-				float muA = it.shapeFriction[tr.shapeA], muB = it.shapeFriction[tr.shapeB];
-				if ( muA > 0.0f )
-					it.gradFriction[tr.shapeA] += gmu * 0.5f * tr.friction / muA;
-				if ( muB > 0.0f )
-					it.gradFriction[tr.shapeB] += gmu * 0.5f * tr.friction / muB;
+				if ( turn == a )
+					reverse_pose( X, mine, gpos, g );
+				__syncwarp();
 			}
 		}
+		else
+		{
+			for ( int a = 0; a <= h.activeCount; ++a )
+			{
+				const bool ov = a == h.activeCount;
+				const int c = ov ? B2G_OVERFLOW : h.active[a];
+				const int lo = ov ? ( lane == 0 ? h.colorStart[c] : h.colorStart[c + 1] ) : h.colorStart[c] + lane;
+				for ( int k = lo; k < h.colorStart[c + 1]; k += ov ? 1 : ADJ_WARP )
+				{
+					float gpos[6];
+					b2gVec g[2];
+					const Row r = reverse_load_row( X, k, sc );
+					const RowAdj ga = radj_load( radj + k, Rs );
+					reverse_prepare( X, k, r, ga, sc, gpos, g, lamNext );
+					mu[k] = ga.mu;
+					reverse_pose( X, r, gpos, g );
+				}
+				__syncwarp();
+			}
+		}
+		for ( int k = R + lane; k < Rs; k += ADJ_WARP )
+			mu[k] = 0.0f;
 		/* position deltas start each step at zero: their adjoints end here */
 		for ( int b = lane; b < N; b += ADJ_WARP )
 		{
-			float* g = L.bodyAdj + (size_t)b * ADJ_BODY;
-			g[7] = g[8] = g[9] = g[10] = 0.0f;
+#pragma unroll
+			for ( int i = 7; i < 11; ++i )
+				X.adj[i * Ns + b] = 0.0f;
 		}
-		__syncwarp();
+		/* the impulse adjoints collected for the step before are its own now */
+		for ( int i = lane; i < 4 * Rs; i += ADJ_WARP )
+		{
+			lam[i] = lamNext[i];
+			lamNext[i] = 0.0f;
+		}
 	}
+	__syncwarp();
 
+	if ( SMEM )
+	{
+		for ( int i = lane; i < ADJ_BODY * Ns; i += ADJ_WARP )
+			G.bodyAdj[i] = X.adj[i];
+		for ( int i = lane; i < 4 * Rs; i += ADJ_WARP )
+			G.lam[i] = lam[i];
+	}
+	if ( first + n < it.stepCount )
+		return;
 	/* gradient with respect to the state at the start of the first recorded step:
 	 * p = c - rotate( q, lc ), angle with dq/dangle = ( -q.s, q.c ) */
 	for ( int b = lane; b < N; b += ADJ_WARP )
 	{
-		const float* st = L.start + (size_t)b * ADJ_START;
-		const float* g = L.bodyAdj + (size_t)b * ADJ_BODY;
+		const float* pose = G.pose + 4 * b;
+		const float* g = X.adj + b;
 		float* out = it.gradInitial + 6 * b;
-		float qc = st[2], qs = st[3], lcx = st[4], lcy = st[5];
+		float qc = pose[0], qs = pose[1], lcx = pose[2], lcy = pose[3];
 		out[0] = g[0];
-		out[1] = g[1];
-		out[2] = g[2] * -qs + g[3] * qc + g[0] * ( -qs * lcx - qc * lcy ) + g[1] * ( qc * lcx - qs * lcy );
-		out[3] = g[4];
-		out[4] = g[5];
-		out[5] = g[6];
-	}
-	for ( int off = 16; off > 0; off >>= 1 )
-	{
-		unsupported += __shfl_down_sync( 0xffffffffu, unsupported, off );
-		mismatches += __shfl_down_sync( 0xffffffffu, mismatches, off );
-		replayDiffs += __shfl_down_sync( 0xffffffffu, replayDiffs, off );
+		out[1] = g[Ns];
+		out[2] = g[2 * Ns] * -qs + g[3 * Ns] * qc + g[0] * ( -qs * lcx - qc * lcy ) + g[Ns] * ( qc * lcx - qs * lcy );
+		out[3] = g[4 * Ns];
+		out[4] = g[5 * Ns];
+		out[5] = g[6 * Ns];
 	}
 	if ( lane == 0 )
+		it.status[1] = it.status[2] + it.status[3];
+}
+
+/* Friction gradient of the chunk's rows, mu_row = sqrt( muA muB ): one thread per shape
+ * adds the rows that touch it, the last step's first, rows in order.  Rows are taken
+ * ADJ_FRICTION at a time through shared memory. */
+#define ADJ_FRICTION 256
+
+__global__ void __launch_bounds__( ADJ_FRICTION ) k_adjoint_friction( const b2gAdjointItem* items, int first, int chunk )
+{
+	const b2gAdjointItem& it = items[blockIdx.x];
+	const AdjStep L = adj_step( it.bodies, it.maxRows, it.maxSub );
+	AdjWorld G;
+	adj_world( &G, it.scratch, L.Ns, L.Rs, it.chunk );
+	const int left = it.stepCount - first;
+	const int n = left < chunk ? left : chunk;
+	const int tid = threadIdx.x;
+	__shared__ int2 shape[ADJ_FRICTION];
+	__shared__ float2 part[ADJ_FRICTION];
+	const int total = n > 0 ? n * L.Rs : 0;
+	for ( int s0 = 0; s0 < it.shapes; s0 += ADJ_FRICTION )
 	{
-		it.status[0] = unsupported;
-		it.status[1] = mismatches + replayDiffs;
-		it.status[2] = mismatches;
-		it.status[3] = replayDiffs;
+		const int s = s0 + tid;
+		float sum = s < it.shapes && first > 0 ? it.gradFriction[s] : 0.0f;
+		for ( int e0 = 0; e0 < total; e0 += ADJ_FRICTION )
+		{
+			const int e = e0 + tid;
+			int2 who = make_int2( -1, -1 );
+			float2 add = make_float2( 0.0f, 0.0f );
+			if ( e < total )
+			{
+				const int t = e / L.Rs, k = e - t * L.Rs;
+				const float gmu = G.mu[e];
+				if ( gmu != 0.0f )
+				{
+					const b2gTapeRow& tr = it.tapeRows[it.steps[it.stepCount - 1 - ( first + t )].rowOff + k];
+					float muA = it.shapeFriction[tr.shapeA], muB = it.shapeFriction[tr.shapeB];
+					if ( muA > 0.0f )
+					{
+						who.x = tr.shapeA;
+						add.x = gmu * 0.5f * tr.friction / muA;
+					}
+					if ( muB > 0.0f )
+					{
+						who.y = tr.shapeB;
+						add.y = gmu * 0.5f * tr.friction / muB;
+					}
+				}
+			}
+			shape[tid] = who;
+			part[tid] = add;
+			__syncthreads();
+			const int m = total - e0 < ADJ_FRICTION ? total - e0 : ADJ_FRICTION;
+			for ( int i = 0; i < m; ++i )
+			{
+				if ( shape[i].x == s )
+					sum += part[i].x;
+				if ( shape[i].y == s )
+					sum += part[i].y;
+			}
+			__syncthreads();
+		}
+		if ( s < it.shapes )
+			it.gradFriction[s] = sum;
 	}
 }
 
-extern "C" int b2gd_adjoint_launch( const b2gAdjointItem* dItems, int count, void* stream )
+/* The backward pass of `count` worlds (device item array), `steps` the most recorded
+ * steps of one, `chunk` steps at a time: one replay, one reverse and one friction launch
+ * each.  bodies, rows, subSteps: the largest of the worlds. */
+extern "C" int b2gd_adjoint_launch( const b2gAdjointItem* dItems, int count, int steps, int chunk, int bodies, int rows, int subSteps, void* stream )
 {
 	if ( count <= 0 )
 		return 0;
-	k_adjoint<<<count, ADJ_WARP, 0, (cudaStream_t)stream>>>( dItems );
+	cudaStream_t s = (cudaStream_t)stream;
+	const AdjStep L = adj_step( bodies, at_least_one( rows ), subSteps );
+	const bool reg = rows <= ADJ_WARP;
+	const size_t bytes = 4u * adj_reverse_floats( L, reg );
+	const bool smem = bytes <= 220u * 1024u;
+	auto kernel = smem ? ( reg ? k_adjoint_reverse<true, true> : k_adjoint_reverse<true, false> ) : k_adjoint_reverse<false, false>;
+	if ( smem )
+	{
+		cudaError_t e = cudaFuncSetAttribute( kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024 );
+		if ( e != cudaSuccess )
+			return (int)e;
+	}
+	for ( int first = 0; first < steps; first += chunk )
+	{
+		const int n = steps - first < chunk ? steps - first : chunk;
+		k_adjoint_replay<<<dim3( (unsigned)n, (unsigned)count ), ADJ_WARP, 0, s>>>( dItems, first );
+		kernel<<<count, ADJ_WARP, smem ? bytes : 0, s>>>( dItems, first, n );
+		k_adjoint_friction<<<count, ADJ_FRICTION, 0, s>>>( dItems, first, n );
+	}
 	return (int)cudaGetLastError();
 }

@@ -228,19 +228,25 @@ typedef struct b2gAdjointItem
 	int shapes;
 	int maxRows;
 	int contactCap;
-	int pad;
+	int maxSub; /* most substeps of a recorded step */
+	int chunk;	/* steps replayed at a time */
 	const float* shapeFriction; /* per shape id */
 	const float* gradFinal;		/* 6 per body id: p.x p.y angle v.x v.y w */
 	float* gradInitial;			/* 6 per body id */
 	float* gradFriction;		/* per shape id */
-	float* scratch;
-	int* status; /* [0] unsupported rows, [1] manifold replay mismatches */
+	float* scratch;		/* carried from step to step */
+	float* stepScratch; /* chunk replays of stepFloats floats */
+	size_t stepFloats;
+	int* status; /* zero at the launch: [0] unsupported rows, [1] mismatches of both kinds, [2] of manifolds, [3] of replayed states */
 } b2gAdjointItem;
 
-/* Scratch floats one world needs for a backward pass. */
-size_t b2gd_adjoint_scratch( int bodies, int maxRows, int contactCap, int subSteps );
-/* Runs the backward pass of `count` worlds (device item array, one CTA each). */
-int b2gd_adjoint_launch( const b2gAdjointItem* dItems, int count, void* stream );
+/* Scratch floats one world needs for a backward pass that replays `chunk` steps at a time,
+ * and of one replayed step. */
+size_t b2gd_adjoint_scratch( int bodies, int maxRows, int chunk );
+size_t b2gd_adjoint_step_scratch( int bodies, int maxRows, int contactCap, int subSteps );
+/* Runs the backward pass of `count` worlds (device item array): steps, bodies, rows and
+ * subSteps are the largest of the worlds. */
+int b2gd_adjoint_launch( const b2gAdjointItem* dItems, int count, int steps, int chunk, int bodies, int rows, int subSteps, void* stream );
 
 /* Device time of the last step's stages in milliseconds (CUDA events recorded when
  * w->timing is set). */
