@@ -132,6 +132,7 @@ extern "C" void b2gd_free( b2gDevWorld* w, b2gHostIO* io )
 	FREE_DEV( w->manifold );
 	FREE_DEV( w->solveList );
 	FREE_DEV( w->jointList );
+	FREE_DEV( w->bins );
 	FREE_DEV( w->kIdx );
 	FREE_DEV( w->kNF );
 	FREE_DEV( w->kMass );
@@ -361,6 +362,19 @@ extern "C" int b2gd_upload_solve_lists( b2gDevWorld* w, const int* solveList, in
 	int e = h2d( w, w->solveList, solveList, 4u * (size_t)solveCount, s );
 	e |= h2d( w, w->jointList, jointList, 4u * (size_t)jointCount, s );
 	return e;
+}
+
+extern "C" int b2gd_upload_bins( b2gDevWorld* w, const int* data, int count )
+{
+	if ( count > w->binCap )
+	{
+		int nc = next_cap( w->binCap, count );
+		int e = grow( (void**)&w->bins, 0, 4u * (size_t)nc, (cudaStream_t)w->stream );
+		w->binCap = e == 0 ? nc : 0;
+		if ( e )
+			return e;
+	}
+	return h2d( w, w->bins, data, 4u * (size_t)count, (cudaStream_t)w->stream );
 }
 
 extern "C" int b2gd_upload_fat( b2gDevWorld* w, int shapeId, const float* fat4 )

@@ -30,7 +30,25 @@ typedef struct b2gSolvePlan
 	 * no grouping (the fused solver is not used). */
 	int bodyBlock;
 	int rowSplit[B2G_OVERFLOW][B2G_FUSED_CTAS];
+	/* Bins of islands, each solved by a CTA of its own (0: none): their number, the most
+	 * rows, bodies and joints of one, and the most rows or joints of one colour of one. */
+	int binCount, binRows, binBodies, binJoints, binWidest;
 } b2gSolvePlan;
+
+/* Shared memory of a CTA that holds a whole bin (or a whole small world): what it may
+ * take, and what rows, bodies and joints take. */
+#define B2G_BIN_BYTES_MAX ( 226 * 1024 )
+#define B2G_BIN_BODY_BYTES 60
+#define B2G_BIN_JOINT_BYTES 260
+static inline size_t b2g_bin_bytes( int rows, int bodies, int joints )
+{
+	size_t b = 144u * (size_t)( rows > 0 ? rows : 1 ) + B2G_BIN_BODY_BYTES * (size_t)( ( bodies + 3 ) & ~3 );
+	return ( b + 15 ) / 16 * 16 + B2G_BIN_JOINT_BYTES * (size_t)joints;
+}
+
+/* Ints of one bin in the bin table: row starts of the colours and the end, joint starts
+ * and the end, first body, bodies. */
+#define B2G_BIN_INTS ( 2 * ( B2G_COLORS + 1 ) + 2 )
 
 /* Pinned host staging owned by the device module (mapped into the device). */
 typedef struct b2gHostIO
@@ -75,6 +93,7 @@ int b2gd_upload_shapes( b2gDevWorld* w, const b2gShapeGeo* geo, const float* aab
 int b2gd_upload_shape_lists( b2gDevWorld* w, const int* range, int bodyCount, const int* list, int listCount );
 int b2gd_upload_joints( b2gDevWorld* w, const b2gJointDev* joints, int count );
 int b2gd_upload_solve_lists( b2gDevWorld* w, const int* solveList, int solveCount, const int* jointList, int jointCount );
+int b2gd_upload_bins( b2gDevWorld* w, const int* data, int count );
 int b2gd_upload_fat( b2gDevWorld* w, int shapeId, const float* fat4 );
 int b2gd_upload_body_velocity( b2gDevWorld* w, int bodyId, const float* v3 );
 /* Pose of one body after a time-of-impact event: transform, centre (with local centre)

@@ -247,15 +247,17 @@ __device__ __forceinline__ void res_joint( b2gJointDev* j, const Bodies& B, int 
 __device__ __forceinline__ int res_first( int n, int k, int ctas ) { return (int)( (long long)n * k / ctas ); }
 
 /* One stage over all colours: the overflow set first (serially, CTA 0), then each active
- * colour with a barrier after it.  JOINTS false compiles the joints out. */
-template <int CL, int PHASE, int T, bool JOINTS, class Bodies>
+ * colour with a barrier after it.  T threads a CTA (0: as launched).  PART:
+ * the one CTA of a bin, which holds a part of the plan's rows and joints.  JOINTS false compiles the joints out. */
+template <int CL, int PHASE, int T, bool JOINTS, bool PART, class Bodies>
 __device__ __forceinline__ void res_stage( const ResidentPlan& P, const ResShare* share, const SmemRows& m, const ResJoints& J, const Bodies& B,
 										   ResBarrier<CL>& bar, int rank, const b2gStepConst& sc, const ResOverflow& ov, int ovSlots )
 {
 	const int* cs = P.colorStart;
-	const int R = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
-	const int jointsAll = JOINTS ? P.jointStart[B2G_COLORS] - P.jointStart[B2G_OVERFLOW] : 0;
+	const int R = PART ? share[B2G_OVERFLOW].count : cs[B2G_COLORS] - cs[B2G_OVERFLOW];
+	const int jointsAll = JOINTS ? ( PART ? share[B2G_OVERFLOW].jcount : P.jointStart[B2G_COLORS] - P.jointStart[B2G_OVERFLOW] ) : 0;
 	const int joints = PHASE == F_RESTITUTION ? 0 : jointsAll;
+	const int step = T ? T : (int)blockDim.x;
 	if ( PHASE == F_RESTITUTION ? R > 0 : R + jointsAll > 0 )
 	{
 		if ( rank == 0 )
@@ -265,7 +267,7 @@ __device__ __forceinline__ void res_stage( const ResidentPlan& P, const ResShare
 			{
 				/* the set's bodies to local slots, the serial pass on them, velocities back:
 				 * nothing else touches a body while the set runs */
-				for ( int s = threadIdx.x; s < ovSlots; s += T )
+				for ( int s = threadIdx.x; s < ovSlots; s += step )
 				{
 					int b = ov.body[s];
 					ov.st0[s] = B.word0( b );
@@ -284,7 +286,7 @@ __device__ __forceinline__ void res_stage( const ResidentPlan& P, const ResShare
 						row_step( mo, OB, i, PHASE, true, sc );
 				}
 				__syncthreads();
-				for ( int s = threadIdx.x; s < ovSlots; s += T )
+				for ( int s = threadIdx.x; s < ovSlots; s += step )
 					B.set_word0( ov.body[s], ov.st0[s] );
 			}
 			else if ( threadIdx.x == 0 )
@@ -309,10 +311,12 @@ __device__ __forceinline__ void res_stage( const ResidentPlan& P, const ResShare
 		if ( JOINTS && PHASE == F_RESTITUTION && cs[c + 1] == cs[c] )
 			continue;
 		const ResShare s = share[c];
-		for ( int j = threadIdx.x; j < s.count; j += T )
+		if ( PART && s.count + ( JOINTS && PHASE != F_RESTITUTION ? s.jcount : 0 ) == 0 )
+			continue;
+		for ( int j = threadIdx.x; j < s.count; j += step )
 			row_step( m, B, s.base + j, PHASE, false, sc );
 		if ( JOINTS && PHASE != F_RESTITUTION )
-			for ( int i = threadIdx.x; i < s.jcount; i += T )
+			for ( int i = threadIdx.x; i < s.jcount; i += step )
 			{
 				b2gJointDev* j = J.at( s.jfirst, s.jbase, i );
 				res_joint( j, B, j->indexA, j->indexB, PHASE, sc );
@@ -323,14 +327,15 @@ __device__ __forceinline__ void res_stage( const ResidentPlan& P, const ResShare
 
 /* All substeps over bodies B.  Integration runs over this CTA's awake bodies: with states
  * in shared memory slots b.awake[0 .. awake), in global memory the ids list[0 .. awake). */
-template <int CL, int T, bool SHARED_STATES, bool JOINTS, class Bodies>
+template <int CL, int T, bool SHARED_STATES, bool JOINTS, bool PART = false, class Bodies>
 __device__ __forceinline__ void res_run( const ResidentPlan& P, const ResShare* share, const SmemRows& m, const ResJoints& J, const Bodies& B,
 										 const ResBodies& rb, float4* gst, const int* list, int awake, ResBarrier<CL>& bar, int rank,
 										 const b2gStepConst& sc, const ResOverflow& ov, int ovSlots )
 {
+	const int step = T ? T : (int)blockDim.x;
 	for ( int sub = 0; sub < sc.subSteps; ++sub )
 	{
-		for ( int j = threadIdx.x; j < awake; j += T )
+		for ( int j = threadIdx.x; j < awake; j += step )
 		{
 			const int s = SHARED_STATES ? rb.awake[j] : list[j];
 			const int k = SHARED_STATES ? s : j;
@@ -349,9 +354,9 @@ __device__ __forceinline__ void res_run( const ResidentPlan& P, const ResShare* 
 				__stcg( p, velocity_word( x ) );
 		}
 		bar.sync();
-		res_stage<CL, F_WARM, T, JOINTS>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
-		res_stage<CL, F_SOLVE, T, JOINTS>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
-		for ( int j = threadIdx.x; j < awake; j += T )
+		res_stage<CL, F_WARM, T, JOINTS, PART>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
+		res_stage<CL, F_SOLVE, T, JOINTS, PART>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
+		for ( int j = threadIdx.x; j < awake; j += step )
 		{
 			const int s = SHARED_STATES ? rb.awake[j] : list[j];
 			float4* p0 = SHARED_STATES ? rb.st0 + s : gst + 2 * s;
@@ -365,9 +370,9 @@ __device__ __forceinline__ void res_run( const ResidentPlan& P, const ResShare* 
 				__stcg( p1, v );
 		}
 		bar.sync();
-		res_stage<CL, F_RELAX, T, JOINTS>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
+		res_stage<CL, F_RELAX, T, JOINTS, PART>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
 	}
-	res_stage<CL, F_RESTITUTION, T, JOINTS>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
+	res_stage<CL, F_RESTITUTION, T, JOINTS, PART>( P, share, m, J, B, bar, rank, sc, ov, ovSlots );
 }
 
 /* Overflow cache: the distinct bodies of the set's ends (joints first) get slots in end
@@ -377,6 +382,7 @@ __device__ __forceinline__ void res_index_overflow( const ResOverflow& ov, const
 													int R, int* slots )
 {
 	const int nj = JOINTS ? joints : 0;
+	const int step = T ? T : (int)blockDim.x;
 	const int E = 2 * ( R + nj );
 	auto end_body = [&]( int e ) {
 		if ( JOINTS && e < 2 * nj )
@@ -387,7 +393,7 @@ __device__ __forceinline__ void res_index_overflow( const ResOverflow& ov, const
 		int4 ix = m.idx[o.base + ( ( e - 2 * nj ) >> 1 )];
 		return ( e & 1 ) ? ix.y : ix.x;
 	};
-	for ( int e = threadIdx.x; e < E; e += T )
+	for ( int e = threadIdx.x; e < E; e += step )
 	{
 		int b = end_body( e );
 		int f = -1;
@@ -420,7 +426,7 @@ __device__ __forceinline__ void res_index_overflow( const ResOverflow& ov, const
 		*slots = K;
 	}
 	__syncthreads();
-	for ( int e = threadIdx.x; e < E; e += T )
+	for ( int e = threadIdx.x; e < E; e += step )
 	{
 		int f = ov.first[e];
 		int s = f < 0 ? -1 : ov.slot[f];
@@ -445,13 +451,15 @@ __device__ __forceinline__ void res_index_overflow( const ResOverflow& ov, const
 	}
 }
 
-/* Preparation of one row into m (reference src/contact_solver.c:597-808, :21-147). */
-__device__ __forceinline__ int2 res_prepare( const b2gDevWorld& W, const SmemRows& m, int k, int local, const b2gStepConst& sc )
+/* Preparation of one row into m (reference src/contact_solver.c:597-808, :21-147): entry k
+ * of the list (null: contact k).  slot, when given, renumbers the row's bodies. */
+__device__ __forceinline__ int2 res_prepare( const b2gDevWorld& W, const SmemRows& m, const int* list, const int* slot, int k, int local,
+											 const b2gStepConst& sc )
 {
 	const float4* gst = (const float4*)W.state;
 	const float4* mass = (const float4*)W.mass;
 	const float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
-	int cid = W.solveList ? W.solveList[k] : k;
+	int cid = list ? list[k] : k;
 	int ia = W.cBodies[2 * cid];
 	int ib = W.cBodies[2 * cid + 1];
 	DevState sA = ia >= 0 ? state_of( gst[2 * ia], gst[2 * ia + 1] ) : identity_state();
@@ -459,6 +467,11 @@ __device__ __forceinline__ int2 res_prepare( const b2gDevWorld& W, const SmemRow
 	Row r;
 	prepare_row( r, W.manifold + cid, ia, ib, ia >= 0 ? mass[ia] : zero, ib >= 0 ? mass[ib] : zero, sA, sB, W.cMix[2 * cid],
 				 W.cMix[2 * cid + 1], ( ia < 0 || ib < 0 ) ? sc.staticSoft : sc.contactSoft, sc.enableWarmStarting ? 1.0f : 0.0f );
+	if ( slot != nullptr )
+	{
+		r.ia = ia >= 0 ? slot[ia] : -1;
+		r.ib = ib >= 0 ? slot[ib] : -1;
+	}
 	store_row_smem( m, local, cid, r );
 	return make_int2( ia, ib );
 }

@@ -255,6 +255,8 @@ typedef struct b2gDevWorld
 	/* colour-major solve lists */
 	int* solveList; /* contact ids */
 	int* jointList; /* joint ids */
+	int* bins;		/* bins of islands (b2gSolvePlan), null until a world has some */
+	int binCap;
 
 	/* constraint rows (B2G_ROW_FLOAT4 arrays; the softness follows from whether a body
 	 * is static and is not stored) */

@@ -1,7 +1,8 @@
 /*
  * fused.cu -- the whole solver stage of one world's step in one launch, by one CTA for a
- * small world and by a cluster of 16 CTAs for a larger one (b2g_resident.h; why one
- * launch, and what bounds it, stands in resident.cu).
+ * small world, by a cluster of 16 CTAs for a larger one, and by a CTA per bin of islands
+ * for a larger one whose islands are small (b2g_resident.h; why one launch, and what
+ * bounds it, stands in resident.cu).
  *
  * Layout (dynamic shared memory of every CTA, rank r of CL):
  *   bodies  body ids are cut into CL contiguous blocks of bodyCap: body b lives in CTA
@@ -31,6 +32,9 @@
 
 #include <string.h>
 
+static_assert( RES_SMEM_MAX == B2G_BIN_BYTES_MAX && RES_JOINT_BYTES == B2G_BIN_JOINT_BYTES && RES_BODY_BYTES == B2G_BIN_BODY_BYTES,
+			   "the host sizes what one CTA holds" );
+
 /* 512 threads and 256 take the same time in the contact sweeps (large pyramid 117 us); joint
  * sweeps want the wider CTA (100 x 100 joint grid: solver stage 354 us with 256, 298 with
  * 512) */
@@ -44,14 +48,35 @@ struct FusedSplit
 	unsigned bodyCapInv; /* ceil(2^32 / bodyCap), for the owner of a body id */
 };
 
-template <int CL, bool JOINTS>
+/* Islands share no constraint and no moving body, so bins of them are worlds of their
+ * own to the solver.  Per bin BIN_INTS ints: row starts of the 12 colours and the end,
+ * joint starts and end, first body and bodies; then the rows' contact ids, the joint ids
+ * and the bodies' awake indices bin by bin, and every body id's slot in its bin.
+ */
+#define BIN_INTS B2G_BIN_INTS
+struct FusedBins
+{
+	const int* table;
+	const int* rows;
+	const int* joints;
+	const int* awake;
+	const int* slot;
+};
+
+template <int CL, bool JOINTS, bool BINS = false>
 __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __grid_constant__ b2gDevWorld W, const __grid_constant__ ResidentPlan P,
-																	 const __grid_constant__ FusedSplit S, const __grid_constant__ b2gStepConst sc )
+																	 const __grid_constant__ FusedSplit S, const __grid_constant__ FusedBins bins,
+																	 const __grid_constant__ b2gStepConst sc )
 {
 	/* every CTA of the cluster takes the same branch: no barrier is left waiting */
 	if ( W.guardEvents && __ldcg( W.counters ) != 0 )
 		return;
-	constexpr int T = FUSED_THREADS;
+	/* bins of small islands are launched with fewer threads */
+	const int T = BINS ? (int)blockDim.x : FUSED_THREADS;
+	constexpr int CT = BINS ? 0 : FUSED_THREADS;
+	const int* const bin = BINS ? bins.table + BIN_INTS * blockIdx.x : nullptr;
+	const int* const rowList = BINS ? bins.rows : W.solveList;
+	const int* const jointList = BINS ? bins.joints : W.jointList;
 	extern __shared__ float4 smem[];
 	__shared__ ResShare share[B2G_COLORS];
 	__shared__ int s_rows, s_joints, s_awake, s_ovSlots;
@@ -69,7 +94,14 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		const bool ov = tid == B2G_OVERFLOW;
 		const int n = cs[tid + 1] - cs[tid], nj = JOINTS ? js[tid + 1] - js[tid] : 0;
 		int f, l, jf, jl;
-		if ( CL == 1 || ov )
+		if ( BINS )
+		{
+			f = bin[tid] - cs[tid];
+			l = bin[tid + 1] - cs[tid];
+			jf = JOINTS ? bin[B2G_COLORS + 1 + tid] - js[tid] : 0;
+			jl = JOINTS ? bin[B2G_COLORS + 2 + tid] - js[tid] : 0;
+		}
+		else if ( CL == 1 || ov )
 		{
 			const bool mine = rank == 0;
 			f = jf = 0;
@@ -89,11 +121,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		share[tid].jcount = jl - jf;
 	}
 	if ( tid == 0 )
-	{
 		s_awake = s_ovSlots = 0;
-		if ( rank == 0 )
-			W.counters[1] = W.counters[3] = 0;
-	}
 	__syncthreads();
 	if ( tid == 0 )
 	{
@@ -113,7 +141,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	ResJoints J;
 	J.local = JOINTS && P.jointCap > 0 ? (char*)( smem + P.jointOffset ) : nullptr;
 	J.array = W.joints;
-	J.list = W.jointList;
+	J.list = jointList;
 	if ( JOINTS && J.local != nullptr )
 	{
 		for ( int t = tid, c = 0; t < 64 * s_joints; t += T )
@@ -121,7 +149,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 			const int k = t >> 6;
 			while ( k >= share[c].jbase + share[c].jcount )
 				++c;
-			const int id = W.jointList[share[c].jfirst + ( k - share[c].jbase )];
+			const int id = jointList[share[c].jfirst + ( k - share[c].jbase )];
 			( (int*)J.local )[RES_JOINT_WORDS * k + ( t & 63 )] = ( (const int*)( W.joints + id ) )[t & 63];
 		}
 	}
@@ -129,11 +157,36 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	{
 		while ( k >= share[c].base + share[c].count )
 			++c;
-		res_prepare( W, m, share[c].first + ( k - share[c].base ), k, sc );
+		res_prepare( W, m, rowList, BINS ? bins.slot : nullptr, share[c].first + ( k - share[c].base ), k, sc );
 	}
-	int bodies = P.bodyIdCount - rank * P.bodyCap;
-	bodies = bodies < 0 ? 0 : ( bodies > P.bodyCap ? P.bodyCap : bodies );
-	for ( int s = tid; s < bodies; s += T )
+	/* one CTA: awake bodies in list order, their awake indices kept for finalisation; a
+	 * cluster: the block of ids that this CTA owns */
+	int bodies = P.awakeCount;
+	if ( BINS )
+		bodies = bin[BIN_INTS - 1];
+	if ( CL == 1 )
+	{
+		const int* mine = BINS ? bins.awake + bin[BIN_INTS - 2] : nullptr;
+		for ( int j = tid; j < bodies; j += T )
+		{
+			const int i = BINS ? mine[j] : j;
+			const int b = W.awake[i];
+			const int s = BINS ? j : b;
+			rb.awake[j] = s;
+			rb.flags[j] = i;
+			rb.st0[s] = gst[2 * b];
+			rb.st1[s] = gst[2 * b + 1];
+			res_terms( W, rb, s, b, sc );
+		}
+		if ( tid == 0 )
+			s_awake = bodies;
+	}
+	else
+	{
+		bodies = P.bodyIdCount - rank * P.bodyCap;
+		bodies = bodies < 0 ? 0 : ( bodies > P.bodyCap ? P.bodyCap : bodies );
+	}
+	for ( int s = tid; CL > 1 && s < bodies; s += T )
 	{
 		const int b = rank * P.bodyCap + s;
 		rb.st0[s] = gst[2 * b];
@@ -151,7 +204,13 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		{
 			while ( k >= share[c].jbase + share[c].jcount )
 				++c;
-			prepare_joint_at( W, J.at( share[c].jfirst, share[c].jbase, k - share[c].jbase ), sc );
+			b2gJointDev* j = J.at( share[c].jfirst, share[c].jbase, k - share[c].jbase );
+			prepare_joint_at( W, j, sc );
+			if ( BINS )
+			{
+				j->indexA = j->indexA >= 0 ? bins.slot[j->indexA] : -1;
+				j->indexB = j->indexB >= 0 ? bins.slot[j->indexB] : -1;
+			}
 		}
 	}
 	const int ovRows = cs[B2G_COLORS] - cs[B2G_OVERFLOW], ovJoints = JOINTS ? js[B2G_COLORS] - js[B2G_OVERFLOW] : 0;
@@ -159,7 +218,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	if ( CL > 1 && rank == 0 && P.ovOffset )
 	{
 		__syncthreads();
-		res_index_overflow<T, JOINTS>( ov, m, J, share[B2G_OVERFLOW], ovJoints, ovRows, &s_ovSlots );
+		res_index_overflow<CT, JOINTS>( ov, m, J, share[B2G_OVERFLOW], ovJoints, ovRows, &s_ovSlots );
 	}
 	ResBarrier<CL> bar{ nullptr, CL, 0 };
 	bar.sync();
@@ -169,12 +228,12 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		LocalBodies B;
 		B.st0 = rb.st0;
 		B.st1 = rb.st1;
-		res_run<CL, T, true, JOINTS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
+		res_run<CL, CT, true, JOINTS, BINS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 	}
 	else
 	{
 		DsmemBodies B{ { cl, rb.st0, rb.st1, P.bodyCap, rank, S.bodyCapInv } };
-		res_run<CL, T, true, JOINTS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
+		res_run<CL, CT, true, JOINTS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 	}
 
 	for ( int k = tid; k < rows; k += T )
@@ -182,7 +241,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	/* owned awake body states back to global memory for finalisation */
 	for ( int j = tid; j < awake; j += T )
 	{
-		const int s = rb.awake[j], b = rank * P.bodyCap + s;
+		const int s = rb.awake[j], b = CL == 1 ? W.awake[rb.flags[j]] : rank * P.bodyCap + s;
 		gst[2 * b] = rb.st0[s];
 		gst[2 * b + 1] = rb.st1[s];
 	}
@@ -193,7 +252,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 			const int k = t >> 6;
 			while ( k >= share[c].jbase + share[c].jcount )
 				++c;
-			const int id = W.jointList[share[c].jfirst + ( k - share[c].jbase )];
+			const int id = jointList[share[c].jfirst + ( k - share[c].jbase )];
 			( (int*)( W.joints + id ) )[t & 63] = ( (const int*)J.local )[RES_JOINT_WORDS * k + ( t & 63 )];
 		}
 	}
@@ -201,31 +260,49 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	/* finalisation (reference src/solver.c:165-351), then the counts of its records and
 	 * sleepy bodies to the host */
 	bar.sync();
-	for ( int i = rank * T + tid; i < P.awakeCount; i += CL * T )
-		finalize_body( W, i, sc );
+	if ( CL == 1 )
+	{
+		for ( int j = tid; j < awake; j += T )
+			finalize_body( W, rb.flags[j], sc );
+	}
+	else
+	{
+		for ( int i = rank * T + tid; i < P.awakeCount; i += CL * T )
+			finalize_body( W, i, sc );
+	}
 	bar.sync();
 	if ( rank == 0 && tid == 0 )
 	{
-		W.hostCounters[1] = __ldcg( W.counters + 1 );
-		W.hostCounters[3] = __ldcg( W.counters + 3 );
-		/* every CTA has passed the guard: the next narrowphase starts from zero */
-		W.counters[0] = 0;
+		bool last = true;
+		if ( BINS )
+		{
+			__threadfence();
+			last = atomicAdd( W.counters + 2, 1 ) == (int)gridDim.x - 1;
+			__threadfence();
+		}
+		if ( last )
+		{
+			W.hostCounters[1] = __ldcg( W.counters + 1 );
+			W.hostCounters[3] = __ldcg( W.counters + 3 );
+			/* every CTA has passed the guard: the next narrowphase starts from zero */
+			W.counters[0] = W.counters[1] = W.counters[2] = W.counters[3] = 0;
+		}
 	}
 }
 
 static_assert( sizeof( b2gJointDev ) == 256, "the joint copies move 64 words" );
 
-typedef void ( *FusedKernel )( const b2gDevWorld, const ResidentPlan, const FusedSplit, const b2gStepConst );
+typedef void ( *FusedKernel )( const b2gDevWorld, const ResidentPlan, const FusedSplit, const FusedBins, const b2gStepConst );
 
-static cudaLaunchConfig_t fused_config( cudaLaunchAttribute* attr, int ctas, size_t smem, cudaStream_t stream )
+static cudaLaunchConfig_t fused_config( cudaLaunchAttribute* attr, int ctas, size_t smem, cudaStream_t stream, int grid = 0, int threads = FUSED_THREADS )
 {
 	cudaLaunchConfig_t cfg = {};
 	attr[0].id = cudaLaunchAttributeClusterDimension;
 	attr[0].val.clusterDim.x = (unsigned)ctas;
 	attr[0].val.clusterDim.y = 1;
 	attr[0].val.clusterDim.z = 1;
-	cfg.gridDim = dim3( (unsigned)ctas, 1, 1 );
-	cfg.blockDim = dim3( FUSED_THREADS, 1, 1 );
+	cfg.gridDim = dim3( (unsigned)( grid > 0 ? grid : ctas ), 1, 1 );
+	cfg.blockDim = dim3( (unsigned)threads, 1, 1 );
 	cfg.dynamicSmemBytes = smem;
 	cfg.stream = stream;
 	cfg.attrs = attr;
@@ -246,7 +323,7 @@ static int fused_cluster_ready( void )
 	if ( ready != 0 )
 		return ready;
 	bool ok = true;
-	for ( FusedKernel k : { k_solve_world<1, false>, k_solve_world<1, true> } )
+	for ( FusedKernel k : { k_solve_world<1, false>, k_solve_world<1, true>, k_solve_world<1, false, true>, k_solve_world<1, true, true> } )
 		ok = ok && cudaFuncSetAttribute( k, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_MAX ) == cudaSuccess;
 	for ( FusedKernel k : { k_solve_world<FUSED_CLUSTER, false>, k_solve_world<FUSED_CLUSTER, true> } )
 	{
@@ -268,10 +345,7 @@ static int fused_cluster_ready( void )
  * caller must use the per-phase kernels, or -1 on a launch error. */
 extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc )
 {
-	/* body ids and slots below 2^16: the owner division is one multiply-high */
-	if ( plan->bodyIdCount <= 0 || plan->bodyBlock <= 0 || plan->bodyIdCount >= 65536 )
-		return 0;
-	if ( fused_cluster_ready() != 1 )
+	if ( plan->bodyIdCount <= 0 || plan->bodyBlock <= 0 || fused_cluster_ready() != 1 )
 		return 0;
 	const int* cs = plan->colorStart;
 	const int* js = plan->jointStart;
@@ -279,6 +353,7 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 	const int ovR = cs[B2G_COLORS] - cs[B2G_OVERFLOW], ovJ = js[B2G_COLORS] - js[B2G_OVERFLOW];
 	ResidentPlan P;
 	FusedSplit S;
+	FusedBins bins = {};
 	memset( &P, 0, sizeof( P ) );
 	memset( &S, 0, sizeof( S ) );
 	memcpy( P.colorStart, cs, sizeof( P.colorStart ) );
@@ -290,9 +365,8 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 
 	/* one CTA when it holds the world, joints included: no barrier crosses SMs (0.45 us a
 	 * sweep for the 20-row pyramid, 0.85 us in a cluster) */
-	size_t one = 144u * (size_t)( cs[B2G_COLORS] > 0 ? cs[B2G_COLORS] : 1 ) + RES_BODY_BYTES * (size_t)( ( plan->bodyIdCount + 3 ) & ~3 );
-	one = ( one + 15 ) / 16 * 16;
-	if ( one + RES_JOINT_BYTES * (size_t)joints <= RES_SMEM_MAX )
+	size_t one = b2g_bin_bytes( cs[B2G_COLORS], plan->bodyIdCount, 0 );
+	if ( b2g_bin_bytes( cs[B2G_COLORS], plan->bodyIdCount, joints ) <= RES_SMEM_MAX )
 	{
 		P.ctas = 1;
 		P.rowCap = cs[B2G_COLORS] > 0 ? cs[B2G_COLORS] : 1;
@@ -302,9 +376,35 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 		cudaLaunchAttribute attr[1];
 		cudaLaunchConfig_t cfg = fused_config( attr, 1, one + RES_JOINT_BYTES * (size_t)joints, (cudaStream_t)w->stream );
 		FusedKernel k = joints > 0 ? k_solve_world<1, true> : k_solve_world<1, false>;
-		return cudaLaunchKernelEx( &cfg, k, *w, P, S, *sc ) == cudaSuccess ? 1 : -1;
+		return cudaLaunchKernelEx( &cfg, k, *w, P, S, bins, *sc ) == cudaSuccess ? 1 : -1;
 	}
 
+	if ( plan->binCount > 0 )
+	{
+		/* a CTA per bin: 128 threads cover the widest colour of small islands, and leave
+		 * room for several CTAs on an SM */
+		const int* at = w->bins;
+		bins.table = at;
+		bins.rows = at + BIN_INTS * plan->binCount;
+		bins.joints = bins.rows + cs[B2G_COLORS];
+		bins.awake = bins.joints + joints;
+		bins.slot = bins.awake + plan->awakeCount;
+		P.ctas = 1;
+		P.rowCap = plan->binRows > 0 ? plan->binRows : 1;
+		P.bodyCap = ( plan->binBodies + 3 ) & ~3;
+		P.jointCap = plan->binJoints;
+		size_t bytes = b2g_bin_bytes( plan->binRows, plan->binBodies, 0 );
+		P.jointOffset = (int)( bytes / 16 );
+		cudaLaunchAttribute attr[1];
+		cudaLaunchConfig_t cfg = fused_config( attr, 1, bytes + RES_JOINT_BYTES * (size_t)plan->binJoints, (cudaStream_t)w->stream, plan->binCount,
+											   plan->binWidest <= 128 ? 128 : FUSED_THREADS );
+		FusedKernel k = joints > 0 ? k_solve_world<1, true, true> : k_solve_world<1, false, true>;
+		return cudaLaunchKernelEx( &cfg, k, *w, P, S, bins, *sc ) == cudaSuccess ? 1 : -1;
+	}
+
+	/* body ids and slots below 2^16: the owner division is one multiply-high */
+	if ( plan->bodyIdCount >= 65536 )
+		return 0;
 	const int CL = FUSED_CLUSTER;
 	P.ctas = CL;
 	P.bodyCap = plan->bodyBlock;
@@ -346,5 +446,5 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 	cudaLaunchAttribute attr[1];
 	cudaLaunchConfig_t cfg = fused_config( attr, CL, bytes, (cudaStream_t)w->stream );
 	FusedKernel k = joints > 0 ? k_solve_world<FUSED_CLUSTER, true> : k_solve_world<FUSED_CLUSTER, false>;
-	return cudaLaunchKernelEx( &cfg, k, *w, P, S, *sc ) == cudaSuccess ? 1 : -1;
+	return cudaLaunchKernelEx( &cfg, k, *w, P, S, bins, *sc ) == cudaSuccess ? 1 : -1;
 }

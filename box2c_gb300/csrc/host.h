@@ -348,6 +348,8 @@ typedef struct gWorld
 	gIntArray jointList;
 	b2gSolvePlan solvePlan; /* plan of the current solve lists */
 	bool solveUploaded;		/* solve lists on the device match the host's */
+	bool binsTried;			/* the plan has its bins of islands, or none are to be had */
+	gIntArray bins;
 	b2gPairQuery* pairQuery; /* device pair query buffers, made on first use */
 	gPairList* pairLists;	 /* per moved proxy, reused every step */
 	int pairListCap;

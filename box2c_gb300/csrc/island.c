@@ -120,6 +120,7 @@ void gbody_remove_from_set( gWorld* w, gBody* b )
 		if ( moved != B2G_NULL )
 			w->bodies[w->awake.data[at]].awakeIndex = at;
 		w->awakeDirty = true;
+		w->solveDirty = true;
 	}
 	else
 	{
@@ -652,6 +653,7 @@ void gsolver_set_wake( gWorld* w, int setIndex )
 		body->awakeIndex = w->awake.count;
 		gia_push( &w->awake, body->id );
 		w->awakeDirty = true;
+		w->solveDirty = true;
 		gbody_stage_op( w, body->id, B2G_BODY_WAKE );
 		for ( int key = body->headContactKey; key != B2G_NULL; )
 		{
@@ -715,6 +717,7 @@ void gisland_try_sleep( gWorld* w, int islandId )
 		if ( moved != B2G_NULL )
 			w->bodies[w->awake.data[awakeIndex]].awakeIndex = awakeIndex;
 		w->awakeDirty = true;
+		w->solveDirty = true;
 		body->setIndex = sleepSetId;
 		body->awakeIndex = B2G_NULL;
 		body->setLocal = sleepIndex;

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	{
 		while ( k >= share[c].base + share[c].count )
 			++c;
-		int2 e = res_prepare( W, m, share[c].first + ( k - share[c].base ), k, sc );
+		int2 e = res_prepare( W, m, nullptr, nullptr, share[c].first + ( k - share[c].base ), k, sc );
 		top = max( top, max( e.x, e.y ) );
 	}
 	for ( int i = af + tid; i < al; i += T )
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 		m = res_global_rows( W );
 	for ( int c = 0; c < B2G_COLORS; ++c )
 		for ( int j = tid; j < share[c].count; j += T )
-			res_prepare( W, m, share[c].first + j, share[c].base + j, sc );
+			res_prepare( W, m, nullptr, nullptr, share[c].first + j, share[c].base + j, sc );
 	ResBodies rb;
 	rb.st0 = rb.st1 = nullptr;
 	rb.flags = rb.awake = nullptr;

@@ -1141,6 +1141,167 @@ static void build_solve_lists( gWorld* w, b2gSolvePlan* plan )
 	w->solvePlan = *plan;
 	w->solveDirty = false;
 	w->solveUploaded = false;
+	w->binsTried = false;
+}
+
+/* Bins of islands for a world that one CTA does not hold: islands share no constraint
+ * and no moving body, so each bin is solved by a CTA of its own, without the barriers of
+ * a cluster or a launch per phase (22000 bodies in 400 pyramids: solver stage 423 us by
+ * phases, 48 by bins).  Only once a step passes without events: building them walks every row, and a
+ * changing colouring would have it done again each step.  Leaves the plan without bins
+ * when an island is too large, or when a kinematic body, which belongs to no island,
+ * could be shared. */
+#define BINS_WANTED ( 4 * 152 ) /* a few CTAs for each SM */
+
+static void build_bins( gWorld* w, b2gSolvePlan* plan )
+{
+	const int rows = plan->colorStart[B2G_COLORS], joints = plan->jointStart[B2G_COLORS];
+	const int bodies = w->awake.count, ids = w->bodyIds.next, islands = w->awakeIslands.count;
+	if ( islands < 2 || b2g_bin_bytes( rows, ids, joints ) <= B2G_BIN_BYTES_MAX )
+		return;
+	for ( int i = 0; i < islands; ++i )
+	{
+		const gIsland* is = w->islands + w->awakeIslands.data[i];
+		if ( b2g_bin_bytes( is->contactCount, is->bodyCount, is->jointCount ) > B2G_BIN_BYTES_MAX )
+			return;
+	}
+	int* islandBin = (int*)b2g_alloc( sizeof( int ) * (size_t)( w->islandCap + ids ) );
+	if ( islandBin == NULL )
+		return;
+	int* bodyBin = islandBin + w->islandCap;
+	/* islands into bins in set order; a static contact or two per body are not counted in
+	 * the island, so leave room for one each */
+	int target = ( rows + bodies ) / BINS_WANTED;
+	target = target < 160 ? 160 : target;
+	int bins = 1, weight = 0, binRows = 0, binBodies = 0, binJoints = 0;
+	for ( int i = 0; i < islands; ++i )
+	{
+		int id = w->awakeIslands.data[i];
+		const gIsland* is = w->islands + id;
+		int more = is->contactCount + is->jointCount + is->bodyCount;
+		if ( weight > 0 && ( weight + more > target || b2g_bin_bytes( binRows + is->contactCount + is->bodyCount, binBodies + is->bodyCount,
+																	   binJoints + is->jointCount ) > B2G_BIN_BYTES_MAX ) )
+		{
+			bins += 1;
+			weight = binRows = binBodies = binJoints = 0;
+		}
+		weight += more;
+		binRows += is->contactCount + is->bodyCount;
+		binBodies += is->bodyCount;
+		binJoints += is->jointCount;
+		islandBin[id] = bins - 1;
+	}
+	for ( int b = 0; b < ids; ++b )
+		bodyBin[b] = B2G_NULL;
+	bool ok = gia_reserve( &w->bins, B2G_BIN_INTS * bins + rows + joints + bodies + ids );
+	for ( int i = 0; i < bodies && ok; ++i )
+	{
+		const gBody* b = w->bodies + w->awake.data[i];
+		ok = b->islandId != B2G_NULL;
+		bodyBin[b->id] = ok ? islandBin[b->islandId] : B2G_NULL;
+	}
+	if ( ok == false )
+	{
+		b2g_free( islandBin );
+		return;
+	}
+	/* counts of every bin and colour, then their starts */
+	int* table = w->bins.data;
+	int* rowAt = table + B2G_BIN_INTS * bins;
+	int* jointAt = rowAt + rows;
+	int* bodyAt = jointAt + joints;
+	int* slotOf = bodyAt + bodies;
+	memset( table, 0, sizeof( int ) * B2G_BIN_INTS * (size_t)bins );
+	const int J = B2G_COLORS + 1, B = 2 * ( B2G_COLORS + 1 );
+#define BIN_OF( a, b ) ( bodyBin[a] != B2G_NULL ? bodyBin[a] : bodyBin[b] )
+	for ( int c = 0; c < B2G_COLORS && ok; ++c )
+	{
+		for ( int k = 0; k < w->colors[c].contacts.count && ok; ++k )
+		{
+			const gContact* e = w->contacts + w->colors[c].contacts.data[k];
+			int bin = BIN_OF( e->edges[0].bodyId, e->edges[1].bodyId );
+			ok = bin != B2G_NULL;
+			if ( ok )
+				table[B2G_BIN_INTS * bin + c] += 1;
+		}
+		for ( int k = 0; k < w->colors[c].joints.count && ok; ++k )
+		{
+			const gJoint* e = w->joints + w->colors[c].joints.data[k];
+			int bin = BIN_OF( e->bodyIdA, e->bodyIdB );
+			ok = bin != B2G_NULL;
+			if ( ok )
+				table[B2G_BIN_INTS * bin + J + c] += 1;
+		}
+	}
+	for ( int i = 0; i < bodies; ++i )
+		table[B2G_BIN_INTS * bodyBin[w->awake.data[i]] + B + 1] += 1;
+	int r = 0, j = 0, n = 0;
+	plan->binRows = plan->binBodies = plan->binJoints = plan->binWidest = 0;
+	for ( int k = 0; k < bins; ++k )
+	{
+		int* t = table + B2G_BIN_INTS * k;
+		int r0 = r, j0 = j;
+		for ( int c = 0; c < B2G_COLORS; ++c )
+		{
+			int nr = t[c], nj = t[J + c];
+			if ( c < B2G_OVERFLOW )
+				plan->binWidest = nr + nj > plan->binWidest ? nr + nj : plan->binWidest;
+			t[c] = r;
+			t[J + c] = j;
+			r += nr;
+			j += nj;
+		}
+		t[B2G_COLORS] = r;
+		t[J + B2G_COLORS] = j;
+		t[B] = n;
+		n += t[B + 1];
+		plan->binRows = r - r0 > plan->binRows ? r - r0 : plan->binRows;
+		plan->binJoints = j - j0 > plan->binJoints ? j - j0 : plan->binJoints;
+		plan->binBodies = t[B + 1] > plan->binBodies ? t[B + 1] : plan->binBodies;
+	}
+	if ( ok == false || b2g_bin_bytes( plan->binRows, plan->binBodies, plan->binJoints ) > B2G_BIN_BYTES_MAX )
+	{
+		b2g_free( islandBin );
+		return;
+	}
+	/* fill: the starts serve as cursors and are put back */
+	for ( int c = 0; c < B2G_COLORS; ++c )
+	{
+		for ( int k = 0; k < w->colors[c].contacts.count; ++k )
+		{
+			const gContact* e = w->contacts + w->colors[c].contacts.data[k];
+			rowAt[table[B2G_BIN_INTS * BIN_OF( e->edges[0].bodyId, e->edges[1].bodyId ) + c]++] = e->id;
+		}
+		for ( int k = 0; k < w->colors[c].joints.count; ++k )
+		{
+			const gJoint* e = w->joints + w->colors[c].joints.data[k];
+			jointAt[table[B2G_BIN_INTS * BIN_OF( e->bodyIdA, e->bodyIdB ) + J + c]++] = e->id;
+		}
+	}
+#undef BIN_OF
+	for ( int k = 0; k < bins; ++k )
+	{
+		int* t = table + B2G_BIN_INTS * k;
+		for ( int c = B2G_COLORS - 1; c > 0; --c )
+		{
+			t[c] = t[c - 1];
+			t[J + c] = t[J + c - 1];
+		}
+		t[0] = k > 0 ? t[B2G_COLORS - B2G_BIN_INTS] : 0;
+		t[J] = k > 0 ? t[J + B2G_COLORS - B2G_BIN_INTS] : 0;
+	}
+	int* cursor = islandBin; /* reused: bodies of a bin so far */
+	memset( cursor, 0, sizeof( int ) * (size_t)bins );
+	memset( slotOf, 0, sizeof( int ) * (size_t)ids );
+	for ( int i = 0; i < bodies; ++i )
+	{
+		int id = w->awake.data[i], bin = bodyBin[id];
+		slotOf[id] = cursor[bin]++;
+		bodyAt[table[B2G_BIN_INTS * bin + B] + slotOf[id]] = i;
+	}
+	b2g_free( islandBin );
+	w->bins.count = B2G_BIN_INTS * bins + rows + joints + bodies + ids;
+	plan->binCount = bins;
 }
 
 /* Host work before the narrowphase: pair update, device capacity, contact staging.
@@ -1265,6 +1426,20 @@ int gstep_after_collide( gWorld* w, float dt, int subSteps, b2gStepConst* sc, b2
 		return 0;
 	plan->awakeCount = w->awake.count;
 	plan->bodyIdCount = w->bodyIds.next;
+	if ( w->binsTried == false && eventCount == 0 && w->batching == false && w->dev.fused )
+	{
+		build_bins( w, plan );
+		if ( gworld_out_of_memory( w, failures ) )
+			return 0;
+		int e = plan->binCount > 0 ? b2gd_upload_bins( &w->dev, w->bins.data, w->bins.count ) : 0;
+		if ( e )
+		{
+			w->status = e;
+			return 0;
+		}
+		w->binsTried = true;
+		w->solvePlan = *plan;
+	}
 	if ( w->solveUploaded == false )
 	{
 		int e = b2gd_upload_solve_lists( &w->dev, w->solveList.data, w->solveList.count, w->jointList.data, w->jointList.count );

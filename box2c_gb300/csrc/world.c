@@ -475,6 +475,7 @@ void b2DestroyWorld( b2WorldId worldId )
 	gia_free( &w->moveArray );
 	gia_free( &w->solveList );
 	gia_free( &w->jointList );
+	gia_free( &w->bins );
 	gset_free( &w->moveSet );
 	gset_free( &w->pairSet );
 	b2g_free( w->bodies );
@@ -701,6 +702,7 @@ b2BodyId b2CreateBody( b2WorldId worldId, const b2BodyDef* def )
 		b->awakeIndex = w->awake.count;
 		gia_push( &w->awake, id );
 		w->awakeDirty = true;
+		w->solveDirty = true;
 		info |= B2G_B_AWAKE;
 		st[0] = def->linearVelocity.x;
 		st[1] = def->linearVelocity.y;

@@ -102,6 +102,26 @@ def test_world_stage_spaces(gpu, oracle, scene, size, steps):
     assert bad is None, detail
 
 
+# worlds that one CTA does not hold, of islands that it does: rows, joints of every type
+# and overflow sets in bins of islands, and steps with events in between, which run
+# without them; then one island too large for a bin
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene,steps", [("pyramids", 40), ("joints", 150), ("mixed", 40)])
+def test_bins_of_islands(gpu, oracle_atan, scene, steps):
+    def make(b):
+        if scene == "joints":
+            return b.joint_zoo(24, 0, 9)
+        if scene == "pyramids":
+            return b.many_pyramids(9, 7, 6)
+        w = b.pyramid(34, 0.01, 3)  # the pyramid's island is too large for a bin
+        for _ in range(40):
+            b.scenes.b2s_add_square(w, 0.25)
+        return w
+
+    bad, detail, _ = lockstep(gpu, oracle_atan, make, steps, check_manifolds=True, check_islands=True)
+    assert bad is None, detail
+
+
 @pytest.mark.gpu
 def test_read_back_follows_every_step(gpu, oracle):
     """Body states read back after each step, after several steps, after body edits and
