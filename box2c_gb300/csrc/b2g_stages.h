@@ -20,6 +20,7 @@
 #pragma once
 
 #include "b2g_collide.h"
+#include "b2g_collide_small.h"
 #include "b2g_device.h"
 #include "b2g_solve.h"
 #include "b2g_toi.h"
@@ -178,8 +179,8 @@ static __device__ __noinline__ void narrowphase_shapes( b2gManifold* m, const b2
 		*packedCache = gcache_pack( &cache );
 }
 
-/* Polygon pairs (the common case) take their own call, whose frame holds only the two
- * polygons in the contact frame; the other pairs' polygon copies stay out of it. */
+/* Polygon pairs take their own call, whose frame holds only the two polygons in the
+ * contact frame; the other pairs' polygon copies stay out of it. */
 static __device__ __noinline__ void narrowphase( b2gManifold* m, const b2gShapeGeo* gA, b2gXf xfA, const b2gShapeGeo* gB, b2gXf xfB,
 												 uint32_t* packedCache )
 {
@@ -189,6 +190,15 @@ static __device__ __noinline__ void narrowphase( b2gManifold* m, const b2gShapeG
 		narrowphase_polygons( m, gA, xfA, gB, xfB );
 	else
 		narrowphase_shapes( m, gA, xfA, gB, xfB, packedCache );
+}
+
+/* By value, so that the caller's manifold keeps its registers. */
+static __device__ __noinline__ b2gManifold narrowphase_general( const b2gShapeGeo* gA, b2gXf xfA, const b2gShapeGeo* gB, b2gXf xfB,
+																uint32_t* packedCache )
+{
+	b2gManifold m;
+	narrowphase( &m, gA, xfA, gB, xfB, packedCache );
+	return m;
 }
 
 /* Sensor contacts: whether the shapes overlap, by their GJK distance with radii,
@@ -276,12 +286,16 @@ static __device__ void collide_contact( const b2gDevWorld& W, int id )
 	const float oldN0 = prev->pts[0].normalImpulse, oldT0 = prev->pts[0].tangentImpulse;
 	const float oldN1 = prev->pts[1].normalImpulse, oldT1 = prev->pts[1].tangentImpulse;
 	b2gManifold m;
-	narrowphase( &m, gA, xfA, gB, xfB, W.cCache + id );
+	if ( small_narrowphase( m, gA, xfA, gB, xfB ) == false )
+		m = narrowphase_general( gA, xfA, gB, xfB, W.cCache + id );
 
 	int pointCount = m.count;
 	bool touching = pointCount > 0;
-	for ( int i = 0; i < pointCount; ++i )
+#pragma unroll
+	for ( int i = 0; i < 2; ++i )
 	{
+		if ( i >= pointCount )
+			break;
 		b2gPoint* mp2 = m.pts + i;
 		mp2->anchorA = gsub( mp2->anchorA, offA );
 		mp2->anchorB = gsub( mp2->anchorB, offB );

@@ -110,6 +110,8 @@ __global__ void __launch_bounds__( BATCH_GRID_THREADS ) k_batch_scatter( const b
 	}
 }
 
+/* Four CTAs an SM (64 registers, a few spilled) beat two (128, none) on a full machine:
+ * 240 us against 260 for 1024 pyramids; for a hundred small worlds two are 3 us faster. */
 __global__ void __launch_bounds__( BATCH_GRID_THREADS, 4 ) k_batch_collide( const b2gBatchItem* items, const int* prefix, int n )
 {
 	int total = prefix[n];
