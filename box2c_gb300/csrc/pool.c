@@ -9,29 +9,42 @@
  * chunks are done.  One job runs at a time: gpool_for waits for the pool, gpool_try_for
  * returns false at once when the pool is busy (another thread's job, or a call from
  * inside a job) and the caller runs the range itself.  gpool_for must not nest.
+ *
+ * A batched step has five short jobs, microseconds of work each for a hundred worlds, so
+ * what counts is what a job costs beside its work.  The caller waits only for workers
+ * that are inside the job, never for one that still has to wake up, and a worker watches
+ * for the next job for POOL_WATCH_US before it sleeps.  Waking every worker and waiting
+ * for all of them took 30 to 60 us a job (96 worlds of 8 bodies: 293 us a step with it,
+ * 142 without).
  */
 #include "host.h"
 
 #include <pthread.h>
+#include <sched.h>
 #include <stdatomic.h>
 #include <stdlib.h>
+#include <time.h>
 #include <unistd.h>
 
 #define POOL_MAX_THREADS 32
+#define POOL_WATCH_US 100
 
 typedef struct gPool
 {
 	pthread_t threads[POOL_MAX_THREADS];
 	int workers;
-	pthread_mutex_t lock;
+	pthread_mutex_t lock; /* sleeping workers */
 	pthread_cond_t wake;
-	pthread_cond_t done;
-	uint64_t generation;
+	int sleeping;
+	/* the open job's number, 0 when none is open: its fields do not change while it is
+	 * open, nor while a worker that found it open is inside */
+	atomic_ullong open;
+	unsigned long long jobs;
 	gTaskFn* fn;
 	void* ctx;
 	int count, grain;
 	atomic_int next;
-	int active; /* workers still inside the current job */
+	atomic_int inside;
 } gPool;
 
 static gPool s_pool;
@@ -50,22 +63,47 @@ static void run_chunks( gPool* p )
 	}
 }
 
+static long long now_us( void )
+{
+	struct timespec t;
+	clock_gettime( CLOCK_MONOTONIC, &t );
+	return 1000000ll * t.tv_sec + t.tv_nsec / 1000;
+}
+
 static void* worker( void* arg )
 {
 	gPool* p = (gPool*)arg;
-	uint64_t seen = 0;
-	pthread_mutex_lock( &p->lock );
+	unsigned long long seen = 0;
 	for ( ;; )
 	{
-		while ( p->generation == seen )
-			pthread_cond_wait( &p->wake, &p->lock );
-		seen = p->generation;
-		pthread_mutex_unlock( &p->lock );
-		run_chunks( p );
-		pthread_mutex_lock( &p->lock );
-		p->active -= 1;
-		if ( p->active == 0 )
-			pthread_cond_signal( &p->done );
+		/* watch for a job, then sleep until one is opened */
+		unsigned long long job = atomic_load( &p->open );
+		for ( long long until = now_us() + POOL_WATCH_US; job == 0 || job == seen; job = atomic_load( &p->open ) )
+		{
+			if ( now_us() < until )
+			{
+				sched_yield();
+				continue;
+			}
+			pthread_mutex_lock( &p->lock );
+			for ( job = atomic_load( &p->open ); job == 0 || job == seen; job = atomic_load( &p->open ) )
+			{
+				p->sleeping += 1;
+				pthread_cond_wait( &p->wake, &p->lock );
+				p->sleeping -= 1;
+			}
+			pthread_mutex_unlock( &p->lock );
+			break;
+		}
+		/* enter it unless it has closed meanwhile */
+		atomic_fetch_add( &p->inside, 1 );
+		job = atomic_load( &p->open );
+		if ( job != 0 && job != seen )
+		{
+			seen = job;
+			run_chunks( p );
+		}
+		atomic_fetch_sub( &p->inside, 1 );
 	}
 	return NULL;
 }
@@ -75,7 +113,6 @@ static void pool_start( void )
 	gPool* p = &s_pool;
 	pthread_mutex_init( &p->lock, NULL );
 	pthread_cond_init( &p->wake, NULL );
-	pthread_cond_init( &p->done, NULL );
 	long cores = sysconf( _SC_NPROCESSORS_ONLN );
 	int n = cores > 1 ? (int)cores - 1 : 0;
 	n = n > POOL_MAX_THREADS ? POOL_MAX_THREADS : n;
@@ -97,21 +134,26 @@ int gpool_threads( void )
 static void run_job( int count, int grain, gTaskFn* fn, void* ctx )
 {
 	gPool* p = &s_pool;
-	pthread_mutex_lock( &p->lock );
 	p->fn = fn;
 	p->ctx = ctx;
 	p->count = count;
 	p->grain = grain;
 	atomic_store( &p->next, 0 );
-	p->active = p->workers;
-	p->generation += 1;
-	pthread_cond_broadcast( &p->wake );
-	pthread_mutex_unlock( &p->lock );
-	run_chunks( p );
+	p->jobs += 1;
+	atomic_store( &p->open, p->jobs );
+	/* wake as many more as there are chunks for */
+	int wanted = ( count + grain - 1 ) / grain - 1;
+	wanted = wanted > p->workers ? p->workers : wanted;
 	pthread_mutex_lock( &p->lock );
-	while ( p->active > 0 )
-		pthread_cond_wait( &p->done, &p->lock );
+	int wakes = wanted - ( p->workers - p->sleeping );
 	pthread_mutex_unlock( &p->lock );
+	for ( int i = 0; i < wakes; ++i )
+		pthread_cond_signal( &p->wake );
+	run_chunks( p );
+	/* no chunk is left to take: close, and wait for those that are being run */
+	atomic_store( &p->open, 0 );
+	while ( atomic_load( &p->inside ) > 0 )
+		sched_yield();
 }
 
 void gpool_for( int count, int grain, gTaskFn* fn, void* ctx )
