@@ -122,6 +122,7 @@ extern "C" void b2gd_free( b2gDevWorld* w, b2gHostIO* io )
 	FREE_DEV( w->shapeRange );
 	FREE_DEV( w->shapeList );
 	FREE_DEV( w->geo );
+	FREE_DEV( w->filter );
 	FREE_DEV( w->aabb );
 	FREE_DEV( w->fat );
 	FREE_DEV( w->cShapes );
@@ -209,6 +210,7 @@ extern "C" int b2gd_reserve( b2gDevWorld* w, b2gHostIO* io, int bodyCap, int sha
 	{
 		int nc = next_cap( w->shapeCap, shapeCap );
 		e |= grow( (void**)&w->geo, sizeof( b2gShapeGeo ) * (size_t)w->shapeCap, sizeof( b2gShapeGeo ) * (size_t)nc, s );
+		e |= grow( &w->filter, 16u * (size_t)w->shapeCap, 16u * (size_t)nc, s );
 		e |= grow( &w->aabb, 16u * (size_t)w->shapeCap, 16u * (size_t)nc, s );
 		e |= grow( &w->fat, 16u * (size_t)w->shapeCap, 16u * (size_t)nc, s );
 		e |= grow( (void**)&w->shapeList, 4u * (size_t)w->shapeCap, 4u * (size_t)nc, s );
@@ -334,10 +336,11 @@ extern "C" int b2gd_upload_awake( b2gDevWorld* w, const int* awake, int count )
 	return h2d( w, w->awake, awake, 4u * (size_t)count, (cudaStream_t)w->stream );
 }
 
-extern "C" int b2gd_upload_shapes( b2gDevWorld* w, const b2gShapeGeo* geo, const float* aabb, const float* fat, int count )
+extern "C" int b2gd_upload_shapes( b2gDevWorld* w, const b2gShapeGeo* geo, const int* filter, const float* aabb, const float* fat, int count )
 {
 	cudaStream_t s = (cudaStream_t)w->stream;
 	int e = h2d( w, w->geo, geo, sizeof( b2gShapeGeo ) * (size_t)count, s );
+	e |= h2d( w, w->filter, filter, 16u * (size_t)count, s );
 	e |= h2d( w, w->aabb, aabb, 16u * (size_t)count, s );
 	e |= h2d( w, w->fat, fat, 16u * (size_t)count, s );
 	return e;

@@ -89,7 +89,7 @@ int b2gd_reserve_body_ops( b2gDevWorld* w, int count );
  * (sleep: stop integrating; wake: identity state, zero sleep timer).  The copy is taken
  * from pageable memory, so ops may be reused when the call returns. */
 int b2gd_body_ops( b2gDevWorld* w, const int* ops, int count );
-int b2gd_upload_shapes( b2gDevWorld* w, const b2gShapeGeo* geo, const float* aabb, const float* fat, int count );
+int b2gd_upload_shapes( b2gDevWorld* w, const b2gShapeGeo* geo, const int* filter, const float* aabb, const float* fat, int count );
 int b2gd_upload_shape_lists( b2gDevWorld* w, const int* range, int bodyCount, const int* list, int listCount );
 int b2gd_upload_joints( b2gDevWorld* w, const b2gJointDev* joints, int count );
 int b2gd_upload_solve_lists( b2gDevWorld* w, const int* solveList, int solveCount, const int* jointList, int jointCount );
@@ -136,7 +136,7 @@ int b2gd_sync( b2gDevWorld* w );
  * (leaf proxy key) and cand[... + 1] (shape id) for k < counts[i]; counts[i] is -1 when
  * the proxy needed more than B2G_QUERY_SLOTS slots or a deeper stack, and the host
  * queries that proxy itself.  Candidates the pair rules reject for the proxy itself, the
- * moved-pair rule or an existing pair (pairTable: the host pair set's table of pairCap
+ * moved-pair rule, shapes of one body, the shapes' filters, two sensors or an existing pair (pairTable: the host pair set's table of pairCap
  * slots, copied when pairVersion changes) are left out.  Synchronises the world's
  * stream; the result arrays are host memory owned by the query and valid until the next
  * call. */

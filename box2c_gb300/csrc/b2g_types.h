@@ -241,6 +241,7 @@ typedef struct b2gDevWorld
 
 	/* shapes, indexed by shape id */
 	b2gShapeGeo* geo;
+	void* filter; /* int4: category bits, mask bits, group index, sensor */
 	void* aabb; /* float4 */
 	void* fat;	/* float4 */
 

@@ -302,6 +302,7 @@ typedef struct gWorld
 	int mirrorCap;
 	void *dState, *dXf, *dCenters; /* the device's view of those mirrors */
 	b2gShapeGeo* hGeo;
+	int* hFilter; /* 4 per shape: category bits, mask bits, group index, sensor */
 	float* hAabb;
 	float* hFat;
 	int shapeMirrorCap;

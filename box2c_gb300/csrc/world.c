@@ -189,11 +189,11 @@ bool gworld_reserve_mirrors( gWorld* w )
 	if ( needS > w->shapeMirrorCap )
 	{
 		int nc = grow_cap( w->shapeMirrorCap, needS );
-		void** ptrs[] = { (void**)&w->hGeo, (void**)&w->hAabb, (void**)&w->hFat };
-		size_t ob[] = { sizeof( b2gShapeGeo ) * (size_t)w->shapeMirrorCap, 16u * (size_t)w->shapeMirrorCap,
-						16u * (size_t)w->shapeMirrorCap };
-		size_t nb[] = { sizeof( b2gShapeGeo ) * (size_t)nc, 16u * (size_t)nc, 16u * (size_t)nc };
-		if ( grow_pinned( ptrs, ob, nb, 3 ) == false )
+		void** ptrs[] = { (void**)&w->hGeo, (void**)&w->hFilter, (void**)&w->hAabb, (void**)&w->hFat };
+		size_t o4 = 16u * (size_t)w->shapeMirrorCap, n4 = 16u * (size_t)nc;
+		size_t ob[] = { sizeof( b2gShapeGeo ) * (size_t)w->shapeMirrorCap, o4, o4, o4 };
+		size_t nb[] = { sizeof( b2gShapeGeo ) * (size_t)nc, n4, n4, n4 };
+		if ( grow_pinned( ptrs, ob, nb, 4 ) == false )
 			return false;
 		w->shapeMirrorCap = nc;
 	}
@@ -327,7 +327,7 @@ void gworld_flush( gWorld* w )
 	}
 	if ( w->shapesDirty )
 	{
-		e |= b2gd_upload_shapes( &w->dev, w->hGeo, w->hAabb, w->hFat, ns );
+		e |= b2gd_upload_shapes( &w->dev, w->hGeo, w->hFilter, w->hAabb, w->hFat, ns );
 		w->shapesDirty = false;
 	}
 	if ( w->shapeListsDirty )
@@ -496,7 +496,7 @@ void b2DestroyWorld( b2WorldId worldId )
 	b2g_free( w->hitEvents );
 	b2g_free( w->sensorBeginEvents );
 	b2g_free( w->sensorEndEvents );
-	void* pinned[] = { w->hState, w->hXf, w->hCenters, w->hPrev, w->hMass, w->hForce, w->hExtent, w->hInfo, w->hGeo, w->hAabb, w->hFat, w->hJoints };
+	void* pinned[] = { w->hState, w->hXf, w->hCenters, w->hPrev, w->hMass, w->hForce, w->hExtent, w->hInfo, w->hGeo, w->hFilter, w->hAabb, w->hFat, w->hJoints };
 	for ( size_t i = 0; i < sizeof( pinned ) / sizeof( pinned[0] ); ++i )
 		if ( pinned[i] )
 			cudaFreeHost( pinned[i] );
@@ -1100,6 +1100,8 @@ static b2ShapeId create_shape_internal( b2BodyId bodyId, const b2ShapeDef* def, 
 	g->bodyId = body->id;
 	g->enableHitEvents = def->enableHitEvents;
 	g->isSensor = def->isSensor;
+	int filter[4] = { (int)def->filter.categoryBits, (int)def->filter.maskBits, def->filter.groupIndex, def->isSensor };
+	memcpy( w->hFilter + 4 * id, filter, sizeof( filter ) );
 
 	/* proxy (reference src/shape.c:38-59, :692-702, src/broad_phase.c:91-102) */
 	const float* xf = w->hXf + 4 * body->id;
