@@ -134,6 +134,160 @@ __device__ __forceinline__ void store_row_smem( const SmemRows& m, int k, int ci
 	m.imp1[k] = make_float4( r.ni[1], r.ti[1], r.maxNi[1], 0.0f );
 }
 
+/* Words of a manifold that a row's preparation reads: both points' anchors, separation,
+ * normal and tangent impulse; the normal; the count. */
+#define ROW_INPUTS 17
+static_assert( sizeof( b2gPoint ) == 48 && sizeof( b2gManifold ) == 108, "manifold words" );
+
+__device__ __forceinline__ void copy4_async( void* to, const void* from )
+{
+	asm volatile( "cp.async.ca.shared.global [%0], [%1], 4;" ::"r"( (unsigned)__cvta_generic_to_shared( to ) ), "l"( from ) );
+}
+
+__device__ __forceinline__ void copy16_async( void* to, const void* from )
+{
+	asm volatile( "cp.async.cg.shared.global [%0], [%1], 16;" ::"r"( (unsigned)__cvta_generic_to_shared( to ) ), "l"( from ) );
+}
+
+/* Preparation of rows [0, rows) in shared memory by T threads, whole warps (reference
+ * src/contact_solver.c:597-808, :21-147): row k is entry source( k ) of the list (null: that
+ * contact); source is called with growing k.  slot, when given, renumbers the bodies.
+ *
+ * Bound by latency: index, contact, bodies and manifold, row by row, is three round trips
+ * to L2 for every T rows.  So a warp first fetches the indices of all its rows, then
+ * starts the copies of all their inputs into the rows' own slots, and computes the rows
+ * when they are there: three round trips in all.  Manifolds are 108 bytes apart; the warp
+ * copies them as one stream of words, lane after lane.  What is left is the issue of the
+ * copies (1130 rows in one CTA 10.4 -> 8.7 us, 1035 rows of a cluster's CTA 9.4 -> 7.7). */
+template <class Source>
+__device__ __forceinline__ void prepare_rows( const b2gDevWorld& W, const SmemRows& m, int rows, const int* list, const int* slot, Source source,
+											  int thread, int T, const b2gStepConst& sc )
+{
+	constexpr int U = 4;
+	for ( int k0 = thread; k0 < rows; k0 += U * T )
+	{
+		int cid[U], ia[U], ib[U];
+#pragma unroll
+		for ( int u = 0; u < U; ++u )
+		{
+			const int k = k0 + u * T;
+			cid[u] = k < rows ? source( k ) : -1;
+			if ( list && cid[u] >= 0 )
+				cid[u] = list[cid[u]];
+		}
+#pragma unroll
+		for ( int u = 0; u < U; ++u )
+		{
+			ia[u] = cid[u] >= 0 ? W.cBodies[2 * cid[u]] : -1;
+			ib[u] = cid[u] >= 0 ? W.cBodies[2 * cid[u] + 1] : -1;
+		}
+#pragma unroll
+		for ( int u = 0; u < U; ++u )
+			if ( cid[u] >= 0 )
+				m.idx[k0 + u * T] = make_int4( ia[u], ib[u], cid[u], 0 );
+	}
+	__syncwarp();
+	const float4* gst = (const float4*)W.state;
+	const float4* mass = (const float4*)W.mass;
+	const int* words = (const int*)W.manifold;
+	const int lane = thread & 31;
+	const float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
+	const int stride = (int)( m.coef1 - m.coef0 );
+	for ( int k0 = thread - lane; k0 < rows; k0 += T )
+	{
+		const int n = min( 32, rows - k0 );
+		const int k = k0 + lane;
+		const int4 own = lane < n ? m.idx[k] : make_int4( -1, -1, 0, 0 );
+#pragma unroll
+		for ( int i = 0; i < ROW_INPUTS; ++i )
+		{
+			const int t = lane + 32 * i, r = t / ROW_INPUTS, j = t - ROW_INPUTS * r;
+			const int w = j < 7 ? j + 2 : ( j < 14 ? j + 7 : j + 10 );
+			int* to = j < 16 ? (int*)( m.coef0 + ( j >> 2 ) * stride + k0 + r ) + ( j & 3 ) : &m.idx[k0 + r].w;
+			const int c = __shfl_sync( 0xffffffffu, own.z, r );
+			if ( r < n )
+				copy4_async( to, words + 27 * (size_t)c + w );
+		}
+		if ( lane < n )
+		{
+			const int ia = own.x, ib = own.y, cid = own.z;
+			copy4_async( &m.nf[k].z, W.cMix + 2 * cid );
+			copy4_async( &m.nf[k].w, W.cMix + 2 * cid + 1 );
+			if ( ia >= 0 )
+			{
+				copy16_async( m.anc0 + k, gst + 2 * ia );
+				copy4_async( &m.ms[k].x, &mass[ia].y );
+				copy4_async( &m.ms[k].y, &mass[ia].w );
+				if ( slot != nullptr )
+					copy4_async( &m.idx[k].x, slot + ia );
+			}
+			else
+			{
+				m.anc0[k] = zero;
+				m.ms[k].x = m.ms[k].y = 0.0f;
+			}
+			if ( ib >= 0 )
+			{
+				copy16_async( m.anc1 + k, gst + 2 * ib );
+				copy4_async( &m.ms[k].z, &mass[ib].y );
+				copy4_async( &m.ms[k].w, &mass[ib].w );
+				if ( slot != nullptr )
+					copy4_async( &m.idx[k].y, slot + ib );
+			}
+			else
+			{
+				m.anc1[k] = zero;
+				m.ms[k].z = m.ms[k].w = 0.0f;
+			}
+		}
+	}
+	asm volatile( "cp.async.wait_all;" ::: "memory" );
+	__syncwarp();
+	for ( int k = thread; k < rows; k += T )
+	{
+		const int4 ix = m.idx[k];
+		const float4 nf = m.nf[k], ms = m.ms[k], a = m.anc0[k], b = m.anc1[k];
+		const float4 q0 = m.coef0[k], q1 = m.coef1[k], q2 = m.imp0[k], q3 = m.imp1[k];
+		b2gManifold in;
+		in.pts[0].anchorA = gv( q0.x, q0.y );
+		in.pts[0].anchorB = gv( q0.z, q0.w );
+		in.pts[0].separation = q1.x;
+		in.pts[0].normalImpulse = q1.y;
+		in.pts[0].tangentImpulse = q1.z;
+		in.pts[1].anchorA = gv( q1.w, q2.x );
+		in.pts[1].anchorB = gv( q2.y, q2.z );
+		in.pts[1].separation = q2.w;
+		in.pts[1].normalImpulse = q3.x;
+		in.pts[1].tangentImpulse = q3.y;
+		in.normal = gv( q3.z, q3.w );
+		in.count = ix.w;
+		DevState sA = state_of( a, zero ), sB = state_of( b, zero );
+		Row r;
+		prepare_row( r, &in, ix.x, ix.y, make_float4( 0.0f, ms.x, 0.0f, ms.y ), make_float4( 0.0f, ms.z, 0.0f, ms.w ), sA, sB, nf.z, nf.w,
+					 ( ix.x < 0 || ix.y < 0 ) ? sc.staticSoft : sc.contactSoft, sc.enableWarmStarting ? 1.0f : 0.0f );
+		store_row_smem( m, k, ix.z, r );
+	}
+}
+
+/* Impulses of rows [0, rows) back to their manifolds (reference src/contact_solver.c:442-471,
+ * :1180-1293) by T threads: colour rows write both point slots, overflow rows
+ * (from colourRows on) their points.  Eight threads a row, a word each, so that a
+ * point's four words go out together: 1130 rows of one CTA 6.2 -> 1.7 us, 1035 rows of a
+ * cluster's CTA 5.0 -> 1.6 us. */
+__device__ __forceinline__ void store_impulses( const b2gDevWorld& W, const SmemRows& m, int rows, int colourRows, int thread, int T )
+{
+	float* words = (float*)W.manifold;
+	for ( int t = thread; t < 8 * rows; t += T )
+	{
+		const int k = t >> 3, p = ( t >> 2 ) & 1, q = t & 3;
+		const int4 idx = m.idx[k];
+		if ( k >= colourRows && p >= idx.w )
+			continue;
+		const float4* from = q < 3 ? ( p ? m.imp1 : m.imp0 ) : ( p ? m.coef1 : m.coef0 );
+		words[27 * (size_t)idx.z + 12 * p + 7 + q] = ( (const float*)( from + k ) )[q];
+	}
+}
+
 /* One row phase on a row in shared memory; Bodies is ClusterBodies (states spread over
  * the cluster) or SharedBodies (states of one CTA, by body id). */
 template <class Bodies>

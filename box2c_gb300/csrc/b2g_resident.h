@@ -451,51 +451,34 @@ __device__ __forceinline__ void res_index_overflow( const ResOverflow& ov, const
 	}
 }
 
-/* Preparation of one row into m (reference src/contact_solver.c:597-808, :21-147): entry k
- * of the list (null: contact k).  slot, when given, renumbers the row's bodies. */
-__device__ __forceinline__ int2 res_prepare( const b2gDevWorld& W, const SmemRows& m, const int* list, const int* slot, int k, int local,
-											 const b2gStepConst& sc )
+/* Preparation of one row in the row arrays: contact k. */
+__device__ __forceinline__ void res_prepare_global( const b2gDevWorld& W, const SmemRows& m, int k, const b2gStepConst& sc )
 {
 	const float4* gst = (const float4*)W.state;
 	const float4* mass = (const float4*)W.mass;
 	const float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
-	int cid = list ? list[k] : k;
-	int ia = W.cBodies[2 * cid];
-	int ib = W.cBodies[2 * cid + 1];
+	int ia = W.cBodies[2 * k];
+	int ib = W.cBodies[2 * k + 1];
 	DevState sA = ia >= 0 ? state_of( gst[2 * ia], gst[2 * ia + 1] ) : identity_state();
 	DevState sB = ib >= 0 ? state_of( gst[2 * ib], gst[2 * ib + 1] ) : identity_state();
 	Row r;
-	prepare_row( r, W.manifold + cid, ia, ib, ia >= 0 ? mass[ia] : zero, ib >= 0 ? mass[ib] : zero, sA, sB, W.cMix[2 * cid],
-				 W.cMix[2 * cid + 1], ( ia < 0 || ib < 0 ) ? sc.staticSoft : sc.contactSoft, sc.enableWarmStarting ? 1.0f : 0.0f );
-	if ( slot != nullptr )
-	{
-		r.ia = ia >= 0 ? slot[ia] : -1;
-		r.ib = ib >= 0 ? slot[ib] : -1;
-	}
-	store_row_smem( m, local, cid, r );
-	return make_int2( ia, ib );
+	prepare_row( r, W.manifold + k, ia, ib, ia >= 0 ? mass[ia] : zero, ib >= 0 ? mass[ib] : zero, sA, sB, W.cMix[2 * k], W.cMix[2 * k + 1],
+				 ( ia < 0 || ib < 0 ) ? sc.staticSoft : sc.contactSoft, sc.enableWarmStarting ? 1.0f : 0.0f );
+	store_row_smem( m, k, k, r );
 }
 
-/* Impulses of local row k back to its manifold (reference src/contact_solver.c:442-471,
- * :1180-1293): colour rows write both point slots, overflow rows their points. */
-__device__ __forceinline__ void res_store( const b2gDevWorld& W, const SmemRows& m, int k, bool overflow )
+/* The list entry of local row k; k grows from call to call of one thread. */
+struct ResSource
 {
-	int4 idx = m.idx[k];
-	b2gManifold* mf = W.manifold + idx.z;
-	int n = overflow ? idx.w : 2;
-	float4 imp[2] = { m.imp0[k], m.imp1[k] };
-	float4 coef[2] = { m.coef0[k], m.coef1[k] };
-#pragma unroll
-	for ( int j = 0; j < 2; ++j )
+	const ResShare* share;
+	int c;
+	__device__ __forceinline__ int operator()( int k )
 	{
-		if ( j >= n )
-			break;
-		mf->pts[j].normalImpulse = imp[j].x;
-		mf->pts[j].tangentImpulse = imp[j].y;
-		mf->pts[j].maxNormalImpulse = imp[j].z;
-		mf->pts[j].normalVelocity = coef[j].w;
+		while ( k >= share[c].base + share[c].count )
+			++c;
+		return share[c].first + ( k - share[c].base );
 	}
-}
+};
 
 __device__ __forceinline__ void res_terms( const b2gDevWorld& W, const ResBodies& rb, int k, int b, const b2gStepConst& sc )
 {

@@ -282,20 +282,7 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 	const int awake = it.awakeCount;
 	if constexpr ( ONCHIP )
 	{
-		const float4 zero = make_float4( 0.0f, 0.0f, 0.0f, 0.0f );
-		const float warm = sc.enableWarmStarting ? 1.0f : 0.0f;
-		for ( int k = tid; k < rows; k += step )
-		{
-			int cid = W.solveList[k];
-			int ia = W.cBodies[2 * cid];
-			int ib = W.cBodies[2 * cid + 1];
-			DevState sA = ia >= 0 ? state_of( gst[2 * ia], gst[2 * ia + 1] ) : identity_state();
-			DevState sB = ib >= 0 ? state_of( gst[2 * ib], gst[2 * ib + 1] ) : identity_state();
-			Row r;
-			prepare_row( r, W.manifold + cid, ia, ib, ia >= 0 ? mass[ia] : zero, ib >= 0 ? mass[ib] : zero, sA, sB, W.cMix[2 * cid],
-						 W.cMix[2 * cid + 1], ( ia < 0 || ib < 0 ) ? sc.staticSoft : sc.contactSoft, warm );
-			store_row_smem( s.m, k, cid, r );
-		}
+		prepare_rows( W, s.m, rows, W.solveList, nullptr, []( int k ) { return k; }, tid, step, sc );
 	}
 	else
 	{
@@ -334,23 +321,7 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 
 	if constexpr ( ONCHIP )
 	{
-		/* colour rows store both point slots, overflow rows their points (as store_row) */
-		const int ov = it.colorStart[B2G_OVERFLOW];
-		for ( int k = tid; k < rows; k += step )
-		{
-			int4 idx = s.m.idx[k];
-			b2gManifold* mf = W.manifold + idx.z;
-			int n = k < ov ? 2 : idx.w;
-			float4 imp[2] = { s.m.imp0[k], s.m.imp1[k] };
-			float4 coef[2] = { s.m.coef0[k], s.m.coef1[k] };
-			for ( int j = 0; j < n; ++j )
-			{
-				mf->pts[j].normalImpulse = imp[j].x;
-				mf->pts[j].tangentImpulse = imp[j].y;
-				mf->pts[j].maxNormalImpulse = imp[j].z;
-				mf->pts[j].normalVelocity = coef[j].w;
-			}
-		}
+		store_impulses( W, s.m, rows, it.colorStart[B2G_OVERFLOW], tid, step );
 	}
 	else
 	{

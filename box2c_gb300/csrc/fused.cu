@@ -153,12 +153,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 			( (int*)J.local )[RES_JOINT_WORDS * k + ( t & 63 )] = ( (const int*)( W.joints + id ) )[t & 63];
 		}
 	}
-	for ( int k = tid, c = 0; k < rows; k += T )
-	{
-		while ( k >= share[c].base + share[c].count )
-			++c;
-		res_prepare( W, m, rowList, BINS ? bins.slot : nullptr, share[c].first + ( k - share[c].base ), k, sc );
-	}
+	prepare_rows( W, m, rows, rowList, BINS ? bins.slot : nullptr, ResSource{ share, 0 }, tid, T, sc );
 	/* one CTA: awake bodies in list order, their awake indices kept for finalisation; a
 	 * cluster: the block of ids that this CTA owns */
 	int bodies = P.awakeCount;
@@ -186,14 +181,22 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		bodies = P.bodyIdCount - rank * P.bodyCap;
 		bodies = bodies < 0 ? 0 : ( bodies > P.bodyCap ? P.bodyCap : bodies );
 	}
-	for ( int s = tid; CL > 1 && s < bodies; s += T )
+	if ( CL > 1 )
 	{
-		const int b = rank * P.bodyCap + s;
-		rb.st0[s] = gst[2 * b];
-		rb.st1[s] = gst[2 * b + 1];
-		if ( W.bodyInfo[b] & B2G_B_AWAKE )
+		const int first = rank * P.bodyCap;
+		for ( int s = tid; s < bodies; s += T )
 		{
+			rb.st0[s] = gst[2 * ( first + s )];
+			rb.st1[s] = gst[2 * ( first + s ) + 1];
+		}
+		/* the awake bodies among them, with their awake indices */
+		for ( int i = tid; i < P.awakeCount; i += T )
+		{
+			const int b = W.awake[i], s = b - first;
+			if ( s < 0 || s >= bodies )
+				continue;
 			rb.awake[atomicAdd( &s_awake, 1 )] = s;
+			rb.flags[s] = i;
 			res_terms( W, rb, s, b, sc );
 		}
 	}
@@ -236,15 +239,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		res_run<CL, CT, true, JOINTS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 	}
 
-	for ( int k = tid; k < rows; k += T )
-		res_store( W, m, k, k >= colourRows );
-	/* owned awake body states back to global memory for finalisation */
-	for ( int j = tid; j < awake; j += T )
-	{
-		const int s = rb.awake[j], b = CL == 1 ? W.awake[rb.flags[j]] : rank * P.bodyCap + s;
-		gst[2 * b] = rb.st0[s];
-		gst[2 * b + 1] = rb.st1[s];
-	}
+	store_impulses( W, m, rows, colourRows, tid, T );
 	if ( JOINTS && J.local != nullptr )
 	{
 		for ( int t = tid, c = 0; t < 64 * s_joints; t += T )
@@ -257,18 +252,14 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		}
 	}
 
-	/* finalisation (reference src/solver.c:165-351), then the counts of its records and
-	 * sleepy bodies to the host */
-	bar.sync();
-	if ( CL == 1 )
+	/* finalisation (reference src/solver.c:165-351) of the bodies whose states are here,
+	 * then the counts of its records and sleepy bodies to the host */
+	for ( int j = tid; j < awake; j += T )
 	{
-		for ( int j = tid; j < awake; j += T )
-			finalize_body( W, rb.flags[j], sc );
-	}
-	else
-	{
-		for ( int i = rank * T + tid; i < P.awakeCount; i += CL * T )
-			finalize_body( W, i, sc );
+		const int s = rb.awake[j], i = CL == 1 ? rb.flags[j] : rb.flags[s];
+		const int b = CL == 1 ? W.awake[i] : rank * P.bodyCap + s;
+		gst[2 * b] = rb.st0[s];
+		finalize_state( W, i, b, rb.st0[s], rb.st1[s], sc );
 	}
 	bar.sync();
 	if ( rank == 0 && tid == 0 )

@@ -95,13 +95,9 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	/* rows, and the largest body index of this CTA's rows and share of the list */
 	const int af = res_first( P.awakeCount, rank, CL ), al = res_first( P.awakeCount, rank + 1, CL );
 	int top = -1;
-	for ( int k = tid, c = 0; k < rows; k += T )
-	{
-		while ( k >= share[c].base + share[c].count )
-			++c;
-		int2 e = res_prepare( W, m, nullptr, nullptr, share[c].first + ( k - share[c].base ), k, sc );
-		top = max( top, max( e.x, e.y ) );
-	}
+	prepare_rows( W, m, rows, nullptr, nullptr, ResSource{ share, 0 }, tid, T, sc );
+	for ( int k = tid; k < rows; k += T )
+		top = max( top, max( m.idx[k].x, m.idx[k].y ) );
 	for ( int i = af + tid; i < al; i += T )
 		top = max( top, W.awake[i] );
 	top = __reduce_max_sync( 0xffffffffu, top );
@@ -212,8 +208,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 			res_run<CL, T, false, false>( P, share, m, J, G, rb, gst, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
 		}
 	}
-	for ( int k = tid; k < rows; k += T )
-		res_store( W, m, k, k >= colourRows );
+	store_impulses( W, m, rows, colourRows, tid, T );
 }
 
 /* The solver stage over a cooperative grid: body states in global memory, rows in shared
@@ -251,9 +246,13 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 		m = res_carve_rows( smem, P.rowCap );
 	else
 		m = res_global_rows( W );
-	for ( int c = 0; c < B2G_COLORS; ++c )
-		for ( int j = tid; j < share[c].count; j += T )
-			res_prepare( W, m, nullptr, nullptr, share[c].first + j, share[c].base + j, sc );
+	const int rows = share[B2G_COLORS - 1].base + share[B2G_COLORS - 1].count;
+	if constexpr ( ONCHIP )
+		prepare_rows( W, m, rows, nullptr, nullptr, ResSource{ share, 0 }, tid, T, sc );
+	else
+		for ( int c = 0; c < B2G_COLORS; ++c )
+			for ( int j = tid; j < share[c].count; j += T )
+				res_prepare_global( W, m, share[c].first + j, sc );
 	ResBodies rb;
 	rb.st0 = rb.st1 = nullptr;
 	rb.flags = rb.awake = nullptr;
@@ -274,9 +273,15 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 	bar.sync();
 	L2Bodies G{ (float4*)W.state };
 	res_run<0, T, false, false>( P, share, m, J, G, rb, (float4*)W.state, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
-	for ( int c = 0; c < B2G_COLORS; ++c )
-		for ( int j = tid; j < share[c].count; j += T )
-			res_store( W, m, share[c].base + j, c == B2G_OVERFLOW );
+	if constexpr ( ONCHIP )
+		store_impulses( W, m, rows, share[B2G_OVERFLOW].base, tid, T );
+	else
+		for ( int c = 0; c < B2G_COLORS; ++c )
+		{
+			const int f = share[c].base;
+			const SmemRows part = { m.idx + f, m.nf + f, m.ms + f, m.anc0 + f, m.anc1 + f, m.coef0 + f, m.coef1 + f, m.imp0 + f, m.imp1 + f };
+			store_impulses( W, part, share[c].count, c == B2G_OVERFLOW ? 0 : share[c].count, tid, T );
+		}
 	if ( tid == 0 && atomicAdd( ctl + 1, 1 ) == ctas - 1 )
 	{
 		/* every CTA is past its last barrier */
