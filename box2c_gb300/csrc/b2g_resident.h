@@ -32,6 +32,8 @@ struct ResidentPlan
 	int bodyCap;  /* body slots per CTA in shared memory; a grid's velocity-term slots */
 	int jointCap; /* joint slots per CTA in shared memory (0: joints in the joint array) */
 	int jointOffset; /* float4 offset of the joint slots */
+	int bodyOffset;	 /* float4 offset of a cluster's body slots */
+	int pushCap;	 /* body copies per CTA (0: no copies) */
 	int ovOffset; /* float4 offset of the overflow cache, 0 without one */
 };
 

@@ -7,14 +7,16 @@
  * Layout (dynamic shared memory of every CTA, rank r of CL):
  *   bodies  body ids are cut into CL contiguous blocks of bodyCap: body b lives in CTA
  *           b / bodyCap at slot b % bodyCap (the owner is found by a multiply-high with a
- *           host-computed reciprocal).  Rows reach a body of another CTA through
- *           distributed shared memory.
+ *           host-computed reciprocal).  Every CTA has copies of the other bodies that its
+ *           rows and joints touch and sends its updates to the other copies
+ *           (b2g_push.h); where the copies do not fit, or joints do not, rows
+ *           reach a body of another CTA through distributed shared memory.
  *   rows    in a cluster the host groups each colour's rows by the CTA owning their first
  *           non-static body (rows of one colour share no body, so the order within a
  *           colour changes no result); CTA o holds rows [split[c][o], split[c][o+1]) of
  *           colour c as nine float4 arrays (structure of arrays, conflict-free).  Most
  *           body accesses of a row are then local.  The overflow colour's rows all live
- *           in CTA 0; thread 0 of CTA 0 solves them serially on CTA-local copies of
+ *           in CTA 0; thread 0 of CTA 0 solves them serially on the CTA's copies of
  *           their bodies.
  *   joints  CTA k takes an equal share of a colour's joints, in shared memory while they
  *           fit, else in the joint array; only one thread reads and writes a joint.
@@ -25,9 +27,13 @@
  *
  * Bound by the chain of about 113 dependent sweeps: a barrier and a row's own chain each.
  * Solver stage of a step before and after the one-CTA space and on-chip joints: pyramid of
- * 20 rows 97 -> 52 us, shape pile of 600 100 -> 68 us, 100 x 100 joint grid 421 -> 298 us;
- * large pyramid 116 -> 117 us, tumbler of 2000 401 -> 393 us.
+ * 20 rows 97 -> 52 us, shape pile of 600 100 -> 68 us, 100 x 100 joint grid 421 -> 298 us.
+ * With preparation and finalisation in the kernel: 47 us, 65 us; large pyramid 112 us, with
+ * body copies 97, tumbler of 2000 370, with them 350 (83 overflow rows, one after the
+ * other, 13 times a step: about 250 of it).  The joint grid's joints stay in L2 (5 us a
+ * sweep); its stage runs beside the host's tree rebuild, which takes longer.
  */
+#include "b2g_push.h"
 #include "b2g_resident.h"
 
 #include <string.h>
@@ -80,13 +86,14 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	extern __shared__ float4 smem[];
 	__shared__ ResShare share[B2G_COLORS];
 	__shared__ int s_rows, s_joints, s_awake, s_ovSlots;
+	__shared__ PushShared push;
 	cg::cluster_group cl = cg::this_cluster();
 	const int rank = CL == 1 ? 0 : (int)cl.block_rank();
 	const int tid = threadIdx.x;
 	const int* cs = P.colorStart;
 	const int* js = P.jointStart;
 	SmemRows m = res_carve_rows( smem, P.rowCap );
-	ResBodies rb = res_carve_bodies( smem + 9 * P.rowCap, P.bodyCap );
+	ResBodies rb = res_carve_bodies( smem + ( CL == 1 ? 9 * P.rowCap : P.bodyOffset ), P.bodyCap );
 	float4* gst = (float4*)W.state;
 
 	if ( tid < B2G_COLORS )
@@ -159,7 +166,43 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	int bodies = P.awakeCount;
 	if ( BINS )
 		bodies = bin[BIN_INTS - 1];
-	if ( CL == 1 )
+	if ( CL > 1 )
+	{
+		bodies = P.bodyIdCount - rank * P.bodyCap;
+		bodies = bodies < 0 ? 0 : ( bodies > P.bodyCap ? P.bodyCap : bodies );
+	}
+	auto load_owned = [&]() {
+		const int first = rank * P.bodyCap;
+		for ( int s = tid; s < bodies; s += T )
+		{
+			rb.st0[s] = gst[2 * ( first + s )];
+			rb.st1[s] = gst[2 * ( first + s ) + 1];
+			rb.flags[s] = -1;
+		}
+		__syncthreads();
+		/* the awake bodies among them, with their awake indices; four of the list at a
+		 * time, and the terms behind it: one round trip each */
+		constexpr int U = 4;
+		for ( int i0 = tid; i0 < P.awakeCount; i0 += U * T )
+		{
+			int s[U];
+#pragma unroll
+			for ( int u = 0; u < U; ++u )
+				s[u] = i0 + u * T < P.awakeCount ? W.awake[i0 + u * T] - first : -1;
+#pragma unroll
+			for ( int u = 0; u < U; ++u )
+				if ( s[u] >= 0 && s[u] < bodies )
+				{
+					rb.awake[atomicAdd( &s_awake, 1 )] = s[u];
+					rb.flags[s[u]] = i0 + u * T;
+				}
+		}
+		__syncthreads();
+		for ( int j = tid; j < s_awake; j += T )
+			res_terms( W, rb, rb.awake[j], first + rb.awake[j], sc );
+	};
+	PushBodies PB;
+	if constexpr ( CL == 1 )
 	{
 		const int* mine = BINS ? bins.awake + bin[BIN_INTS - 2] : nullptr;
 		for ( int j = tid; j < bodies; j += T )
@@ -178,27 +221,12 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	}
 	else
 	{
-		bodies = P.bodyIdCount - rank * P.bodyCap;
-		bodies = bodies < 0 ? 0 : ( bodies > P.bodyCap ? P.bodyCap : bodies );
-	}
-	if ( CL > 1 )
-	{
-		const int first = rank * P.bodyCap;
-		for ( int s = tid; s < bodies; s += T )
+		if ( P.pushCap > 0 )
 		{
-			rb.st0[s] = gst[2 * ( first + s )];
-			rb.st1[s] = gst[2 * ( first + s ) + 1];
+			push_carve( smem + P.bodyOffset, P.pushCap, P.bodyCap, PB, rb );
+			push_init( PB, push, P, P.bodyCap, rank );
 		}
-		/* the awake bodies among them, with their awake indices */
-		for ( int i = tid; i < P.awakeCount; i += T )
-		{
-			const int b = W.awake[i], s = b - first;
-			if ( s < 0 || s >= bodies )
-				continue;
-			rb.awake[atomicAdd( &s_awake, 1 )] = s;
-			rb.flags[s] = i;
-			res_terms( W, rb, s, b, sc );
-		}
+		load_owned();
 	}
 	if ( JOINTS )
 	{
@@ -216,14 +244,33 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 			}
 		}
 	}
+	ResBarrier<CL> bar{ nullptr, CL, 0 };
+	bool pushes = false;
+	int* const ovList = rb.awake + P.bodyCap;
+	if constexpr ( CL > 1 )
+	{
+		if ( P.pushCap > 0 )
+		{
+			pushes = push_exchange<JOINTS>( cl, PB, push, P.pushCap, P.bodyCap, S.bodyCapInv, rank, rows, s_joints, share, m, J, ovList,
+											[&]( int owner, int at ) { return *cl.map_shared_rank( rb.flags + at, owner ) >= 0; } );
+			if ( pushes == false )
+			{
+				/* more copies than a CTA can hold: states in their owners' CTAs only */
+				rb = res_carve_bodies( smem + P.bodyOffset, P.bodyCap );
+				if ( tid == 0 )
+					s_awake = 0;
+				__syncthreads();
+				load_owned();
+			}
+		}
+	}
 	const int ovRows = cs[B2G_COLORS] - cs[B2G_OVERFLOW], ovJoints = JOINTS ? js[B2G_COLORS] - js[B2G_OVERFLOW] : 0;
 	ResOverflow ov = res_carve_overflow( smem + P.ovOffset, P.ovOffset ? ovRows : 0, P.ovOffset ? ovJoints : 0 );
-	if ( CL > 1 && rank == 0 && P.ovOffset )
+	if ( CL > 1 && rank == 0 && P.ovOffset && pushes == false )
 	{
 		__syncthreads();
 		res_index_overflow<CT, JOINTS>( ov, m, J, share[B2G_OVERFLOW], ovJoints, ovRows, &s_ovSlots );
 	}
-	ResBarrier<CL> bar{ nullptr, CL, 0 };
 	bar.sync();
 	const int awake = s_awake;
 	if constexpr ( CL == 1 )
@@ -233,6 +280,8 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		B.st1 = rb.st1;
 		res_run<CL, CT, true, JOINTS, BINS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 	}
+	else if ( pushes )
+		push_run<CT, JOINTS>( P, share, m, J, PB, push, rb, awake, rank, ovList, sc );
 	else
 	{
 		DsmemBodies B{ { cl, rb.st0, rb.st1, P.bodyCap, rank, S.bodyCapInv } };
@@ -262,6 +311,8 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		finalize_state( W, i, b, rb.st0[s], rb.st1[s], sc );
 	}
 	bar.sync();
+	if ( CL > 1 && pushes && tid == 0 && push.gaveUp )
+		W.hostCounters[2] = 1;
 	if ( rank == 0 && tid == 0 )
 	{
 		bool last = true;
@@ -419,21 +470,38 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 	P.rowCap = 1;
 	for ( int o = 0; o < CL; ++o )
 		P.rowCap = perCta[o] > P.rowCap ? perCta[o] : P.rowCap;
-	size_t bytes = ( 144u * (size_t)P.rowCap + RES_BODY_BYTES * (size_t)P.bodyCap + 15 ) / 16 * 16;
+	/* rows, joints while they fit, then the bodies with the overflow cache or, in their
+	 * place, the copies of push_run: as many as there is room for */
+	const size_t rowBytes = 144u * (size_t)P.rowCap;
+	const size_t bodyBytes = ( RES_BODY_BYTES * (size_t)P.bodyCap + 15 ) / 16 * 16;
+	size_t bytes = rowBytes + bodyBytes;
 	if ( bytes > RES_SMEM_MAX )
 		return 0;
+	size_t ovBytes = 0;
 	if ( ovR + ovJ > 0 && ovR + ovJ <= RES_OVERFLOW_MAX && bytes + res_overflow_bytes( ovR, ovJ ) <= RES_SMEM_MAX )
-	{
-		P.ovOffset = (int)( bytes / 16 );
-		bytes = ( bytes + res_overflow_bytes( ovR, ovJ ) + 15 ) / 16 * 16;
-	}
-	if ( bytes + RES_JOINT_BYTES * (size_t)P.jointCap <= RES_SMEM_MAX )
-	{
-		P.jointOffset = (int)( bytes / 16 );
-		bytes += RES_JOINT_BYTES * (size_t)P.jointCap;
-	}
+		ovBytes = ( res_overflow_bytes( ovR, ovJ ) + 15 ) / 16 * 16;
+	bytes += ovBytes;
+	size_t jointBytes = ( RES_JOINT_BYTES * (size_t)P.jointCap + 15 ) / 16 * 16;
+	if ( bytes + jointBytes <= RES_SMEM_MAX )
+		P.jointOffset = (int)( rowBytes / 16 );
 	else
+	{
 		P.jointCap = 0;
+		jointBytes = 0;
+	}
+	bytes += jointBytes;
+	P.bodyOffset = (int)( ( rowBytes + jointBytes ) / 16 );
+	if ( ovBytes > 0 )
+		P.ovOffset = P.bodyOffset + (int)( bodyBytes / 16 );
+	const size_t fixed = rowBytes + jointBytes + PUSH_OWNED_BYTES * (size_t)P.bodyCap + 8u * (size_t)( ovR + ovJ );
+	if ( ( joints == 0 || jointBytes > 0 ) && fixed + PUSH_COPY_BYTES * (size_t)P.bodyCap <= RES_SMEM_MAX )
+	{
+		size_t cap = ( RES_SMEM_MAX - fixed ) / PUSH_COPY_BYTES;
+		P.pushCap = cap < (size_t)P.bodyIdCount ? (int)cap : P.bodyIdCount;
+		P.pushCap = P.pushCap < P.bodyCap ? P.bodyCap : P.pushCap;
+		const size_t need = fixed + PUSH_COPY_BYTES * (size_t)P.pushCap;
+		bytes = need > bytes ? need : bytes;
+	}
 	cudaLaunchAttribute attr[1];
 	cudaLaunchConfig_t cfg = fused_config( attr, CL, bytes, (cudaStream_t)w->stream );
 	FusedKernel k = joints > 0 ? k_solve_world<FUSED_CLUSTER, true> : k_solve_world<FUSED_CLUSTER, false>;

@@ -1464,6 +1464,8 @@ void gstep_finish( gWorld* w )
 	w->profile.solve = (float)( t3 - w->stepStart );
 	int recordCount = w->io.counters[1];
 	w->lastRecordCount = recordCount;
+	if ( w->io.counters[2] != 0 )
+		w->status = -1; /* a solver CTA gave up waiting for another */
 	report_hits( w );
 	double tr = b2g_now_ms();
 	/* records reach the host through mapped memory: 48 bytes, 80 for fast shapes */

@@ -102,6 +102,20 @@ def test_world_stage_spaces(gpu, oracle, scene, size, steps):
     assert bad is None, detail
 
 
+# a cluster's body copies: they fit (100, 111), do not fit beside the rows (113), are not
+# tried (115, 117), the world does not fit a cluster (119); bodies mixed over all CTAs,
+# overflow rows and a joint (tumbler)
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene,size,steps", [("pyramid", 100, 6), ("pyramid", 111, 3), ("pyramid", 113, 3), ("pyramid", 115, 3), ("pyramid", 117, 3),
+                                              ("pyramid", 119, 3), ("tumbler", 1500, 40)])
+def test_cluster_copies(gpu, oracle, scene, size, steps):
+    def make(b):
+        return b.pyramid(size, 0.01, 3) if scene == "pyramid" else b.tumbler(size, 5, 0)
+
+    bad, detail, _ = lockstep(gpu, oracle, make, steps, check_manifolds=True)
+    assert bad is None, detail
+
+
 # worlds that one CTA does not hold, of islands that it does: rows, joints of every type
 # and overflow sets in bins of islands, and steps with events in between, which run
 # without them; then one island too large for a bin
