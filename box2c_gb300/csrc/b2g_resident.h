@@ -34,6 +34,7 @@ struct ResidentPlan
 	int jointOffset; /* float4 offset of the joint slots */
 	int bodyOffset;	 /* float4 offset of a cluster's body slots */
 	int pushCap;	 /* body copies per CTA (0: no copies) */
+	int pushBytes;	 /* caller buffers, whose copies the kernel counts: their shared memory */
 	int ovOffset; /* float4 offset of the overflow cache, 0 without one */
 };
 

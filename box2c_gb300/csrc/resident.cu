@@ -13,8 +13,10 @@
  *   CL == 1   one CTA: rows and body states in its shared memory, __syncthreads between
  *             sweeps.
  *   CL > 1    a thread-block cluster of CL CTAs: rows in the shared memory of the CTA
- *             that solves them, body b in CTA b / block, reached through distributed
- *             shared memory; hardware cluster barriers.
+ *             that solves them, body b in CTA b / block with copies in the CTAs whose
+ *             rows touch it, which updates are pushed to (b2g_push.h); where the copies
+ *             do not fit, reached through distributed shared memory, with hardware
+ *             cluster barriers.
  *   CL == 0   a cooperative grid of up to one CTA per SM: rows in shared memory while
  *             they fit (in the world's row arrays otherwise), body states in global
  *             memory read and written at L2; a counter barrier in global memory, every
@@ -30,12 +32,14 @@
  * the same bits.
  *
  * What bounds it: the chain of sweeps.  Per sweep 0.33 us in one CTA (0.5 us at 200 rows
- * a colour, where shared-memory bandwidth shows), 0.75 to 1 us in a cluster, 2 us in a
+ * a colour), 0.6 us in a cluster with body copies and 0.75 to 1 us without, 2 us in a
  * grid (an L2 round trip to arrive and one to see it).  b2SolveContacts, one kernel per
  * phase before and one resident kernel now, four substeps: 900 contacts 420 -> 52 us (a
- * cluster takes 82), 15000 420 -> 102 (a grid takes 199), 60000 424 -> 207; with 17
- * overflow rows at 15000 contacts 799 -> 185.
+ * cluster without copies takes 82), 15000 420 -> 102 without copies (a grid takes 199),
+ * 60000 424 -> 207; with 17 overflow rows at 15000 contacts 799 -> 185, with body copies
+ * 162.
  */
+#include "b2g_push.h"
 #include "b2g_resident.h"
 
 #include <string.h>
@@ -51,6 +55,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	extern __shared__ float4 smem[];
 	__shared__ ResShare share[B2G_COLORS];
 	__shared__ int s_rows, s_awake, s_top, s_ovSlots;
+	__shared__ PushShared push;
 	cg::cluster_group cl = cg::this_cluster();
 	const int rank = CL == 1 ? 0 : (int)cl.block_rank();
 	const int tid = threadIdx.x;
@@ -120,56 +125,97 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	ResBarrier<CL> bar{ nullptr, CL, 0 };
 	const ResJoints J{};
 	ResOverflow ov = res_carve_overflow( smem + P.ovOffset, P.ovOffset ? cs[B2G_COLORS] - cs[B2G_OVERFLOW] : 0, 0 );
-	if ( CL > 1 && rank == 0 && P.ovOffset )
-	{
-		res_index_overflow<T, false>( ov, m, J, share[B2G_OVERFLOW], 0, cs[B2G_COLORS] - cs[B2G_OVERFLOW], &s_ovSlots );
-		__syncthreads();
-	}
+	auto index_overflow = [&]() {
+		if ( CL > 1 && rank == 0 && P.ovOffset )
+		{
+			res_index_overflow<T, false>( ov, m, J, share[B2G_OVERFLOW], 0, cs[B2G_COLORS] - cs[B2G_OVERFLOW], &s_ovSlots );
+			__syncthreads();
+		}
+	};
 	const int ids = top + 1;
 	const int block = ids > 0 ? ( ids + CL - 1 ) / CL : 1;
 	/* owners by a multiply-high with ceil(2^32 / block): exact for ids below 2^16 */
 	if ( block <= P.bodyCap && ids < 65536 )
 	{
 		const unsigned inv = block > 1 ? (unsigned)( ( ( 1ull << 32 ) + (unsigned)block - 1 ) / (unsigned)block ) : 0u;
-		DsmemBodies D{ { cl, rb.st0, rb.st1, block, rank, inv } };
+		const int owned = min( block, ids - rank * block );
 		auto place = [&]( int b, int& r, int& s ) {
 			r = CL == 1 ? 0 : ( block == 1 ? b : (int)__umulhi( (unsigned)b, inv ) );
 			s = b - r * block;
 		};
 		auto there = [&]( int* p, int r ) { return CL == 1 ? p : cl.map_shared_rank( p, r ); };
-		for ( int k = tid; k < rows; k += T )
-		{
-			int4 ix = m.idx[k];
-			int r, s;
-			if ( ix.x >= 0 )
+		auto mark_and_load = [&]() {
+			for ( int k = tid; k < rows; k += T )
 			{
-				place( ix.x, r, s );
-				atomicOr( there( rb.flags + s, r ), RES_TOUCHED );
+				int4 ix = m.idx[k];
+				int r, s;
+				if ( ix.x >= 0 )
+				{
+					place( ix.x, r, s );
+					atomicOr( there( rb.flags + s, r ), RES_TOUCHED );
+				}
+				if ( ix.y >= 0 )
+				{
+					place( ix.y, r, s );
+					atomicOr( there( rb.flags + s, r ), RES_TOUCHED );
+				}
 			}
-			if ( ix.y >= 0 )
+			/* the listed bodies to their owners' lists, each once */
+			for ( int i = af + tid; i < al; i += T )
 			{
-				place( ix.y, r, s );
-				atomicOr( there( rb.flags + s, r ), RES_TOUCHED );
+				int b = W.awake[i];
+				if ( b < 0 )
+					continue;
+				int r, s;
+				place( b, r, s );
+				if ( atomicOr( there( rb.flags + s, r ), RES_AWAKE ) & RES_AWAKE )
+					continue;
+				*there( rb.awake + atomicAdd( there( &s_awake, r ), 1 ), r ) = s;
+			}
+			for ( int s = tid; s < owned; s += T )
+			{
+				int b = rank * block + s;
+				rb.st0[s] = gst[2 * b];
+				rb.st1[s] = gst[2 * b + 1];
+			}
+		};
+		auto clear = [&]() {
+			for ( int s = tid; s < block; s += T )
+				rb.flags[s] = 0;
+			if ( tid == 0 )
+				s_awake = 0;
+		};
+		/* a cluster whose CTAs can hold copies of the bodies that their rows touch; states
+		 * in their owners' CTAs only where they cannot */
+		bool pushes = false;
+		PushBodies PB;
+		int* ovList = nullptr;
+		if constexpr ( CL > 1 )
+		{
+			const int space = P.pushBytes - PUSH_OWNED_BYTES * block - 8 * ( cs[B2G_COLORS] - cs[B2G_OVERFLOW] );
+			const int cap = min( space / PUSH_COPY_BYTES, 65535 );
+			if ( space > 0 && cap > block )
+			{
+				push_carve( smem + 9 * P.rowCap, cap, block, PB, rb );
+				push_init( PB, push, P, block, rank );
+				ovList = rb.awake + block;
+				clear();
+				cl.sync();
+				mark_and_load();
+				pushes = push_exchange<false>( cl, PB, push, cap, block, inv, rank, rows, 0, share, m, J, ovList,
+											   [&]( int owner, int at ) { return ( *cl.map_shared_rank( rb.flags + at, owner ) & RES_AWAKE ) != 0; } );
+				if ( pushes == false )
+				{
+					rb = res_carve_bodies( smem + 9 * P.rowCap, P.bodyCap );
+					clear();
+					cl.sync();
+				}
 			}
 		}
-		/* the listed bodies to their owners' lists, each once */
-		for ( int i = af + tid; i < al; i += T )
+		if ( pushes == false )
 		{
-			int b = W.awake[i];
-			if ( b < 0 )
-				continue;
-			int r, s;
-			place( b, r, s );
-			if ( atomicOr( there( rb.flags + s, r ), RES_AWAKE ) & RES_AWAKE )
-				continue;
-			*there( rb.awake + atomicAdd( there( &s_awake, r ), 1 ), r ) = s;
-		}
-		const int owned = min( block, ids - rank * block );
-		for ( int s = tid; s < owned; s += T )
-		{
-			int b = rank * block + s;
-			rb.st0[s] = gst[2 * b];
-			rb.st1[s] = gst[2 * b + 1];
+			index_overflow();
+			mark_and_load();
 		}
 		bar.sync();
 		const int awake = s_awake;
@@ -183,12 +229,23 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 			/* a thread's terms are its own: no barrier before the first integration */
 			res_run<CL, T, true, false>( P, share, m, J, LB, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 		}
+		else if ( pushes )
+		{
+			push_run<T, false>( P, share, m, J, PB, push, rb, awake, rank, ovList, sc );
+			cl.sync(); /* no CTA ends before what was sent to it, or by it, is there */
+		}
 		else
+		{
+			const DsmemBodies D{ { cl, rb.st0, rb.st1, block, rank, inv } };
 			res_run<CL, T, true, false>( P, share, m, J, D, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
+		}
 		for ( int s = tid; s < owned; s += T )
 		{
 			int b = rank * block + s;
 			int f = rb.flags[s];
+			/* a CTA that gave up on another has no result */
+			if ( CL > 1 && pushes && push.gaveUp )
+				rb.st0[s].x = rb.st0[s].y = rb.st0[s].z = __int_as_float( 0x7fffffff );
 			if ( f )
 				gst[2 * b] = rb.st0[s];
 			if ( f & RES_AWAKE )
@@ -197,6 +254,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	}
 	else
 	{
+		index_overflow();
 		/* states at L2; the terms of this CTA's share of the list as far as they fit */
 		L2Bodies G{ gst };
 		const int n = al - af;
@@ -443,6 +501,11 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 		size_t bytes = rows + RES_BODY_BYTES * (size_t)P.bodyCap;
 		if ( tail )
 			bytes = res_with_overflow( &P, bytes, ovRows );
+		if ( ctas > 1 )
+		{
+			P.pushBytes = RES_SMEM_MAX - (int)rows;
+			bytes = RES_SMEM_MAX;
+		}
 		auto kernel = ctas == 1 ? (ResClusterKernel)k_solve_cluster<1, CLUSTER_THREADS> : (ResClusterKernel)k_solve_cluster<B2G_FUSED_CTAS, CLUSTER_THREADS>;
 		cudaLaunchConfig_t cfg = res_config( attr, ctas, ctas, CLUSTER_THREADS, bytes, s );
 		return cudaLaunchKernelEx( &cfg, kernel, *w, P, *sc ) == cudaSuccess ? 1 : -1;

@@ -56,6 +56,31 @@ def test_resident_solver_matches_oracle(gpu, oracle, scene, stride):
     assert np.array_equal(manifolds, cap["manifoldsOut"])
 
 
+# contacts in random order within their colours: a cluster's CTAs touch bodies of all
+# others, and their copies fit (60) or do not (100)
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene,stride", [("60", 1), ("100", 1), ("100", 3)])
+def test_resident_solver_mixed_order(gpu, oracle, scene, stride):
+    torch = pytest.importorskip("torch")
+    w, warm = _scene(oracle, scene)
+    oracle.step(w, count=warm)
+    cap = capture_step(oracle, w)
+    oracle.destroy(w)
+    rng = np.random.default_rng(3)
+    starts = cap["colorStart"]
+    order = np.concatenate([rng.permutation(np.arange(a, b)) for a, b in zip(starts[:11], starts[1:12])]
+                           + [np.arange(starts[11], starts[12])]).astype(np.int64)
+    assert len(order) == len(cap["contactBodies"])
+    for k in ("contactBodies", "mix"):
+        cap[k] = cap[k][order]
+    for k in ("manifoldsIn", "manifoldsOut"):
+        cap[k] = cap[k].reshape(len(order), -1)[order].reshape(-1)
+    cap = _spread(cap, stride)
+    states, manifolds = solve_on_device(gpu, torch, cap)
+    assert np.array_equal(states.view(np.uint32), cap["statesOut"].view(np.uint32))
+    assert np.array_equal(manifolds, cap["manifoldsOut"])
+
+
 @pytest.mark.gpu
 def test_resident_solver_captured(gpu, oracle):
     """Both entry points inside a stream capture, replayed twice on the same inputs."""
