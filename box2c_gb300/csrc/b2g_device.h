@@ -169,7 +169,7 @@ typedef struct b2gBatchItem
 	void* tapeBodies; /* adjoint tape destinations, or null when not recording */
 	void* tapeRowDst;
 	int widest;		/* most rows + joints of any colour but the overflow colour */
-	int rowsOnChip; /* 1 when the solver keeps this world's rows in shared memory (set at launch) */
+	int rowsOnChip; /* 1 when the solver keeps all rows of this world in shared memory (set at launch) */
 } b2gBatchItem;
 
 /* Device context of batched steps: pinned staging of items and counters, device copies,

@@ -18,8 +18,8 @@
 #endif
 
 /* Shared-memory image of one world on its solver group: body states (two float4) by
- * body id; after them, for a world that fits, its constraint rows by solve-list
- * position (nine float4 each).  Velocity terms are recomputed every substep from the
+ * body id; after them its constraint rows by solve-list position (nine float4 each), for
+ * a world that does not fit the last ones.  Velocity terms are recomputed every substep from the
  * body's mass, force and extent rather than held, which keeps the image small. */
 B2G_PACK_HD inline int body_float4s( int bodies ) { return 2 * bodies; }
 B2G_PACK_HD inline size_t world_smem_bytes( int bodies, int rows )

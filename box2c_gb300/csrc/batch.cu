@@ -7,8 +7,8 @@
  * queue: worlds of similar size side by side, each on a group of threads (one warp, a
  * named-barrier group or the whole CTA) that runs the world's whole solver stage and
  * finalisation with the group's barrier between the dependent phases.  Body states
- * always live in shared memory; a world whose constraint rows fit beside them keeps the
- * rows there too, a larger one in its own row arrays.  The per-row work is
+ * always live in shared memory; a world keeps as many of its constraint rows beside them
+ * as fit, from the end of the colour-major order, and the others in its row arrays.  The per-row work is
  * b2g_stages.h's and b2g_cluster.h's, the same functions the single-world kernels use,
  * so every world gets the bits it would get from b2World_Step alone.
  *
@@ -136,10 +136,17 @@ __global__ void __launch_bounds__( BATCH_GRID_THREADS ) k_batch_tape( const b2gB
 	}
 }
 
+/* A world on its group: rows [base, rows) of the colour-major order are in shared memory
+ * at k - base, the ones before in the world's row arrays.  A sweep with any row in the
+ * arrays takes about 1 us, one without 0.4: the overflow rows and the small colours come
+ * last in the order, so the split frees as many sweeps of L2 as it can (all rows in the
+ * arrays before, when not all fit: 160 pyramids of 4 to 40 rows 221 -> 194 us, 1024 of
+ * them 800 -> 627). */
 struct WorldImage
 {
 	SharedBodies B;
 	SmemRows m;
+	int base;
 };
 
 /* Asks L2 for rows [first, first + n) of the world's row arrays: one bulk prefetch per
@@ -155,13 +162,14 @@ __device__ __forceinline__ void prefetch_rows( const b2gDevWorld& W, int first, 
 	}
 }
 
-/* One row phase: the row in shared memory (ONCHIP) or in the world's row arrays. */
+/* One row phase: the row in shared memory, or (ONCHIP false only) in the world's row
+ * arrays. */
 template <bool ONCHIP>
 __device__ __forceinline__ void world_row( const b2gDevWorld& W, const WorldImage& s, int k, int phase, bool scalar,
 										   const b2gStepConst& sc )
 {
-	if constexpr ( ONCHIP )
-		row_step( s.m, s.B, k, phase, scalar, sc );
+	if ( ONCHIP || k >= s.base )
+		row_step( s.m, s.B, k - ( ONCHIP ? 0 : s.base ), phase, scalar, sc );
 	else
 		row_work( W, s.B, k, phase, scalar, sc );
 }
@@ -224,8 +232,9 @@ __device__ void world_stage( const b2gBatchItem& it, const WorldImage& s, const 
 			if ( G.t == G.g - 1 )
 			{
 				int cn = it.active[a + 1 < it.activeCount ? a + 1 : 0];
-				if ( cs[cn + 1] > cs[cn] )
-					prefetch_rows( W, cs[cn], cs[cn + 1] - cs[cn] );
+				int end = min( cs[cn + 1], s.base );
+				if ( end > cs[cn] )
+					prefetch_rows( W, cs[cn], end - cs[cn] );
 			}
 		}
 		for ( int t = G.t; t < nj + nr; t += G.g )
@@ -245,7 +254,7 @@ __device__ void world_stage( const b2gBatchItem& it, const WorldImage& s, const 
  * ONCHIP the rows are prepared straight into shared memory (reference
  * src/contact_solver.c:597-808) and only their impulses go back to the manifolds. */
 template <int T, bool ONCHIP>
-__device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, float4* sm, const Group& G )
+__device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, float4* sm, int room, const Group& G )
 {
 	const b2gDevWorld& W = it.W;
 	const int tid = G.t;
@@ -255,15 +264,17 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 	WorldImage s;
 	s.B = SharedBodies{ sm, sm + N };
 	float4* rb = sm + body_float4s( N );
+	const int chip = ONCHIP ? rows : min( rows, ( room - body_float4s( N ) ) / 9 );
+	s.base = rows - chip;
 	s.m.idx = (int4*)rb;
-	s.m.nf = rb + rows;
-	s.m.ms = rb + 2 * rows;
-	s.m.anc0 = rb + 3 * rows;
-	s.m.anc1 = rb + 4 * rows;
-	s.m.coef0 = rb + 5 * rows;
-	s.m.coef1 = rb + 6 * rows;
-	s.m.imp0 = rb + 7 * rows;
-	s.m.imp1 = rb + 8 * rows;
+	s.m.nf = rb + chip;
+	s.m.ms = rb + 2 * chip;
+	s.m.anc0 = rb + 3 * chip;
+	s.m.anc1 = rb + 4 * chip;
+	s.m.coef0 = rb + 5 * chip;
+	s.m.coef1 = rb + 6 * chip;
+	s.m.imp0 = rb + 7 * chip;
+	s.m.imp1 = rb + 8 * chip;
 	float4* st0 = s.B.st0;
 	float4* st1 = s.B.st1;
 	float4* gst = (float4*)W.state;
@@ -280,15 +291,10 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 		st1[b] = gst[2 * b + 1];
 	}
 	const int awake = it.awakeCount;
-	if constexpr ( ONCHIP )
-	{
-		prepare_rows( W, s.m, rows, W.solveList, nullptr, []( int k ) { return k; }, tid, step, sc );
-	}
-	else
-	{
-		for ( int k = tid; k < rows; k += step )
-			prepare_contact_row( W, k, sc );
-	}
+	const int base = s.base;
+	for ( int k = tid; k < base; k += step )
+		prepare_contact_row( W, k, sc );
+	prepare_rows( W, s.m, chip, W.solveList, nullptr, [base]( int k ) { return base + k; }, tid, step, sc );
 	const int joints = it.jointStart[B2G_COLORS];
 	for ( int t = tid; t < joints; t += step )
 		prepare_joint( W, t, sc );
@@ -319,15 +325,9 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 	}
 	world_stage<T, ONCHIP>( it, s, G, F_RESTITUTION, sc );
 
-	if constexpr ( ONCHIP )
-	{
-		store_impulses( W, s.m, rows, it.colorStart[B2G_OVERFLOW], tid, step );
-	}
-	else
-	{
-		for ( int k = tid; k < rows; k += step )
-			store_row( W, k, it.colorStart[B2G_OVERFLOW] );
-	}
+	for ( int k = tid; k < base; k += step )
+		store_row( W, k, it.colorStart[B2G_OVERFLOW] );
+	store_impulses( W, s.m, chip, max( it.colorStart[B2G_OVERFLOW] - base, 0 ), tid, step );
 	for ( int i = tid; i < awake; i += step )
 	{
 		int b = W.awake[i];
@@ -371,11 +371,11 @@ __global__ void __launch_bounds__( T, MINB ) k_batch_solve( const b2gBatchItem* 
 			for ( int i = G.t; i < (int)( sizeof( b2gBatchItem ) / 4 ); i += G.g )
 				( (int*)&it )[i] = ( (const int*)( items + w ) )[i];
 			group_sync<T>( G );
-			float4* region = sm + ( smemFloat4 / ( T / G.g ) ) * G.gi;
+			const int room = smemFloat4 / ( T / G.g );
 			if ( it.rowsOnChip )
-				solve_world<T, true>( it, it.sc, region, G );
+				solve_world<T, true>( it, it.sc, sm + room * G.gi, room, G );
 			else
-				solve_world<T, false>( it, it.sc, region, G );
+				solve_world<T, false>( it, it.sc, sm + room * G.gi, room, G );
 		}
 		__syncthreads();
 	}

@@ -204,3 +204,29 @@ def test_read_back_follows_every_step(gpu, oracle):
                 assert np.array_equal(got[both][:, :4].view(np.uint32), full[both][:, :4].view(np.uint32)), (k, step)
         gpu.destroy(w)
         oracle.destroy(o)
+
+
+@pytest.mark.gpu
+def test_batched_rows_beside_the_chip(gpu, oracle):
+    """Batched worlds whose rows fit their group's shared memory, fit it in part (pyramids
+    of 30 rows and more; overflow rows and a joint in the tumbler) and lie in it alone, over
+    every launch shape the first steps try.  Tolerance: none."""
+    from box2c_gb300.capi import bind_batch_api, world_array
+
+    bind_batch_api(gpu.lib)
+
+    def make(b):
+        return [b.pyramid(n, 0.01, 3) for n in (2, 12, 20, 29, 30, 31, 38, 45)] + [b.tumbler(900, 5, 0)]
+
+    batch, alone = make(gpu), make(oracle)
+    ids = world_array(batch)
+    for step in range(24):
+        gpu.lib.b2World_StepBatch(ids, len(batch), 1.0 / 60.0, 4)
+        for w in alone:
+            oracle.step(w)
+    for i, (w, o) in enumerate(zip(batch, alone)):
+        got, want = gpu.bodies(w)[:, :7], oracle.bodies(o)[:, :7]
+        live = np.isfinite(want).all(1)
+        assert np.array_equal(got[live].view(np.uint32), want[live].view(np.uint32)), i
+        gpu.destroy(w)
+        oracle.destroy(o)
