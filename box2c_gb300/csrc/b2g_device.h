@@ -180,7 +180,7 @@ b2gBatch* b2gd_batch_create( void );
 void b2gd_batch_destroy( b2gBatch* b );
 /* Grows the item and counter buffers; returns the pinned item array or null. */
 b2gBatchItem* b2gd_batch_items( b2gBatch* b, int count );
-void* b2gd_batch_stream( b2gBatch* b );
+void* b2gd_batch_stream( b2gBatch* b, int half );
 /* Worlds with more body ids than this are stepped alone (b2World_Step) by the batch. */
 int b2gd_batch_max_bodies( void );
 /* Host copy of world i's 4 counters after the last sync. */

@@ -5,8 +5,9 @@
  *
  * The host work of each world is the single-world step's, phase by phase (step.c:
  * gstep_begin, gstep_rebuild_trees, gstep_after_collide, gstep_finish); only the device
- * launches are shared.  While the batch runs, every world's uploads go to the batch's
- * stream, so they are ordered before the graphs that read them.
+ * launches are shared.  While the batch runs, every world's uploads go to the stream of
+ * its half of the batch, so they are ordered before the graphs that read them; both
+ * streams are idle when the call returns.
  */
 #include "host.h"
 
@@ -230,7 +231,7 @@ void b2World_StepBatch( const b2WorldId* worldIds, int count, float timeStep, in
 	for ( int h = 0; h < 2; ++h )
 	{
 		c[h].items = items;
-		c[h].stream = b2gd_batch_stream( s_batch );
+		c[h].stream = b2gd_batch_stream( s_batch, h );
 		c[h].timeStep = timeStep;
 		c[h].subStepCount = subStepCount;
 		c[h].first = h == 0 ? 0 : split;

@@ -12,9 +12,11 @@
  * b2g_stages.h's and b2g_cluster.h's, the same functions the single-world kernels use,
  * so every world gets the bits it would get from b2World_Step alone.
  *
- * A step's worlds run in two halves, each with its own graphs (uploads, kernels,
- * counter download), captured once and replayed every step, so that the host work of
- * one half overlaps the device work of the other; the kernels read their counts from
+ * A step's worlds run in two halves, each with its own stream and graphs (uploads,
+ * kernels, counter download), captured once and replayed every step, so that the host
+ * work of one half overlaps the device work of the other, and the halves share the
+ * device: a half's solver runs as long as its largest world, with SMs idle (1024
+ * pyramids of 4 to 40 rows, a step: 965 us on one stream, 803 on two); the kernels read their counts from
  * device memory, so the graphs do not change while the number of worlds and the
  * shared-memory size stay the same.  The solver's launch shape (threads per CTA, CTAs
  * per SM and so shared memory per world) is chosen by timing the candidates on the
@@ -48,6 +50,7 @@
  * timing events, so that the host phases of one half overlap the other's device work. */
 struct BatchHalf
 {
+	cudaStream_t stream;
 	int* hPrefix; /* scatter prefix [n+1], then narrowphase prefix [n+1] */
 	int* dPrefix;
 	int* hOrder; /* [0] = packs to solve, then PACK_INTS ints per pack; then scratch */
@@ -63,12 +66,12 @@ struct BatchHalf
 	int solveN[TUNE_CANDIDATES];
 	int solveSmem[TUNE_CANDIDATES];
 	int solvePerSm[TUNE_CANDIDATES]; /* resident CTAs per SM of each captured launch */
+	int used; /* this step has worlds in the half */
 	int collideTimed, solveTimed;
 };
 
 struct b2gBatch
 {
-	cudaStream_t stream;
 	int capacity;
 	b2gBatchItem* hItems;
 	b2gBatchItem* dItems;
@@ -399,9 +402,9 @@ static int solve_occupancy( size_t smem )
 }
 
 template <int T, int MINB>
-static void launch_solve( b2gBatch* b, int grid, size_t smem, const int* packs, int* queue )
+static void launch_solve( b2gBatch* b, cudaStream_t stream, int grid, size_t smem, const int* packs, int* queue )
 {
-	k_batch_solve<T, MINB><<<grid, T, smem, b->stream>>>( b->dItems, packs, queue, (int)( smem / 16u ) );
+	k_batch_solve<T, MINB><<<grid, T, smem, stream>>>( b->dItems, packs, queue, (int)( smem / 16u ) );
 }
 
 /* Solver launch shapes tried on the first steps: threads per CTA and CTAs per SM (which
@@ -410,7 +413,7 @@ struct TuneCandidate
 {
 	int threads, perSM;
 	int ( *occupancy )( size_t smem );
-	void ( *launch )( b2gBatch* b, int grid, size_t smem, const int* packs, int* queue );
+	void ( *launch )( b2gBatch* b, cudaStream_t stream, int grid, size_t smem, const int* packs, int* queue );
 };
 #define TUNE_SHAPE( T, B ) { T, B, solve_occupancy<T, B>, launch_solve<T, B> }
 static const TuneCandidate s_tune[TUNE_CANDIDATES] = { TUNE_SHAPE( 128, 6 ), TUNE_SHAPE( 512, 1 ), TUNE_SHAPE( 128, 8 ),
@@ -422,11 +425,14 @@ extern "C" b2gBatch* b2gd_batch_create( void )
 	b2gBatch* b = (b2gBatch*)b2g_calloc( 1, sizeof( b2gBatch ) );
 	if ( b == nullptr )
 		return nullptr;
-	if ( cudaStreamCreateWithFlags( &b->stream, cudaStreamNonBlocking ) != cudaSuccess )
-	{
-		b2g_free( b );
-		return nullptr;
-	}
+	for ( int h = 0; h < B2G_BATCH_HALVES; ++h )
+		if ( cudaStreamCreateWithFlags( &b->half[h].stream, cudaStreamNonBlocking ) != cudaSuccess )
+		{
+			for ( int k = 0; k < h; ++k )
+				cudaStreamDestroy( b->half[k].stream );
+			b2g_free( b );
+			return nullptr;
+		}
 	int dev = 0;
 	cudaGetDevice( &dev );
 	cudaDeviceGetAttribute( &b->sms, cudaDevAttrMultiProcessorCount, dev );
@@ -437,6 +443,17 @@ extern "C" b2gBatch* b2gd_batch_create( void )
 		cudaMalloc( &b->half[h].dQueue, sizeof( int ) );
 	}
 	return b;
+}
+
+static cudaError_t sync_streams( b2gBatch* b )
+{
+	cudaError_t e = cudaSuccess;
+	for ( int h = 0; h < B2G_BATCH_HALVES; ++h )
+	{
+		cudaError_t one = cudaStreamSynchronize( b->half[h].stream );
+		e = e == cudaSuccess ? one : e;
+	}
+	return e;
 }
 
 static void release_graphs( b2gBatch* b )
@@ -481,16 +498,16 @@ extern "C" void b2gd_batch_destroy( b2gBatch* b )
 {
 	if ( b == nullptr )
 		return;
-	cudaStreamSynchronize( b->stream );
+	sync_streams( b );
 	release_graphs( b );
 	release_buffers( b );
 	for ( int h = 0; h < B2G_BATCH_HALVES; ++h )
 	{
+		cudaStreamDestroy( b->half[h].stream );
 		cudaFree( b->half[h].dQueue );
 		for ( int i = 0; i < 4; ++i )
 			cudaEventDestroy( b->half[h].ev[i] );
 	}
-	cudaStreamDestroy( b->stream );
 	b2g_free( b );
 }
 
@@ -498,7 +515,7 @@ extern "C" b2gBatchItem* b2gd_batch_items( b2gBatch* b, int count )
 {
 	if ( count <= b->capacity )
 		return b->hItems;
-	cudaStreamSynchronize( b->stream );
+	sync_streams( b );
 	release_graphs( b );
 	release_buffers( b );
 	int cap = count < 64 ? 64 : count;
@@ -526,7 +543,7 @@ extern "C" b2gBatchItem* b2gd_batch_items( b2gBatch* b, int count )
 	return b->hItems;
 }
 
-extern "C" void* b2gd_batch_stream( b2gBatch* b ) { return (void*)b->stream; }
+extern "C" void* b2gd_batch_stream( b2gBatch* b, int h ) { return (void*)b->half[h].stream; }
 
 /* Largest body-id count the batched solver holds (bodies in shared memory, 32 bytes each,
  * rounded up to 256 ids). */
@@ -569,7 +586,7 @@ extern "C" void b2gd_batch_begin_step( b2gBatch* b )
 	b->choice = b->tuned ? b->choice : b->tuneStep % TUNE_CANDIDATES;
 	b->launches = 0;
 	for ( int h = 0; h < B2G_BATCH_HALVES; ++h )
-		b->half[h].collideTimed = b->half[h].solveTimed = 0;
+		b->half[h].used = b->half[h].collideTimed = b->half[h].solveTimed = 0;
 }
 
 extern "C" int b2gd_batch_collide( b2gBatch* b, int h, int first, int n )
@@ -577,6 +594,7 @@ extern "C" int b2gd_batch_collide( b2gBatch* b, int h, int first, int n )
 	if ( n <= 0 )
 		return 0;
 	BatchHalf& H = b->half[h];
+	H.used = 1;
 	point_counters( b, first, n );
 	int* ps = H.hPrefix;
 	int* pc = H.hPrefix + n + 1;
@@ -595,23 +613,23 @@ extern "C" int b2gd_batch_collide( b2gBatch* b, int h, int first, int n )
 		int grid = b->sms * 8;
 		const b2gBatchItem* items = b->dItems + first;
 		cudaGetLastError();
-		cudaStreamBeginCapture( b->stream, cudaStreamCaptureModeThreadLocal );
-		cudaMemcpyAsync( b->dItems + first, b->hItems + first, sizeof( b2gBatchItem ) * n, cudaMemcpyHostToDevice, b->stream );
-		cudaMemcpyAsync( H.dPrefix, H.hPrefix, sizeof( int ) * 2 * ( n + 1 ), cudaMemcpyHostToDevice, b->stream );
-		cudaMemsetAsync( b->dCounters + 4 * first, 0, sizeof( int ) * 4 * n, b->stream );
-		k_batch_scatter<<<grid, BATCH_GRID_THREADS, 0, b->stream>>>( items, H.dPrefix, n );
-		k_batch_collide<<<grid, BATCH_GRID_THREADS, 0, b->stream>>>( items, H.dPrefix + n + 1, n );
+		cudaStreamBeginCapture( H.stream, cudaStreamCaptureModeThreadLocal );
+		cudaMemcpyAsync( b->dItems + first, b->hItems + first, sizeof( b2gBatchItem ) * n, cudaMemcpyHostToDevice, H.stream );
+		cudaMemcpyAsync( H.dPrefix, H.hPrefix, sizeof( int ) * 2 * ( n + 1 ), cudaMemcpyHostToDevice, H.stream );
+		cudaMemsetAsync( b->dCounters + 4 * first, 0, sizeof( int ) * 4 * n, H.stream );
+		k_batch_scatter<<<grid, BATCH_GRID_THREADS, 0, H.stream>>>( items, H.dPrefix, n );
+		k_batch_collide<<<grid, BATCH_GRID_THREADS, 0, H.stream>>>( items, H.dPrefix + n + 1, n );
 		cudaError_t launch = cudaGetLastError();
-		cudaMemcpyAsync( b->hCounters + 4 * first, b->dCounters + 4 * first, sizeof( int ) * 4 * n, cudaMemcpyDeviceToHost, b->stream );
-		cudaError_t e = finish_capture( b->stream, launch, &H.collideExec );
+		cudaMemcpyAsync( b->hCounters + 4 * first, b->dCounters + 4 * first, sizeof( int ) * 4 * n, cudaMemcpyDeviceToHost, H.stream );
+		cudaError_t e = finish_capture( H.stream, launch, &H.collideExec );
 		if ( e != cudaSuccess )
 			return (int)e;
 		H.collideN = n;
 		H.collideFirst = first;
 	}
-	cudaEventRecord( H.ev[0], b->stream );
-	cudaError_t e = cudaGraphLaunch( H.collideExec, b->stream );
-	cudaEventRecord( H.ev[1], b->stream );
+	cudaEventRecord( H.ev[0], H.stream );
+	cudaError_t e = cudaGraphLaunch( H.collideExec, H.stream );
+	cudaEventRecord( H.ev[1], H.stream );
 	H.collideTimed = 1;
 	b->launches += 2;
 	return (int)e;
@@ -652,24 +670,24 @@ extern "C" int b2gd_batch_solve( b2gBatch* b, int h, int first, int n )
 		H.solvePerSm[choice] = occ;
 		int grid = b->sms * occ;
 		cudaGetLastError();
-		cudaStreamBeginCapture( b->stream, cudaStreamCaptureModeThreadLocal );
-		cudaMemcpyAsync( b->dItems + first, b->hItems + first, sizeof( b2gBatchItem ) * n, cudaMemcpyHostToDevice, b->stream );
-		cudaMemcpyAsync( H.dOrder, H.hOrder, sizeof( int ) * ( 1 + PACK_INTS * (size_t)n ), cudaMemcpyHostToDevice, b->stream );
-		cudaMemsetAsync( H.dQueue, 0, sizeof( int ), b->stream );
-		k_batch_tape<<<b->sms * 4, BATCH_GRID_THREADS, 0, b->stream>>>( b->dItems + first, n );
-		tc.launch( b, grid, smem, H.dOrder, H.dQueue );
+		cudaStreamBeginCapture( H.stream, cudaStreamCaptureModeThreadLocal );
+		cudaMemcpyAsync( b->dItems + first, b->hItems + first, sizeof( b2gBatchItem ) * n, cudaMemcpyHostToDevice, H.stream );
+		cudaMemcpyAsync( H.dOrder, H.hOrder, sizeof( int ) * ( 1 + PACK_INTS * (size_t)n ), cudaMemcpyHostToDevice, H.stream );
+		cudaMemsetAsync( H.dQueue, 0, sizeof( int ), H.stream );
+		k_batch_tape<<<b->sms * 4, BATCH_GRID_THREADS, 0, H.stream>>>( b->dItems + first, n );
+		tc.launch( b, H.stream, grid, smem, H.dOrder, H.dQueue );
 		cudaError_t launch = cudaGetLastError();
-		cudaMemcpyAsync( b->hCounters + 4 * first, b->dCounters + 4 * first, sizeof( int ) * 4 * n, cudaMemcpyDeviceToHost, b->stream );
-		cudaError_t e = finish_capture( b->stream, launch, &H.solveExec[choice] );
+		cudaMemcpyAsync( b->hCounters + 4 * first, b->dCounters + 4 * first, sizeof( int ) * 4 * n, cudaMemcpyDeviceToHost, H.stream );
+		cudaError_t e = finish_capture( H.stream, launch, &H.solveExec[choice] );
 		if ( e != cudaSuccess )
 			return (int)e;
 		H.solveN[choice] = n;
 		H.solveFirst[choice] = first;
 		H.solveSmem[choice] = (int)smem;
 	}
-	cudaEventRecord( H.ev[2], b->stream );
-	cudaError_t e = cudaGraphLaunch( H.solveExec[choice], b->stream );
-	cudaEventRecord( H.ev[3], b->stream );
+	cudaEventRecord( H.ev[2], H.stream );
+	cudaError_t e = cudaGraphLaunch( H.solveExec[choice], H.stream );
+	cudaEventRecord( H.ev[3], H.stream );
 	H.solveTimed = 1;
 	b->launches += 2; /* tape records, solver */
 	return (int)e;
@@ -691,23 +709,42 @@ extern "C" int b2gd_batch_wait_solve( b2gBatch* b, int h )
 
 extern "C" int b2gd_batch_end_step( b2gBatch* b )
 {
-	cudaError_t e = cudaStreamSynchronize( b->stream );
+	cudaError_t e = cudaSuccess;
+	for ( int h = 0; h < B2G_BATCH_HALVES && e == cudaSuccess; ++h )
+		if ( b->half[h].used )
+			e = cudaStreamSynchronize( b->half[h].stream );
 	if ( e != cudaSuccess )
-		return (int)e;
-	float collide = 0.0f, solve = 0.0f;
-	int solved = 0;
-	for ( int h = 0; h < B2G_BATCH_HALVES; ++h )
 	{
-		BatchHalf& H = b->half[h];
-		float ms = 0.0f;
-		if ( H.collideTimed && cudaEventElapsedTime( &ms, H.ev[0], H.ev[1] ) == cudaSuccess )
-			collide += ms;
-		if ( H.solveTimed && cudaEventElapsedTime( &ms, H.ev[2], H.ev[3] ) == cudaSuccess )
-		{
-			solve += ms;
-			solved = 1;
-		}
+		sync_streams( b );
+		return (int)e;
 	}
+	/* a stage's time: what its halves' intervals cover together */
+	float covered[2] = { 0.0f, 0.0f };
+	int solved = 0;
+	for ( int stage = 0; stage < 2; ++stage )
+	{
+		cudaEvent_t from[2], to[2];
+		int n = 0;
+		for ( int h = 0; h < B2G_BATCH_HALVES; ++h )
+			if ( stage == 0 ? b->half[h].collideTimed : b->half[h].solveTimed )
+			{
+				from[n] = b->half[h].ev[2 * stage];
+				to[n++] = b->half[h].ev[2 * stage + 1];
+			}
+		float own[2] = { 0.0f, 0.0f }, gap = 0.0f, end = 0.0f;
+		for ( int k = 0; k < n; ++k )
+			cudaEventElapsedTime( own + k, from[k], to[k] );
+		covered[stage] = own[0] + own[1];
+		if ( n == 2 && cudaEventElapsedTime( &gap, from[0], from[1] ) == cudaSuccess )
+		{
+			/* the second from gap to gap + own[1] of the first's clock */
+			end = fminf( own[0], gap + own[1] ) - fmaxf( 0.0f, gap );
+			covered[stage] -= fmaxf( end, 0.0f );
+		}
+		if ( stage == 1 )
+			solved = n > 0;
+	}
+	const float collide = covered[0], solve = covered[1];
 	b->collideMs = collide;
 	b->solveMs = solve;
 	if ( solved && b->tuned == 0 )
