@@ -254,12 +254,12 @@ def run_tumbler(g, steps=1000, cpu=True):
 
 
 BATCH_WORLDS = 4096
-# DRAM bytes of the solver stage of one large-pyramid step (k_fused_stage 2.35 MB +
-# k_solve_fused 2.76 MB), from the committed ncu capture of the same workload
-SOLVER_DRAM_BYTES = 5.10e6
+# DRAM bytes of the solver stage of one large-pyramid step (k_solve_world), from the
+# committed ncu capture of the same workload
+SOLVER_DRAM_BYTES = 3.66e6
 # DRAM bytes of the batched solver over 2048 of the batched worlds (both halves), from the
 # committed ncu capture of that workload
-BATCH_SOLVE_DRAM_BYTES = 3.33e9
+BATCH_SOLVE_DRAM_BYTES = 0.724e9
 BATCH_SEED = 1237
 
 
@@ -335,8 +335,8 @@ def run_batch(g, steps, warmup, n_worlds=BATCH_WORLDS):
         "gpu_launches_per_step": st.launches,
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": BATCH_SOLVE_DRAM_BYTES * n / 2048,
-                     "traffic_source": "ncu dram__bytes_read+write of k_batch_solve, 2048 worlds (a capture "
-                                       "before the per-group descriptor copy) scaled to the worlds stepped "
+                     "traffic_source": "ncu dram__bytes_read+write of k_batch_solve, 2048 worlds, "
+                                       "scaled to the worlds stepped "
                                        "(profiles/batch_solver_4096_worlds.txt)",
                      "kernel": "k_batch_solve (solver stage + finalisation, both halves)",
                      "algorithmic_bytes_per_step": int(solve_bytes), "peak_kind": peak_kind},
@@ -628,7 +628,7 @@ def run_gpu(args):
                    "settled_solve_ms": round(float(np.mean(settled["solve"])), 4)},
         "scene": {"bodies": n_bodies - 1, "contacts": int(len(contacts)), "touching": int(len(touching)),
                   "colors": list(counters.colorCounts), "l2": "flushed between timed steps (256 MB write)",
-                  "solver": "fused cluster kernel" if rec["fused"] == args.steps else "per-phase kernels"},
+                  "solver": "one-launch solver" if rec["fused"] == args.steps else "per-phase kernels"},
         "stages_ms": {"collide": round(float(np.mean(collide_ms)), 4), "solve": round(solve_dev, 4),
                       "finalize": round(float(np.mean(finalize_ms)), 4)},
         "host_ms": dict(zip(("step", "pairs", "collide_and_events", "solve_and_sync", "records"),
@@ -638,7 +638,7 @@ def run_gpu(args):
                                               [round(float(x), 4) for x in np.mean(np.array(settled["phases"]), 0)]))},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "traffic": SOLVER_DRAM_BYTES,
-                     "traffic_source": "ncu dram__bytes_read+write of k_fused_stage + k_solve_fused, one step "
+                     "traffic_source": "ncu dram__bytes_read+write of k_solve_world, one step "
                                        "(profiles/solver_fused_large_pyramid.txt)",
                      "kernel": "solver stage (prepare..store)",
                      "algorithmic_bytes_per_step": solver_bytes, "peak_kind": peak_kind},

@@ -1,6 +1,6 @@
 /*
  * b2g_solve.h -- per-constraint solver arithmetic shared by the per-phase kernels
- * (kernels.cu) and the fused cluster solver (fused.cu).
+ * (kernels.cu) and the resident solvers (fused.cu, resident.cu, batch.cu).
  *
  * Every routine works on values already loaded into registers: one constraint row
  * (Row) or joint (b2gJointDev), and the two body states it couples (DevState).

@@ -291,7 +291,7 @@ typedef struct b2gDevWorld
 	int timing;
 	int launches;
 	long long h2dBytes, d2hBytes; /* host <-> device bytes of the current step */
-	int fused;	   /* use the fused cluster solver when the world fits on chip */
+	int fused;	   /* use the one-launch solver when the world fits on chip */
 	int fusedUsed; /* the last step's solver stage ran fused */
 	/* set for a solver stage launched before the host has seen the narrowphase's events:
 	 * its kernels return at once when the narrowphase reported any (counters[0] != 0) */

@@ -17,6 +17,9 @@
  * finalize bodies      src/solver.c:165-351 (+ fast-body sweep
  *                      boxes, :787-1105)                           k_finalize
  *
+ * From preparation on, these are the kernels of a world that fits none of the one-launch
+ * solvers (fused.cu), and of caller buffers that fit none (resident.cu).
+ *
  * Within one graph colour no two constraints share a non-static body
  * (src/constraint_graph.c:84-131), so a colour runs fully in parallel and still gives
  * the reference's results bit for bit: one thread owns one constraint row (or joint),

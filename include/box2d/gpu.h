@@ -63,10 +63,10 @@ typedef struct b2DeviceTimes
 B2_API void b2World_EnableDeviceTiming( b2WorldId worldId, bool flag );
 B2_API b2DeviceTimes b2World_GetDeviceTimes( b2WorldId worldId );
 
-/* Solver-stage implementation: one fused launch of a 16-CTA cluster that keeps the
- * world's bodies and constraint rows in shared memory (the default; used whenever the
- * world fits, roughly 20k contacts), or one kernel launch per phase.  Both give
- * bit-identical results. */
+/* Solver-stage implementation: one launch that keeps the world's bodies and constraint
+ * rows in shared memory and finalises the bodies (the default; by one CTA, a 16-CTA
+ * cluster up to roughly 20k contacts, or a CTA per bin of islands for larger worlds whose
+ * islands are small), or one kernel launch per phase.  All give bit-identical results. */
 B2_API void b2World_EnableFusedSolver( b2WorldId worldId, bool flag );
 
 /* Steps `count` independent worlds by one b2World_Step each.  The device work of all of

@@ -56,6 +56,42 @@ def test_resident_solver_matches_oracle(gpu, oracle, scene, stride):
     assert np.array_equal(manifolds, cap["manifoldsOut"])
 
 
+def _tile(cap, copies):
+    """The same set `copies` times over, side by side."""
+    n = len(cap["statesIn"])
+    starts = cap["colorStart"]
+    out = dict(cap)
+    for k in ("statesIn", "statesOut", "mass", "force", "damping"):
+        out[k] = np.concatenate([cap[k]] * copies)
+    out["awake"] = np.concatenate([cap["awake"] + i * n for i in range(copies)]).astype(np.int32)
+    order = np.concatenate([np.arange(a, b) for a, b in zip(starts[:12], starts[1:13]) for _ in range(copies)])
+    shift = np.concatenate([np.full(b - a, i * n) for a, b in zip(starts[:12], starts[1:13]) for i in range(copies)])
+    bodies = cap["contactBodies"][order]
+    out["contactBodies"] = np.where(bodies < 0, -1, bodies + shift[:, None]).astype(np.int32)
+    out["mix"] = cap["mix"][order]
+    for k in ("manifoldsIn", "manifoldsOut"):
+        out[k] = cap[k].reshape(starts[12], -1)[order].reshape(-1)
+    out["colorStart"] = [copies * c for c in starts]
+    return out
+
+
+# a grid's rows in shared memory, and in the row arrays when a CTA's share does not fit
+# (about 240000 contacts)
+@pytest.mark.gpu
+@pytest.mark.parametrize("copies", [2, 5])
+def test_resident_solver_large_sets(gpu, oracle, copies):
+    torch = pytest.importorskip("torch")
+    w, warm = _scene(oracle, "many")
+    oracle.step(w, count=warm)
+    cap = capture_step(oracle, w, body_cap=30000, contact_cap=80000)
+    oracle.destroy(w)
+    cap = _tile(cap, copies)
+    assert (len(cap["contactBodies"]) > 250000) == (copies == 5)
+    states, manifolds = solve_on_device(gpu, torch, cap)
+    assert np.array_equal(states.view(np.uint32), cap["statesOut"].view(np.uint32))
+    assert np.array_equal(manifolds, cap["manifoldsOut"])
+
+
 # contacts in random order within their colours: a cluster's CTAs touch bodies of all
 # others, and their copies fit (60) or do not (100)
 @pytest.mark.gpu
