@@ -277,6 +277,7 @@ typedef struct b2gDevWorld
 	 * hostCounters: the device view of the host's copy, which the kernels write */
 	int* counters;
 	int* hostCounters;
+	int collideLast;   /* the last step's narrowphase launched its kernel (host only) */
 	int countersClean; /* the events and blocks are zero once the stream gets there */
 	int* events;	   /* device view of the mapped event buffer */
 	b2gRecord* records; /* device view of the mapped record buffer */

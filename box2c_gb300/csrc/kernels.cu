@@ -54,6 +54,9 @@ __global__ void k_body_ops( b2gDevWorld W, const int* ops, int n )
  * the kernel. */
 __global__ void __launch_bounds__( BLOCK ) k_collide( b2gDevWorld W, int idCount )
 {
+	/* once every block has started, a solver launched behind this kernel may start on
+	 * what the narrowphase does not write */
+	asm volatile( "griddepcontrol.launch_dependents;" ::: "memory" );
 	int id = blockIdx.x * blockDim.x + threadIdx.x;
 	if ( id < idCount )
 		collide_contact( W, id );
@@ -186,6 +189,7 @@ extern "C" int b2gd_collide( b2gDevWorld* w, b2gHostIO* io, int newCount, int id
 		k_scatter_contacts<<<blocks_for( newCount ), BLOCK, 0, s>>>( *w, w->newContacts, newCount );
 		w->launches += 1;
 	}
+	w->collideLast = idCount > 0;
 	if ( idCount > 0 )
 	{
 		k_collide<<<blocks_for( idCount ), BLOCK, 0, s>>>( *w, idCount );
