@@ -87,7 +87,7 @@ struct ResBodies
 	float4* st1;  /* dp.x dp.y dq.c dq.s */
 	float4* term; /* lvd.x lvd.y avd ld */
 	float* ad;	  /* angular damping factor */
-	int* flags;	  /* RES_AWAKE, RES_TOUCHED */
+	int* flags;	  /* RES_AWAKE, RES_TOUCHED; of a world: awake indices */
 	int* awake;	  /* local awake slots */
 };
 
