@@ -12,8 +12,9 @@
  * b2g_stages.h's and b2g_cluster.h's, the same functions the single-world kernels use,
  * so every world gets the bits it would get from b2World_Step alone.
  *
- * A step's worlds run in two halves, each with its own stream and graphs (uploads,
- * kernels, counter download), captured once and replayed every step, so that the host
+ * A step's worlds run in two halves, each with its own stream and graphs (uploads and
+ * kernels; counts are cleared and written to the host by the kernels, which took a step
+ * of 96 small worlds from 144 to 135 us), captured once and replayed every step, so that the host
  * work of one half overlaps the device work of the other, and the halves share the
  * device: a half's solver runs as long as its largest world, with SMs idle (1024
  * pyramids of 4 to 40 rows, a step: 965 us on one stream, 803 on two); the kernels read their counts from
@@ -56,7 +57,7 @@ struct BatchHalf
 	int* hOrder; /* [0] = packs to solve, then PACK_INTS ints per pack; then scratch */
 	int* dOrder;
 	int* hScratch; /* 5 ints per item */
-	int* dQueue;
+	int* dQueue; /* next pack, finished narrowphase blocks */
 	cudaEvent_t ev[4]; /* narrowphase start / end, solver start / end */
 
 	cudaGraphExec_t collideExec;
@@ -77,6 +78,7 @@ struct b2gBatch
 	b2gBatchItem* dItems;
 	int* hCounters; /* 4 per item */
 	int* dCounters;
+	int* dHostCounters; /* hCounters as the device sees it */
 	int sms;
 	BatchHalf half[B2G_BATCH_HALVES];
 
@@ -102,9 +104,16 @@ __device__ __forceinline__ int find_world( const int* prefix, int n, int t )
 	return lo;
 }
 
-__global__ void __launch_bounds__( BATCH_GRID_THREADS ) k_batch_scatter( const b2gBatchItem* items, const int* prefix, int n )
+/* Contact creation; it also clears what the half's other kernels count in, which saves
+ * two memset nodes: the worlds' counters, the pack queue and the finished blocks. */
+__global__ void __launch_bounds__( BATCH_GRID_THREADS ) k_batch_scatter( const b2gBatchItem* items, const int* prefix, int n, int* counters,
+																		 int* queue )
 {
 	int total = prefix[n];
+	for ( int t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * n; t += gridDim.x * blockDim.x )
+		counters[t] = 0;
+	if ( blockIdx.x == 0 && threadIdx.x < 2 )
+		queue[threadIdx.x] = 0;
 	for ( int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x )
 	{
 		int w = find_world( prefix, n, t );
@@ -115,14 +124,28 @@ __global__ void __launch_bounds__( BATCH_GRID_THREADS ) k_batch_scatter( const b
 
 /* Four CTAs an SM (64 registers, a few spilled) beat two (128, none) on a full machine:
  * 240 us against 260 for 1024 pyramids; for a hundred small worlds two are 3 us faster. */
-__global__ void __launch_bounds__( BATCH_GRID_THREADS, 4 ) k_batch_collide( const b2gBatchItem* items, const int* prefix, int n )
+__global__ void __launch_bounds__( BATCH_GRID_THREADS, 4 ) k_batch_collide( const b2gBatchItem* items, const int* prefix, int n, const int* counters,
+																			int* hostCounters, int* finished )
 {
+	__shared__ int s_last;
 	int total = prefix[n];
 	for ( int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x )
 	{
 		int w = find_world( prefix, n, t );
 		collide_contact( items[w].W, t - prefix[w] );
 	}
+	/* the last block writes the worlds' event counts to the host, which saves a copy node */
+	__syncthreads();
+	if ( threadIdx.x == 0 )
+	{
+		__threadfence();
+		s_last = atomicAdd( finished, 1 ) == (int)gridDim.x - 1;
+		__threadfence();
+	}
+	__syncthreads();
+	if ( s_last )
+		for ( int i = threadIdx.x; i < n; i += blockDim.x )
+			hostCounters[4 * i] = __ldcg( counters + 4 * i );
 }
 
 /* Adjoint tape records of the worlds that are recording (one CTA per world in turn). */
@@ -283,11 +306,6 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 	float4* gst = (float4*)W.state;
 	const float4* mass = (const float4*)W.mass;
 
-	if ( tid == 0 )
-	{
-		W.counters[1] = 0;
-		W.counters[3] = 0;
-	}
 	for ( int b = tid; b < N; b += step )
 	{
 		st0[b] = gst[2 * b];
@@ -340,6 +358,13 @@ __device__ void solve_world( const b2gBatchItem& it, const b2gStepConst& sc, flo
 	group_sync<T>( G );
 	for ( int i = tid; i < awake; i += step )
 		finalize_body( W, i, sc );
+	/* the counts of records and sleepy bodies to the host */
+	group_sync<T>( G );
+	if ( tid == 0 )
+	{
+		W.hostCounters[1] = __ldcg( W.counters + 1 );
+		W.hostCounters[3] = __ldcg( W.counters + 3 );
+	}
 }
 
 
@@ -440,7 +465,7 @@ extern "C" b2gBatch* b2gd_batch_create( void )
 	{
 		for ( int i = 0; i < 4; ++i )
 			cudaEventCreate( &b->half[h].ev[i] );
-		cudaMalloc( &b->half[h].dQueue, sizeof( int ) );
+		cudaMalloc( &b->half[h].dQueue, 2 * sizeof( int ) );
 	}
 	return b;
 }
@@ -521,7 +546,8 @@ extern "C" b2gBatchItem* b2gd_batch_items( b2gBatch* b, int count )
 	int cap = count < 64 ? 64 : count;
 	size_t ints = (size_t)cap + 1;
 	bool ok = cudaMallocHost( &b->hItems, sizeof( b2gBatchItem ) * cap ) == cudaSuccess &&
-			  cudaMallocHost( &b->hCounters, sizeof( int ) * 4 * cap ) == cudaSuccess &&
+			  cudaHostAlloc( &b->hCounters, sizeof( int ) * 4 * cap, cudaHostAllocMapped ) == cudaSuccess &&
+			  cudaHostGetDevicePointer( &b->dHostCounters, b->hCounters, 0 ) == cudaSuccess &&
 			  cudaMalloc( &b->dItems, sizeof( b2gBatchItem ) * cap ) == cudaSuccess &&
 			  cudaMalloc( &b->dCounters, sizeof( int ) * 4 * cap ) == cudaSuccess;
 	for ( int h = 0; h < B2G_BATCH_HALVES && ok; ++h )
@@ -562,7 +588,10 @@ extern "C" int b2gd_stage_contacts( b2gDevWorld* w, b2gHostIO* io, int count )
 static void point_counters( b2gBatch* b, int first, int count )
 {
 	for ( int i = first; i < first + count; ++i )
+	{
 		b->hItems[i].W.counters = b->dCounters + 4 * i;
+		b->hItems[i].W.hostCounters = b->dHostCounters + 4 * i;
+	}
 }
 
 /* Ends a capture; on a failed launch or capture nothing is instantiated. */
@@ -616,11 +645,11 @@ extern "C" int b2gd_batch_collide( b2gBatch* b, int h, int first, int n )
 		cudaStreamBeginCapture( H.stream, cudaStreamCaptureModeThreadLocal );
 		cudaMemcpyAsync( b->dItems + first, b->hItems + first, sizeof( b2gBatchItem ) * n, cudaMemcpyHostToDevice, H.stream );
 		cudaMemcpyAsync( H.dPrefix, H.hPrefix, sizeof( int ) * 2 * ( n + 1 ), cudaMemcpyHostToDevice, H.stream );
-		cudaMemsetAsync( b->dCounters + 4 * first, 0, sizeof( int ) * 4 * n, H.stream );
-		k_batch_scatter<<<grid, BATCH_GRID_THREADS, 0, H.stream>>>( items, H.dPrefix, n );
-		k_batch_collide<<<grid, BATCH_GRID_THREADS, 0, H.stream>>>( items, H.dPrefix + n + 1, n );
+		int* counters = b->dCounters + 4 * first;
+		k_batch_scatter<<<grid, BATCH_GRID_THREADS, 0, H.stream>>>( items, H.dPrefix, n, counters, H.dQueue );
+		k_batch_collide<<<grid, BATCH_GRID_THREADS, 0, H.stream>>>( items, H.dPrefix + n + 1, n, counters, b->dHostCounters + 4 * first,
+																	H.dQueue + 1 );
 		cudaError_t launch = cudaGetLastError();
-		cudaMemcpyAsync( b->hCounters + 4 * first, b->dCounters + 4 * first, sizeof( int ) * 4 * n, cudaMemcpyDeviceToHost, H.stream );
 		cudaError_t e = finish_capture( H.stream, launch, &H.collideExec );
 		if ( e != cudaSuccess )
 			return (int)e;
@@ -673,11 +702,9 @@ extern "C" int b2gd_batch_solve( b2gBatch* b, int h, int first, int n )
 		cudaStreamBeginCapture( H.stream, cudaStreamCaptureModeThreadLocal );
 		cudaMemcpyAsync( b->dItems + first, b->hItems + first, sizeof( b2gBatchItem ) * n, cudaMemcpyHostToDevice, H.stream );
 		cudaMemcpyAsync( H.dOrder, H.hOrder, sizeof( int ) * ( 1 + PACK_INTS * (size_t)n ), cudaMemcpyHostToDevice, H.stream );
-		cudaMemsetAsync( H.dQueue, 0, sizeof( int ), H.stream );
 		k_batch_tape<<<b->sms * 4, BATCH_GRID_THREADS, 0, H.stream>>>( b->dItems + first, n );
 		tc.launch( b, H.stream, grid, smem, H.dOrder, H.dQueue );
 		cudaError_t launch = cudaGetLastError();
-		cudaMemcpyAsync( b->hCounters + 4 * first, b->dCounters + 4 * first, sizeof( int ) * 4 * n, cudaMemcpyDeviceToHost, H.stream );
 		cudaError_t e = finish_capture( H.stream, launch, &H.solveExec[choice] );
 		if ( e != cudaSuccess )
 			return (int)e;
