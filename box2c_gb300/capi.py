@@ -164,6 +164,8 @@ class Backend:
         S.b2s_joint_grid.restype = WorldId
         S.b2s_many_pyramids.argtypes = [C.c_int, C.c_int, C.c_int]
         S.b2s_many_pyramids.restype = WorldId
+        S.b2s_shelves.argtypes = [C.c_int, C.c_int, C.c_int]
+        S.b2s_shelves.restype = WorldId
         S.b2s_shape_pile.argtypes = [C.c_int, C.c_uint64]
         S.b2s_shape_pile.restype = WorldId
         S.b2s_joint_hub.argtypes = [C.c_int, C.c_int, C.c_int, C.c_uint64]
@@ -229,6 +231,9 @@ class Backend:
 
     def joint_grid(self, n: int = 100, gravity_y: float = 0.0) -> WorldId:
         return self._made(self.scenes.b2s_joint_grid(n, gravity_y))
+
+    def shelves(self, count: int, wide: int = 16, narrow: int = 8) -> WorldId:
+        return self._made(self.scenes.b2s_shelves(count, wide, narrow))
 
     def many_pyramids(self, rows: int = 20, columns: int = 20, base: int = 10) -> WorldId:
         return self._made(self.scenes.b2s_many_pyramids(rows, columns, base))

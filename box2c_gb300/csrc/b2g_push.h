@@ -47,9 +47,10 @@ struct PushShared
 	unsigned long long bar[PUSH_BARS];
 	int colorBytes[B2G_COLORS]; /* received in a sweep of the active colour */
 	int restBytes[B2G_COLORS];	/* in its restitution sweep */
-	int ovBytes, ownedBytes;	/* in an overflow sweep, in an integration */
+	int ovBytes;				/* in an overflow sweep */
 	int place[B2G_COLORS];		/* active index of a colour */
 	int copies, fail, failAll, gaveUp, ovCount;
+	int forwards; /* owned bodies that are sent but not integrated */
 };
 
 struct PushBodies : SharedBodies
@@ -180,38 +181,43 @@ __device__ __forceinline__ void push_stage( const ResidentPlan& P, const ResShar
 	}
 }
 
-/* All substeps; rb: the owned bodies' terms and awake slots. */
+/* All substeps; rb: the owned bodies' terms and awake slots, the forwarded ones behind the
+ * awake ones.  others: this CTA's copies of other CTAs' bodies. */
 template <int T, bool JOINTS>
 __device__ __forceinline__ void push_run( const ResidentPlan& P, const ResShare* share, const SmemRows& m, const ResJoints& J, PushBodies& B,
-										  PushShared& S, const ResBodies& rb, int awake, int rank, const int* ovList, const b2gStepConst& sc )
+										  PushShared& S, const ResBodies& rb, int awake, int others, int rank, const int* ovList, const b2gStepConst& sc )
 {
 	const unsigned bars = (unsigned)__cvta_generic_to_shared( S.bar );
-	const int bytes = S.ownedBytes;
+	const int bytes = 16 * others, sent = awake + S.forwards;
 	for ( int sub = 0; sub < sc.subSteps; ++sub )
 	{
 		push_expect( B, bars, 0, bytes );
-		for ( int j = threadIdx.x; j < awake; j += T )
+		for ( int j = threadIdx.x; j < sent; j += T )
 		{
 			const int s = rb.awake[j];
 			DevState x = state_of( B.st0[s], make_float4( 0.0f, 0.0f, 1.0f, 0.0f ) );
-			float4 t4 = rb.term[s];
-			VelocityTerms t;
-			t.lvd = gv( t4.x, t4.y );
-			t.avd = t4.z;
-			t.ld = t4.w;
-			t.ad = rb.ad[s];
-			integrate_velocity( x, t, sc );
+			if ( j < awake )
+			{
+				float4 t4 = rb.term[s];
+				VelocityTerms t;
+				t.lvd = gv( t4.x, t4.y );
+				t.avd = t4.z;
+				t.ld = t4.w;
+				t.ad = rb.ad[s];
+				integrate_velocity( x, t, sc );
+			}
 			B.store( s, x );
 		}
 		push_wait( B, S, bytes, sub & 1 );
 		push_stage<F_WARM, T, JOINTS>( P, share, m, J, B, S, bars, rank, sub, ovList, sc );
 		push_stage<F_SOLVE, T, JOINTS>( P, share, m, J, B, S, bars, rank, sub, ovList, sc );
 		push_expect( B, bars, PUSH_BAR_POSITION, bytes );
-		for ( int j = threadIdx.x; j < awake; j += T )
+		for ( int j = threadIdx.x; j < sent; j += T )
 		{
 			const int s = rb.awake[j];
 			DevState x = state_of( B.st0[s], B.st1[s] );
-			integrate_position( x, sc.h );
+			if ( j < awake )
+				integrate_position( x, sc.h );
 			const float4 v = make_float4( x.dp.x, x.dp.y, x.dq.c, x.dq.s );
 			B.st1[s] = v;
 			B.send( B.st1At, s, v );
@@ -252,9 +258,9 @@ __device__ __forceinline__ void push_init( PushBodies& B, PushShared& S, const R
 		for ( int i = 0; i < PUSH_BARS; ++i )
 			asm volatile( "mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"( bars + 8u * (unsigned)i ) : "memory" );
 		asm volatile( "fence.mbarrier_init.release.cluster;" ::: "memory" );
-		S.ovBytes = S.ownedBytes = 0;
+		S.ovBytes = 0;
 		S.copies = owned;
-		S.fail = S.failAll = S.gaveUp = S.ovCount = 0;
+		S.fail = S.failAll = S.gaveUp = S.ovCount = S.forwards = 0;
 		for ( int a = 0; a < P.activeCount; ++a )
 			S.place[P.active[a]] = a;
 	}
@@ -288,10 +294,8 @@ __device__ __forceinline__ void push_meet( const cg::cluster_group& cl, const Pu
 	B.slot[PUSH_CTAS * s + 1] = (unsigned short)at;
 }
 
-/* Fills this CTA's copies of other CTAs' bodies.  integrated( owner, at ): whether the
- * owner integrates the body. */
-template <class F>
-__device__ __forceinline__ void push_fill( const cg::cluster_group& cl, PushBodies& B, PushShared& S, int owned, int rank, F integrated )
+/* Fills this CTA's copies of other CTAs' bodies. */
+__device__ __forceinline__ void push_fill( const cg::cluster_group& cl, PushBodies& B, PushShared& S, int owned, int rank )
 {
 	for ( int s = owned + threadIdx.x; s < S.copies; s += blockDim.x )
 	{
@@ -305,8 +309,6 @@ __device__ __forceinline__ void push_fill( const cg::cluster_group& cl, PushBodi
 		const uint4 w0 = from[0], w1 = from[1];
 		to[0] = w0;
 		to[1] = w1;
-		if ( integrated( owner, at ) )
-			atomicAdd( &S.ownedBytes, 16 );
 	}
 }
 
@@ -345,12 +347,13 @@ __device__ __forceinline__ void push_count( const cg::cluster_group& cl, const P
 /* From rows and joints on body ids to rows and joints on copies, with the expected bytes
  * counted; false, on every CTA, when a CTA's copies do not fit: the ids are unchanged
  * then.  Owned bodies (of block ids a CTA, inv its reciprocal) are in the first slots of
- * their owners; integrated( owner, at ) as in push_fill.  All threads of the cluster; the
- * caller meets the other CTAs before the first sweep. */
+ * their owners; behind the `awake` ones of rb.awake, which integrated( s ) knows, come the
+ * others with copies elsewhere.  All threads of the cluster; the caller meets the other
+ * CTAs before the first sweep. */
 template <bool JOINTS, class F>
 __device__ __forceinline__ bool push_exchange( const cg::cluster_group& cl, PushBodies& B, PushShared& S, int cap, int block, unsigned inv, int rank,
 											   int rows, int joints, const ResShare* share, const SmemRows& m, const ResJoints& J, int* ovList,
-											   F integrated )
+											   const ResBodies& rb, const int& awake, F integrated )
 {
 	const int tid = threadIdx.x, T = blockDim.x;
 	auto owner_of = [&]( int b ) { return block == 1 ? b : (int)__umulhi( (unsigned)b, inv ); };
@@ -387,7 +390,10 @@ __device__ __forceinline__ bool push_exchange( const cg::cluster_group& cl, Push
 	cl.sync();
 	if ( S.failAll )
 		return false;
-	push_fill( cl, B, S, block, rank, integrated );
+	push_fill( cl, B, S, block, rank );
+	for ( int s = tid; s < block; s += T )
+		if ( ( B.mask[s] & 0xffffu ) != 0 && integrated( s ) == false )
+			rb.awake[awake + atomicAdd( &S.forwards, 1 )] = s;
 	__syncthreads();
 	for ( int k = tid, c = 0; k < rows; k += T )
 	{

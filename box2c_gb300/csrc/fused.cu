@@ -255,7 +255,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		if ( P.pushCap > 0 )
 		{
 			pushes = push_exchange<JOINTS>( cl, PB, push, P.pushCap, P.bodyCap, S.bodyCapInv, rank, rows, s_joints, share, m, J, ovList,
-											[&]( int owner, int at ) { return *cl.map_shared_rank( rb.flags + at, owner ) >= 0; } );
+											rb, s_awake, [&]( int s ) { return rb.flags[s] >= 0; } );
 			if ( pushes == false )
 			{
 				/* more copies than a CTA can hold: states in their owners' CTAs only */
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		res_run<CL, CT, true, JOINTS, BINS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 	}
 	else if ( pushes )
-		push_run<CT, JOINTS>( P, share, m, J, PB, push, rb, awake, rank, ovList, sc );
+		push_run<CT, JOINTS>( P, share, m, J, PB, push, rb, awake, push.copies - P.bodyCap, rank, ovList, sc );
 	else
 	{
 		DsmemBodies B{ { cl, rb.st0, rb.st1, P.bodyCap, rank, S.bodyCapInv } };

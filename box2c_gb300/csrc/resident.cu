@@ -202,8 +202,8 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 				clear();
 				cl.sync();
 				mark_and_load();
-				pushes = push_exchange<false>( cl, PB, push, cap, block, inv, rank, rows, 0, share, m, J, ovList,
-											   [&]( int owner, int at ) { return ( *cl.map_shared_rank( rb.flags + at, owner ) & RES_AWAKE ) != 0; } );
+				pushes = push_exchange<false>( cl, PB, push, cap, block, inv, rank, rows, 0, share, m, J, ovList, rb,
+											   s_awake, [&]( int s ) { return ( rb.flags[s] & RES_AWAKE ) != 0; } );
 				if ( pushes == false )
 				{
 					rb = res_carve_bodies( smem + 9 * P.rowCap, P.bodyCap );
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 		}
 		else if ( pushes )
 		{
-			push_run<T, false>( P, share, m, J, PB, push, rb, awake, rank, ovList, sc );
+			push_run<T, false>( P, share, m, J, PB, push, rb, awake, push.copies - block, rank, ovList, sc );
 			cl.sync(); /* no CTA ends before what was sent to it, or by it, is there */
 		}
 		else

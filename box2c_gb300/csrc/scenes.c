@@ -459,6 +459,37 @@ b2WorldId b2s_many_pyramids( int rowCount, int columnCount, int baseCount )
 	return worldId;
 }
 
+b2WorldId b2s_shelves( int shelfCount, int wide, int narrow )
+{
+	b2WorldDef wd = b2s_world_def();
+	b2WorldId worldId = b2CreateWorld( &wd );
+	if ( B2_IS_NULL( worldId ) )
+		return worldId;
+
+	b2BodyDef bd = b2DefaultBodyDef();
+	bd.enableSleep = false;
+	b2ShapeDef sd = b2DefaultShapeDef();
+	b2Polygon box = b2MakeSquare( 0.5f );
+	for ( int k = 0; k < shelfCount; ++k )
+	{
+		int stacks = ( k & 1 ) ? narrow : wide;
+		float y = 4.0f * k;
+		bd.type = b2_kinematicBody;
+		bd.position = ( b2Vec2 ){ 0.0f, y };
+		b2BodyId shelfId = b2CreateBody( worldId, &bd );
+		b2Polygon slab = b2MakeBox( 0.75f * (float)stacks + 0.5f, 0.25f );
+		b2CreatePolygonShape( shelfId, &sd, &slab );
+		bd.type = b2_dynamicBody;
+		for ( int i = 0; i < 2 * stacks; ++i )
+		{
+			bd.position = ( b2Vec2 ){ 1.5f * ( (float)( i >> 1 ) - 0.5f * (float)( stacks - 1 ) ), y + 0.75f + ( i & 1 ) };
+			b2BodyId bodyId = b2CreateBody( worldId, &bd );
+			b2CreatePolygonShape( bodyId, &sd, &box );
+		}
+	}
+	return worldId;
+}
+
 b2WorldId b2s_shape_pile( int count, uint64_t seed )
 {
 	b2WorldDef wd = b2s_world_def();

@@ -71,6 +71,11 @@ b2WorldId b2s_joint_grid( int n, float gravityY );
  * static segment; sleep off.  The benchmark has 20 x 20 pyramids of base 10. */
 b2WorldId b2s_many_pyramids( int rowCount, int columnCount, int baseCount );
 
+/* Kinematic shelves at rest, each under a row of stacks of two boxes: `wide` stacks on the
+ * even shelves, `narrow` on the odd ones.  A shelf is one body of all its boxes' contacts:
+ * with more than 11 stacks some of them are in the overflow set.  Sleep off. */
+b2WorldId b2s_shelves( int shelfCount, int wide, int narrow );
+
 /* Mixed-shape pile in a static funnel of segments (floor, two slopes) with a static
  * capsule bar and a static box ledge: `count` bodies dropped from a seeded jittered
  * grid, in turn a horizontal capsule, a box, a circle, a rounded box and an upright

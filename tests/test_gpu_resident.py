@@ -266,3 +266,36 @@ def test_batched_rows_beside_the_chip(gpu, oracle):
         assert np.array_equal(got[live].view(np.uint32), want[live].view(np.uint32)), i
         gpu.destroy(w)
         oracle.destroy(o)
+
+
+# bodies that contacts touch and the list leaves out: kinematic shelves at rest, whose
+# integration changes nothing, so that the oracle's step is the expected result.  One CTA
+# (8 shelves), a cluster (80, 120) with the contacts of the shelves spread over CTAs that do not
+# own them, CTA 0 held up by an overflow set (wide shelves of 16), and a grid with its rows in memory (1000).
+# Tolerance: none but the sign of a zero.
+@pytest.mark.gpu
+@pytest.mark.parametrize("shelves,wide,narrow", [(8, 8, 4), (8, 16, 8), (120, 8, 5), (80, 16, 8), (1000, 16, 8)])
+def test_resident_solver_unlisted_bodies(gpu, oracle, shelves, wide, narrow):
+    torch = pytest.importorskip("torch")
+    w = oracle.shelves(shelves, wide, narrow)
+    oracle.step(w, count=12)
+    cap = capture_step(oracle, w, body_cap=30000, contact_cap=80000)
+    oracle.destroy(w)
+    kinematic = cap["mass"][cap["awake"], 1] == 0
+    assert kinematic.sum() == shelves and (cap["colorStart"][12] > cap["colorStart"][11]) == (wide > 11)
+    # the narrow shelves, whose contacts are the last of their colours, first
+    n = len(cap["statesIn"])
+    shelf = np.sort(cap["awake"][kinematic])
+    order = np.concatenate([shelf[1::2], np.setdiff1d(np.arange(n), shelf[1::2])])
+    place = np.empty(n, np.int32)
+    place[order] = np.arange(n)
+    for k in ("statesIn", "statesOut", "mass", "force", "damping"):
+        cap[k] = cap[k][order]
+    cap["contactBodies"] = np.where(cap["contactBodies"] < 0, -1, place[cap["contactBodies"]]).astype(np.int32)
+    rng = np.random.default_rng(11)
+    for drop in (kinematic, kinematic & (rng.random(len(kinematic)) < 0.5)):
+        part = dict(cap, awake=place[cap["awake"][~drop]])
+        states, manifolds = solve_on_device(gpu, torch, part)
+        assert np.array_equal(states, cap["statesOut"])
+        got, want = manifolds.view(np.float32), cap["manifoldsOut"].view(np.float32)
+        assert np.all((got == want) | (got.view(np.uint32) == want.view(np.uint32)))

@@ -97,3 +97,16 @@ def test_joint_angle_atan2(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.startswith("ok"), r.stdout
+
+
+def test_pushed_copies_keep_their_order(tmp_path):
+    """A host model of the cluster solver's pushed body copies (box2c_gb300/csrc/b2g_push.h)
+    on seeded random sets and schedules, bodies that no CTA integrates among them
+    (tests/c/push_check.cpp)."""
+    exe = str(tmp_path / "push_check")
+    src = os.path.join(REPO, "box2c_gb300", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I", src, os.path.join(REPO, "tests", "c", "push_check.cpp"), "-o", exe],
+                   check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.startswith("ok"), r.stdout
