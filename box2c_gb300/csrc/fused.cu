@@ -204,8 +204,8 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	{
 		if ( P.pushCap > 0 )
 		{
-			push_carve( smem + P.bodyOffset, P.pushCap, P.bodyCap, PB, rb );
-			push_init( PB, push, P, P.bodyCap, rank );
+			push_carve( smem + P.bodyOffset, P.pushCap, P.bodyCap, rank, PB, rb );
+			push_init( PB, push, P, P.bodyCap );
 		}
 		load_owned();
 	}
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 	{
 		if ( P.pushCap > 0 )
 		{
-			pushes = push_exchange<JOINTS>( cl, PB, push, P.pushCap, P.bodyCap, S.bodyCapInv, rank, rows, s_joints, share, m, J, ovList,
+			pushes = push_exchange<JOINTS>( cl, PB, push, P.pushCap, P.bodyCap, S.bodyCapInv, rows, s_joints, share, m, J, ovList,
 											rb, s_awake, [&]( int s ) { return rb.flags[s] >= 0; } );
 			if ( pushes == false )
 			{
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		res_run<CL, CT, true, JOINTS, BINS>( P, share, m, J, B, rb, gst, nullptr, awake, bar, rank, sc, ov, s_ovSlots );
 	}
 	else if ( pushes )
-		push_run<CT, JOINTS>( P, share, m, J, PB, push, rb, awake, push.copies - P.bodyCap, rank, ovList, sc );
+		push_run<CT, JOINTS>( P, share, m, J, PB, push, rb, awake, push.copies - P.bodyCap, ovList, sc );
 	else
 	{
 		DsmemBodies B{ { cl, rb.st0, rb.st1, P.bodyCap, rank, S.bodyCapInv } };

@@ -196,13 +196,13 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 			const int cap = min( space / PUSH_COPY_BYTES, 65535 );
 			if ( space > 0 && cap > block )
 			{
-				push_carve( smem + 9 * P.rowCap, cap, block, PB, rb );
-				push_init( PB, push, P, block, rank );
+				push_carve( smem + 9 * P.rowCap, cap, block, rank, PB, rb );
+				push_init( PB, push, P, block );
 				ovList = rb.awake + block;
 				clear();
 				cl.sync();
 				mark_and_load();
-				pushes = push_exchange<false>( cl, PB, push, cap, block, inv, rank, rows, 0, share, m, J, ovList, rb,
+				pushes = push_exchange<false>( cl, PB, push, cap, block, inv, rows, 0, share, m, J, ovList, rb,
 											   s_awake, [&]( int s ) { return ( rb.flags[s] & RES_AWAKE ) != 0; } );
 				if ( pushes == false )
 				{
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 		}
 		else if ( pushes )
 		{
-			push_run<T, false>( P, share, m, J, PB, push, rb, awake, push.copies - block, rank, ovList, sc );
+			push_run<T, false>( P, share, m, J, PB, push, rb, awake, push.copies - block, ovList, sc );
 			cl.sync(); /* no CTA ends before what was sent to it, or by it, is there */
 		}
 		else

@@ -2,13 +2,16 @@
  * push_check.cpp -- host model of the pushed body copies (box2c_gb300/csrc/b2g_push.h): CTAs
  * that sweep over coloured constraints, each with copies of the bodies its constraints
  * touch, an update of a body travelling as a message that completes on the receiver's
- * mbarrier of that sweep.  Messages arrive in any order and CTAs lag as they please; the
- * mbarriers count as the hardware's do.
+ * mbarrier of that sweep, to the CTA that box2c_gb300/csrc/b2g_chain.h names.  Messages
+ * arrive in any order, CTAs lag as they please, and the mbarriers count as the hardware's
+ * do.
  *
  * Checked on seeded random sets, some bodies of which are not integrated: every wait
- * ends, no transaction counts into a phase before its own, and every update starts from
- * the one before it.  Prints "ok" or the first failure.
+ * ends, no transaction counts into a phase before its own, every update starts from the
+ * one before it, and the owner ends with the last one.  Prints "ok" or the first failure.
  */
+#include "b2g_chain.h"
+
 #include <algorithm>
 #include <stdio.h>
 #include <stdlib.h>
@@ -29,9 +32,18 @@ enum
 	SUBSTEPS = 4,
 	/* sweeps of a substep: integrate, warm start, solve, positions, relax */
 	SWEEPS = 2 + 3 * COLORS,
-	/* then a restitution stage */
-	TOTAL = SUBSTEPS * SWEEPS + COLORS,
-	BARS = SWEEPS + COLORS,
+	/* then the start of restitution and its stage */
+	TOTAL = SUBSTEPS * SWEEPS + 1 + COLORS,
+	BARS = SWEEPS + 1 + COLORS,
+};
+
+/* How updates travel: to the next updater, or to all copies; with the latter, owners may
+ * send nothing of the bodies that they do not integrate. */
+enum Policy
+{
+	CHAIN,
+	ALL,
+	ALL_LISTED,
 };
 
 enum Word
@@ -42,7 +54,7 @@ enum Word
 
 struct Constraint
 {
-	int cta, color, body[2];
+	int cta, color, joint, body[2];
 };
 
 /* An mbarrier of arrival count 1. */
@@ -71,12 +83,13 @@ struct Set
 	std::vector<int> owner, listed;
 	std::vector<Constraint> rows;
 	std::vector<unsigned> holders; /* CTAs with a copy, the owner among them */
+	std::vector<b2gChain> chain;
 };
 
 struct Model
 {
 	const Set* set;
-	bool forward; /* owners send the bodies they do not integrate as well */
+	Policy policy;
 	Bar bar[CTAS][BARS];
 	int sweep[CTAS], armed[CTAS];
 	std::vector<std::vector<int>> slot[2]; /* [word][cta][body]: the version held */
@@ -84,84 +97,100 @@ struct Model
 	const char* fault = nullptr;
 };
 
-/* What sweep i is: its stage (-1 integrate, -2 positions, 0 to 3) and colour, and the
- * mbarrier it completes on. */
-static void decode( int i, int* stage, int* color, int* bar, int* phase )
+enum Stage
+{
+	WARM,
+	SOLVE,
+	RELAX,
+	RESTITUTION,
+	INTEGRATE,
+	POSITIONS,
+	RESTITUTION_START,
+};
+
+/* What sweep i is: its stage and colour, and the mbarrier it completes on. */
+static Stage decode( int i, int* color, int* bar, int* phase )
 {
 	*phase = i / SWEEPS;
+	*color = 0;
 	int k = i % SWEEPS;
 	if ( i >= SUBSTEPS * SWEEPS )
 	{
-		*stage = 3;
-		*color = i - SUBSTEPS * SWEEPS;
-		*bar = SWEEPS + *color;
+		k = i - SUBSTEPS * SWEEPS;
 		*phase = 0;
-		return;
+		*bar = SWEEPS + k;
+		*color = k > 0 ? k - 1 : 0;
+		return k == 0 ? RESTITUTION_START : RESTITUTION;
 	}
 	*bar = k;
-	*color = 0;
 	if ( k == 0 )
-		*stage = -1;
-	else if ( k == 1 + 2 * COLORS )
-		*stage = -2;
-	else
-	{
-		k -= k > 2 * COLORS ? 2 : 1;
-		*stage = k / COLORS;
-		*color = k % COLORS;
-	}
+		return INTEGRATE;
+	if ( k == 1 + 2 * COLORS )
+		return POSITIONS;
+	k -= k > 2 * COLORS ? 2 : 1;
+	*color = k % COLORS;
+	return (Stage)( k / COLORS );
 }
 
-static bool moves( const Set& s, const Constraint& r, int b, int color ) { return r.color == color && ( r.body[0] == b || r.body[1] == b ); }
+static bool sent_by_owner( const Model& m, int b ) { return m.set->listed[b] || m.policy != ALL_LISTED; }
 
-/* The CTA that updates body b's velocity in sweep i, or -1. */
-static int updater( const Model& m, int b, int i )
+/* The CTA that updates a word of body b in sweep i, or -1. */
+static int updater( const Model& m, int b, int i, Word word )
 {
-	const Set& s = *m.set;
-	int stage, color, bar, phase;
-	decode( i, &stage, &color, &bar, &phase );
-	if ( stage == -1 )
-		return s.listed[b] || m.forward ? s.owner[b] : -1;
-	for ( const Constraint& r : s.rows )
-		if ( stage >= 0 && moves( s, r, b, color ) )
+	int color, bar, phase;
+	const Stage stage = decode( i, &color, &bar, &phase );
+	if ( stage == ( word == VELOCITY ? INTEGRATE : POSITIONS ) )
+		return sent_by_owner( m, b ) ? m.set->owner[b] : -1;
+	if ( word == POSITION || stage > RESTITUTION )
+		return -1;
+	for ( const Constraint& r : m.set->rows )
+		if ( r.color == color && ( r.body[0] == b || r.body[1] == b ) && ( r.joint == 0 || stage != RESTITUTION ) )
 			return r.cta;
 	return -1;
 }
 
-/* The CTA that updates its position, or -1. */
-static int mover( const Model& m, int b, int i )
-{
-	int stage, color, bar, phase;
-	decode( i, &stage, &color, &bar, &phase );
-	return stage == -2 && ( m.set->listed[b] || m.forward ) ? m.set->owner[b] : -1;
-}
-
-/* The CTAs that the updater of sweep i sends the word of body b to. */
-static unsigned receivers( const Model& m, int b, int i, Word word )
+/* The CTA that sends a word in sweep i, or -1, and the CTAs it goes to. */
+static int sender( const Model& m, int b, int i, Word word, unsigned* to )
 {
 	const Set& s = *m.set;
-	int stage, color, bar, phase;
-	decode( i, &stage, &color, &bar, &phase );
-	int from = word == VELOCITY ? updater( m, b, i ) : mover( m, b, i );
+	int color, bar, phase;
+	const Stage stage = decode( i, &color, &bar, &phase );
+	int from = updater( m, b, i, word );
+	*to = 0;
+	if ( m.policy != CHAIN || word == POSITION )
+	{
+		if ( from >= 0 )
+			*to = s.holders[b] & ~( 1u << from );
+		return from;
+	}
+	if ( stage == POSITIONS || stage == RESTITUTION_START )
+		from = s.owner[b];
 	if ( from < 0 )
-		return 0;
-	return s.holders[b] & ~( 1u << from );
+		return -1;
+	int t = b2g_chain_next( s.chain[b], stage > RESTITUTION ? -1 : color, stage == WARM, stage == RESTITUTION || stage == RESTITUTION_START,
+							s.owner[b] );
+	*to = 1u << t & ~( 1u << from );
+	return from;
 }
 
 static int version_before( const Model& m, int b, int i, Word word )
 {
 	int v = 0;
 	for ( int k = 0; k < i; ++k )
-		v += ( word == POSITION ? mover( m, b, k ) : updater( m, b, k ) ) >= 0;
+		v += updater( m, b, k, word ) >= 0;
 	return v;
 }
 
 static int expected( const Model& m, int cta, int i )
 {
 	int n = 0;
+	unsigned to;
 	for ( int b = 0; b < m.set->bodies; ++b )
 		for ( Word w : { VELOCITY, POSITION } )
-			n += ( receivers( m, b, i, w ) >> cta ) & 1;
+		{
+			sender( m, b, i, w, &to );
+			n += ( to >> cta ) & 1;
+		}
 	return n;
 }
 
@@ -170,8 +199,8 @@ static void begin_sweep( Model& m, int cta )
 {
 	const Set& s = *m.set;
 	const int i = m.sweep[cta];
-	int stage, color, bar, phase;
-	decode( i, &stage, &color, &bar, &phase );
+	int color, bar, phase;
+	const Stage stage = decode( i, &color, &bar, &phase );
 	int n = expected( m, cta, i );
 	if ( n > 0 )
 	{
@@ -186,17 +215,18 @@ static void begin_sweep( Model& m, int cta )
 	for ( int b = 0; b < s.bodies; ++b )
 		for ( Word w : { VELOCITY, POSITION } )
 		{
-			int from = w == VELOCITY ? updater( m, b, i ) : mover( m, b, i );
-			if ( from != cta )
+			unsigned to;
+			if ( sender( m, b, i, w, &to ) != cta )
 				continue;
-			int v = version_before( m, b, i, VELOCITY );
-			if ( m.slot[VELOCITY][cta][b] != v && ( w == VELOCITY || s.listed[b] ) )
+			const bool update = updater( m, b, i, w ) == cta;
+			if ( ( update || to ) && m.slot[VELOCITY][cta][b] != version_before( m, b, i, VELOCITY ) )
 				m.fault = "an update starts from an older one";
-			if ( stage >= 1 && stage <= 2 && m.slot[POSITION][cta][b] != version_before( m, b, i, POSITION ) )
+			if ( ( stage == SOLVE || stage == RELAX ) && m.slot[POSITION][cta][b] != version_before( m, b, i, POSITION ) )
 				m.fault = "a constraint reads an older position";
-			v = version_before( m, b, i, w ) + 1;
-			m.slot[w][cta][b] = v;
-			unsigned to = receivers( m, b, i, w );
+			const int v = version_before( m, b, i, w ) + update;
+			/* a velocity that goes to the next updater is not kept */
+			if ( m.policy != CHAIN || w == POSITION || to == 0 )
+				m.slot[w][cta][b] = v;
 			for ( int t = 0; t < CTAS; ++t )
 				if ( ( to >> t ) & 1 )
 					m.flight.push_back( { t, b, i, v, w } );
@@ -207,8 +237,8 @@ static void deliver( Model& m, size_t k )
 {
 	Message g = m.flight[k];
 	m.flight.erase( m.flight.begin() + (long)k );
-	int stage, color, bar, phase;
-	decode( g.sweep, &stage, &color, &bar, &phase );
+	int color, bar, phase;
+	decode( g.sweep, &color, &bar, &phase );
 	Bar& B = m.bar[g.to][bar];
 	if ( B.phase != phase )
 		m.fault = "a transaction counts into a phase before its own";
@@ -217,13 +247,13 @@ static void deliver( Model& m, size_t k )
 	B.settle();
 }
 
-/* Runs the set under one schedule: CTA `lag` moves seldom.  Messages of one sweep may
- * overtake one another, later ones none of the same body. */
-static const char* run( const Set& s, bool forward, int lag )
+/* Runs the set under one schedule: CTA `lag` moves seldom.  A message may overtake any
+ * other, or with `ordered` none of the same copy. */
+static const char* run( const Set& s, Policy policy, int lag, bool ordered )
 {
 	Model m;
 	m.set = &s;
-	m.forward = forward;
+	m.policy = policy;
 	for ( int w = 0; w < 2; ++w )
 		m.slot[w].assign( CTAS, std::vector<int>( (size_t)s.bodies, 0 ) );
 	for ( int c = 0; c < CTAS; ++c )
@@ -236,11 +266,16 @@ static const char* run( const Set& s, bool forward, int lag )
 		if ( m.fault )
 			return m.fault;
 		if ( left == 0 && m.flight.empty() )
+		{
+			for ( int b = 0; b < s.bodies; ++b )
+				if ( m.slot[VELOCITY][s.owner[b]][b] != version_before( m, b, TOTAL, VELOCITY ) )
+					return "an owner ends with an older velocity";
 			return nullptr;
+		}
 		if ( m.flight.empty() == false && rnd( 3 ) != 0 )
 		{
 			int k = rnd( (int)m.flight.size() );
-			for ( int j = 0; j < k; ++j )
+			for ( int j = 0; j < k && ordered; ++j )
 				if ( m.flight[j].to == m.flight[k].to && m.flight[j].body == m.flight[k].body )
 				{
 					k = j;
@@ -259,8 +294,8 @@ static const char* run( const Set& s, bool forward, int lag )
 			idle = 0;
 			continue;
 		}
-		int stage, color, bar, phase;
-		decode( m.sweep[c], &stage, &color, &bar, &phase );
+		int color, bar, phase;
+		decode( m.sweep[c], &color, &bar, &phase );
 		if ( expected( m, c, m.sweep[c] ) > 0 && m.bar[c][bar].phase == phase )
 			continue;
 		m.sweep[c] += 1;
@@ -282,7 +317,7 @@ static Set make_set()
 	int want = 1 + rnd( 3 * s.bodies );
 	for ( int k = 0; k < want; ++k )
 	{
-		Constraint r = { rnd( CTAS ), 1 + rnd( COLORS - 1 ), { rnd( s.bodies ), rnd( s.bodies ) } };
+		Constraint r = { rnd( CTAS ), 1 + rnd( COLORS - 1 ), rnd( 5 ) == 0, { rnd( s.bodies ), rnd( s.bodies ) } };
 		if ( rnd( 8 ) == 0 )
 			r.body[1] = -1;
 		if ( r.body[0] == r.body[1] )
@@ -306,37 +341,90 @@ static Set make_set()
 		s.rows.push_back( r );
 	}
 	s.holders.assign( (size_t)s.bodies, 0u );
+	s.chain.assign( (size_t)s.bodies, b2gChain{ 0u, { 0u, 0u } } );
 	for ( int b = 0; b < s.bodies; ++b )
 		s.holders[b] = 1u << s.owner[b];
 	for ( const Constraint& r : s.rows )
 		for ( int b : r.body )
 			if ( b >= 0 )
+			{
 				s.holders[b] |= 1u << r.cta;
+				s.chain[b].who |= 1u << ( r.color + ( r.joint ? 16 : 0 ) );
+				s.chain[b].cta[r.color >> 3] |= (unsigned)r.cta << ( 4 * ( r.color & 7 ) );
+			}
 	return s;
+}
+
+/* b2g_chain_next over all 12 places, CTAs and subsets against a walk of the stages. */
+static const char* check_chain( void )
+{
+	for ( int n = 0; n < 20000; ++n )
+	{
+		b2gChain c = { 0u, { 0u, 0u } };
+		int cta[B2G_CHAIN_PLACES], kind[B2G_CHAIN_PLACES];
+		const int owner = rnd( 16 );
+		for ( int p = 0; p < B2G_CHAIN_PLACES; ++p )
+		{
+			kind[p] = rnd( 3 ) == 0 ? 1 + rnd( 2 ) : 0; /* 1 a row, 2 a joint */
+			cta[p] = p == 0 ? 0 : rnd( 16 );
+			if ( kind[p] )
+			{
+				c.who |= 1u << ( p + ( kind[p] == 2 ? 16 : 0 ) );
+				c.cta[p >> 3] |= (unsigned)cta[p] << ( 4 * ( p & 7 ) );
+			}
+		}
+		for ( int restitution = 0; restitution < 2; ++restitution )
+			for ( int warm = 0; warm < 2 - restitution; ++warm )
+				for ( int p = -1; p < B2G_CHAIN_PLACES; ++p )
+				{
+					int want = -1;
+					for ( int lap = 0; lap < ( warm ? 2 : 1 ) && want < 0; ++lap )
+						for ( int q = lap ? 0 : p + 1; q < B2G_CHAIN_PLACES && want < 0; ++q )
+							want = kind[q] == 1 || ( kind[q] == 2 && restitution == 0 ) ? cta[q] : -1;
+					want = want < 0 ? owner : want;
+					if ( b2g_chain_next( c, p, warm, restitution, owner ) != want )
+						return "the next CTA of a chain";
+				}
+	}
+	return nullptr;
 }
 
 int main()
 {
-	int caught = 0;
-	for ( int k = 0; k < 800; ++k )
+	const char* wrong = check_chain();
+	if ( wrong )
+	{
+		printf( "failed: %s\n", wrong );
+		return 1;
+	}
+	int ahead = 0, stale = 0;
+	for ( int k = 0; k < 500; ++k )
 	{
 		Set s = make_set();
 		int lag = rnd( CTAS + 1 );
-		const char* fault = run( s, true, lag );
+		const char* fault = run( s, CHAIN, lag, false );
 		if ( fault )
 		{
 			printf( "failed: %s (set %d, %d bodies)\n", fault, k, s.bodies );
 			return 1;
 		}
-		/* with owners silent about the bodies they do not integrate, a CTA runs ahead of one */
-		fault = run( s, false, lag );
-		caught += fault != nullptr && strstr( fault, "before its own" ) != nullptr;
+		/* updates sent to all copies overtake one another; with owners silent about the bodies
+		 * that they do not integrate, a CTA runs ahead of one even where they do not */
+		fault = run( s, ALL, lag, false );
+		stale += fault != nullptr && strstr( fault, "older" ) != nullptr;
+		fault = run( s, ALL_LISTED, lag, true );
+		ahead += fault != nullptr && strstr( fault, "before its own" ) != nullptr;
+		if ( ( fault = run( s, ALL, lag, true ) ) != nullptr )
+		{
+			printf( "failed: %s with ordered messages (set %d)\n", fault, k );
+			return 1;
+		}
 	}
-	if ( caught < 8 )
+	if ( ahead < 5 || stale < 5 )
 	{
-		printf( "failed: the planted mistake was met %d times\n", caught );
+		printf( "failed: planted mistakes were met %d and %d times\n", ahead, stale );
 		return 1;
 	}
-	printf( "ok: 800 sets, planted mistake met %d times\n", caught );
+	printf( "ok: 500 sets, planted mistakes met %d and %d times\n", ahead, stale );
 	return 0;
 }
