@@ -42,9 +42,14 @@
 #define PUSH_BARS ( 3 + 4 * B2G_CHAIN_PLACES )
 #define PUSH_BAR_POSITION ( PUSH_BARS - 2 )
 #define PUSH_BAR_RESTITUTION ( PUSH_BARS - 1 )
-/* a CTA gives up on an mbarrier after this many polls or nanoseconds */
+/* a CTA gives up on an mbarrier after this many polls or nanoseconds; then all of the
+ * cluster leave the solve at the next substep, and its results are marked */
+#ifndef PUSH_SPIN_LIMIT
 #define PUSH_SPIN_LIMIT ( 1 << 22 )
+#endif
 #define PUSH_SPIN_NS 1000000000ull
+/* what a store under way to another CTA may take: a cluster that gave up waits it out */
+#define PUSH_FLIGHT_NS 100000ull
 /* bytes of a copy: two state float4, its slots in the 16 CTAs, the mask of the others; of
  * an owned body besides: velocity terms, chain, damping, flags, an entry of the awake list */
 #define PUSH_COPY_BYTES ( 32 + 2 * PUSH_CTAS + 4 )
@@ -141,6 +146,13 @@ __device__ __forceinline__ void push_expect( PushBodies& B, unsigned bars, int b
 		asm volatile( "mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"( B.barAt ), "r"( bytes ) : "memory" );
 }
 
+__device__ __forceinline__ unsigned long long push_clock()
+{
+	unsigned long long now;
+	asm volatile( "mov.u64 %0, %globaltimer;" : "=l"( now ) );
+	return now;
+}
+
 /* Ends it: this CTA's own updates, then the ones it receives. */
 __device__ __forceinline__ void push_wait( const PushBodies& B, PushShared& S, int bytes, int parity )
 {
@@ -151,26 +163,47 @@ __device__ __forceinline__ void push_wait( const PushBodies& B, PushShared& S, i
 	for ( int left = PUSH_SPIN_LIMIT;; )
 	{
 		unsigned done;
-		asm volatile( "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-					  : "=r"( done )
-					  : "r"( B.barAt ), "r"( parity )
-					  : "memory" );
-		if ( done )
+		if ( PUSH_SPIN_LIMIT > 1 )
+			asm volatile( "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+						  : "=r"( done )
+						  : "r"( B.barAt ), "r"( parity )
+						  : "memory" );
+		else /* one look */
+			asm volatile( "{ .reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+						  : "=r"( done )
+						  : "r"( B.barAt ), "r"( parity )
+						  : "memory" );
+		if ( done || *(volatile int*)&S.gaveUp != 0 )
 			return;
-		bool late = --left == 0 || *(volatile int*)&S.gaveUp != 0;
+		bool late = --left == 0;
 		if ( ( left & 255 ) == 0 )
 		{
-			unsigned long long now;
-			asm volatile( "mov.u64 %0, %globaltimer;" : "=l"( now ) );
+			const unsigned long long now = push_clock();
 			start = start == 0 ? now : start;
 			late = late || now - start > PUSH_SPIN_NS;
 		}
 		if ( late )
 		{
-			*(volatile int*)&S.gaveUp = 1;
+			for ( int t = 0; t < PUSH_CTAS; ++t )
+				*(volatile int*)cg::this_cluster().map_shared_rank( &S.gaveUp, t ) = 1;
 			return;
 		}
 	}
+}
+
+/* After the run: no CTA ends before what was sent to it, or by it, is there.  True, on every
+ * CTA, when one gave up. */
+__device__ __forceinline__ bool push_end( const cg::cluster_group& cl, const PushShared& S )
+{
+	cl.sync();
+	if ( S.gaveUp == 0 )
+		return false;
+	/* stores that no wait has seen */
+	const unsigned long long start = push_clock();
+	for ( int left = 1 << 20; push_clock() - start < PUSH_FLIGHT_NS && left > 0; --left )
+		;
+	cl.sync();
+	return true;
 }
 
 /* Bytes received in the sweep of a place. */
@@ -256,6 +289,9 @@ __device__ __forceinline__ void push_run( const ResidentPlan& P, const ResShare*
 	const int sent = awake + S.forwards, firstBytes = 16 * S.firsts, restBytes = 16 * S.restFirsts;
 	for ( int sub = 0; sub < sc.subSteps; ++sub )
 	{
+		/* an mbarrier whose wait ran out is not armed again */
+		if ( __syncthreads_or( *(volatile int*)&S.gaveUp ) )
+			return;
 		push_expect( B, bars, 0, firstBytes );
 		for ( int j = threadIdx.x; j < sent; j += T )
 		{
@@ -293,6 +329,8 @@ __device__ __forceinline__ void push_run( const ResidentPlan& P, const ResShare*
 		push_wait( B, S, 16 * others + firstBytes, sub & 1 );
 		push_stage<F_RELAX, T, JOINTS>( P, share, m, J, B, S, bars, sub, ovList, sc );
 	}
+	if ( __syncthreads_or( *(volatile int*)&S.gaveUp ) )
+		return;
 	push_expect( B, bars, PUSH_BAR_RESTITUTION, restBytes );
 	for ( int j = threadIdx.x; j < sent; j += T )
 	{

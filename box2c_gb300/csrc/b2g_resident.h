@@ -17,7 +17,9 @@
 #define RES_OVERFLOW_MAX 512
 /* polls of a grid barrier before it gives up (seconds; a cooperative launch never gets
  * there) */
+#ifndef RES_SPIN_LIMIT
 #define RES_SPIN_LIMIT ( 1 << 22 )
+#endif
 
 struct ResidentPlan
 {

@@ -313,8 +313,9 @@ __global__ void __launch_bounds__( FUSED_THREADS, 1 ) k_solve_world( const __gri
 		gst[2 * b] = rb.st0[s];
 		finalize_state( W, i, b, rb.st0[s], rb.st1[s], sc );
 	}
-	bar.sync();
-	if ( CL > 1 && pushes && tid == 0 && push.gaveUp )
+	if ( pushes == false )
+		bar.sync();
+	else if ( push_end( cl, push ) && tid == 0 )
 		W.hostCounters[2] = 1;
 	if ( rank == 0 && tid == 0 )
 	{

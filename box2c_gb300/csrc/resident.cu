@@ -187,7 +187,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 		};
 		/* a cluster whose CTAs can hold copies of the bodies that their rows touch; states
 		 * in their owners' CTAs only where they cannot */
-		bool pushes = false;
+		bool pushes = false, lost = false;
 		PushBodies PB;
 		int* ovList = nullptr;
 		if constexpr ( CL > 1 )
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 		else if ( pushes )
 		{
 			push_run<T, false>( P, share, m, J, PB, push, rb, awake, push.copies - block, ovList, sc );
-			cl.sync(); /* no CTA ends before what was sent to it, or by it, is there */
+			lost = push_end( cl, push );
 		}
 		else
 		{
@@ -243,8 +243,8 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 		{
 			int b = rank * block + s;
 			int f = rb.flags[s];
-			/* a CTA that gave up on another has no result */
-			if ( CL > 1 && pushes && push.gaveUp )
+			/* a cluster of which a CTA gave up on another has no result */
+			if ( lost )
 				rb.st0[s].x = rb.st0[s].y = rb.st0[s].z = __int_as_float( 0x7fffffff );
 			if ( f )
 				gst[2 * b] = rb.st0[s];
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 {
 	extern __shared__ float4 smem[];
 	__shared__ ResShare share[B2G_COLORS];
-	__shared__ int s_ovSlots;
+	__shared__ int s_ovSlots, s_last;
 	const int rank = blockIdx.x, ctas = gridDim.x, tid = threadIdx.x;
 	const int* cs = P.colorStart;
 	const int ovRows = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
@@ -340,13 +340,32 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 			const SmemRows part = { m.idx + f, m.nf + f, m.ms + f, m.anc0 + f, m.anc1 + f, m.coef0 + f, m.coef1 + f, m.imp0 + f, m.imp1 + f };
 			store_impulses( W, part, share[c].count, c == B2G_OVERFLOW ? 0 : share[c].count, tid, T );
 		}
-	if ( tid == 0 && atomicAdd( ctl + 1, 1 ) == ctas - 1 )
+	__syncthreads();
+	if ( tid == 0 )
 	{
-		/* every CTA is past its last barrier */
-		ctl[0] = 0;
-		ctl[1] = 0;
-		ctl[2] = 0;
+		__threadfence();
+		s_last = atomicAdd( ctl + 1, 1 ) == ctas - 1;
+		__threadfence();
 	}
+	__syncthreads();
+	if ( s_last == 0 )
+		return;
+	/* every CTA is past its last barrier, and its last write of a state */
+	if ( *(volatile int*)( ctl + 2 ) != 0 )
+	{
+		/* a grid of which a CTA gave up on another has no result */
+		float* st = (float*)W.state;
+		const int total = cs[B2G_COLORS];
+		for ( int i = tid; i < P.awakeCount + 2 * total; i += T )
+		{
+			const int b = i < P.awakeCount ? W.awake[i] : W.cBodies[i - P.awakeCount];
+			for ( int k = 0; k < 3 && b >= 0; ++k )
+				st[8 * (size_t)b + k] = __int_as_float( 0x7fffffff );
+		}
+	}
+	__syncthreads();
+	if ( tid < 3 )
+		ctl[tid] = 0;
 }
 
 /* ------------------------------------------------------------------ host side */

@@ -146,7 +146,9 @@ B2_API int b2World_GetBodyStates( b2WorldId worldId, float* out, int capacity );
  * coloured contacts (no two contacts of one colour share a non-static body; colour 11
  * is the overflow set, solved serially in array order) and receives updated body
  * velocities, position/rotation deltas and accumulated impulses.  All pointers are
- * device pointers except colorStart; the call is asynchronous on `stream`. */
+ * device pointers except colorStart; the call is asynchronous on `stream`.  Its CTAs wait
+ * for one another with a limit of about a second; a solve in which a wait ran out ends with
+ * NaN velocities of all bodies that it lists, or has contacts on. */
 typedef struct b2ContactSolveDesc
 {
 	/* bodies, indexed by body index */

@@ -2,6 +2,8 @@
 cluster, a cooperative grid, body indices that do not fit on chip, overflow rows and an
 empty set.  The reference is the oracle's captured solver stage; tolerance: none."""
 import ctypes as C
+import os
+import subprocess
 
 import numpy as np
 import pytest
@@ -299,3 +301,21 @@ def test_resident_solver_unlisted_bodies(gpu, oracle, shelves, wide, narrow):
         assert np.array_equal(states, cap["statesOut"])
         got, want = manifolds.view(np.float32), cap["manifoldsOut"].view(np.float32)
         assert np.all((got == want) | (got.view(np.uint32) == want.view(np.uint32)))
+
+
+@pytest.mark.gpu
+def test_solve_that_gives_up_is_marked(tmp_path):
+    """A cluster or grid whose waits run out (tests/cuda/give_up_check.cu, compiled with limits
+    of one poll) writes NaN velocities of all listed bodies."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    src = os.path.join(os.path.dirname(here), "box2c_gb300", "csrc")
+    nvcc = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
+    flags = ["-gencode", "arch=compute_103a,code=sm_103a", "-O2", "--fmad=false", "-std=c++17", "-DPUSH_SPIN_LIMIT=1", "-DRES_SPIN_LIMIT=1",
+             "-I", os.path.join(os.path.dirname(here), "include"), "-I", src]
+    exe = str(tmp_path / "give_up_check")
+    files = ["solve_api.cu", "resident.cu", "kernels.cu", "fused.cu", "arena.cu", "util.c"]
+    subprocess.run([nvcc, "-t", "0", *flags, os.path.join(here, "cuda", "give_up_check.cu"), *[os.path.join(src, f) for f in files], "-o", exe],
+                   check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "MISMATCH" not in r.stdout and "status no error" in r.stdout
