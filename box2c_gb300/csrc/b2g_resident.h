@@ -8,13 +8,11 @@
 
 #include "b2g_cluster.h"
 #include "b2g_device.h"
+#include "b2g_space.h"
 #include "b2g_stages.h"
 
 #include <cuda_runtime.h>
 
-/* dynamic shared memory per CTA, leaving 1 KB of the 227 KB opt-in limit for statics */
-#define RES_SMEM_MAX ( 226 * 1024 )
-#define RES_OVERFLOW_MAX 512
 /* polls of a grid barrier before it gives up (seconds; a cooperative launch never gets
  * there) */
 #ifndef RES_SPIN_LIMIT
@@ -54,12 +52,6 @@ struct ResOverflow
 	int2* jslot;
 };
 
-static inline __host__ __device__ size_t res_overflow_bytes( int R, int J )
-{
-	size_t E = 2u * (size_t)( R + J );
-	return 16u * ( (size_t)R + 2u * E ) + 4u * ( 3u * E + 2u * (size_t)J );
-}
-
 __device__ __forceinline__ ResOverflow res_carve_overflow( float4* base, int R, int J )
 {
 	int E = 2 * ( R + J );
@@ -78,10 +70,6 @@ __device__ __forceinline__ ResOverflow res_carve_overflow( float4* base, int R, 
  * on its own joint, read different banks. */
 #define RES_JOINT_WORDS ( (int)( sizeof( b2gJointDev ) / 4 ) + 1 )
 #define RES_JOINT_BYTES ( 4 * RES_JOINT_WORDS )
-
-/* Bytes of one body slot in shared memory: two state float4, the velocity terms (float4
- * and float), flags and an entry of the awake list. */
-#define RES_BODY_BYTES 60
 
 struct ResBodies
 {

@@ -255,16 +255,13 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	else
 	{
 		index_overflow();
-		/* states at L2; the terms of this CTA's share of the list as far as they fit */
+		/* states at L2; the terms of this CTA's share of the list, which fit (res_body_cap) */
 		L2Bodies G{ gst };
 		const int n = al - af;
-		if ( n <= P.bodyCap )
-		{
-			for ( int j = tid; j < n; j += T )
-				res_terms( W, rb, j, W.awake[af + j], sc );
-			bar.sync();
-			res_run<CL, T, false, false>( P, share, m, J, G, rb, gst, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
-		}
+		for ( int j = tid; j < n; j += T )
+			res_terms( W, rb, j, W.awake[af + j], sc );
+		bar.sync();
+		res_run<CL, T, false, false>( P, share, m, J, G, rb, gst, W.awake + af, n, bar, rank, sc, ov, s_ovSlots );
 	}
 	store_impulses( W, m, rows, colourRows, tid, T );
 }
@@ -452,16 +449,6 @@ static const ResDevice* res_device( void )
 	return d;
 }
 
-/* Row slots of the fullest CTA: every colour splits into shares that differ by one, CTA
- * 0 also holds the overflow rows. */
-static int res_row_cap( const int* cs, int ctas )
-{
-	int cap = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
-	for ( int c = 0; c < B2G_OVERFLOW; ++c )
-		cap += ( cs[c + 1] - cs[c] + ctas - 1 ) / ctas;
-	return cap > 0 ? cap : 1;
-}
-
 /* Shared memory of CTA 0 with its overflow cache, which is left out when it does not fit. */
 static size_t res_with_overflow( ResidentPlan* P, size_t bytes, int ovRows )
 {
@@ -494,9 +481,8 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 	cudaStream_t s = (cudaStream_t)w->stream;
 	cudaLaunchAttribute attr[1];
 
-	/* One CTA, else a whole cluster, when the rows fit with as many bodies as the list
-	 * has and one for every two rows (body indices are the caller's: the kernel copes
-	 * with more, at L2).  One CTA is the faster one as long as it holds the set (1200
+	/* One CTA, else a whole cluster, when it holds the set (res_body_cap).  One CTA is the
+	 * faster one as long as it does (1200
 	 * contacts: 58 us, 80 in a cluster); clusters of 2, 4 or 8 take what 16 take (2000
 	 * contacts: 78 to 82 us), so there is no space between the two; a grid is slower
 	 * wherever a cluster holds the set (20000 contacts: 201 us, 110 in a cluster). */
@@ -505,20 +491,14 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 	{
 		if ( ctas > 1 && d->cluster == 0 )
 			break;
+		P.bodyCap = res_body_cap( cs, P.awakeCount, ctas );
+		if ( P.bodyCap == 0 )
+			continue;
 		P.ctas = ctas;
 		P.rowCap = res_row_cap( cs, ctas );
-		int want = P.awakeCount > cs[B2G_COLORS] / 2 ? P.awakeCount : cs[B2G_COLORS] / 2;
-		want = ( want + ctas - 1 ) / ctas + 1;
-		size_t rows = 144u * (size_t)P.rowCap;
-		size_t tail = ctas > 1 && ovRows > 0 && ovRows <= RES_OVERFLOW_MAX ? res_overflow_bytes( ovRows, 0 ) + 16 : 0;
-		if ( rows + RES_BODY_BYTES * (size_t)want + tail > RES_SMEM_MAX )
-			continue;
-		/* the body slots take what the rows leave */
-		P.bodyCap = (int)( ( RES_SMEM_MAX - rows - tail ) / RES_BODY_BYTES ) & ~3;
-		if ( P.bodyCap > 4 * want )
-			P.bodyCap = ( 4 * want + 3 ) & ~3;
+		size_t rows = RES_ROW_BYTES * (size_t)P.rowCap;
 		size_t bytes = rows + RES_BODY_BYTES * (size_t)P.bodyCap;
-		if ( tail )
+		if ( ctas > 1 )
 			bytes = res_with_overflow( &P, bytes, ovRows );
 		if ( ctas > 1 )
 		{

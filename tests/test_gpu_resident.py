@@ -319,3 +319,39 @@ def test_solve_that_gives_up_is_marked(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert "MISMATCH" not in r.stdout and "status no error" in r.stdout
+
+
+def _slots(starts, ctas):
+    """Body slots that the rows of a set without overflow leave a CTA of 226 KB."""
+    rows = sum(-(-(b - a) // ctas) for a, b in zip(starts[:11], starts[1:12]))
+    return (226 * 1024 - 144 * rows) // 60
+
+
+# sets with as many listed bodies as a space holds beside their rows, and a few fewer and
+# more: the contacts of a pyramid with bodies in free fall added, one CTA and a cluster
+@pytest.mark.gpu
+@pytest.mark.parametrize("scene,ctas", [("21", 1), ("24", 1), ("27", 1), ("60", 16), ("100", 16), ("105", 16)])
+def test_resident_solver_body_edges(gpu, oracle, scene, ctas):
+    torch = pytest.importorskip("torch")
+    w, warm = _scene(oracle, scene)
+    oracle.step(w, count=warm)
+    cap = capture_step(oracle, w)
+    oracle.destroy(w)
+    w = oracle.drop_boxes(np.array([9.0], np.float32), np.array([0.5]), np.array([-1.0]), 0.6)
+    free = capture_step(oracle, w)
+    oracle.destroy(w)
+    one = free["awake"][0]
+    assert len(free["awake"]) == 1 and len(free["contactBodies"]) == 0
+    edge = _slots(cap["colorStart"], ctas)
+    n, listed = len(cap["statesIn"]), len(cap["awake"])
+    for slots in range(edge - 4, edge + 2):
+        for bodies in {ctas * slots - ctas + 1, ctas * slots}:
+            more = bodies - listed
+            assert more > 0
+            part = dict(cap)
+            for k in ("statesIn", "statesOut", "mass", "force", "damping"):
+                part[k] = np.concatenate([cap[k], np.repeat(free[k][one:one + 1], more, axis=0)])
+            part["awake"] = np.concatenate([cap["awake"], n + np.arange(more)]).astype(np.int32)
+            states, manifolds = solve_on_device(gpu, torch, part)
+            assert np.array_equal(states.view(np.uint32), part["statesOut"].view(np.uint32)), (slots, bodies)
+            assert np.array_equal(manifolds, cap["manifoldsOut"]), (slots, bodies)

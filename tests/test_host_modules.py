@@ -110,3 +110,15 @@ def test_pushed_copies_keep_their_order(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.startswith("ok"), r.stdout
+
+
+def test_resident_solver_spaces(tmp_path):
+    """Body slots of the resident contact solve's CTAs (box2c_gb300/csrc/b2g_space.h) over
+    every number of bodies up to the edge of each space (tests/c/space_check.c)."""
+    exe = str(tmp_path / "space_check")
+    src = os.path.join(REPO, "box2c_gb300", "csrc")
+    subprocess.run(["gcc", "-std=gnu17", "-O2", "-I", src, "-I", os.path.join(REPO, "include"),
+                    os.path.join(REPO, "tests", "c", "space_check.c"), "-o", exe], check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.startswith("ok"), r.stdout
