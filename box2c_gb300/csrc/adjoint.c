@@ -15,6 +15,7 @@
 
 #include <cuda_runtime_api.h>
 
+#include <stdatomic.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -28,6 +29,9 @@ typedef struct gTape
 	b2gTapeStep* hdr;
 } gTape;
 
+static atomic_int s_tapes; /* worlds with a tape */
+static void release_ctx( void );
+
 void gtape_free( gWorld* w )
 {
 	gTape* t = w->tape;
@@ -38,6 +42,8 @@ void gtape_free( gWorld* w )
 	b2g_free( t->hdr );
 	b2g_free( t );
 	w->tape = NULL;
+	if ( atomic_fetch_sub( &s_tapes, 1 ) == 1 )
+		release_ctx();
 }
 
 void b2World_BeginTape( b2WorldId worldId, int maxSteps )
@@ -57,6 +63,7 @@ void b2World_BeginTape( b2WorldId worldId, int maxSteps )
 		if ( t == NULL )
 			return;
 		w->tape = t;
+		atomic_fetch_add( &s_tapes, 1 );
 	}
 	if ( maxSteps > t->maxSteps )
 	{
@@ -171,7 +178,8 @@ typedef struct gAdjointCtx
 } gAdjointCtx;
 
 /* Device memory for the replays of a chunk of steps (a step that needs more is replayed
- * alone). */
+ * alone).  Kept from call to call while a world has a tape: allocating it takes about as
+ * long as a backward pass. */
 #define ADJOINT_CHUNK_BYTES ( (size_t)512 << 20 )
 
 static gAdjointCtx s_adj;
@@ -183,7 +191,19 @@ void b2World_GetBackwardCheck( int* manifoldMismatches, int* replayMismatches )
 	*replayMismatches = s_lastCheck[1];
 }
 
-static int ensure_ctx( int count, size_t bufBytes, size_t scratchFloats )
+static void release_ctx( void )
+{
+	cudaFreeHost( s_adj.hItems );
+	cudaFree( s_adj.dItems );
+	cudaFreeHost( s_adj.hBuf );
+	cudaFree( s_adj.dBuf );
+	cudaFree( s_adj.scratch );
+	cudaStream_t stream = s_adj.stream;
+	memset( &s_adj, 0, sizeof( s_adj ) );
+	s_adj.stream = stream;
+}
+
+static int ensure_ctx( int count, size_t bufBytes )
 {
 	if ( s_adj.stream == NULL && cudaStreamCreateWithFlags( &s_adj.stream, cudaStreamNonBlocking ) != cudaSuccess )
 		return -1;
@@ -210,15 +230,23 @@ static int ensure_ctx( int count, size_t bufBytes, size_t scratchFloats )
 			return -1;
 		s_adj.bufCap = bufBytes;
 	}
-	if ( scratchFloats > s_adj.scratchCap )
+	return 0;
+}
+
+static int ensure_scratch( size_t floats )
+{
+	if ( floats <= s_adj.scratchCap )
+		return 0;
+	cudaFree( s_adj.scratch );
+	s_adj.scratch = NULL;
+	s_adj.scratchCap = 0;
+	if ( cudaMalloc( (void**)&s_adj.scratch, sizeof( float ) * floats ) != cudaSuccess )
 	{
-		cudaFree( s_adj.scratch );
+		cudaGetLastError();
 		s_adj.scratch = NULL;
-		s_adj.scratchCap = 0;
-		if ( cudaMalloc( (void**)&s_adj.scratch, sizeof( float ) * scratchFloats ) != cudaSuccess )
-			return -1;
-		s_adj.scratchCap = scratchFloats;
+		return -1;
 	}
+	s_adj.scratchCap = floats;
 	return 0;
 }
 
@@ -227,7 +255,7 @@ int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStr
 {
 	if ( worldIds == NULL || count <= 0 || gradFinal == NULL || gradInitial == NULL )
 		return -1;
-	size_t headerBytes = 0, scratchFloats = 0, stepFloats = 0;
+	size_t headerBytes = 0, stepFloats = 0;
 	int steps = 1, bodies = 1, rows = 1, sub = 1;
 	for ( int i = 0; i < count; ++i )
 	{
@@ -251,20 +279,28 @@ int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStr
 		gWorld* w = gworld_get( worldIds[i] );
 		stepFloats += b2gd_adjoint_step_scratch( w->tape->bodies, w->tape->maxRows, w->dev.contactCap, sub );
 	}
-	/* as many steps at a time as fit the budget: the replays of a chunk run side by side */
-	int chunk = (int)( ADJOINT_CHUNK_BYTES / ( sizeof( float ) * stepFloats ) );
-	chunk = chunk < 1 ? 1 : ( chunk > steps ? steps : chunk );
-	for ( int i = 0; i < count; ++i )
-	{
-		gWorld* w = gworld_get( worldIds[i] );
-		scratchFloats += b2gd_adjoint_scratch( w->tape->bodies, w->tape->maxRows, chunk );
-	}
-	scratchFloats += stepFloats * (size_t)chunk;
 	size_t gradBytes = sizeof( float ) * (size_t)count * ( 12u * (size_t)bodyStride + 2u * (size_t)shapeStride );
 	size_t statusBytes = sizeof( int ) * 4u * (size_t)count;
 	size_t bufBytes = round_up( headerBytes, 256 ) + round_up( gradBytes, 256 ) + statusBytes;
-	if ( ensure_ctx( count, bufBytes, scratchFloats ) != 0 )
+	if ( ensure_ctx( count, bufBytes ) != 0 )
 		return -1;
+	/* as many steps at a time as fit the budget, as the replays of a chunk run side by side;
+	 * fewer when the device has less */
+	size_t budget = ADJOINT_CHUNK_BYTES / ( sizeof( float ) * stepFloats );
+	int chunk = budget > (size_t)steps ? steps : ( budget < 1 ? 1 : (int)budget );
+	for ( ;; chunk /= 2 )
+	{
+		size_t floats = stepFloats * (size_t)chunk;
+		for ( int i = 0; i < count; ++i )
+		{
+			gTape* t = gworld_get( worldIds[i] )->tape;
+			floats += b2gd_adjoint_scratch( t->bodies, t->maxRows, chunk );
+		}
+		if ( ensure_scratch( floats ) == 0 )
+			break;
+		if ( chunk == 1 )
+			return -1;
+	}
 
 	char* hb = s_adj.hBuf;
 	char* db = s_adj.dBuf;

@@ -125,8 +125,10 @@ B2_API void b2World_BeginTape( b2WorldId worldId, int maxSteps );
 B2_API int b2World_GetTapeSteps( b2WorldId worldId );
 B2_API int b2World_StepBackward( b2WorldId worldId, const float* gradFinal, float* gradInitial, float* gradFriction );
 
-/* The backward pass of `count` recorded worlds in one launch (one warp per world).
- * Arrays are per world with fixed strides: gradFinal / gradInitial 6 * bodyStride
+/* The backward pass of `count` recorded worlds.  Their steps are replayed side by side, as
+ * many as 512 MiB of device memory hold at a time, or fewer when that much cannot be had;
+ * the memory is kept for the next call until the last recording is freed (with its world,
+ * or by b2World_BeginTape with 0 steps).  Arrays are per world with fixed strides: gradFinal / gradInitial 6 * bodyStride
  * floats per world, gradFriction shapeStride floats per world. */
 B2_API int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStride, int shapeStride, const float* gradFinal,
 									  float* gradInitial, float* gradFriction );

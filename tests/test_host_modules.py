@@ -122,3 +122,17 @@ def test_resident_solver_spaces(tmp_path):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.startswith("ok"), r.stdout
+
+
+def test_backward_pass_with_little_memory(tmp_path):
+    """The backward call's device memory (box2c_gb300/csrc/adjoint.c) against a runtime that
+    has only so much (tests/c/adjoint_memory.c)."""
+    exe = str(tmp_path / "adjoint_memory")
+    src = os.path.join(REPO, "box2c_gb300", "csrc")
+    cuda = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+    subprocess.run(["gcc", "-std=gnu17", "-O2", "-I", src, "-I", os.path.join(REPO, "include"), "-I", cuda,
+                    os.path.join(REPO, "tests", "c", "adjoint_memory.c"), os.path.join(src, "adjoint.c"), "-o", exe],
+                   check=True, capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.startswith("ok"), r.stdout
