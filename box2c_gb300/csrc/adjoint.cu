@@ -942,19 +942,21 @@ __device__ void snapshot( const AdjStep& L, float* D, int N, int index )
 	__syncwarp();
 }
 
-/* The replay of step stepCount - 1 - (first + blockIdx.x) of world blockIdx.y.  Reads the
- * tape and the world; writes that step's scratch and, added, the world's status. */
-__global__ void __launch_bounds__( ADJ_WARP ) k_adjoint_replay( const b2gAdjointItem* items, int first )
+/* Block n i + t of a chunk of n steps: the replay of step stepCount - 1 - (first + t) of
+ * world i.  Reads the tape and the world; writes that step's scratch and, added, the
+ * world's status. */
+__global__ void __launch_bounds__( ADJ_WARP ) k_adjoint_replay( const b2gAdjointItem* items, int first, int n )
 {
-	const b2gAdjointItem& it = items[blockIdx.y];
-	const int ts = it.stepCount - 1 - ( first + (int)blockIdx.x );
+	const int t = (int)( blockIdx.x % (unsigned)n );
+	const b2gAdjointItem& it = items[blockIdx.x / (unsigned)n];
+	const int ts = it.stepCount - 1 - ( first + t );
 	if ( ts < 0 )
 		return;
 	const b2gDevWorld& W = it.W;
 	const int lane = threadIdx.x;
 	const int N = it.bodies;
 	const AdjStep L = adj_step( N, it.maxRows, it.maxSub );
-	float* D = it.stepScratch + (size_t)blockIdx.x * it.stepFloats;
+	float* D = it.stepScratch + (size_t)t * it.stepFloats;
 	int* table = (int*)( D + L.total ); /* rows of the step before by contact id, where set */
 	const b2gTapeStep& h = it.steps[ts];
 	const b2gStepConst& sc = h.sc;
@@ -1922,7 +1924,8 @@ extern "C" int b2gd_adjoint_launch( const b2gAdjointItem* dItems, int count, int
 	for ( int first = 0; first < steps; first += chunk )
 	{
 		const int n = steps - first < chunk ? steps - first : chunk;
-		k_adjoint_replay<<<dim3( (unsigned)n, (unsigned)count ), ADJ_WARP, 0, s>>>( dItems, first );
+		/* in one dimension of the grid, the only one for more than 65535 worlds or steps */
+		k_adjoint_replay<<<(unsigned)n * (unsigned)count, ADJ_WARP, 0, s>>>( dItems, first, n );
 		kernel<<<count, ADJ_WARP, smem ? bytes : 0, s>>>( dItems, first, n );
 		k_adjoint_friction<<<count, ADJ_FRICTION, 0, s>>>( dItems, first, n );
 	}

@@ -89,3 +89,20 @@ def test_backward_in_chunks(gpu, maker, copies):
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
     for w in one + many:
         gpu.destroy(w)
+
+
+def test_backward_of_many_worlds(gpu):
+    """More worlds than a grid's second dimension holds, each without a recorded step: the
+    kernels are launched and do nothing."""
+    import ctypes as C
+
+    torch = pytest.importorskip("torch")
+    launch = gpu.lib.b2gd_adjoint_launch
+    launch.argtypes = [C.c_void_p] + [C.c_int] * 6 + [C.c_void_p]
+    launch.restype = C.c_int
+    worlds = 70000
+    items = torch.zeros(worlds * 4096, dtype=torch.uint8, device="cuda:0")  # an item is smaller
+    torch.cuda.synchronize()
+    assert launch(items.data_ptr(), worlds, 1, 1, 1, 1, 4, None) == 0
+    torch.cuda.synchronize()
+    assert not items.any()
