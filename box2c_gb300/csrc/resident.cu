@@ -269,7 +269,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 /* The solver stage over a cooperative grid: body states in global memory, rows in shared
  * memory (ONCHIP) or in the row arrays, where row k of the colour-major order is entry k.
  * ctl: the barrier's arrival count, the count of finished CTAs and the give-up flag, all
- * zero at the launch and again when the kernel ends. */
+ * zero at the launch. */
 template <int T, bool ONCHIP>
 __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ b2gDevWorld W, const __grid_constant__ ResidentPlan P,
 														const __grid_constant__ b2gStepConst sc, int* ctl )
@@ -360,9 +360,6 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 				st[8 * (size_t)b + k] = __int_as_float( 0x7fffffff );
 		}
 	}
-	__syncthreads();
-	if ( tid < 3 )
-		ctl[tid] = 0;
 }
 
 /* ------------------------------------------------------------------ host side */
@@ -464,8 +461,8 @@ static size_t res_with_overflow( ResidentPlan* P, size_t bytes, int ovRows )
 
 /* The solver stage of caller buffers in one launch: the number of launches, 0 when this
  * device or set needs the per-phase kernels, or -1 on a launch error.  ctl: four ints of
- * device memory, zero, or cleared here when `clear` is set. */
-extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl, int clear )
+ * device memory for a grid's barrier. */
+extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl )
 {
 	const ResDevice* d = res_device();
 	if ( d == nullptr )
@@ -530,7 +527,7 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 		if ( terms > RES_SMEM_MAX )
 			return 0;
 	}
-	if ( clear && cudaMemsetAsync( ctl, 0, 4 * sizeof( int ), s ) != cudaSuccess )
+	if ( cudaMemsetAsync( ctl, 0, 4 * sizeof( int ), s ) != cudaSuccess )
 		return -1;
 	size_t bytes = res_with_overflow( &P, 144u * (size_t)P.rowCap + terms, ovRows );
 	auto kernel = onChip ? (ResGridKernel)k_solve_grid<GRID_THREADS, true> : (ResGridKernel)k_solve_grid<GRID_THREADS, false>;

@@ -7,7 +7,7 @@
  * integrate positions / relax, restitution, store impulses) as one resident kernel
  * (resident.cu), or as one kernel per phase (b2gd_contact_solver) where the device
  * launches neither a cluster nor a cooperative grid.  The scratch (barrier words, and
- * rows for sets larger than all shared memory) is taken from the stream-ordered device
+ * rows for sets of which a CTA's share exceeds its shared memory) is taken from the stream-ordered device
  * allocator for the call.
  */
 #include "b2g_device.h"
@@ -22,7 +22,7 @@ static_assert( sizeof( b2gManifold ) == sizeof( b2Manifold ), "device manifold m
 static_assert( sizeof( b2gPoint ) == sizeof( b2ManifoldPoint ), "device manifold point must have the b2ManifoldPoint layout" );
 
 extern "C" int b2gd_contact_solver( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc );
-extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl, int clear );
+extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl );
 
 static void make_soft( float hertz, float zeta, float h, float* out )
 {
@@ -122,14 +122,14 @@ extern "C" int b2SolveContacts( const b2ContactSolveDesc* desc )
 	if ( b2gd_contact_desc( desc, &w, &plan, &sc ) != 0 )
 		return -1;
 	cudaStream_t s = (cudaStream_t)desc->stream;
-	/* a grid's barrier words, then the rows of a set too large for shared memory */
+	/* a grid's barrier words, then rows that do not fit in shared memory */
 	char* scratch = nullptr;
 	int n = desc->contactCount > 0 ? desc->contactCount : 1;
 	cudaError_t e = cudaMallocAsync( (void**)&scratch, 256u + 16u * B2G_ROW_FLOAT4 * (size_t)n, s );
 	if ( e != cudaSuccess )
 		return (int)e;
 	b2gd_contact_rows( &w, scratch + 256, n );
-	if ( b2gd_contact_resident( &w, &plan, &sc, (int*)scratch, 1 ) == 0 )
+	if ( b2gd_contact_resident( &w, &plan, &sc, (int*)scratch ) == 0 )
 		b2gd_contact_solver( &w, &plan, &sc );
 	e = cudaGetLastError();
 	cudaError_t f = cudaFreeAsync( scratch, s );

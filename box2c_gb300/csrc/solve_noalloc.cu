@@ -8,8 +8,10 @@
  * that may block on other work or fail under memory pressure halfway through a run.
  * Both pass their own buffers and want the solver to take no memory of its own.
  *
- * Such sets fit on chip (resident.cu), so the array is read only where the device
- * launches neither a cluster nor a cooperative grid.
+ * Nearly all such sets fit on chip (resident.cu).  The array holds the rows of those that
+ * do not, whose overflow rows (more than about 1600 contacts) or listed bodies are more
+ * than one CTA takes, and of all where the device launches neither a cluster nor a
+ * cooperative grid.
  *
  * The rows: B2G_ROW_FLOAT4 float4 arrays of `contactCount` entries carved from one block, the same
  * layout b2SolveContacts uses (b2gd_contact_rows).  k_prepare writes every field of
@@ -17,8 +19,9 @@
  * cleared between calls.
  *
  * One array per device: calls that overlap on one device (two host threads, or two
- * streams whose calls are not ordered) write the same rows and race.  The caller orders
- * them.
+ * streams whose calls are not ordered) write the same rows, and those that run as a grid
+ * pass one another's barriers, so they race.  The caller orders them.  The barrier's words
+ * are cleared in every call, so that calls that did overlap leave nothing behind.
  */
 #include "b2g_device.h"
 
@@ -29,12 +32,12 @@
 #include <mutex>
 
 extern "C" int b2gd_contact_solver( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc );
-extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl, int clear );
+extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, const b2gStepConst* sc, int* ctl );
 extern "C" int b2gd_contact_desc( const b2ContactSolveDesc* d, b2gDevWorld* w, b2gSolvePlan* plan, b2gStepConst* sc );
 extern "C" void b2gd_contact_rows( b2gDevWorld* w, void* base, int rows );
 
 /* 144 bytes per contact row: B2G_ROW_FLOAT4 float4; then the barrier words of a
- * cooperative grid, zero between calls (the kernel leaves them so) */
+ * cooperative grid */
 static __device__ __align__( 256 ) float4 g_contactRows[B2G_ROW_FLOAT4 * B2_SOLVE_NOALLOC_MAX_CONTACTS + 1];
 
 enum
@@ -129,7 +132,7 @@ extern "C" int b2SolveContactsNoAlloc( const b2ContactSolveDesc* desc )
 	int n = desc->contactCount > 0 ? desc->contactCount : 1;
 	b2gd_contact_rows( &w, rows, n );
 	int* ctl = (int*)( (float4*)rows + B2G_ROW_FLOAT4 * B2_SOLVE_NOALLOC_MAX_CONTACTS );
-	if ( b2gd_contact_resident( &w, &plan, &sc, ctl, 0 ) == 0 )
+	if ( b2gd_contact_resident( &w, &plan, &sc, ctl ) == 0 )
 		b2gd_contact_solver( &w, &plan, &sc );
 	return (int)cudaGetLastError();
 }

@@ -196,8 +196,9 @@ B2_API int b2SolveContacts( const b2ContactSolveDesc* desc );
  *   address, and again after the device's context was replaced (cudaDeviceReset); make
  *   such calls before any stream capture starts.
  * - Nothing in the array has to start at zero: every row is written before it is read.
- * - Calls that overlap on one device share the array and race: order them (one stream,
- *   or events between streams, and one host thread at a time). */
+ * - Calls that overlap on one device share the array, and the barrier of sets too large
+ *   for a cluster, and race: order them (one stream, or events between streams, and one
+ *   host thread at a time). */
 #define B2_SOLVE_NOALLOC_MAX_CONTACTS 16384
 #define B2_SOLVE_NOALLOC_TOO_LARGE ( -2 )
 #define B2_SOLVE_NOALLOC_DEVICE_LIMIT ( -3 )

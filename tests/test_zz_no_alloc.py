@@ -123,3 +123,17 @@ def test_no_alloc_takes_no_device_memory(gpu, oracle):
     assert gpu.lib.b2SolveContacts(C.byref(d)) == 0
     torch.cuda.synchronize()
     assert _default_pool_used_high(reset=False) > base
+
+
+@pytest.mark.gpu
+def test_no_alloc_rows_in_the_array(gpu, oracle):
+    """More overflow rows than a CTA holds: a grid with its rows in the fixed array, twice."""
+    torch = pytest.importorskip("torch")
+    _bind(gpu.lib)
+    cap = _capture(oracle, oracle.shelves(640, 16, 8), 6)
+    assert 144 * (cap["colorStart"][12] - cap["colorStart"][11] + 115) > 226 * 1024
+    assert len(cap["contactBodies"]) <= MAX_CONTACTS
+    for _ in range(2):
+        got = _run(torch, gpu.lib.b2SolveContactsNoAlloc, cap)
+        assert np.array_equal(got[0], cap["statesOut"])  # shelves: the sign of a zero
+        assert np.array_equal(got[1], cap["manifoldsOut"])
