@@ -444,6 +444,14 @@ extern "C" void* b2gd_device_view( void* pinned )
 	return d;
 }
 
+extern "C" int b2gd_sms( void )
+{
+	int dev = 0, n = 0;
+	if ( cudaGetDevice( &dev ) != cudaSuccess || cudaDeviceGetAttribute( &n, cudaDevAttrMultiProcessorCount, dev ) != cudaSuccess || n < 1 )
+		return 1;
+	return n;
+}
+
 /* Hit test of one contact (reference src/solver.c:1688-1712): the point with the largest
  * approach speed above the threshold among the points that carry a normal impulse. */
 __global__ void k_hit_events( const b2gManifold* manifolds, const int* ids, int n, float threshold, float4* out )

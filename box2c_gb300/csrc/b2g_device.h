@@ -106,6 +106,8 @@ int b2gd_upload_shape_boxes( b2gDevWorld* w, int shapeId, const float* aabb4, co
 int b2gd_download_bodies( b2gDevWorld* w, void* state, void* xf, void* centers, int count );
 /* The device's view of pinned host memory; null when there is none. */
 void* b2gd_device_view( void* pinned );
+/* SMs of the current device, at least 1. */
+int b2gd_sms( void );
 int b2gd_download_manifolds( b2gDevWorld* w, b2gManifold* out, uint32_t* flags, int count );
 /* Hit test of the contacts ids[0..n) after the solver stage (reference
  * src/solver.c:1670-1723): out[8 k ..] = hit flag, approach speed and point of the

@@ -27,7 +27,6 @@ struct ResidentPlan
 	int activeCount;
 	int awakeCount;
 	int bodyIdCount; /* body ids of a world (0: caller buffers, ids unknown) */
-	int ctas;
 	int rowCap;	  /* row slots per CTA (0: rows in the row arrays) */
 	int bodyCap;  /* body slots per CTA in shared memory; a grid's velocity-term slots */
 	int jointCap; /* joint slots per CTA in shared memory (0: joints in the joint array) */

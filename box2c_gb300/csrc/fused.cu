@@ -430,7 +430,6 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 	size_t one = b2g_bin_bytes( cs[B2G_COLORS], plan->bodyIdCount, 0 );
 	if ( b2g_bin_bytes( cs[B2G_COLORS], plan->bodyIdCount, joints ) <= RES_SMEM_MAX )
 	{
-		P.ctas = 1;
 		P.rowCap = cs[B2G_COLORS] > 0 ? cs[B2G_COLORS] : 1;
 		P.bodyCap = ( plan->bodyIdCount + 3 ) & ~3;
 		P.jointCap = joints;
@@ -451,7 +450,6 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 		bins.joints = bins.rows + cs[B2G_COLORS];
 		bins.awake = bins.joints + joints;
 		bins.slot = bins.awake + plan->awakeCount;
-		P.ctas = 1;
 		P.rowCap = plan->binRows > 0 ? plan->binRows : 1;
 		P.bodyCap = ( plan->binBodies + 3 ) & ~3;
 		P.jointCap = plan->binJoints;
@@ -468,7 +466,6 @@ extern "C" int b2gd_solver_fused( b2gDevWorld* w, const b2gSolvePlan* plan, cons
 	if ( plan->bodyIdCount >= 65536 )
 		return 0;
 	const int CL = FUSED_CLUSTER;
-	P.ctas = CL;
 	P.bodyCap = plan->bodyBlock;
 	S.bodyCapInv = P.bodyCap > 1 ? (unsigned)( ( ( 1ull << 32 ) + (unsigned long long)P.bodyCap - 1 ) / (unsigned long long)P.bodyCap ) : 0u;
 	int perCta[B2G_FUSED_CTAS] = { ovR };

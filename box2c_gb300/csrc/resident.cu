@@ -491,7 +491,6 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 		P.bodyCap = res_body_cap( cs, P.awakeCount, ctas );
 		if ( P.bodyCap == 0 )
 			continue;
-		P.ctas = ctas;
 		P.rowCap = res_row_cap( cs, ctas );
 		size_t rows = RES_ROW_BYTES * (size_t)P.rowCap;
 		size_t bytes = rows + RES_BODY_BYTES * (size_t)P.bodyCap;
@@ -516,7 +515,6 @@ extern "C" int b2gd_contact_resident( b2gDevWorld* w, const b2gSolvePlan* plan, 
 		widest = cs[c + 1] - cs[c] > widest ? cs[c + 1] - cs[c] : widest;
 	int ctas = ( widest + 63 ) / 64;
 	ctas = ctas < 1 ? 1 : ( ctas > d->sms ? d->sms : ctas );
-	P.ctas = ctas;
 	P.rowCap = res_row_cap( cs, ctas );
 	P.bodyCap = ( ( P.awakeCount + ctas - 1 ) / ctas + 3 ) & ~3;
 	size_t terms = 20u * (size_t)P.bodyCap;

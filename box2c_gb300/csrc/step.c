@@ -1151,7 +1151,7 @@ static void build_solve_lists( gWorld* w, b2gSolvePlan* plan )
  * changing colouring would have it done again each step.  Leaves the plan without bins
  * when an island is too large, or when a kinematic body, which belongs to no island,
  * could be shared. */
-#define BINS_WANTED ( 4 * 152 ) /* a few CTAs for each SM */
+#define BINS_PER_SM 4
 
 static void build_bins( gWorld* w, b2gSolvePlan* plan )
 {
@@ -1171,7 +1171,7 @@ static void build_bins( gWorld* w, b2gSolvePlan* plan )
 	int* bodyBin = islandBin + w->islandCap;
 	/* islands into bins in set order; a static contact or two per body are not counted in
 	 * the island, so leave room for one each */
-	int target = ( rows + bodies ) / BINS_WANTED;
+	int target = ( rows + bodies ) / ( BINS_PER_SM * b2gd_sms() );
 	target = target < 160 ? 160 : target;
 	int bins = 1, weight = 0, binRows = 0, binBodies = 0, binJoints = 0;
 	for ( int i = 0; i < islands; ++i )
