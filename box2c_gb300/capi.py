@@ -178,6 +178,8 @@ class Backend:
         S.b2s_chain_scene.restype = WorldId
         S.b2s_event_scene.argtypes = [C.c_int, C.c_uint64]
         S.b2s_event_scene.restype = WorldId
+        S.b2s_filter_scene.argtypes = [C.c_int, C.c_uint64]
+        S.b2s_filter_scene.restype = WorldId
         S.b2s_empty_world.argtypes = []
         S.b2s_empty_world.restype = WorldId
         S.b2s_add_body.argtypes = [WorldId, C.c_int]
@@ -256,6 +258,9 @@ class Backend:
     def joint_zoo(self, copies: int = 2, flags: int = 0, seed: int = 1250) -> WorldId:
         """Every joint type: ropes, pendulum, elevators, car, welds, motor and mouse joints, an overflowing spider."""
         return self._made(self.scenes.b2s_joint_zoo(copies, flags, seed))
+
+    def filter_scene(self, count: int, seed: int = 7) -> WorldId:
+        return self._made(self.scenes.b2s_filter_scene(count, seed))
 
     def event_scene(self, count: int = 40, seed: int = 1243) -> WorldId:
         return self._made(self.scenes.b2s_event_scene(count, seed))

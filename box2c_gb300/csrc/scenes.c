@@ -1021,6 +1021,44 @@ b2BodyId b2s_add_square( b2WorldId worldId, float h )
 	return bodyId;
 }
 
+b2WorldId b2s_filter_scene( int count, uint64_t seed )
+{
+	b2WorldDef wd = b2s_world_def();
+	b2WorldId worldId = b2CreateWorld( &wd );
+	if ( B2_IS_NULL( worldId ) )
+		return worldId;
+	b2s_ground( worldId, 0.6f );
+
+	static const int groups[] = { 0, 0, -1, 1, 2, -2 };
+	b2sRandom rng;
+	b2s_seed( &rng, seed );
+	b2BodyDef bd = b2DefaultBodyDef();
+	bd.type = b2_dynamicBody;
+	bd.enableSleep = false;
+	int row = 1;
+	while ( row * row < count )
+		row += 1;
+	for ( int k = 0; k < count; ++k )
+	{
+		bd.position = ( b2Vec2 ){ 0.9f * (float)( k % row - row / 2 ), 1.0f + 0.9f * (float)( k / row ) };
+		b2BodyId bodyId = b2CreateBody( worldId, &bd );
+		for ( int i = 0; i < 2; ++i )
+		{
+			b2ShapeDef sd = b2DefaultShapeDef();
+			sd.density = 1.0f;
+			uint32_t category = b2s_next( &rng ) % 3u, mask = 1u + b2s_next( &rng ) % 7u, group = b2s_next( &rng ) % 6u;
+			uint32_t sensor = b2s_next( &rng ) % 4u;
+			sd.filter.categoryBits = 1u << category;
+			sd.filter.maskBits = mask;
+			sd.filter.groupIndex = groups[group];
+			sd.isSensor = sensor == 0;
+			b2Polygon box = b2MakeOffsetBox( 0.4f, 0.3f, ( b2Vec2 ){ i == 0 ? -0.2f : 0.2f, 0.0f }, 0.0f );
+			b2CreatePolygonShape( bodyId, &sd, &box );
+		}
+	}
+	return worldId;
+}
+
 b2WorldId b2s_event_scene( int count, uint64_t seed )
 {
 	b2WorldDef wd = b2s_world_def();

@@ -120,6 +120,11 @@ b2BodyId b2s_add_square( b2WorldId worldId, float h );
  * carries a sensor ring of radius 0.8. */
 b2WorldId b2s_event_scene( int count, uint64_t seed );
 
+/* A grid of overlapping bodies of two shapes each, in free fall onto a ground, with drawn
+ * filter categories, masks and groups (zero, equal or not, of both signs) and sensors.
+ * Sleep off. */
+b2WorldId b2s_filter_scene( int count, uint64_t seed );
+
 /* Joint scene with every joint type: `copies` copies 40 m apart on one static ground,
  * each with a distance-joint rope (soft with length limits, rigid, motorised), a
  * revolute pendulum (spring, limits, motor), two prismatic elevators (motor and limits;

@@ -282,3 +282,12 @@ def test_gpu_events_match_oracle(gpu, oracle):
         gpu.destroy(wg)
         oracle.destroy(wo)
     assert all(t > 0 for t in totals), totals
+
+
+# the device pair query (256 moved proxies and more; below, the host's) applies the shape
+# filters: categories and masks, equal groups of both signs, shapes of one body, two sensors
+@pytest.mark.gpu
+@pytest.mark.parametrize("count,seed", [(100, 7), (400, 7), (1500, 8)])
+def test_pair_filters(gpu, oracle, count, seed):
+    bad, detail, _ = lockstep(gpu, oracle, lambda b: b.filter_scene(count, seed), 40, check_manifolds=True)
+    assert bad is None, detail
