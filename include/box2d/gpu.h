@@ -30,7 +30,11 @@ B2_API int b2World_GetStatus( b2WorldId worldId );
 B2_API int b2World_GetToiEventCount( b2WorldId worldId );
 
 /* Device stage timings of the last step (milliseconds, CUDA events on the world's
- * stream): whole step, narrowphase, solver (prepare .. store impulses), finalisation. */
+ * stream): whole step, narrowphase, solver (prepare .. store impulses), finalisation.  A
+ * solver stage in one launch finalises the bodies too: its time is in `solve`, and
+ * `finalize` is about zero.  While timing is on, the solver does not start beside the
+ * narrowphase, so that the stages can be told apart; such a step takes a few microseconds
+ * longer. */
 typedef struct b2DeviceTimes
 {
 	float step; /* whole b2World_Step, host work included */
@@ -77,7 +81,12 @@ B2_API void b2World_EnableFusedSolver( b2WorldId worldId, bool flag );
  * with more bodies than the batched solver holds (about 6900) is stepped alone in the
  * same call.  Every world gets exactly the results b2World_Step would give it alone.
  * Invalid, failed or repeated ids are skipped.  Not thread-safe: one batch at a time
- * per process. */
+ * per process.
+ *
+ * Host work of a batch, and the pair rules of large single steps, run on one thread per
+ * core (at most 32).  After a job its threads watch for the next one for 100 microseconds,
+ * yielding their core to any other thread, before they sleep: a program that steps more
+ * often than that keeps them running between steps. */
 B2_API void b2World_StepBatch( const b2WorldId* worldIds, int count, float timeStep, int subStepCount );
 
 /* Device milliseconds of the last batched step's narrowphase and solver segments (both
@@ -112,9 +121,9 @@ B2_API b2BatchStats b2World_GetBatchStats( void );
  *   gradInitial   dL/d(state before the first recorded step)    (6 x bodies, out)
  *   gradFriction  dL/d(shape friction) per shape id             (shapes, out, may be null)
  * The discrete choices of each step (pairs, colours, contact features, active clamps)
- * are those of the recorded steps.  Supported: polygon, capsule and segment shapes
- * without joints or overflow-colour constraints, and steps without time-of-impact
- * events; otherwise B2_ADJOINT_UNSUPPORTED.
+ * are those of the recorded steps.  Supported: polygon, capsule, segment and circle shapes
+ * without joints or chain links, and steps without time-of-impact events; otherwise
+ * B2_ADJOINT_UNSUPPORTED.
  * B2_ADJOINT_REPLAY_MISMATCH reports that the recomputed contact geometry differed from
  * the recorded one (the world changed after recording).  No counterpart in the
  * reference API. */
@@ -128,8 +137,9 @@ B2_API int b2World_StepBackward( b2WorldId worldId, const float* gradFinal, floa
 /* The backward pass of `count` recorded worlds.  Their steps are replayed side by side, as
  * many as 512 MiB of device memory hold at a time, or fewer when that much cannot be had;
  * the memory is kept for the next call until the last recording is freed (with its world,
- * or by b2World_BeginTape with 0 steps).  Arrays are per world with fixed strides: gradFinal / gradInitial 6 * bodyStride
- * floats per world, gradFriction shapeStride floats per world. */
+ * or by b2World_BeginTape with 0 steps).  Arrays are per world with fixed strides:
+ * gradFinal / gradInitial 6 * bodyStride floats per world, gradFriction shapeStride
+ * floats per world. */
 B2_API int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int bodyStride, int shapeStride, const float* gradFinal,
 									  float* gradInitial, float* gradFriction );
 
@@ -139,7 +149,9 @@ B2_API int b2World_StepBackwardBatch( const b2WorldId* worldIds, int count, int 
 B2_API void b2World_GetBackwardCheck( int* manifoldMismatches, int* replayMismatches );
 
 /* Copies p.x p.y q.c q.s v.x v.y w (7 floats) of every body id into out (7 * capacity
- * floats).  One device-to-host copy per call.  Returns the number of body ids. */
+ * floats).  In the 64 steps after a read, steps leave the states in host memory as they
+ * go, and a read copies nothing from the device; otherwise it is one device-to-host copy.
+ * Returns the number of body ids. */
 B2_API int b2World_GetBodyStates( b2WorldId worldId, float* out, int capacity );
 
 /* One soft-step contact solve on caller-owned device buffers: the solver stage of
