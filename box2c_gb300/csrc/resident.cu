@@ -266,6 +266,27 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_cluster( const __grid_constant
 	store_impulses( W, m, rows, colourRows, tid, T );
 }
 
+/* CTAs of a grid that ended before this one. */
+__device__ __forceinline__ int grid_ended( int* ctl )
+{
+	int n;
+	asm volatile( "atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"( n ) : "l"( ctl + 1 ) : "memory" );
+	return n;
+}
+
+/* A grid of which a CTA gave up on another has no result: NaN velocities of the listed bodies
+ * and of those with contacts, by one thread, as it is hardly ever called. */
+__device__ __noinline__ void mark_lost( const b2gDevWorld& W, int listed, int contacts )
+{
+	float* st = (float*)W.state;
+	for ( int i = 0; i < listed + 2 * contacts; ++i )
+	{
+		const int b = i < listed ? W.awake[i] : W.cBodies[i - listed];
+		for ( int k = 0; k < 3 && b >= 0; ++k )
+			st[8 * (size_t)b + k] = __int_as_float( 0x7fffffff );
+	}
+}
+
 /* The solver stage over a cooperative grid: body states in global memory, rows in shared
  * memory (ONCHIP) or in the row arrays, where row k of the colour-major order is entry k.
  * ctl: the barrier's arrival count, the count of finished CTAs and the give-up flag, all
@@ -276,7 +297,7 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 {
 	extern __shared__ float4 smem[];
 	__shared__ ResShare share[B2G_COLORS];
-	__shared__ int s_ovSlots, s_last;
+	__shared__ int s_ovSlots;
 	const int rank = blockIdx.x, ctas = gridDim.x, tid = threadIdx.x;
 	const int* cs = P.colorStart;
 	const int ovRows = cs[B2G_COLORS] - cs[B2G_OVERFLOW];
@@ -337,29 +358,9 @@ __global__ void __launch_bounds__( T, 1 ) k_solve_grid( const __grid_constant__ 
 			const SmemRows part = { m.idx + f, m.nf + f, m.ms + f, m.anc0 + f, m.anc1 + f, m.coef0 + f, m.coef1 + f, m.imp0 + f, m.imp1 + f };
 			store_impulses( W, part, share[c].count, c == B2G_OVERFLOW ? 0 : share[c].count, tid, T );
 		}
-	__syncthreads();
-	if ( tid == 0 )
-	{
-		__threadfence();
-		s_last = atomicAdd( ctl + 1, 1 ) == ctas - 1;
-		__threadfence();
-	}
-	__syncthreads();
-	if ( s_last == 0 )
-		return;
-	/* every CTA is past its last barrier, and its last write of a state */
-	if ( *(volatile int*)( ctl + 2 ) != 0 )
-	{
-		/* a grid of which a CTA gave up on another has no result */
-		float* st = (float*)W.state;
-		const int total = cs[B2G_COLORS];
-		for ( int i = tid; i < P.awakeCount + 2 * total; i += T )
-		{
-			const int b = i < P.awakeCount ? W.awake[i] : W.cBodies[i - P.awakeCount];
-			for ( int k = 0; k < 3 && b >= 0; ++k )
-				st[8 * (size_t)b + k] = __int_as_float( 0x7fffffff );
-		}
-	}
+	/* no CTA writes a state after its last barrier */
+	if ( tid == 0 && grid_ended( ctl ) == ctas - 1 && *(volatile int*)( ctl + 2 ) != 0 )
+		mark_lost( W, P.awakeCount, cs[B2G_COLORS] );
 }
 
 /* ------------------------------------------------------------------ host side */
