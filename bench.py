@@ -647,8 +647,8 @@ def run_gpu(args):
         "e2e": {"value": round(e2e_ms, 4), "unit": "ms/step", "h2d_bytes_per_step": int(np.mean(h2d)),
                 "d2h_bytes_per_step": int(np.mean(d2h)),
                 "bytes_source": "counted by the library per step (b2DeviceTimes host/device bytes): staged contacts, "
-                                "solve lists, counters, mapped events and records, and the body-state download of "
-                                "b2World_GetBodyStates"},
+                                "solve lists, counters, mapped events and records, and the body states that a step "
+                                "writes into host memory for b2World_GetBodyStates, or the call downloads"},
         "gpu_launches": int(sum(rec["launches"])),
         "cpu_baseline": cpu,
         "clocks": clocks, "status": status, "toi_events": toi,

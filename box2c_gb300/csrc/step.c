@@ -1466,6 +1466,9 @@ void gstep_finish( gWorld* w )
 	w->lastRecordCount = recordCount;
 	if ( w->io.counters[2] != 0 )
 		w->status = -1; /* a solver CTA gave up waiting for another */
+	/* finalisation wrote each awake body's pose and velocity into the mirrors */
+	if ( w->dev.mirrorXf != NULL )
+		w->dev.d2hBytes += 48 * (long long)w->awake.count;
 	report_hits( w );
 	double tr = b2g_now_ms();
 	/* records reach the host through mapped memory: 48 bytes, 80 for fast shapes */

@@ -47,7 +47,8 @@ typedef struct b2DeviceTimes
 	int fusedSolver; /* 1 when the last step's solver stage ran as one fused launch */
 	/* bytes the last step moved between host and device: copies (setup changes, new
 	 * contacts, solve lists, tree nodes, counters, time-of-impact poses) and device
-	 * reads or writes of mapped host memory (events, records, pair candidates) */
+	 * reads or writes of mapped host memory (events, records, pair candidates, body
+	 * states of a world that is read) */
 	long long hostToDeviceBytes;
 	long long deviceToHostBytes;
 	/* host phases of the last step (milliseconds): tree walks of the moved proxies on the

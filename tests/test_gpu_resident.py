@@ -355,3 +355,33 @@ def test_resident_solver_body_edges(gpu, oracle, scene, ctas):
             states, manifolds = solve_on_device(gpu, torch, part)
             assert np.array_equal(states.view(np.uint32), part["statesOut"].view(np.uint32)), (slots, bodies)
             assert np.array_equal(manifolds, cap["manifoldsOut"]), (slots, bodies)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batched", [False, True])
+def test_bytes_of_read_back_states(gpu, batched):
+    """A step of a world that is read counts the 48 bytes a body that it writes to the host."""
+    from box2c_gb300.capi import bind_batch_api, bind_gpu_api, world_array
+
+    bind_gpu_api(gpu.lib)
+    bind_batch_api(gpu.lib)
+    w = gpu.pyramid(12, 0.0, 1)
+    ids = world_array([w])
+
+    def moved():
+        if batched:
+            gpu.lib.b2World_StepBatch(ids, 1, 1.0 / 60.0, 4)
+        else:
+            gpu.step(w)
+        return gpu.lib.b2World_GetDeviceTimes(w).deviceToHostBytes
+
+    for _ in range(40):
+        before = moved()
+    n = gpu.lib.b2World_GetBodyStates(w, None, 0)
+    out = np.zeros((n, 7), np.float32)
+    gpu.lib.b2World_GetBodyStates(w, out.ctypes.data, n)
+    times = gpu.lib.b2World_GetDeviceTimes(w)
+    after = moved()
+    grown = 48 * (gpu.lib.b2World_GetDeviceTimes(w).recordCount - times.recordCount)
+    assert after - before == 48 * 78 + grown
+    gpu.destroy(w)
