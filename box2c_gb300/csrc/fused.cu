@@ -8,7 +8,7 @@
  *   bodies  body ids are cut into CL contiguous blocks of bodyCap: body b lives in CTA
  *           b / bodyCap at slot b % bodyCap (the owner is found by a multiply-high with a
  *           host-computed reciprocal).  Every CTA has copies of the other bodies that its
- *           rows and joints touch and sends its updates to the other copies
+ *           rows and joints touch and sends an update to the copy that is moved next
  *           (b2g_push.h); where the copies do not fit, or joints do not, rows
  *           reach a body of another CTA through distributed shared memory.
  *   rows    in a cluster the host groups each colour's rows by the CTA owning their first
@@ -29,7 +29,7 @@
  * Solver stage of a step before and after the one-CTA space and on-chip joints: pyramid of
  * 20 rows 97 -> 52 us, shape pile of 600 100 -> 68 us, 100 x 100 joint grid 421 -> 298 us.
  * With preparation and finalisation in the kernel: 47 us, 65 us; large pyramid 112 us, with
- * body copies 97, tumbler of 2000 370, with them 350 (83 overflow rows, one after the
+ * body copies 94, tumbler of 2000 370, with them 337 (83 to 95 overflow rows, one after the
  * other, 13 times a step: about 250 of it).  The joint grid's joints stay in L2 (5 us a
  * sweep); its stage runs beside the host's tree rebuild, which takes longer.
  */

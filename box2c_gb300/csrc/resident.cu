@@ -14,7 +14,7 @@
  *             sweeps.
  *   CL > 1    a thread-block cluster of CL CTAs: rows in the shared memory of the CTA
  *             that solves them, body b in CTA b / block with copies in the CTAs whose
- *             rows touch it, which updates are pushed to (b2g_push.h); where the copies
+ *             rows touch it, between which updates are passed (b2g_push.h); where the copies
  *             do not fit, reached through distributed shared memory, with hardware
  *             cluster barriers.
  *   CL == 0   a cooperative grid of up to one CTA per SM: rows in shared memory while
@@ -36,7 +36,7 @@
  * grid (an L2 round trip to arrive and one to see it).  b2SolveContacts, one kernel per
  * phase before and one resident kernel now, four substeps: 900 contacts 420 -> 52 us (a
  * cluster without copies takes 82), 15000 420 -> 102 without copies (a grid takes 199),
- * 60000 424 -> 207; with 17 overflow rows at 15000 contacts 799 -> 185, with body copies
+ * 60000 424 -> 206; with 17 overflow rows at 15000 contacts 799 -> 185, with body copies
  * 162.
  */
 #include "b2g_push.h"
